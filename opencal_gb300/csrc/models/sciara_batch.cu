@@ -21,9 +21,9 @@
  *      only its own state and the compact outflows; it joins the next lava
  *      list if it still holds lava.  Any other cell has no lava and no
  *      inflow, so it is unchanged (border cells hold 0 from the start).
- *   For the adjoint, K1 also flags the 32 x 16 tiles of the lava cells and
- *   receivers, and a tape kernel between K1 and K2 copies those tiles'
- *   state before the update.
+ *   For the adjoint, K1 leaves its compact slots and K2 what the update's
+ *   adjoint needs of every cell it visits on a tape, one entry per visited
+ *   cell and step.
  *
  * Arithmetic is the reference's, operation by operation (--fmad=false),
  * except the transcendental forms of sciara_math.cuh (exp10, the shear test
@@ -55,6 +55,7 @@ namespace sci2 {
 
 constexpr int T = 256;
 constexpr int K1T = 64;
+constexpr int BT = 64; /* reverse sweep: entries per block */
 constexpr int TW = 32, TH = 16; /* K2 tile; 2 cells per thread */
 constexpr int K2_BLOCKS = 152 * 4;
 constexpr int MAX_INST = 1024;
@@ -72,10 +73,9 @@ struct Inst {
 };
 
 /* counts[]: [0] lava list length, [5] K2 ticket, [6] epoch, [7] tiles
- * flagged in this step, [8] lava- or receiver-list overflow flag, [9] tape
- * slots used so far (counted on past the capacity), [10] tape overflow
- * flag, [11] receiver list length, [12] tiles flagged in the previous step,
- * [13] lava cells after the last update */
+ * flagged in this step, [8] lava- or receiver-list overflow flag, [9] tiles
+ * flagged in all steps so far, [11] receiver list length, [12] tiles flagged
+ * in the previous step, [13] lava cells after the last update */
 struct Dev {
     const Inst* inst;
     const long long* offs;
@@ -96,16 +96,11 @@ struct Dev {
     int* tlist;
     long long ncells;
     int capacity;
-    int nvents;
-    const int* vent_cell;  /* packed cell index of each vent */
-    const int* vent_first; /* B + 1: vents of instance b are [vent_first[b], vent_first[b + 1]) */
-    /* vent cells: the vents of one scenario at one cell form a group, led
-     * by its first vent; per group and phase the vent whose emission takes
-     * effect (the last with a positive one, -1: none) and its thickness */
+    /* vent cells: the vents of one scenario at one cell form a group; per
+     * group and phase the vent whose emission takes effect (the last with a
+     * positive one, -1: none) and its thickness */
     int ngroups;
     const int* g_cell;    /* packed cell */
-    const int* g_member;  /* g_mfirst[g]..g_mfirst[g+1]: the group's vents, leader first */
-    const int* g_mfirst;
     const int* g_eff;     /* ngroups x nphases */
     const double* g_emit; /* ngroups x nphases */
     int nphases;
@@ -162,32 +157,19 @@ static __device__ __forceinline__ void flag_tile(const Dev& d, int t, int epoch)
  * warp reads a tile's 16 mask words and reserves the tile's run of list
  * slots with one atomic.  (The first step uses the list the priming kernel
  * built.)  Block 0 also emits at the vents, one thread per scenario; a
- * vent cell that had no lava is appended.  With a vent tape (one record of
- * 3 doubles per vent and step) the first vent of each cell records the
- * cell's thickness and temperature before the emission and which vent's
- * emission took effect. */
-__global__ void __launch_bounds__(T) k_collect(const __grid_constant__ Dev d, unsigned phase, double* vtape,
-                                               int rebuild)
+ * vent cell that had no lava is appended. */
+__global__ void __launch_bounds__(T) k_collect(const __grid_constant__ Dev d, unsigned phase, int rebuild)
 {
     if (blockIdx.x == 0) {
         if (threadIdx.x == 0)
             d.counts[13] = 0;
         for (int g = threadIdx.x; g < d.ngroups; g += blockDim.x) {
             const int c = d.g_cell[g];
-            const int m0 = d.g_mfirst[g], m1 = d.g_mfirst[g + 1];
             const int eff = phase < (unsigned)d.nphases ? d.g_eff[(size_t)g * d.nphases + phase] : -1;
             /* the process reads the current thickness: the cell's vents add
              * to the value before this step's emission, the last positive
              * one wins */
             const double orig = d.Slt[c];
-            if (vtape) {
-                const int lead = d.g_member[m0];
-                vtape[3 * lead] = orig;
-                vtape[3 * lead + 1] = d.St[c];
-                vtape[3 * lead + 2] = (double)eff;
-                for (int m = m0 + 1; m < m1; m++)
-                    vtape[3 * d.g_member[m] + 2] = -2.0; /* handled with the cell's first vent */
-            }
             if (eff >= 0) {
                 d.Slt[c] = orig + d.g_emit[(size_t)g * d.nphases + phase];
                 d.St[c] = d.ph.PTvent;
@@ -351,13 +333,47 @@ static __device__ __forceinline__ void compute_flows(const Dev& d, const Inst& I
     }
 }
 
+/* The tape of a run whose gradient is wanted: per step one entry for every
+ * cell K2 visits, in K2's order (the lava list, then the receivers), at
+ * consecutive slots from the step's base.  It holds everything the reverse
+ * sweep reads, so the sweep neither restores the state nor evaluates the
+ * flows, the mixing or the cooling again: 200 bytes an entry, where copying
+ * the visited 32 x 16 tiles' state took 12 KB a tile (16 scenarios of
+ * 700 x 768, 240 steps: 4.6 GB of tiles).  Lava entries: the sixteen
+ * doubles of K1's slot (K2 reads them here too), the power law Pr and the
+ * masks; every entry: the update's intermediate values. */
+struct Tape {
+    int* cell;
+    unsigned* mask;      /* lava entries: F | S << 9 | in-grid neighbours << 18 */
+    unsigned char* flag; /* E_* */
+    double* pr;          /* lava entries */
+    double* fc;          /* 16 per entry */
+    double* val;         /* NVAL arrays of cap: t, t', h', residual, D, aus, cooled t */
+    long long cap;       /* entries; 0: the run is not taped */
+    long long* used;     /* entries of the steps so far, counted on past the capacity */
+    long long* step_base;
+    int* step_lava; /* lava entries of each step */
+    int* step_n;    /* all entries */
+};
+constexpr int NVAL = 7;
+constexpr size_t ENTRY_BYTES = sizeof(int) * 2 + 1 + sizeof(double) * (1 + 16 + NVAL);
+constexpr unsigned char E_FLOW = 1, E_BORDER = 2, E_LAVA = 4, E_SOLID = 8;
+
+/* where this step's compact slots are: the list's scratch, or the tape
+ * while the step's lava entries fit (a run that outgrows the tape is
+ * repeated with a larger one); K1 and K2 decide alike */
+static __device__ __forceinline__ double* slots_of(const Dev& d, const Tape& tp, int nlava, long long* base)
+{
+    *base = tp.cap ? *tp.used : 0;
+    return tp.cap && *base + nlava <= tp.cap ? tp.fc + 16 * (size_t)*base : d.fc;
+}
+
 /* K1: outflows of every lava cell into compact slots.  A receiver without
  * lava joins the receiver list once (epoch stamp), so that K2 visits
  * exactly the lava cells and the cells they flow into.  The tiles of the
  * lava cells and receivers are flagged: they hold every cell that can hold
- * lava after K2 (K0 of the next step collects the list from them) and every
- * cell the step changes besides the vents (the tape copies them). */
-__global__ void __launch_bounds__(K1T) k_flows(const __grid_constant__ Dev d)
+ * lava after K2 (K0 of the next step collects the list from them). */
+__global__ void __launch_bounds__(K1T) k_flows(const __grid_constant__ Dev d, const __grid_constant__ Tape tp)
 {
     __shared__ long long s_offs[MAX_INST + 1];
     for (int k = threadIdx.x; k <= d.B; k += blockDim.x)
@@ -365,6 +381,8 @@ __global__ void __launch_bounds__(K1T) k_flows(const __grid_constant__ Dev d)
     __syncthreads();
     const int epoch = d.counts[6];
     const int n = min(d.counts[0], d.capacity);
+    long long base;
+    double* slots = slots_of(d, tp, n, &base);
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const int c = d.list[k];
         const Inst I = d.inst[locate(s_offs, d.B, c)];
@@ -372,7 +390,11 @@ __global__ void __launch_bounds__(K1T) k_flows(const __grid_constant__ Dev d)
         const int i = (int)(lc / I.cols), j = (int)(lc - (long long)i * I.cols);
         Flow F;
         compute_flows(d, I, c, i, j, F);
-        double* slot = d.fc + (size_t)k * 16;
+        if (slots != d.fc) {
+            tp.mask[base + k] = F.F | (F.S << 9) | (F.inside << 18);
+            tp.pr[base + k] = F.Pr;
+        }
+        double* slot = slots + (size_t)k * 16;
 #pragma unroll
         for (int q = 1; q < 9; q++) {
             slot[q - 1] = F.f[q];
@@ -400,15 +422,15 @@ struct CellFwd {
     bool flowcond, border, lava, solid;
 };
 
-static __device__ __forceinline__ void compute_cell(const Dev& d, const Inst& I, int i, int j, long long x, int epoch,
-                                                    CellFwd& Cf)
+static __device__ __forceinline__ void compute_cell(const Dev& d, const double* slots, const Inst& I, int i, int j,
+                                                    long long x, int epoch, CellFwd& Cf)
 {
     const int opp[8] = {3, 2, 1, 0, 6, 7, 4, 5};
     Cf.h = d.Slt[x];
     Cf.t = d.St[x];
     Cf.sz = d.Sz[x];
     const int2 me = d.map[x];
-    const double* mine = me.x == epoch ? d.fc + (size_t)me.y * 16 : nullptr;
+    const double* mine = me.x == epoch ? slots + (size_t)me.y * 16 : nullptr;
     double ht = 0, in_sum = 0, out_sum = 0;
 #pragma unroll
     for (int n = 1; n < 9; n++) {
@@ -417,7 +439,7 @@ static __device__ __forceinline__ void compute_cell(const Dev& d, const Inst& I,
         if (nbr(I, i, j, n, &cn)) {
             const int2 m = d.map[cn];
             if (m.x == epoch) {
-                const double* s = d.fc + (size_t)m.y * 16;
+                const double* s = slots + (size_t)m.y * 16;
                 in_flow = s[opp[n - 1]];
                 in_ft = s[8 + opp[n - 1]];
             }
@@ -456,12 +478,23 @@ static __device__ __forceinline__ void compute_cell(const Dev& d, const Inst& I,
     }
 }
 
-/* the step at one cell, in place (the border reset of the steering last) */
-static __device__ __forceinline__ bool update_cell(const Dev& d, const Inst& I, int i, int j, int epoch)
+/* the step at one cell, in place (the border reset of the steering last);
+ * with a tape slot (entry >= 0) the values its adjoint needs go there */
+static __device__ __forceinline__ bool update_cell(const Dev& d, const double* slots, const Inst& I, int i, int j,
+                                                   int epoch, const Tape& tp, long long entry)
 {
     const long long x = I.off + (long long)i * I.cols + j;
     CellFwd Cf;
-    compute_cell(d, I, i, j, x, epoch, Cf);
+    compute_cell(d, slots, I, i, j, x, epoch, Cf);
+    if (entry >= 0) {
+        tp.cell[entry] = (int)x;
+        tp.flag[entry] = (unsigned char)((Cf.flowcond ? E_FLOW : 0) | (Cf.border ? E_BORDER : 0) |
+                                         (Cf.lava ? E_LAVA : 0) | (Cf.solid ? E_SOLID : 0));
+        const double v[NVAL] = {Cf.t, Cf.tn, Cf.hn, Cf.residual, Cf.D, Cf.aus, Cf.st};
+#pragma unroll
+        for (int q = 0; q < NVAL; q++)
+            tp.val[q * tp.cap + entry] = v[q];
+    }
     double sh = Cf.hn, st = Cf.tn;
     if (Cf.lava) {
         st = Cf.st;
@@ -481,60 +514,6 @@ static __device__ __forceinline__ bool update_cell(const Dev& d, const Inst& I, 
     return sh > 0;
 }
 
-/* undo tape of a run whose gradient is wanted: per flagged tile and step,
- * the tile's (Slt, St, Sz) before the update; per step and vent cell, its
- * thickness and temperature before the emission and the vent that emitted */
-struct Tape {
-    int* tile;        /* per slot: tile */
-    double* state;    /* per slot: 3 x TW*TH */
-    int* step_base;   /* per step: first slot */
-    int* step_count;  /* per step: slots */
-    double* vent;     /* per step and vent: orig Slt, orig St, emitting vent (-1: none, -2: not the cell's first) */
-    long long cap;    /* slots */
-};
-
-/* With a tape: every cell of the flagged tiles, (Slt, St, Sz) before the
- * update, into the tape slot of the tile.  The flagged tiles hold every
- * cell K0 and K2 change in this step besides the vent cells, which the
- * vent tape records. */
-__global__ void __launch_bounds__(T) k_tape(const __grid_constant__ Dev d, const __grid_constant__ Tape tp)
-{
-    const int ntiles = d.counts[7];
-    const int base = d.counts[9];
-    for (int item = blockIdx.x; item < ntiles; item += gridDim.x) {
-        const int t = d.tlist[item];
-        int lo = 0, hi = d.B - 1; /* the tile's instance: largest b with tile0 <= t */
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (d.inst[mid].tile0 <= t)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-        const Inst I = d.inst[lo];
-        const int lt = t - I.tile0;
-        const int ty = lt / I.tiles_x, tx = lt - ty * I.tiles_x;
-        const long long slot = (long long)base + item;
-        if (slot >= tp.cap) {
-            if (threadIdx.x == 0)
-                atomicExch(d.counts + 10, 1);
-            continue;
-        }
-        if (threadIdx.x == 0)
-            tp.tile[slot] = t;
-        double* s = tp.state + (size_t)slot * 3 * TW * TH;
-        for (int q = threadIdx.x; q < TW * TH; q += T) {
-            const int i = ty * TH + q / TW, j = tx * TW + q % TW;
-            if (i < I.rows && j < I.cols) {
-                const long long x = I.off + (long long)i * I.cols + j;
-                s[q] = d.Slt[x];
-                s[TW * TH + q] = d.St[x];
-                s[2 * TW * TH + q] = d.Sz[x];
-            }
-        }
-    }
-}
-
 /* K2: width_update, updateTemperature and the border reset at every lava
  * cell and every receiver (the only cells whose state can change: any
  * other cell has no lava and no inflow, so h + (0 - 0) = h and the
@@ -552,6 +531,9 @@ __global__ void __launch_bounds__(K1T) k_update(const __grid_constant__ Dev d, c
     const int epoch = d.counts[6];
     const int nl = min(d.counts[0], d.capacity);
     const int n = nl + min(d.counts[11], d.capacity);
+    long long base;
+    const double* slots = slots_of(d, tp, nl, &base);
+    const bool taped = tp.cap && base + n <= tp.cap;
     const int lane = threadIdx.x & 31;
     const int stride = gridDim.x * blockDim.x;
     for (int k0 = blockIdx.x * blockDim.x; k0 < n; k0 += stride) {
@@ -562,7 +544,7 @@ __global__ void __launch_bounds__(K1T) k_update(const __grid_constant__ Dev d, c
             const Inst I = d.inst[locate(s_offs, d.B, c)];
             const long long lc = c - I.off;
             const int i = (int)(lc / I.cols), j = (int)(lc - (long long)i * I.cols);
-            lava = update_cell(d, I, i, j, epoch);
+            lava = update_cell(d, slots, I, i, j, epoch, tp, taped ? base + k : -1);
             if (lava)
                 atomicOr(d.mask + (size_t)(I.tile0 + (i / TH) * I.tiles_x + j / TW) * 16 + (i % TH), 1u << (j % TW));
         }
@@ -574,12 +556,13 @@ __global__ void __launch_bounds__(K1T) k_update(const __grid_constant__ Dev d, c
     if (threadIdx.x == 0) {
         __threadfence();
         if (atomicAdd(reinterpret_cast<unsigned*>(d.counts + 5), 1u) == gridDim.x - 1) {
-            if (tp.state) {
-                const int ntiles = d.counts[7], base = d.counts[9];
+            if (tp.cap) {
                 tp.step_base[step] = base;
-                tp.step_count[step] = ntiles;
-                d.counts[9] = base + ntiles;
+                tp.step_lava[step] = nl;
+                tp.step_n[step] = n;
+                *tp.used = base + n;
             }
+            d.counts[9] += d.counts[7];
             d.counts[0] = 0; /* K0 of the next step collects the list from the masks */
             d.counts[5] = 0;
             d.counts[6] = epoch + 1;
@@ -596,273 +579,214 @@ __global__ void __launch_bounds__(K1T) k_update(const __grid_constant__ Dev d, c
  * discrete decisions are frozen: the minimisation's elimination sets and the
  * shear-resistance test, whether a cell has any flow, whether it holds lava,
  * whether it solidifies, the border mask.  Reverse mode, step by step from
- * the last: restore the step's taped tiles (the state after its emission),
- * recompute its outflows, then
- *   B2 (per cell of the step's tiles): mixing and cooling backward, in
- *      place on the cell's own adjoints; keeps, per cell, dL/dh' (A_h),
- *      dL/dt' / D (A_t) and t' for the outflow adjoints;
- *   B1 (per lava cell): the adjoint of each outflow gathered from the two
+ * the last, over the step's tape entries, one thread each:
+ *   B2 (every entry): mixing and cooling backward, in place on the cell's
+ *      own adjoints; keeps, per entry, dL/dh' (A_h), dL/dt' / D (A_t) and
+ *      t' for the outflow adjoints;
+ *   B1 (lava entries): the adjoint of each outflow gathered from the two
  *      cells it connects, then the minimisation backward, scattered (FP64
  *      atomics) to the thickness, altitude and temperature adjoints of the
- *      nine cells it read;
- *   B0 (per scenario): the emission backward -- dL/drate += dL/dSlt(vent) *
- *      Pclock / Pac for the vent whose emission took effect, the temperature
- *      adjoint of the vent cell reset (the emission overwrote it) -- and the
- *      vent cells restored to their state before the emission. */
+ *      nine cells it read; then, by its last block, the emission backward --
+ *      dL/drate += dL/dSlt(vent) * Pclock / Pac for the vent whose emission
+ *      took effect, the temperature adjoint of the vent cell reset (the
+ *      emission overwrote it).
+ * Both are bound by the FP64 pipe, and the entries spread over every SM.
+ * The sweep before took the visited tiles as its unit (a block per 32 x 16
+ * tile, so that the few hundred tiles left SMs idle) and evaluated the flows
+ * twice and the cooling once more per step from a restored state; 16
+ * scenarios of 700 x 768, 240 steps: 211 us per step in four kernels (ncu:
+ * FP64 pipe 57 % on the 88 SMs with tiles). */
+struct __align__(32) Mix {
+    double Ah, At, tp, unused;
+};
 struct Adj {
     double* lh;   /* dense: dL/dSlt */
     double* lt;   /* dense: dL/dSt */
     double* lz;   /* dense: dL/dSz */
-    double* fcb;  /* per compact cell: recomputed outflows (16 doubles) */
-    double* Ah;   /* per compact cell */
-    double* At;
-    double* tp;
+    Mix* mix;     /* per entry of the step */
     double* grad; /* nvents x nphases, internal vent order */
 };
 
-static __device__ __forceinline__ int tile_instance(const Dev& d, int t)
+__global__ void __launch_bounds__(BT) k_bcells(const __grid_constant__ Dev d, const __grid_constant__ Tape tp,
+                                               const __grid_constant__ Adj a, long long base, int n, int epoch_b)
 {
-    int lo = 0, hi = d.B - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (d.inst[mid].tile0 <= t)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return lo;
-}
-
-__global__ void __launch_bounds__(T) k_brestore(const __grid_constant__ Dev d, const __grid_constant__ Tape tp, int base,
-                                                int count)
-{
-    for (int item = blockIdx.x; item < count; item += gridDim.x) {
-        const long long slot = (long long)base + item;
-        const int t = tp.tile[slot];
-        const Inst I = d.inst[tile_instance(d, t)];
-        const int lt = t - I.tile0;
-        const int ty = lt / I.tiles_x, tx = lt - ty * I.tiles_x;
-        const double* s = tp.state + (size_t)slot * 3 * TW * TH;
-        for (int q = threadIdx.x; q < TW * TH; q += T) {
-            const int i = ty * TH + q / TW, j = tx * TW + q % TW;
-            if (i < I.rows && j < I.cols) {
-                const long long x = I.off + (long long)i * I.cols + j;
-                d.Slt[x] = s[q];
-                d.St[x] = s[TW * TH + q];
-                d.Sz[x] = s[2 * TW * TH + q];
-            }
-        }
-    }
-}
-
-/* the step's outflows again, from the restored state, into compact cells */
-__global__ void __launch_bounds__(T) k_bflows(const __grid_constant__ Dev db, const __grid_constant__ Tape tp,
-                                              int base, int count, int epoch_b)
-{
-    for (int item = blockIdx.x; item < count; item += gridDim.x) {
-        const int t = tp.tile[(long long)base + item];
-        const Inst I = db.inst[tile_instance(db, t)];
-        const int lt = t - I.tile0;
-        const int ty = lt / I.tiles_x, tx = lt - ty * I.tiles_x;
-        for (int q = threadIdx.x; q < TW * TH; q += T) {
-            const int i = ty * TH + q / TW, j = tx * TW + q % TW;
-            if (i >= I.rows || j >= I.cols)
-                continue;
-            const long long x = I.off + (long long)i * I.cols + j;
-            const int idx = item * TW * TH + q;
-            double* slot = db.fc + (size_t)idx * 16;
-            db.map[x] = make_int2(epoch_b, idx);
-            if (db.Slt[x] > 0) {
-                Flow F;
-                compute_flows(db, I, x, i, j, F);
-#pragma unroll
-                for (int k = 1; k < 9; k++) {
-                    slot[k - 1] = F.f[k];
-                    slot[8 + k - 1] = F.f[k] * F.t;
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < 16; k++)
-                    slot[k] = 0.0;
-            }
-        }
-    }
-}
-
-__global__ void __launch_bounds__(T) k_bcells(const __grid_constant__ Dev db, const __grid_constant__ Tape tp,
-                                              const __grid_constant__ Adj a, int base, int count, int epoch_b)
-{
-    for (int item = blockIdx.x; item < count; item += gridDim.x) {
-        const int t = tp.tile[(long long)base + item];
-        const Inst I = db.inst[tile_instance(db, t)];
-        const int lt = t - I.tile0;
-        const int ty = lt / I.tiles_x, tx = lt - ty * I.tiles_x;
-        for (int q = threadIdx.x; q < TW * TH; q += T) {
-            const int i = ty * TH + q / TW, j = tx * TW + q % TW;
-            if (i >= I.rows || j >= I.cols)
-                continue;
-            const long long x = I.off + (long long)i * I.cols + j;
-            const int idx = item * TW * TH + q;
-            CellFwd Cf;
-            compute_cell(db, I, i, j, x, epoch_b, Cf);
-            const double lh = a.lh[x], lt_ = a.lt[x];
-            double Lh = lh, Lt = lt_; /* adjoints of h', t' */
-            if (Cf.border) {
-                Lh = 0.0;
-                Lt = 0.0;
-            } else if (Cf.lava) {
-                if (Cf.solid) {
-                    Lh = a.lz[x]; /* Sz += h' */
-                    Lt = 0.0;
-                } else {
-                    /* st = nT / aus^(1/3), aus = 1 + 3 K nT^3 / (C h') */
-                    const double K = db.ph.Pepsilon * db.ph.Psigma * db.ph.Pclock * db.ph.Pcool;
-                    const double Cc = db.ph.Prho * db.ph.Pcv * db.ph.Pac;
-                    const double nT = Cf.tn, hn = Cf.hn;
-                    const double dst_daus = -Cf.st / (3.0 * Cf.aus);
-                    const double daus_dT = 9.0 * K * nT * nT / (Cc * hn);
-                    const double daus_dh = -3.0 * K * nT * nT * nT / (Cc * hn * hn);
-                    const double dst_dT = Cf.st / nT + dst_daus * daus_dT;
-                    Lh = lh + lt_ * (dst_daus * daus_dh);
-                    Lt = lt_ * dst_dT;
-                }
-            }
-            double new_lh = Lh, new_lt = Lt, At = 0.0;
-            if (Cf.flowcond) {
-                new_lh = Lh + Lt * (Cf.t - Cf.tn) / Cf.D;
-                new_lt = Lt * Cf.residual / Cf.D;
-                At = Lt / Cf.D;
-            }
-            a.lh[x] = new_lh;
-            a.lt[x] = new_lt;
-            a.Ah[idx] = Lh;
-            a.At[idx] = At;
-            a.tp[idx] = Cf.tn;
-        }
-    }
-}
-
-__global__ void __launch_bounds__(T) k_bflowadj(const __grid_constant__ Dev db, const __grid_constant__ Tape tp,
-                                                const __grid_constant__ Adj a, int base, int count, int epoch_b)
-{
-    for (int item = blockIdx.x; item < count; item += gridDim.x) {
-        const int t = tp.tile[(long long)base + item];
-        const Inst I = db.inst[tile_instance(db, t)];
-        const int lt = t - I.tile0;
-        const int ty = lt / I.tiles_x, tx = lt - ty * I.tiles_x;
-        for (int q0 = threadIdx.x; q0 < TW * TH; q0 += T) {
-            const int i = ty * TH + q0 / TW, j = tx * TW + q0 % TW;
-            if (i >= I.rows || j >= I.cols)
-                continue;
-            const long long x = I.off + (long long)i * I.cols + j;
-            if (!(db.Slt[x] > 0))
-                continue;
-            Flow F;
-            compute_flows(db, I, x, i, j, F);
-            if (!F.F)
-                continue;
-            const int idx = item * TW * TH + q0;
-            const double Ahc = a.Ah[idx], Atc = a.At[idx], tpc = a.tp[idx];
-            double lf[9];
-            double lt_add = 0.0;
-#pragma unroll
-            for (int k = 0; k < 9; k++)
-                lf[k] = 0.0;
-#pragma unroll
-            for (int k = 1; k < 9; k++) {
-                if (!((F.F >> k) & 1u))
-                    continue;
-                double v = -Ahc + Atc * (tpc - F.t); /* this cell's outflow */
-                if ((F.inside >> k) & 1u) {
-                    const int2 m = db.map[F.cn[k]];
-                    if (m.x == epoch_b) { /* the receiver's inflow (its tile is in the list) */
-                        const double Ahr = a.Ah[m.y], Atr = a.At[m.y], tpr = a.tp[m.y];
-                        v += Ahr + Atr * (F.t - tpr);
-                        lt_add += Atr * F.f[k]; /* the receiver's heat term f * t */
-                    }
-                }
-                lf[k] = v;
-            }
-            /* f[k] = Pr(t) (avg - H[k]), avg = (h0 + sum_S H) / |S| */
-            const double dPr = F.Pr * db.ph.b * 2.302585092994045684;
-            double G = 0.0, lH[9];
-#pragma unroll
-            for (int k = 0; k < 9; k++)
-                lH[k] = 0.0;
-#pragma unroll
-            for (int k = 1; k < 9; k++)
-                if ((F.F >> k) & 1u) {
-                    G += lf[k] * F.Pr;
-                    lH[k] -= lf[k] * F.Pr;
-                    lt_add += lf[k] * dPr * (F.avg - F.H[k]);
-                }
-            const double g = G / (double)F.nS;
-#pragma unroll
-            for (int k = 0; k < 9; k++)
-                if ((F.S >> k) & 1u)
-                    lH[k] += g;
-            atomicAdd(a.lh + x, g); /* avg's h[0] */
-            atomicAdd(a.lt + x, lt_add);
-            const double inv = 1.0 / db.ph.rad2;
-#pragma unroll
-            for (int k = 0; k < 9; k++) {
-                if (lH[k] == 0.0)
-                    continue;
-                const bool in = (F.inside >> k) & 1u;
-                /* H[k] = z[k] + h[k] for k >= 1, H[0] = z[0] */
-                if (k >= 1 && in)
-                    atomicAdd(a.lh + F.cn[k], lH[k]);
-                if (k < 5) {
-                    if (in)
-                        atomicAdd(a.lz + F.cn[k], lH[k]);
-                } else {
-                    /* z[k] = sz0 - (sz0 - sz_k) / rad2 */
-                    if (in)
-                        atomicAdd(a.lz + F.cn[k], lH[k] * inv);
-                    atomicAdd(a.lz + x, lH[k] * (1.0 - inv));
-                }
-            }
-        }
-    }
-}
-
-__global__ void k_bvents(const __grid_constant__ Dev d, const __grid_constant__ Adj a, const double* vtape, int phase)
-{
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= d.B)
+    const int k = blockIdx.x * BT + threadIdx.x;
+    if (k >= n)
         return;
-    for (int v = d.vent_first[b]; v < d.vent_first[b + 1]; v++) {
-        const double* rec = vtape + 3 * v;
-        const int eff = (int)rec[2];
-        if (eff < 0)
-            continue; /* not the cell's first vent, or no emission */
-        const int c = d.vent_cell[v];
-        if (phase < d.nphases)
-            a.grad[(size_t)eff * d.nphases + phase] += a.lh[c] * d.ph.Pclock / d.ph.Pac;
-        a.lt[c] = 0.0;
-        d.Slt[c] = rec[0];
-        d.St[c] = rec[1];
+    const long long e = base + k;
+    const int x = tp.cell[e];
+    const unsigned flag = tp.flag[e];
+    const double t = tp.val[e], tn = tp.val[tp.cap + e];
+    const double lh = a.lh[x], lt = a.lt[x];
+    double Lh = lh, Lt = lt; /* adjoints of h', t' */
+    if (flag & E_BORDER) {
+        Lh = 0.0;
+        Lt = 0.0;
+    } else if (flag & E_SOLID) {
+        Lh = a.lz[x]; /* Sz += h' */
+        Lt = 0.0;
+    } else if (flag & E_LAVA) {
+        /* st = t' / aus^(1/3), aus = 1 + 3 K t'^3 / (C h') */
+        const double K = d.ph.Pepsilon * d.ph.Psigma * d.ph.Pclock * d.ph.Pcool;
+        const double Cc = d.ph.Prho * d.ph.Pcv * d.ph.Pac;
+        const double hn = tp.val[2 * tp.cap + e], aus = tp.val[5 * tp.cap + e], st = tp.val[6 * tp.cap + e];
+        const double dst_daus = -st / (3.0 * aus);
+        const double daus_dT = 9.0 * K * tn * tn / (Cc * hn);
+        const double daus_dh = -3.0 * K * tn * tn * tn / (Cc * hn * hn);
+        Lh = lh + lt * (dst_daus * daus_dh);
+        Lt = lt * (st / tn + dst_daus * daus_dT);
     }
+    Mix m = {Lh, 0.0, tn, 0.0};
+    if (flag & E_FLOW) {
+        const double residual = tp.val[3 * tp.cap + e], D = tp.val[4 * tp.cap + e];
+        m.At = Lt / D;
+        Lh = Lh + Lt * (t - tn) / D;
+        Lt = Lt * residual / D;
+    }
+    a.lh[x] = Lh;
+    a.lt[x] = Lt;
+    a.mix[k] = m;
+    d.map[x] = make_int2(epoch_b, k);
 }
 
-/* dL/dSlt_T = 2 (Slt_T - target), the other adjoints 0; per-scenario loss */
-__global__ void k_bloss(const __grid_constant__ Dev d, const __grid_constant__ Adj a, const double* tgt, double* loss)
+__global__ void __launch_bounds__(BT) k_bflows(const __grid_constant__ Dev d, const __grid_constant__ Tape tp,
+                                               const __grid_constant__ Adj a, long long base, int nlava, int epoch_b,
+                                               unsigned phase)
 {
-    __shared__ long long s_offs[MAX_INST + 1];
+    extern __shared__ long long s_offs[];
+    __shared__ int s_last;
+    for (int k = threadIdx.x; k <= d.B; k += BT)
+        s_offs[k] = d.offs[k];
+    __syncthreads();
+    const int k0 = blockIdx.x * BT + threadIdx.x;
+    const unsigned mask = k0 < nlava ? tp.mask[base + k0] : 0u;
+    const unsigned F = mask & 511u, S = (mask >> 9) & 511u, inside = mask >> 18;
+    if (F) { /* no positive outflow: nothing was moved from the cell */
+        const int x = tp.cell[base + k0];
+        const int cols = d.inst[locate(s_offs, d.B, x)].cols;
+        const double* f = tp.fc + 16 * (size_t)(base + k0) - 1; /* f[1..8] */
+        const double t = tp.val[base + k0], Pr = tp.pr[base + k0];
+        const double dlog = d.ph.b * 2.302585092994045684;
+        const Mix me = a.mix[k0];
+        /* v_k = dL/df[k] from the cell the flow left and the one it reached;
+         * f[k] = Pr(t) (avg - H[k]), avg = (h0 + sum_S H) / |S|, so
+         * dPr/dt (avg - H[k]) = b ln(10) f[k] */
+        double lt_add = 0.0, G = 0.0, lH[9];
+        lH[0] = 0.0;
+#pragma unroll
+        for (int k = 1; k < 9; k++) {
+            lH[k] = 0.0;
+            if (!((F >> k) & 1u))
+                continue;
+            const double fk = f[k];
+            double v = -me.Ah + me.At * (me.tp - t); /* this cell's outflow */
+            if ((inside >> k) & 1u) {
+                const int2 m = d.map[x + kMi[k] * cols + kMj[k]];
+                if (m.x == epoch_b) { /* the receiver's inflow */
+                    const Mix r = a.mix[m.y];
+                    v += r.Ah + r.At * (t - r.tp);
+                    lt_add += r.At * fk; /* the receiver's heat term f * t */
+                }
+            }
+            G += v * Pr;
+            lH[k] = -(v * Pr);
+            lt_add += v * dlog * fk;
+        }
+        const double g = cal_div_small(G, __popc(S));
+        const double inv = 1.0 / d.ph.rad2;
+        double lz_own = 0.0;
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            if ((S >> k) & 1u)
+                lH[k] += g;
+            if (lH[k] == 0.0)
+                continue;
+            /* H[k] = z[k] + h[k] for k >= 1, H[0] = z[0];
+             * z[k] = sz0 - (sz0 - sz_k) / rad2 for k >= 5 */
+            if (k == 0)
+                lz_own += lH[k];
+            if (k >= 5)
+                lz_own += lH[k] * (1.0 - inv);
+            if (k >= 1 && ((inside >> k) & 1u)) {
+                const int cn = x + kMi[k] * cols + kMj[k];
+                atomicAdd(a.lh + cn, lH[k]);
+                atomicAdd(a.lz + cn, k < 5 ? lH[k] : lH[k] * inv);
+            }
+        }
+        atomicAdd(a.lh + x, g); /* avg's h[0] */
+        atomicAdd(a.lt + x, lt_add);
+        if (lz_own != 0.0)
+            atomicAdd(a.lz + x, lz_own);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(reinterpret_cast<unsigned*>(d.counts + 5), 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last)
+        return;
+    __threadfence();
+    for (int q = threadIdx.x; q < d.ngroups; q += BT) {
+        const int eff = phase < (unsigned)d.nphases ? d.g_eff[(size_t)q * d.nphases + phase] : -1;
+        if (eff >= 0) {
+            const int c = d.g_cell[q];
+            a.grad[(size_t)eff * d.nphases + phase] += __ldcg(a.lh + c) * d.ph.Pclock / d.ph.Pac;
+            a.lt[c] = 0.0;
+        }
+    }
+    if (threadIdx.x == 0)
+        d.counts[5] = 0;
+}
+
+/* dL/dSlt_T = 2 (Slt_T - target), the other adjoints 0; per-scenario loss.
+ * A block takes one run of consecutive cells, so that a warp's cells are of
+ * one scenario but where two meet: its sum is kept in registers and added
+ * to the scenario's loss when the scenario changes (one atomic per cell
+ * queued them all on a few words: 8.6M cells 1.30 ms). */
+__global__ void __launch_bounds__(T) k_bloss(const __grid_constant__ Dev d, const __grid_constant__ Adj a,
+                                             const double* tgt, double* loss)
+{
+    extern __shared__ long long s_offs[];
     for (int k = threadIdx.x; k <= d.B; k += blockDim.x)
         s_offs[k] = d.offs[k];
     __syncthreads();
-    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < d.ncells; c += (long long)gridDim.x * blockDim.x) {
-        const int b = locate(s_offs, d.B, c);
-        const Inst I = d.inst[b];
-        const bool valid = c - I.off < (long long)I.rows * I.cols;
-        const double diff = valid ? d.Slt[c] - tgt[c] : 0.0;
-        a.lh[c] = 2.0 * diff;
-        a.lt[c] = 0.0;
-        a.lz[c] = 0.0;
-        if (valid && diff != 0.0)
+    const long long per = ((d.ncells + gridDim.x - 1) / gridDim.x + T - 1) / T * T;
+    const long long c1 = min(d.ncells, per * (blockIdx.x + 1));
+    double acc = 0.0;
+    int cur = -1; /* the scenario acc belongs to, the same in every lane */
+    auto flush = [&]() {
+        double v = acc;
+        for (int o = 16; o > 0; o >>= 1)
+            v += __shfl_down_sync(0xffffffffu, v, o);
+        if ((threadIdx.x & 31) == 0 && cur >= 0 && v != 0.0)
+            atomicAdd(loss + cur, v);
+        acc = 0.0;
+    };
+    for (long long c0 = per * blockIdx.x; c0 < c1; c0 += T) {
+        const long long c = c0 + threadIdx.x;
+        int b = -1;
+        double diff = 0.0;
+        if (c < c1) {
+            b = locate(s_offs, d.B, c);
+            if (c - s_offs[b] < (long long)d.inst[b].rows * d.inst[b].cols)
+                diff = d.Slt[c] - tgt[c];
+            a.lh[c] = 2.0 * diff;
+            a.lt[c] = 0.0;
+            a.lz[c] = 0.0;
+        }
+        const int b0 = __shfl_sync(0xffffffffu, b, 0);
+        if (__all_sync(0xffffffffu, b == b0 || b < 0)) {
+            if (b0 >= 0 && b0 != cur) {
+                flush();
+                cur = b0;
+            }
+            acc += diff * diff;
+        } else if (b >= 0 && diff != 0.0) {
             atomicAdd(loss + b, diff * diff);
+        }
     }
+    flush();
 }
 
 /* MakeBorder (Sciara.cpp:206-250) on the device, the border reset of the
@@ -939,6 +863,13 @@ struct Batch {
     void* allocs[32] = {};
     int nalloc = 0;
     bool primed = false;
+    /* loss_grad's workspace: kept for the next call while it is a small
+     * part of the device's memory (free_work) */
+    Tape tp = {};
+    Adj adj = {};
+    double* tgt = nullptr;  /* target, padded layout */
+    double* loss = nullptr; /* B */
+    int tape_steps = 0, mix_cap = 0;
 };
 
 template <typename T>
@@ -950,10 +881,76 @@ static bool dalloc(Batch& bt, T** p, size_t bytes)
     return true;
 }
 
+template <typename T>
+static bool walloc(T** p, size_t count)
+{
+    if (*p)
+        return true;
+    if (cudaMalloc(p, std::max<size_t>(1, count) * sizeof(T)) == cudaSuccess)
+        return true;
+    (void)cudaGetLastError();
+    *p = nullptr;
+    return false;
+}
+
+template <typename T>
+static void wfree(T** p)
+{
+    cudaFree(*p);
+    *p = nullptr;
+}
+
+static void free_tape(Batch& bt)
+{
+    Tape& tp = bt.tp;
+    wfree(&tp.cell);
+    wfree(&tp.mask);
+    wfree(&tp.flag);
+    wfree(&tp.pr);
+    wfree(&tp.fc);
+    wfree(&tp.val);
+    tp.cap = 0;
+}
+
+/* a tape for `entries` entries (kept when it is large enough already) */
+static bool grow_tape(Batch& bt, long long entries)
+{
+    Tape& tp = bt.tp;
+    if (tp.cap >= entries)
+        return true;
+    free_tape(bt);
+    const size_t n = (size_t)entries;
+    if (walloc(&tp.cell, n) && walloc(&tp.mask, n) && walloc(&tp.flag, n) && walloc(&tp.pr, n) &&
+        walloc(&tp.fc, 16 * n) && walloc(&tp.val, NVAL * n)) {
+        tp.cap = entries;
+        return true;
+    }
+    free_tape(bt);
+    return false;
+}
+
+static void free_work(Batch& bt)
+{
+    free_tape(bt);
+    wfree(&bt.tp.used);
+    wfree(&bt.tp.step_base);
+    wfree(&bt.tp.step_lava);
+    wfree(&bt.tp.step_n);
+    wfree(&bt.adj.lh);
+    wfree(&bt.adj.lt);
+    wfree(&bt.adj.lz);
+    wfree(&bt.adj.mix);
+    wfree(&bt.adj.grad);
+    wfree(&bt.tgt);
+    wfree(&bt.loss);
+    bt.tape_steps = bt.mix_cap = 0;
+}
+
 static void destroy(Batch* bt)
 {
     if (bt->st)
         cudaStreamSynchronize(bt->st);
+    free_work(*bt);
     for (int k = 0; k < bt->nalloc; k++)
         cudaFree(bt->allocs[k]);
     if (bt->st)
@@ -1080,7 +1077,6 @@ extern "C" void* cal_sciara_batch_create(int B, const int* dims, const double* z
     d.B = B;
     d.ncells = bt->N;
     d.capacity = bt->capacity;
-    d.nvents = nvents;
     d.nphases = nphases;
     d.emission_time = emission_time;
     d.ph.Pclock = params[0];
@@ -1120,11 +1116,7 @@ extern "C" void* cal_sciara_batch_create(int B, const int* dims, const double* z
               sci2::dalloc(*bt, &d.counts, 16 * sizeof(int)) &&
               sci2::dalloc(*bt, &d.tflag, sizeof(int) * (size_t)tiles) &&
               sci2::dalloc(*bt, &d.tlist, sizeof(int) * (size_t)tiles) &&
-              sci2::dalloc(*bt, (int**)&d.vent_cell, sizeof(int) * std::max(1, nvents)) &&
-              sci2::dalloc(*bt, (int**)&d.vent_first, sizeof(int) * (B + 1)) &&
               sci2::dalloc(*bt, (int**)&d.g_cell, sizeof(int) * std::max(1, ngroups)) &&
-              sci2::dalloc(*bt, (int**)&d.g_member, sizeof(int) * std::max(1, nvents)) &&
-              sci2::dalloc(*bt, (int**)&d.g_mfirst, sizeof(int) * (ngroups + 1)) &&
               sci2::dalloc(*bt, (int**)&d.g_eff, sizeof(int) * std::max<size_t>(1, g_eff.size())) &&
               sci2::dalloc(*bt, (double**)&d.g_emit, sizeof(double) * std::max<size_t>(1, g_emit.size())) &&
               sci2::dalloc(*bt, &bt->Sz0, nb) && sci2::dalloc(*bt, &bt->Slt0, nb) && sci2::dalloc(*bt, &bt->St0, nb);
@@ -1136,17 +1128,13 @@ extern "C" void* cal_sciara_batch_create(int B, const int* dims, const double* z
     cudaMemcpy((void*)d.inst, bt->inst.data(), sizeof(sci2::Inst) * B, cudaMemcpyHostToDevice);
     cudaMemcpy((void*)d.offs, bt->offs.data(), sizeof(long long) * (B + 1), cudaMemcpyHostToDevice);
     d.ngroups = ngroups;
-    cudaMemcpy((void*)d.g_mfirst, g_mfirst.data(), sizeof(int) * (ngroups + 1), cudaMemcpyHostToDevice);
     if (nvents) {
-        cudaMemcpy((void*)d.vent_cell, vcell.data(), sizeof(int) * nvents, cudaMemcpyHostToDevice);
         cudaMemcpy((void*)d.g_cell, g_cell.data(), sizeof(int) * ngroups, cudaMemcpyHostToDevice);
-        cudaMemcpy((void*)d.g_member, g_member.data(), sizeof(int) * g_member.size(), cudaMemcpyHostToDevice);
         if (!g_eff.empty()) {
             cudaMemcpy((void*)d.g_eff, g_eff.data(), sizeof(int) * g_eff.size(), cudaMemcpyHostToDevice);
             cudaMemcpy((void*)d.g_emit, g_emit.data(), sizeof(double) * g_emit.size(), cudaMemcpyHostToDevice);
         }
     }
-    cudaMemcpy((void*)d.vent_first, vfirst.data(), sizeof(int) * (B + 1), cudaMemcpyHostToDevice);
     cudaMemset(d.Sz, 0, nb);
     cudaMemset(d.Slt, 0, nb);
     cudaMemset(d.St, 0, nb);
@@ -1181,10 +1169,10 @@ extern "C" void cal_sciara_batch_destroy(void* handle)
 namespace sci2 {
 
 /* the run from the initial state: calRun2D's loop with the stop condition
- * of Sciara.cpp:177-183 (elapsed time >= emission's end).  With a tape the
- * undo records of every step are kept (vtape: steps x nvents x 3). */
-static int forward(Batch* bt, int max_steps, const Tape* tape, double* vtape, std::vector<double>* elapsed_of,
-                   int* steps_done, float* ms)
+ * of Sciara.cpp:177-183 (elapsed time >= emission's end).  With a tape
+ * every step's entries are kept. */
+static int forward(Batch* bt, int max_steps, const Tape* tape, std::vector<double>* elapsed_of, int* steps_done,
+                   float* ms)
 {
     Dev& d = bt->d;
     cudaStream_t st = bt->st;
@@ -1204,8 +1192,10 @@ static int forward(Batch* bt, int max_steps, const Tape* tape, double* vtape, st
     k_prime<<<blocks, T, 0, st>>>(d);
     Tape tp;
     memset(&tp, 0, sizeof(tp));
-    if (tape)
+    if (tape) {
         tp = *tape;
+        cudaMemsetAsync(tp.used, 0, sizeof(long long), st);
+    }
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -1217,11 +1207,8 @@ static int forward(Batch* bt, int max_steps, const Tape* tape, double* vtape, st
             elapsed_of->push_back(elapsed);
         /* the phase as the vent process forms it: (unsigned)(elapsed / emission_time) */
         const unsigned phase = (unsigned)(elapsed / (double)bt->emission_time);
-        k_collect<<<K2_BLOCKS, T, 0, st>>>(d, phase, vtape ? vtape + (size_t)done * 3 * bt->nvents : nullptr,
-                                           done > 0);
-        k_flows<<<152 * 32, K1T, 0, st>>>(d);
-        if (tp.state)
-            k_tape<<<K2_BLOCKS, T, 0, st>>>(d, tp);
+        k_collect<<<K2_BLOCKS, T, 0, st>>>(d, phase, done > 0);
+        k_flows<<<152 * 32, K1T, 0, st>>>(d, tp);
         k_update<<<152 * 32, K1T, 0, st>>>(d, tp, done);
         done++;
         elapsed += d.ph.Pclock;
@@ -1238,11 +1225,11 @@ static int forward(Batch* bt, int max_steps, const Tape* tape, double* vtape, st
         *ms = t;
     if (steps_done)
         *steps_done = done;
-    int flags[3] = {0, 0, 0};
-    cudaMemcpy(flags, d.counts + 8, sizeof(flags), cudaMemcpyDeviceToHost);
+    int overflow = 0;
+    cudaMemcpy(&overflow, d.counts + 8, sizeof(overflow), cudaMemcpyDeviceToHost);
     if (cudaGetLastError() != cudaSuccess)
         return 3; /* CAL_ERROR_CUDA */
-    return (flags[0] || flags[2]) ? 2 /* CAL_ERROR_OUT_OF_MEMORY: lava list or tape too small */ : 0;
+    return overflow ? 2 /* CAL_ERROR_OUT_OF_MEMORY: lava list too small */ : 0;
 }
 
 /* steps a run takes (the stop condition's accumulation of the clock) */
@@ -1267,174 +1254,152 @@ static int run_length(const Batch* bt, int max_steps)
  * loop.  0, or a CALError code (CAL_ERROR_OUT_OF_MEMORY = list overflow). */
 extern "C" int cal_sciara_batch_run(void* handle, int max_steps, int* steps_done, float* ms)
 {
-    return sci2::forward((Batch*)handle, max_steps, nullptr, nullptr, nullptr, steps_done, ms);
+    return sci2::forward((Batch*)handle, max_steps, nullptr, nullptr, steps_done, ms);
 }
 
-/* Loss L_b = sum over scenario b of (Slt_T - target)^2 and its gradient
- * with respect to every emission rate, by the adjoint with the forward's
- * decisions frozen.  target: host array, the scenarios' grids back to back
- * (unpadded); loss_out[B]; grad_out[nvents x nphases] in the caller's vent
- * order.  tape_slots: undo-tape capacity in tiles summed over the steps
- * (0: twice the scenarios' tiles + 4096, and when that proves too small,
- * the forward runs once more with a tape of the size it asked for; a given
- * tape_slots that is too small is an error).  The state after the call is the
- * run's final one for Slt, St, Sz (Msl is not restored).  0 or a CALError
- * code; ms: device time of forward + adjoint. */
-extern "C" int cal_sciara_batch_loss_grad(void* handle, const double* target, int max_steps, double* loss_out,
-                                          double* grad_out, int* steps_done, long long tape_slots, float* ms)
+namespace sci2 {
+
+/* tape entries a run is first given room for: a vent's lava spreads over
+ * some 15 cells more each step (10..50 m3/s on 10 m cells), half as many
+ * again for receivers and slower lava, at most a quarter of the free memory;
+ * a run that visits more is repeated with the size it asked for */
+static long long first_tape(const Batch& bt, int steps)
 {
-    Batch* bt = (Batch*)handle;
-    sci2::Dev& d = bt->d;
+    long long sum = 0;
+    for (int t = 1; t <= steps; t++)
+        sum += std::min<long long>(bt.N, 64 + 24LL * std::max(1, bt.nvents) * t);
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    return std::max<long long>(4096, std::min<long long>(sum, (long long)(free_b / 4 / ENTRY_BYTES)));
+}
+
+static int loss_grad(Batch* bt, const double* target, int max_steps, double* loss_out, double* grad_out,
+                     int* steps_done, long long tape_slots, float* ms, cudaEvent_t e0, cudaEvent_t e1)
+{
+    constexpr int OOM = 2, CUDA = 3; /* CAL_ERROR_OUT_OF_MEMORY, CAL_ERROR_CUDA */
+    Dev& d = bt->d;
+    Tape& tp = bt->tp;
+    Adj& a = bt->adj;
     cudaStream_t st = bt->st;
-    const int steps = sci2::run_length(bt, max_steps);
-    const long long cap = tape_slots > 0 ? tape_slots : 2LL * bt->ntiles + 4096;
-    const size_t tile_cells = (size_t)sci2::TW * sci2::TH;
-    sci2::Tape tp;
-    memset(&tp, 0, sizeof(tp));
-    tp.cap = cap;
-    double* vtape = nullptr;
-    double* tgt = nullptr;
-    double* dloss = nullptr;
-    sci2::Adj a;
-    memset(&a, 0, sizeof(a));
-    std::vector<void*> mem;
-    auto alloc = [&](void** p, size_t bytes) {
-        if (cudaMalloc(p, bytes) != cudaSuccess)
-            return false;
-        mem.push_back(*p);
-        return true;
-    };
-    const size_t nb = (size_t)bt->N * sizeof(double);
-    bool ok = alloc((void**)&tp.step_base, sizeof(int) * (steps + 1)) &&
-              alloc((void**)&tp.step_count, sizeof(int) * (steps + 1)) &&
-              alloc((void**)&vtape, sizeof(double) * 3 * std::max(1, bt->nvents) * (size_t)steps) &&
-              alloc((void**)&tgt, nb) && alloc((void**)&dloss, sizeof(double) * bt->B) &&
-              alloc((void**)&a.lh, nb) && alloc((void**)&a.lt, nb) && alloc((void**)&a.lz, nb) &&
-              alloc((void**)&a.grad, sizeof(double) * std::max(1, bt->nvents * bt->nphases));
-    auto free_tape = [&]() {
-        cudaStreamSynchronize(st);
-        cudaFree(tp.tile);
-        cudaFree(tp.state);
-        tp.tile = nullptr;
-        tp.state = nullptr;
-    };
-    auto alloc_tape = [&](long long slots) {
-        tp.cap = slots;
-        if (cudaMalloc((void**)&tp.tile, sizeof(int) * slots) != cudaSuccess ||
-            cudaMalloc((void**)&tp.state, sizeof(double) * 3 * tile_cells * slots) != cudaSuccess) {
-            cudaGetLastError();
-            free_tape();
-            return false;
-        }
-        return true;
-    };
-    auto release = [&]() {
-        free_tape();
-        for (void* p : mem)
-            cudaFree(p);
-    };
-    if (!ok || !alloc_tape(cap)) {
-        release();
-        return 2; /* CAL_ERROR_OUT_OF_MEMORY */
+    const int steps = run_length(bt, max_steps);
+    const size_t ngrad = (size_t)std::max(1, bt->nvents * bt->nphases);
+    if (steps > bt->tape_steps) {
+        wfree(&tp.step_base);
+        wfree(&tp.step_lava);
+        wfree(&tp.step_n);
+        bt->tape_steps = steps;
     }
+    if (!walloc(&tp.used, 1) || !walloc(&tp.step_base, (size_t)bt->tape_steps) ||
+        !walloc(&tp.step_lava, (size_t)bt->tape_steps) || !walloc(&tp.step_n, (size_t)bt->tape_steps) ||
+        !walloc(&bt->tgt, (size_t)bt->N) || !walloc(&bt->loss, (size_t)bt->B) || !walloc(&a.lh, (size_t)bt->N) ||
+        !walloc(&a.lt, (size_t)bt->N) || !walloc(&a.lz, (size_t)bt->N) || !walloc(&a.grad, ngrad))
+        return OOM;
+    if (!tp.cap && !grow_tape(*bt, first_tape(*bt, steps)) && !grow_tape(*bt, 4096))
+        return OOM;
     /* target in the padded layout: an input, copied before the timed region */
-    cudaMemsetAsync(tgt, 0, nb, st);
+    cudaMemsetAsync(bt->tgt, 0, (size_t)bt->N * sizeof(double), st);
     size_t src = 0;
     for (int b = 0; b < bt->B; b++) {
         const size_t n = (size_t)bt->inst[b].rows * bt->inst[b].cols;
-        cudaMemcpyAsync(tgt + bt->offs[b], target + src, n * sizeof(double), cudaMemcpyHostToDevice, st);
+        cudaMemcpyAsync(bt->tgt + bt->offs[b], target + src, n * sizeof(double), cudaMemcpyHostToDevice, st);
         src += n;
     }
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    cudaEventRecord(e0, st);
     std::vector<double> elapsed_of;
     int done = 0;
-    int rc = sci2::forward(bt, max_steps, &tp, vtape, &elapsed_of, &done, nullptr);
-    if (rc == 2 && tape_slots <= 0) {
-        /* the default tape was too small but the lava list was not: the
-         * forward counted every slot it wanted, so run it again once with
-         * a tape of exactly that size */
-        int c[3] = {0, 0, 0};
-        cudaMemcpy(c, d.counts + 8, sizeof(c), cudaMemcpyDeviceToHost);
-        if (!c[0] && c[2] && c[1] > cap) {
-            const long long need = c[1];
-            free_tape();
-            if (!alloc_tape(need)) {
-                release();
-                cudaEventDestroy(e0);
-                cudaEventDestroy(e1);
-                return 2;
-            }
-            elapsed_of.clear();
-            cudaEventRecord(e0, st);
-            rc = sci2::forward(bt, max_steps, &tp, vtape, &elapsed_of, &done, nullptr);
-        }
+    for (int attempt = 0;; attempt++) {
+        elapsed_of.clear();
+        cudaEventRecord(e0, st);
+        const int rc = forward(bt, max_steps, &tp, &elapsed_of, &done, nullptr);
+        if (rc)
+            return rc;
+        long long need = 0;
+        int tiles = 0;
+        cudaMemcpy(&need, tp.used, sizeof(need), cudaMemcpyDeviceToHost);
+        cudaMemcpy(&tiles, d.counts + 9, sizeof(tiles), cudaMemcpyDeviceToHost);
+        if (tape_slots > 0 && tiles > tape_slots)
+            return OOM; /* the caller's limit */
+        if (need <= tp.cap)
+            break;
+        if (attempt || !grow_tape(*bt, need))
+            return OOM;
     }
-    if (rc) {
-        release();
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        return rc;
-    }
-    cudaMemsetAsync(dloss, 0, sizeof(double) * bt->B, st);
-    cudaMemsetAsync(a.grad, 0, sizeof(double) * std::max(1, bt->nvents * bt->nphases), st);
-    const int blocks = (int)std::min<long long>((bt->N + sci2::T - 1) / sci2::T, 152 * 16);
-    sci2::k_bloss<<<blocks, sci2::T, 0, st>>>(d, a, tgt, dloss);
-    /* backward scratch: the largest step's tiles */
-    std::vector<int> base(done), count(done);
-    cudaMemcpyAsync(base.data(), tp.step_base, sizeof(int) * done, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(count.data(), tp.step_count, sizeof(int) * done, cudaMemcpyDeviceToHost, st);
+    cudaMemsetAsync(bt->loss, 0, sizeof(double) * bt->B, st);
+    cudaMemsetAsync(a.grad, 0, sizeof(double) * ngrad, st);
+    const size_t offs_bytes = sizeof(long long) * (bt->B + 1);
+    k_bloss<<<(int)std::min<long long>((bt->N + T - 1) / T, 152 * 8), T, offs_bytes, st>>>(d, a, bt->tgt, bt->loss);
+    std::vector<long long> base(done);
+    std::vector<int> nlava(done), n(done);
+    cudaMemcpyAsync(base.data(), tp.step_base, sizeof(long long) * done, cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(nlava.data(), tp.step_lava, sizeof(int) * done, cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(n.data(), tp.step_n, sizeof(int) * done, cudaMemcpyDeviceToHost, st);
     cudaStreamSynchronize(st);
-    int maxc = 1;
+    int most = 1;
     for (int t = 0; t < done; t++)
-        maxc = std::max(maxc, count[t]);
-    const size_t nc = (size_t)maxc * tile_cells;
-    ok = alloc((void**)&a.fcb, sizeof(double) * 16 * nc) && alloc((void**)&a.Ah, sizeof(double) * nc) &&
-         alloc((void**)&a.At, sizeof(double) * nc) && alloc((void**)&a.tp, sizeof(double) * nc);
-    if (!ok) {
-        release();
-        return 2;
+        most = std::max(most, n[t]);
+    if (most > bt->mix_cap) {
+        wfree(&a.mix);
+        bt->mix_cap = 0;
+        if (!walloc(&a.mix, (size_t)most))
+            return OOM;
+        bt->mix_cap = most;
     }
-    sci2::Dev db = d;
-    db.fc = a.fcb;
     for (int t = done - 1; t >= 0; t--) {
         const int epoch_b = -(t + 1);
-        const int g = std::max(1, std::min(count[t], sci2::K2_BLOCKS));
-        if (count[t] > 0) {
-            sci2::k_brestore<<<g, sci2::T, 0, st>>>(d, tp, base[t], count[t]);
-            sci2::k_bflows<<<g, sci2::T, 0, st>>>(db, tp, base[t], count[t], epoch_b);
-            sci2::k_bcells<<<g, sci2::T, 0, st>>>(db, tp, a, base[t], count[t], epoch_b);
-            sci2::k_bflowadj<<<g, sci2::T, 0, st>>>(db, tp, a, base[t], count[t], epoch_b);
-        }
-        const int phase = (int)(unsigned)(elapsed_of[t] / bt->emission_time);
-        sci2::k_bvents<<<(bt->B + 63) / 64, 64, 0, st>>>(d, a, vtape + (size_t)t * 3 * bt->nvents, phase);
+        const unsigned phase = (unsigned)(elapsed_of[t] / bt->emission_time);
+        if (n[t] > 0)
+            k_bcells<<<(n[t] + BT - 1) / BT, BT, 0, st>>>(d, tp, a, base[t], n[t], epoch_b);
+        /* an emitting vent cell is a lava cell of the step */
+        if (nlava[t] > 0)
+            k_bflows<<<(nlava[t] + BT - 1) / BT, BT, offs_bytes, st>>>(d, tp, a, base[t], nlava[t], epoch_b, phase);
     }
     cudaEventRecord(e1, st);
-    std::vector<double> grad((size_t)std::max(1, bt->nvents * bt->nphases));
-    cudaMemcpyAsync(grad.data(), a.grad, sizeof(double) * grad.size(), cudaMemcpyDeviceToHost, st);
+    std::vector<double> grad(ngrad);
+    cudaMemcpyAsync(grad.data(), a.grad, sizeof(double) * ngrad, cudaMemcpyDeviceToHost, st);
     if (loss_out)
-        cudaMemcpyAsync(loss_out, dloss, sizeof(double) * bt->B, cudaMemcpyDeviceToHost, st);
-    cudaEventSynchronize(e1);
-    float t_ms = 0.f;
-    cudaEventElapsedTime(&t_ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+        cudaMemcpyAsync(loss_out, bt->loss, sizeof(double) * bt->B, cudaMemcpyDeviceToHost, st);
+    cudaStreamSynchronize(st);
     if (ms)
-        *ms = t_ms;
+        cudaEventElapsedTime(ms, e0, e1);
     if (steps_done)
         *steps_done = done;
     if (grad_out)
         for (int k = 0; k < bt->nvents; k++)
             for (int p = 0; p < bt->nphases; p++)
                 grad_out[(size_t)bt->vent_order[k] * bt->nphases + p] = grad[(size_t)k * bt->nphases + p];
-    rc = cudaGetLastError() == cudaSuccess ? 0 : 3;
-    release();
-    /* the tape undid the run: run again so that reads see the final state,
-     * as after cal_sciara_batch_run */
-    if (!rc)
-        rc = sci2::forward(bt, max_steps, nullptr, nullptr, nullptr, nullptr, nullptr);
+    return cudaGetLastError() == cudaSuccess ? 0 : CUDA;
+}
+
+} // namespace sci2
+
+/* Loss L_b = sum over scenario b of (Slt_T - target)^2 and its gradient
+ * with respect to every emission rate, by the adjoint with the forward's
+ * decisions frozen.  target: host array, the scenarios' grids back to back
+ * (unpadded); loss_out[B]; grad_out[nvents x nphases] in the caller's vent
+ * order.  tape_slots: a limit on the tiles flagged, summed over the steps
+ * (0: none); a run that flags more is an error.  The tape grows to the run:
+ * when it proves too small the forward runs once more with a tape of the
+ * size it asked for.  The state after the call is the run's final one.  0
+ * or a CALError code; ms: device time of forward + adjoint. */
+extern "C" int cal_sciara_batch_loss_grad(void* handle, const double* target, int max_steps, double* loss_out,
+                                          double* grad_out, int* steps_done, long long tape_slots, float* ms)
+{
+    Batch* bt = (Batch*)handle;
+    cudaEvent_t e0, e1;
+    cudaEventCreate(&e0);
+    cudaEventCreate(&e1);
+    const int rc = sci2::loss_grad(bt, target, max_steps, loss_out, grad_out, steps_done, tape_slots, ms, e0, e1);
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    /* the workspace stays for the next call while it takes at most a
+     * sixteenth of the device's memory */
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    const size_t held = (size_t)bt->tp.cap * sci2::ENTRY_BYTES + sizeof(double) * 4 * (size_t)bt->N +
+                        sizeof(sci2::Mix) * (size_t)bt->mix_cap;
+    if (rc || held > total_b / 16) {
+        cudaStreamSynchronize(bt->st);
+        sci2::free_work(*bt);
+    }
     return rc;
 }
 
