@@ -46,6 +46,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <thread>
 #include <vector>
 
 #include "exact_div.cuh"
@@ -1403,6 +1404,41 @@ extern "C" int cal_sciara_batch_loss_grad(void* handle, const double* target, in
     return rc;
 }
 
+namespace sci2 {
+
+/* Host pages under a result, before the copy into it.  Pages of a freshly
+ * allocated array do not exist yet; when the device's copy is the first to
+ * touch them, each fault is a round trip of the GPU to the operating system
+ * (134 MB: 37-72 ms), while a few host threads map them in a fraction of
+ * that.  Every byte written here is overwritten by the copy. */
+static void touch_pages(void* dst, size_t bytes)
+{
+    constexpr size_t STEP = 4096, MIN_SHARE = 4u << 20;
+    const int nthreads = (int)std::min<size_t>(4, bytes / MIN_SHARE);
+    volatile char* p = (volatile char*)dst;
+    auto share = [=](int k, int n) {
+        for (size_t q = bytes / n * k; q < (k + 1 == n ? bytes : bytes / n * (k + 1)); q += STEP)
+            p[q] = 0;
+    };
+    if (nthreads < 1)
+        return; /* small results: the faults cost less than the threads */
+    std::vector<std::thread> others;
+    int started = 1;
+    try {
+        others.reserve(nthreads - 1);
+        for (; started < nthreads; started++)
+            others.emplace_back(share, started, nthreads);
+    } catch (...) { /* no more threads: the rest here */
+    }
+    share(0, nthreads);
+    for (int k = started; k < nthreads; k++)
+        share(k, nthreads);
+    for (std::thread& t : others)
+        t.join();
+}
+
+} // namespace sci2
+
 /* the scenarios' final Sz, Slt, St, Msl, back to back and unpadded (any may be NULL) */
 extern "C" int cal_sciara_batch_read(void* handle, double* z, double* slt, double* st, double* msl)
 {
@@ -1413,7 +1449,15 @@ extern "C" int cal_sciara_batch_read(void* handle, double* z, double* slt, doubl
     for (int q = 0; q < 4; q++) {
         if (!outs[q])
             continue;
-        size_t pos = 0;
+        size_t pos = 0, total = 0;
+        for (int b = 0; b < bt->B; b++)
+            total += (size_t)bt->inst[b].rows * bt->inst[b].cols;
+        cudaPointerAttributes at;
+        const bool known = cudaPointerGetAttributes(&at, outs[q]) == cudaSuccess;
+        if (!known)
+            (void)cudaGetLastError();
+        if (!known || at.type == cudaMemoryTypeUnregistered)
+            sci2::touch_pages(outs[q], total * sizeof(double));
         for (int b = 0; b < bt->B; b++) {
             const size_t n = (size_t)bt->inst[b].rows * bt->inst[b].cols;
             cudaMemcpy(outs[q] + pos, src[q] + bt->offs[b], n * sizeof(double), cudaMemcpyDeviceToHost);
