@@ -168,7 +168,8 @@ struct CalGrid {
     bool fill(int type, int slot, int layer, const void* value, bool at_active);
     bool fill_both(int type, int slot, const void* value); /* calInitSubstate: both layers, all (or active) cells */
     void untrack(int type, int slot);                    /* device pointer handed out: no tracking from now on */
-    bool copy_next_to_current(const std::vector<std::pair<int, int>>& which, bool use_dirty, bool at_active);
+    bool copy_next_to_current(const std::vector<std::pair<int, int>>& which, bool use_dirty, bool at_active,
+                              bool* cleared = nullptr);
     bool update_all();                         /* calUpdate: compaction + copies */
     bool compact();                            /* calUpdateActiveCells */
     bool clear_dirty();
