@@ -109,6 +109,12 @@ struct CALDevModel2D {
     signed char stage_of[3][CAL_MAX_SUBSTATES];
     int* stage_err; /* set when a box did not arrive in time (the tile then reads global memory) */
     CUtensorMap stage_map[CAL_MAX_STAGED];
+    /* cells that a neighbour read cannot leave the grid from: at least
+     * reach_i rows and reach_j columns off every edge; there neighbour n is
+     * at off[n] = xi[n] * cols + xj[n] from the cell */
+    int reach_i, reach_j;
+    int off[CAL_MAX_NEIGHBORS];
+    int spread; /* plain launches give the rows of a tile to different blocks */
 };
 
 
@@ -120,7 +126,7 @@ static __shared__ unsigned char cal_written2D[3 * CAL_MAX_SUBSTATES];
 /* per warp: substates whose next layer this warp changed in the current
  * tile (flushed into the chg bitmaps after each tile row), and per block:
  * substates written by unsafe operations */
-static __shared__ unsigned char cal_chg2D[CAL_EP_THREADS / 32][3 * CAL_MAX_SUBSTATES];
+static __shared__ __align__(4) unsigned char cal_chg2D[CAL_EP_THREADS / 32][3 * CAL_MAX_SUBSTATES];
 static __shared__ unsigned char cal_untracked2D[3 * CAL_MAX_SUBSTATES];
 /* per block: a process changed an active-cell flag */
 static __shared__ unsigned char cal_flagchg2D;
@@ -212,6 +218,41 @@ static __device__ __forceinline__ struct CALModel2D cal_model_view2D(const struc
     return v;
 }
 
+/* What the kernel knows about the cell it runs the process on travels in two
+ * fields of the view that mean nothing on the device (the host's arrays of
+ * handles): pQb_array holds the cell (i, j), pQi_array the traits below.
+ * Once the process is inlined they are values in registers or compile-time
+ * constants, and an accessor called with the cell's own i, j drops the tests
+ * they settle: a neighbour read of a cell off the edges (most cells) is one
+ * address offset instead of a table look-up per coordinate, the wrap or the
+ * bounds test, a 64-bit index and the test for a staged copy.  Any other
+ * coordinates, and views without traits (stop conditions), take the general
+ * path.  A process of a few reads is bound by instruction issue; Life (nine
+ * reads a cell): 441 -> 249 instructions a cell, 15.1 -> 12.0 us a launch on
+ * 1024 x 1024, 190 -> 123 us on 4096 x 4096. */
+#define CAL_VIEW_INSIDE 1u /* every neighbour of the cell lies in the grid */
+#define CAL_VIEW_STAGED 2u /* the launch may stage declared reads */
+#define CAL_VIEW_SQUARE 4u /* the neighbourhood is not hexagonal */
+static __device__ __forceinline__ void cal_view_cell2D(struct CALModel2D& v, int i, int j, unsigned traits)
+{
+    v.pQb_array = reinterpret_cast<struct CALSubstate2Db**>(((unsigned long long)(unsigned)i << 32) | (unsigned)j);
+    v.pQi_array = reinterpret_cast<struct CALSubstate2Di**>((unsigned long long)traits);
+}
+static __device__ __forceinline__ bool cal_view_is2D(const struct CALModel2D* ca, unsigned trait)
+{
+    return (reinterpret_cast<unsigned long long>(ca->pQi_array) & trait) != 0;
+}
+static __device__ __forceinline__ bool cal_view_inside2D(const struct CALModel2D* ca, int i, int j)
+{
+    return cal_view_is2D(ca, CAL_VIEW_INSIDE) &&
+           reinterpret_cast<unsigned long long>(ca->pQb_array) ==
+               (((unsigned long long)(unsigned)i << 32) | (unsigned)j);
+}
+static __device__ __forceinline__ bool cal_cell_inside2D(const struct CALDevModel2D& m, int i, int j)
+{
+    return i >= m.reach_i && i < m.rows - m.reach_i && j >= m.reach_j && j < m.cols - m.reach_j;
+}
+
 static __device__ __forceinline__ int cal_slot2D(const struct CALDevModel2D* m, int t, const void* q)
 {
     return (int)(((unsigned long long)(uintptr_t)q - m->pool[t]) >> CAL_HANDLE_SHIFT);
@@ -262,8 +303,9 @@ static __device__ __forceinline__ T cal_get2D(const struct CALModel2D* ca, int t
 {
     const struct CALDevModel2D* m = cal_dm2D(ca);
     const int s = cal_slot2D(m, t, q);
-    if (const T* p = cal_staged2D<T>(m, t, s, i, j))
-        return *p;
+    if (cal_view_is2D(ca, CAL_VIEW_STAGED))
+        if (const T* p = cal_staged2D<T>(m, t, s, i, j))
+            return *p;
     return static_cast<const T*>(m->cur[t][s])[cal_lin2D(m, i, j)];
 }
 
@@ -272,7 +314,12 @@ static __device__ __forceinline__ T cal_getx2D(const struct CALModel2D* ca, int 
 {
     const struct CALDevModel2D* m = cal_dm2D(ca);
     const int s = cal_slot2D(m, t, q);
-    if (m->nstage && cal_stage_on2D) {
+    if (cal_view_inside2D(ca, i, j)) {
+        if (!cal_view_is2D(ca, CAL_VIEW_SQUARE) && ((m->hex == 1 && (j & 1)) || (m->hex == 2 && (i & 1))))
+            n += CAL_HEXAGONAL_SHIFT;
+        return (static_cast<const T*>(m->cur[t][s]) + cal_lin2D(m, i, j))[m->off[n]];
+    }
+    if (cal_view_is2D(ca, CAL_VIEW_STAGED) && m->nstage && cal_stage_on2D) {
         /* a staged tile lies inside a toroidal grid or the box's zero fill
          * is the flat boundary: the neighbour is read without wrapping */
         const int nn = ((m->hex == 1 && (j & 1)) || (m->hex == 2 && (i & 1))) ? n + CAL_HEXAGONAL_SHIFT : n;
@@ -379,6 +426,27 @@ static __device__ __forceinline__ int calGetActiveCellCountDevice2D(const struct
     return m->count ? *m->count : 0;
 }
 
+/* the warp's marks of the tile into the chg bitmaps; whether this lane found
+ * one.  A lane reads the marks of four substates in one word. */
+static __device__ __forceinline__ bool cal_flush_chg2D(const struct CALDevModel2D& m, int tile, unsigned tbit)
+{
+    const int lane = threadIdx.x & 31;
+    unsigned* marks = reinterpret_cast<unsigned*>(cal_chg2D[threadIdx.x >> 5]);
+    __syncwarp();
+    unsigned v = lane < 3 * CAL_MAX_SUBSTATES / 4 ? marks[lane] : 0u;
+    const bool changed = v != 0;
+    if (changed) {
+        marks[lane] = 0;
+        do {
+            const int t = 4 * lane + ((__ffs(v) - 1) >> 3);
+            atomicOr(&m.chg[(long long)t * m.tile_words + (tile >> 5)], tbit);
+            v &= v - 1; /* a mark is a byte of value 1 */
+        } while (v);
+    }
+    __syncwarp();
+    return changed;
+}
+
 /* One elementary process over every cell, or over the active list when the
  * optimisation is on and the list is non-empty (cal2D.c:717-734).  The grid
  * is sized by the host to a few waves of the GPU; both loops are
@@ -424,6 +492,9 @@ __global__ void __launch_bounds__(CAL_EP_THREADS) cal_ep2D_kernel(const __grid_c
         const int stride = nblocks * blockDim.x;
         for (int n = bid * blockDim.x + threadIdx.x; n < listed; n += stride) {
             const struct CALCell2D c = m.cells[n];
+            cal_view_cell2D(view, c.i, c.j,
+                            (STAGED ? CAL_VIEW_STAGED : 0u) |
+                                (cal_cell_inside2D(m, c.i, c.j) ? CAL_VIEW_INSIDE : 0u));
             EP(ca, c.i, c.j);
         }
     } else {
@@ -480,10 +551,10 @@ __global__ void __launch_bounds__(CAL_EP_THREADS) cal_ep2D_kernel(const __grid_c
          * skipping a tile where the process changed nothing has its bit
          * cleared (or, when the launch deals its tiles, gathered in quiet for
          * the last block to clear) */
-        auto run_tile = [&](int tile) {
+        auto run_tile = [&](int tile, int row) {
             const unsigned tbit = 1u << (tile & 31);
             const int ty = tile / m.tiles_x;
-            const int i = ty * CAL_TILE_H + warp, j = (tile - ty * m.tiles_x) * CAL_TILE_W + lane;
+            const int i = ty * CAL_TILE_H + row, j = (tile - ty * m.tiles_x) * CAL_TILE_W + lane;
             if (MODE == 3) {
                 /* the cells that pass the guard, in tile order, onto threads
                  * 0, 1, ... (the counting barrier comes first: the previous
@@ -505,9 +576,8 @@ __global__ void __launch_bounds__(CAL_EP_THREADS) cal_ep2D_kernel(const __grid_c
                 /* one barrier settles a tile where no cell or every cell
                  * passes; the others are packed */
                 const int total = __syncthreads_count(pass);
-                if (total == CAL_EP_THREADS) {
-                    EP(ca, i, j);
-                } else if (total > 0) {
+                int q = (int)threadIdx.x;
+                if (total > 0 && total < CAL_EP_THREADS) {
                     const unsigned bal = __ballot_sync(0xffffffffu, pass);
                     if (lane == 0)
                         cal_gcount2D[warp] = __popc(bal);
@@ -518,25 +588,26 @@ __global__ void __launch_bounds__(CAL_EP_THREADS) cal_ep2D_kernel(const __grid_c
                     if (pass)
                         cal_gcell2D[off + __popc(bal & ((1u << lane) - 1u))] = (unsigned char)threadIdx.x;
                     __syncthreads();
-                    if ((int)threadIdx.x < total) {
-                        const int q = cal_gcell2D[threadIdx.x];
-                        EP(ca, ty * CAL_TILE_H + (q >> 5), (tile - ty * m.tiles_x) * CAL_TILE_W + (q & 31));
-                    }
+                    q = cal_gcell2D[threadIdx.x];
                 }
+                if ((int)threadIdx.x < total) {
+                    const int a = ty * CAL_TILE_H + (q >> 5), b = (tile - ty * m.tiles_x) * CAL_TILE_W + (q & 31);
+                    cal_view_cell2D(view, a, b, cal_cell_inside2D(m, a, b) ? CAL_VIEW_INSIDE : 0u);
+                    EP(ca, a, b);
+                }
+            } else if ((NX == 7 || NX == 0 || !m.hex) && cal_cell_inside2D(m, i, j - lane) &&
+                       cal_cell_inside2D(m, i, j - lane + CAL_TILE_W - 1)) {
+                /* the warp's whole row is off the edges: its own copy of the
+                 * process, with nothing left to test per read */
+                cal_view_cell2D(view, i, j, CAL_VIEW_INSIDE | (NX == 7 || NX == 0 ? 0u : CAL_VIEW_SQUARE));
+                EP(ca, i, j);
             } else if (i < m.rows && j < m.cols) {
+                cal_view_cell2D(view, i, j, 0u);
                 EP(ca, i, j);
             }
             if (m.track) {
-                bool changed = false;
-                __syncwarp();
-                for (int t = lane; t < 3 * CAL_MAX_SUBSTATES; t += 32)
-                    if (cal_chg2D[warp][t]) {
-                        cal_chg2D[warp][t] = 0;
-                        changed = true;
-                        atomicOr(&m.chg[(long long)t * m.tile_words + (tile >> 5)], tbit);
-                    }
-                __syncwarp();
-                if (m.run && !__syncthreads_or(changed) && threadIdx.x == 0) {
+                const bool changed = cal_flush_chg2D(m, tile, tbit);
+                if (MODE != 0 && m.run && !__syncthreads_or(changed) && threadIdx.x == 0) {
                     if (m.quiet)
                         atomicOr(&m.quiet[tile >> 5], tbit);
                     else
@@ -546,7 +617,7 @@ __global__ void __launch_bounds__(CAL_EP_THREADS) cal_ep2D_kernel(const __grid_c
         };
         if (ntodo >= 0) {
             for (int k = 0; k < ntodo; k++)
-                run_tile(cal_dtile2D[k]);
+                run_tile(cal_dtile2D[k], warp);
         } else if (MODE == 2 || (MODE == 3 && m.run)) {
             /* the block's tiles bid, bid + nblocks, ..., only those whose run
              * bit is set.  The bits of 32 of them come in one load per lane
@@ -561,12 +632,27 @@ __global__ void __launch_bounds__(CAL_EP_THREADS) cal_ep2D_kernel(const __grid_c
                 if (need && m.run)
                     need = (m.run[t >> 5] >> (t & 31)) & 1u;
                 for (unsigned todo = __ballot_sync(0xffffffffu, need); todo; todo &= todo - 1)
-                    run_tile(base + (__ffs(todo) - 1) * nblocks);
+                    run_tile(base + (__ffs(todo) - 1) * nblocks, warp);
+            }
+        } else if (MODE == 0) {
+            /* a row of a tile per warp.  With spread, consecutive rows go to
+             * consecutive blocks: nothing here waits for the block's other
+             * warps, and a tile where the process does much work (a flow's
+             * wet cells) loads eight SMs' narrow FP64 pipes instead of one's
+             * (SCIDDICA-T's flows, 610 x 496: 23.1 -> 12.0 us; the dense
+             * width update 9.6 -> 8.8).  Without, the rows stay together and
+             * share their neighbour rows in L1 (Life 1024 x 1024: 12.6 us
+             * against 14.8 spread). */
+            for (int k = 0;; k++) {
+                const int u = bid + (warp + k * (CAL_EP_THREADS / 32)) * nblocks;
+                const int tile = m.spread ? u / CAL_TILE_H : bid + k * nblocks;
+                if (tile >= ntiles)
+                    break;
+                run_tile(tile, m.spread ? u % CAL_TILE_H : warp);
             }
         } else {
             for (int tile = bid; tile < ntiles; tile += nblocks)
-                if (!m.run || (m.run[tile >> 5] >> (tile & 31)) & 1u)
-                    run_tile(tile);
+                run_tile(tile, warp);
         }
         } else {
         /* staged: the tiles dealt to the block, or the block's tiles bid,
@@ -653,20 +739,14 @@ __global__ void __launch_bounds__(CAL_EP_THREADS) cal_ep2D_kernel(const __grid_c
                     nstage = 0;
                 }
             }
-            if (i < m.rows && j < m.cols)
+            if (i < m.rows && j < m.cols) {
+                cal_view_cell2D(view, i, j, CAL_VIEW_STAGED);
                 EP(ca, i, j);
+            }
             if (nstage)
                 __syncthreads(); /* every read of this buffer done before it is refilled */
             if (m.track) {
-                bool changed = false;
-                __syncwarp();
-                for (int t = lane; t < 3 * CAL_MAX_SUBSTATES; t += 32)
-                    if (cal_chg2D[warp][t]) {
-                        cal_chg2D[warp][t] = 0;
-                        changed = true;
-                        atomicOr(&m.chg[(long long)t * m.tile_words + (tile >> 5)], tbit);
-                    }
-                __syncwarp();
+                const bool changed = cal_flush_chg2D(m, tile, tbit);
                 if (m.run && !__syncthreads_or(changed) && threadIdx.x == 0) {
                     if (m.quiet)
                         atomicOr(&m.quiet[tile >> 5], tbit);
@@ -719,6 +799,22 @@ __global__ void __launch_bounds__(CAL_EP_THREADS) cal_ep2D_kernel(const __grid_c
  * of declared reads, with tile skipping, and for a guarded process (the
  * staging, skipping and packing loops cost registers and barriers that the
  * plain loop does not pay) */
+template <void (*EP)(struct CALModel2D*, int, int), int NX>
+static void cal_launch_plain2D(const struct CALDevModel2D* m, int nblocks, cudaStream_t st)
+{
+    /* one resident wave: a second wave's blocks would pay the start of a
+     * block (the handles' managed memory, the written bits) once more */
+    static int wave = 0;
+    if (!wave) {
+        int dev = 0, sms = 0, per_sm = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cal_ep2D_kernel<EP, NX, 0>, CAL_EP_THREADS, 0);
+        wave = sms * per_sm > 0 ? sms * per_sm : nblocks;
+    }
+    cal_ep2D_kernel<EP, NX, 0><<<nblocks < wave ? nblocks : wave, CAL_EP_THREADS, 0, st>>>(*m);
+}
+
 template <void (*EP)(struct CALModel2D*, int, int)>
 static int cal_launch_ep2D(const struct CALDevModel2D* m, int gx, int gy, void* stream)
 {
@@ -749,10 +845,10 @@ static int cal_launch_ep2D(const struct CALDevModel2D* m, int gx, int gy, void* 
         }
     } else {
         switch (m->model.sizeof_X) {
-        case 5: cal_ep2D_kernel<EP, 5, 0><<<grid, CAL_EP_THREADS, 0, st>>>(*m); break;
-        case 7: cal_ep2D_kernel<EP, 7, 0><<<grid, CAL_EP_THREADS, 0, st>>>(*m); break;
-        case 9: cal_ep2D_kernel<EP, 9, 0><<<grid, CAL_EP_THREADS, 0, st>>>(*m); break;
-        default: cal_ep2D_kernel<EP, 0, 0><<<grid, CAL_EP_THREADS, 0, st>>>(*m); break;
+        case 5: cal_launch_plain2D<EP, 5>(m, gx * gy, st); break;
+        case 7: cal_launch_plain2D<EP, 7>(m, gx * gy, st); break;
+        case 9: cal_launch_plain2D<EP, 9>(m, gx * gy, st); break;
+        default: cal_launch_plain2D<EP, 0>(m, gx * gy, st); break;
         }
     }
     return (int)cudaGetLastError();

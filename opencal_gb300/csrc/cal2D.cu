@@ -160,7 +160,12 @@ static bool build_desc(struct CALModel2D* ca, CALDevModel2D* d)
     for (int n = 0; n < len; n++) {
         d->xi[n] = ca->X[n].i;
         d->xj[n] = ca->X[n].j;
+        d->reach_i = std::max(d->reach_i, std::abs(ca->X[n].i));
+        d->reach_j = std::max(d->reach_j, std::abs(ca->X[n].j));
+        d->off[n] = ca->X[n].i * ca->columns + ca->X[n].j;
     }
+    if (d->reach_i >= ca->rows) /* no cell is that far off the edges (and off[] may not fit) */
+        d->reach_i = ca->rows;
     /* process tiles (every launch) and change tracking (models without
      * active cells) */
     d->tiles_x = (ca->columns + CAL_TILE_W - 1) / CAL_TILE_W;
@@ -169,6 +174,8 @@ static bool build_desc(struct CALModel2D* ca, CALDevModel2D* d)
     d->tile_words = g.tile_words;
     d->chg = g.d_chg;
     d->untracked = g.d_untracked;
+    for (int k = 0; k < g.nslot[CAL_TYPE_R]; k++)
+        d->spread |= g.sub[CAL_TYPE_R][k].used; /* real substates: the work is FP64 */
     return true;
 }
 
