@@ -92,6 +92,9 @@ void cal_sciddicaT_close(void* session);
 /* ---- SCIDDICA-T adjoint (one grid; device arrays) ---- */
 void* cal_sdt_adj_create(int rows, int cols, int steps, int toroidal);
 void cal_sdt_adj_destroy(void* work);
+/* 0: the next forwards leave no tape for a backward (which then runs the
+ * forward again); 1 (default): they do */
+int cal_sdt_adj_set_tape(void* work, int on);
 int cal_sdt_adj_forward(void* work, const double* z_dem, const double* h0, double p_r, double p_eps, double* hT,
                         void* stream);
 int cal_sdt_adj_backward(void* work, const double* dL_dhT, double* dL_dh0, double* dL_dpr, double* dL_dpeps,
@@ -111,14 +114,13 @@ int cal_sdt_batch_set_shape(void* ensemble, int shape /* 0: 32x16, 1: 64x16, 2: 
 int cal_sdt_batch_autotune(void* ensemble, int probe_steps, float* ms /* 5: 32x16, 64x16, 64x32, 16x8, 32x8 */);
 int cal_sdt_batch_set_params(void* ensemble, const double* params);
 int cal_sdt_batch_forward(void* ensemble, double* hT /* device, or NULL */);
-int cal_sdt_batch_active_tiles(void* ensemble, int* counts /* steps + 1 */);
+int cal_sdt_batch_active_tiles(void* ensemble, int* counts /* tiles updated by each step, then 0: steps + 1 */);
 int cal_sdt_batch_loss_grad(void* ensemble, const double* target /* device */, double* loss /* B */,
                             double* grad /* 2B */, double* dL_dh0 /* device, or NULL */);
 /* 1 (default): cal_sdt_batch_loss_grad is one launch of a recorded CUDA graph
- * (forward, loss, tape layout computed on the device, reverse sweep, results
+ * (forward, loss, tape offsets chained on the device, reverse sweep, results
  * to pinned host memory); 0: launch by launch.  Segmented tapes of more than
- * 32 steps a segment (rollouts over 1024 steps) are laid out on the host and
- * run launch by launch. */
+ * 32 steps a segment (rollouts over 1024 steps) are run launch by launch. */
 int cal_sdt_batch_set_graph(void* ensemble, int on);
 int cal_sdt_batch_graph_stats(void* ensemble, long long* launches, long long* nodes);
 /* What the adjoint's tape holds: -1 (default) the whole rollout (the

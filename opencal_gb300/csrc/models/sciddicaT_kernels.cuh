@@ -45,26 +45,15 @@ static __device__ __forceinline__ bool is_wet(double h, long long eps_bits)
     return (b & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL; /* -NaN; other negatives are dry */
 }
 
-/* The outflows of one wet cell, exactly as sciddicaT_flows_computation:
- * the same additions in the same order; the division by the number of
- * remaining cells and the comparisons are done on the integer pipe with
- * bit-identical results (exact_div.cuh). */
-static __device__ __forceinline__ void outflows_u0(double hc, double u0, const double u1, const double u2,
-                                                   const double u3, const double u4, double eps, double r,
-                                                   double f[4], unsigned* elim_out = nullptr);
-
-static __device__ __forceinline__ void outflows(double hc, double zc, const double u1, const double u2,
-                                                const double u3, const double u4, double eps, double r, double f[4],
-                                                unsigned* elim_out = nullptr)
-{
-    outflows_u0(hc, zc + eps, u1, u2, u3, u4, eps, r, f, elim_out);
-}
-
-/* the same with u[0] = z + eps of the cell given (a caller that keeps it
- * per cell saves the addition) */
-static __device__ __forceinline__ void outflows_u0(double hc, double u0, const double u1, const double u2,
-                                                   const double u3, const double u4, double eps, double r,
-                                                   double f[4], unsigned* elim_out)
+/* The minimisation of differences of one wet cell, exactly as
+ * sciddicaT_flows_computation: the same additions in the same order; the
+ * division by the number of remaining cells and the comparisons are done on
+ * the integer pipe with bit-identical results (exact_div.cuh).  u0 = z +
+ * epsilon of the cell, u1..u4 = z + h of its neighbours.  diff[n - 1] =
+ * average - u[n] of neighbour n, or 0 when it was eliminated; the result's
+ * bit n: neighbour n (1..4) eliminated; bit 0: the cell itself. */
+static __device__ __forceinline__ unsigned minimise(double hc, double u0, const double u1, const double u2,
+                                                    const double u3, const double u4, double eps, double diff[4])
 {
     double u[5];
     const double m = hc - eps;
@@ -97,9 +86,29 @@ static __device__ __forceinline__ void outflows_u0(double hc, double u0, const d
     } while (again);
 #pragma unroll
     for (int n = 1; n < 5; n++)
-        f[n - 1] = (elim & (1u << n)) ? 0.0 : (average - u[n]) * r;
+        diff[n - 1] = (elim & (1u << n)) ? 0.0 : average - u[n];
+    return elim;
+}
+
+/* the outflows (average - u[n]) * r of the kept neighbours, u0 = z + eps */
+static __device__ __forceinline__ void outflows_u0(double hc, double u0, const double u1, const double u2,
+                                                   const double u3, const double u4, double eps, double r,
+                                                   double f[4], unsigned* elim_out = nullptr)
+{
+    const unsigned elim = minimise(hc, u0, u1, u2, u3, u4, eps, f);
+#pragma unroll
+    for (int n = 1; n < 5; n++)
+        if (!(elim & (1u << n)))
+            f[n - 1] *= r;
     if (elim_out)
-        *elim_out = elim; /* bit n: neighbour n (1..4) eliminated; bit 0: the cell itself */
+        *elim_out = elim;
+}
+
+static __device__ __forceinline__ void outflows(double hc, double zc, const double u1, const double u2,
+                                                const double u3, const double u4, double eps, double r, double f[4],
+                                                unsigned* elim_out = nullptr)
+{
+    outflows_u0(hc, zc + eps, u1, u2, u3, u4, eps, r, f, elim_out);
 }
 
 static __device__ __forceinline__ int wrapi(int x, int n)

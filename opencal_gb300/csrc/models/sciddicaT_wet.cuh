@@ -1,0 +1,590 @@
+/*
+ * sciddicaT_wet.cuh -- many SCIDDICA-T grids (or one) advanced together over
+ * one list of their wet cells, forward and adjoint: the kernels of the
+ * ensembles (sciddicaT_batch.cu) and of the single rollout
+ * (sciddicaT_adjoint.cu).
+ *
+ * The flow covers a small part of its grids (calibration ensembles: 1 % of
+ * the cells, 8 % of the cells of the tiles that hold some), and a wet cell's
+ * FP64 chain is the expensive part, so the unit of work is the wet cell:
+ * whatever tiles they lie in, the cells of the list spread evenly over the
+ * SMs.  A step is two launches:
+ *
+ *   k_outflows  one thread per listed wet cell: its outflows into f (zero
+ *               everywhere else), and the tiles that hold the cell or a
+ *               receiver flagged once (epoch stamps) in the step's tile
+ *               list.  With a tape, the cell, its elimination set and the
+ *               differences average - u[n] of its kept neighbours go to
+ *               entry off + k of the tape.
+ *   k_update    the flagged tiles: h in place, z + h beside it, and the next
+ *               list (wet cells, and ~c for a cell that dried, whose outflows
+ *               the next k_outflows clears); wet cells of other tiles are
+ *               carried over.
+ *
+ * The adjoint of a step reads the tape and lambda alone -- neither h nor z,
+ * nothing is restored or minimised again -- and is two launches:
+ *
+ *   k_coeffs    one thread per taped wet cell: g and the four w (the
+ *               formulas of sciddicaT_adjoint.cu) beside the step's stamp,
+ *               and the sums dL/dr, dL/deps of its instance;
+ *   k_gather    the step's flagged tiles: lambda = lambda + g + the
+ *               neighbours' w, in place, in a fixed order (results do not
+ *               depend on the order of the list).
+ *
+ * mu = lambda - lambda_z, kept only when dL/dh0 is wanted: both take the same
+ * w, so mu changes only by g at a wet cell that eliminated itself, and
+ * dL/dh0 = lambda_0 - [h0 > 0] lambda_z is mu where h0 > 0, lambda elsewhere.
+ *
+ * Measured against the tile-by-tile step this replaced (fused tiles of 64 x
+ * 16 cells with their rings, the adjoint on whole tiles after restoring
+ * them), 64 instances of 128..1024 cells a side, 500 steps, us per step:
+ * forward 92 -> 16 (k_outflows) + 16 (k_update); reverse 10 + 65 + 29 -> 15
+ * (k_coeffs) + 10 (k_gather).  k_outflows is bound by the FP64 pipe (60 % of
+ * it over the launch, the rest is its chain of loads), the others by the
+ * latency of theirs.
+ */
+#pragma once
+
+#include "sciddicaT_kernels.cuh"
+
+namespace sdtw {
+
+constexpr int T = 256;
+/* 608 blocks: launch cost grows with the blocks, and four resident blocks on
+ * each SM keep the FP64 pipes fed (the split step of the single grid,
+ * sciddicaT.cu, measured the same) */
+constexpr int BLOCKS = 152 * 4;
+
+struct Inst {
+    int rows, cols;
+    long long off;
+    double r, eps;
+    long long eps_bits;
+    int tiles_x, tiles_y, tile0, toroidal;
+};
+
+struct __align__(32) D4 {
+    double v[4];
+};
+
+/* cell (packed index; ~cell: dried in the previous step) and its instance */
+typedef int2 Entry;
+
+struct Dev {
+    const Inst* inst;
+    const long long* offs; /* B + 1 */
+    const int* tile_inst;
+    int B, ntiles, lw, lh; /* tiles of 2^lw x 2^lh cells */
+    long long N;
+    const double* z;
+    double* h;
+    double* zh; /* z + h */
+    D4* f;
+    Entry* list[2]; /* list t in list[t & 1] */
+    int* nlist;     /* per step: entries of its list */
+    int* tiles;     /* per step: ntiles places for its flagged tiles */
+    int* counts;    /* per step: flagged tiles */
+    int* stamps;    /* per tile: epoch it was flagged in */
+    Entry* t_entry; /* tape */
+    unsigned char* t_elim;
+    D4* t_diff;
+    long long cap;   /* its entries */
+    long long* toff; /* per step: first entry; toff[t + 1] chained by step t */
+    long long* need; /* the most entries any rollout or segment asked for */
+};
+
+constexpr size_t TAPE_BYTES = sizeof(Entry) + 1 + sizeof(D4); /* per entry */
+
+struct Adj {
+    double* lam;
+    double* mu; /* or NULL */
+    int* stamp; /* per cell: step whose coefficients it holds */
+    D4* w;
+    double* g;
+    double* part; /* COPIES x 2B partial sums of grad */
+    double* grad; /* 2B: dL/dr[0..B), dL/deps[B..2B) */
+};
+constexpr int COPIES = 32;
+
+/* neighbour q = 0..3 (north, west, east, south) of (i, j); false where a
+ * flat grid ends */
+static __device__ __forceinline__ bool nbr(const Inst& I, int i, int j, int q, int* a, int* b)
+{
+    *a = i + (q == 0 ? -1 : (q == 3 ? 1 : 0));
+    *b = j + (q == 1 ? -1 : (q == 2 ? 1 : 0));
+    if (I.toroidal) {
+        *a = sdt::wrapi(*a, I.rows);
+        *b = sdt::wrapi(*b, I.cols);
+        return true;
+    }
+    return (unsigned)*a < (unsigned)I.rows && (unsigned)*b < (unsigned)I.cols;
+}
+
+/* the tape entries of step t start here; -1: they do not fit (the
+ * evaluation is discarded and repeated with a larger tape) */
+static __device__ __forceinline__ long long tape_base(const Dev& d, int t, int n)
+{
+    const long long off = d.toff[t];
+    return off + n <= d.cap ? off : -1;
+}
+
+static __global__ void __launch_bounds__(T) k_outflows(const __grid_constant__ Dev d, int t, int epoch, int taped)
+{
+    const int n = d.nlist[t];
+    const Entry* list = d.list[t & 1];
+    long long base = -1;
+    if (taped) {
+        base = tape_base(d, t, n);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            const long long end = d.toff[t] + n;
+            d.toff[t + 1] = end;
+            if (*d.need < end) /* one step at a time runs */
+                *d.need = end;
+        }
+    }
+    int* tiles = d.tiles + (size_t)t * d.ntiles;
+    /* chunks of 32 entries on consecutive blocks */
+    const int stride = gridDim.x * T;
+    for (int k = ((threadIdx.x >> 5) * (int)gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31); k < n; k += stride) {
+        const Entry e = list[k];
+        if (base >= 0)
+            d.t_entry[base + k] = e;
+        if (e.x < 0) {
+            const D4 zero = {{0.0, 0.0, 0.0, 0.0}};
+            d.f[~e.x] = zero;
+            continue;
+        }
+        const Inst I = d.inst[e.y];
+        const int lc = (int)(e.x - I.off);
+        const int i = lc / I.cols, j = lc - i * I.cols;
+        double u[4];
+        /* the cell's tile and its receivers' where they differ, and their
+         * stamps, loaded here so that they arrive while the minimisation
+         * runs (one after another behind it they added up to 2 us a step) */
+        const int own = I.tile0 + (i >> d.lh) * I.tiles_x + (j >> d.lw);
+        int rt[4], stamp[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            int a, b;
+            const bool in = nbr(I, i, j, q, &a, &b);
+            u[q] = in ? d.zh[I.off + (long long)a * I.cols + b] : 0.0; /* an absent neighbour: 0.0 + 0.0 */
+            rt[q] = in ? I.tile0 + (a >> d.lh) * I.tiles_x + (b >> d.lw) : own;
+            stamp[q] = rt[q] != own ? d.stamps[rt[q]] : epoch;
+        }
+        const int own_stamp = d.stamps[own];
+        D4 diff, f;
+        const unsigned elim = sdt::minimise(d.h[e.x], d.z[e.x] + I.eps, u[0], u[1], u[2], u[3], I.eps, diff.v);
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            f.v[q] = (elim & (2u << q)) ? 0.0 : diff.v[q] * I.r;
+        d.f[e.x] = f;
+        if (base >= 0) {
+            d.t_elim[base + k] = (unsigned char)elim;
+            d.t_diff[base + k] = diff;
+        }
+        /* the tiles the update must visit: the receivers', and the own tile
+         * once per distinct tile of the lanes here */
+        const bool any = (elim & 0x1eu) != 0x1eu;
+        auto flag = [&](int tile) {
+            if (atomicExch(d.stamps + tile, epoch) != epoch)
+                tiles[atomicAdd(d.counts + t, 1)] = tile;
+        };
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (!(elim & (2u << q)) && stamp[q] != epoch)
+                flag(rt[q]);
+        const bool mine = any && own_stamp != epoch;
+        const unsigned act = __activemask();
+        const unsigned peers = __match_any_sync(act, mine ? own : -1);
+        if (mine && (threadIdx.x & 31) == __ffs(peers) - 1)
+            flag(own);
+    }
+}
+
+/* one entry per thread at most onto the next list, one atomic per block */
+static __device__ __forceinline__ void block_append(bool want, Entry e, Entry* list, int* count, int* s_warp)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned m = __ballot_sync(0xffffffffu, want);
+    if (lane == 0)
+        s_warp[warp] = __popc(m);
+    __syncthreads();
+    if (warp == 0) {
+        const int v = lane < T / 32 ? s_warp[lane] : 0;
+        int incl = v;
+#pragma unroll
+        for (int o = 1; o < T / 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o)
+                incl += y;
+        }
+        int at = 0;
+        if (lane == T / 32 - 1 && incl > 0)
+            at = atomicAdd(count, incl);
+        at = __shfl_sync(0xffffffffu, at, T / 32 - 1);
+        if (lane < T / 32)
+            s_warp[lane] = at + incl - v;
+    }
+    __syncthreads();
+    if (want)
+        list[s_warp[warp] + __popc(m & ((1u << lane) - 1u))] = e;
+    __syncthreads(); /* s_warp is reused */
+}
+
+static __global__ void __launch_bounds__(T) k_update(const __grid_constant__ Dev d, int t, int epoch)
+{
+    __shared__ int s_warp[T / 32];
+    const int ntiles = d.counts[t], nlist = d.nlist[t];
+    const int* tiles = d.tiles + (size_t)t * d.ntiles;
+    const Entry* cur = d.list[t & 1];
+    Entry* next = d.list[(t + 1) & 1];
+    const int items = ntiles + (nlist + T - 1) / T;
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+        if (item >= ntiles) {
+            /* wet cells of tiles that no flow touched: they stay wet */
+            const int k = (item - ntiles) * T + threadIdx.x;
+            bool carry = false;
+            Entry e = make_int2(-1, 0);
+            if (k < nlist) {
+                e = cur[k];
+                if (e.x >= 0) {
+                    const Inst& I = d.inst[e.y];
+                    const int lc = (int)(e.x - I.off);
+                    const int i = lc / I.cols, j = lc - i * I.cols;
+                    carry = d.stamps[I.tile0 + (i >> d.lh) * I.tiles_x + (j >> d.lw)] != epoch;
+                }
+            }
+            block_append(carry, e, next, d.nlist + t + 1, s_warp);
+            continue;
+        }
+        const int tile = tiles[item];
+        const int bi = d.tile_inst[tile];
+        const Inst I = d.inst[bi];
+        const int lt = tile - I.tile0;
+        const int ty = lt / I.tiles_x, tx = lt - ty * I.tiles_x;
+        for (int q0 = 0; q0 < 1 << (d.lw + d.lh); q0 += T) {
+            const int q = q0 + threadIdx.x;
+            const int i = (ty << d.lh) + (q >> d.lw), j = (tx << d.lw) + (q & ((1 << d.lw) - 1));
+            bool want = false;
+            Entry e = make_int2(-1, bi);
+            if (q < 1 << (d.lw + d.lh) && i < I.rows && j < I.cols) {
+                const int c = (int)(I.off + (long long)i * I.cols + j);
+                const double hc = d.h[c];
+                const D4 o = d.f[c];
+                double in[4]; /* inflow from neighbour q is its outflow towards here */
+#pragma unroll
+                for (int s = 0; s < 4; s++) {
+                    int a, b;
+                    in[s] = nbr(I, i, j, s, &a, &b) ? d.f[I.off + (long long)a * I.cols + b].v[3 - s] : 0.0;
+                }
+                long long any = 0;
+#pragma unroll
+                for (int s = 0; s < 4; s++)
+                    any |= __double_as_longlong(in[s]) | __double_as_longlong(o.v[s]);
+                double hn = hc;
+                if (any != 0) {
+#pragma unroll
+                    for (int s = 0; s < 4; s++)
+                        hn += in[s] - o.v[s];
+                    d.h[c] = hn;
+                    d.zh[c] = d.z[c] + hn;
+                }
+                const bool wet = sdt::is_wet(hn, I.eps_bits);
+                want = wet || sdt::is_wet(hc, I.eps_bits);
+                e.x = wet ? c : ~c;
+            }
+            block_append(want, e, next, d.nlist + t + 1, s_warp);
+        }
+    }
+}
+
+/* f back to zero after the last step run: the cells wet in step t */
+static __global__ void __launch_bounds__(T) k_clear_flows(const __grid_constant__ Dev d, int t)
+{
+    const int n = d.nlist[t];
+    const D4 zero = {{0.0, 0.0, 0.0, 0.0}};
+    for (int k = blockIdx.x * T + threadIdx.x; k < n; k += gridDim.x * T) {
+        const Entry e = d.list[t & 1][k];
+        d.f[e.x < 0 ? ~e.x : e.x] = zero;
+    }
+}
+
+/* Every cell of every instance, a run of consecutive cells per block, with
+ * the instance carried along (offsets in shared memory): fn(c, b, inside)
+ * for all lanes of the warp together; inside is false on padding and past
+ * the end (b then still names an instance). */
+template <typename FN>
+static __device__ __forceinline__ void each_cell(const Dev& d, long long* s_offs, FN fn)
+{
+    for (int k = threadIdx.x; k <= d.B; k += T)
+        s_offs[k] = d.offs[k];
+    __syncthreads();
+    const long long per = ((d.N + gridDim.x - 1) / gridDim.x + T - 1) / T * T;
+    const long long c1 = min(d.N, per * (blockIdx.x + 1));
+    int b = 0, hi = d.B - 1; /* the last instance that starts at or before the run */
+    while (b < hi) {
+        const int mid = (b + hi + 1) >> 1;
+        if (s_offs[mid] <= per * blockIdx.x)
+            b = mid;
+        else
+            hi = mid - 1;
+    }
+    for (long long c0 = per * blockIdx.x; c0 < c1; c0 += T) {
+        const long long c = c0 + threadIdx.x;
+        while (b + 1 < d.B && s_offs[b + 1] <= c)
+            b++;
+        fn(c, b, c < c1 && c - s_offs[b] < (long long)d.inst[b].rows * d.inst[b].cols);
+    }
+}
+
+/* z after the initialisation (z_dem - h0 where h0 > 0), h = h0 with -0 made
+ * +0 (the first reference step adds 0.0 to every cell), z + h, and list 0 */
+static __global__ void __launch_bounds__(T) k_init(const __grid_constant__ Dev d, const double* __restrict__ z_dem,
+                                            const double* __restrict__ h0, double* z)
+{
+    extern __shared__ long long s_offs[];
+    each_cell(d, s_offs, [&](long long c, int b, bool inside) {
+        bool wet = false;
+        if (inside) {
+            const double hv = h0[c];
+            const double zv = hv > 0.0 ? z_dem[c] - hv : z_dem[c];
+            const double hc = sdt::plus_zero(hv);
+            z[c] = zv;
+            d.h[c] = hc;
+            d.zh[c] = zv + hc;
+            wet = sdt::is_wet(hc, d.inst[b].eps_bits);
+        } else if (c < d.N) {
+            z[c] = d.h[c] = d.zh[c] = 0.0;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, wet);
+        if (m) {
+            const int lane = threadIdx.x & 31;
+            int at = 0;
+            if (lane == 0)
+                at = atomicAdd(d.nlist, __popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (wet)
+                d.list[0][at + __popc(m & ((1u << lane) - 1u))] = make_int2((int)c, b);
+        }
+    });
+}
+
+/* list t and z + h again from h (a checkpoint just copied into it) */
+static __global__ void __launch_bounds__(T) k_relist(const __grid_constant__ Dev d, int t)
+{
+    extern __shared__ long long s_offs[];
+    each_cell(d, s_offs, [&](long long c, int b, bool inside) {
+        bool wet = false;
+        if (inside) {
+            const double hc = d.h[c];
+            d.zh[c] = d.z[c] + hc;
+            wet = sdt::is_wet(hc, d.inst[b].eps_bits);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, wet);
+        if (m) {
+            const int lane = threadIdx.x & 31;
+            int at = 0;
+            if (lane == 0)
+                at = atomicAdd(d.nlist + t, __popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (wet)
+                d.list[t & 1][at + __popc(m & ((1u << lane) - 1u))] = make_int2((int)c, b);
+        }
+    });
+}
+
+/* The coefficients of step t's wet cells and their parts of dL/dr, dL/deps.
+ * Neighbouring entries come from a few tiles, so a warp holds a few runs of
+ * entries of one instance: a segmented scan sums each run, and its last lane
+ * adds it to one of COPIES partial sums of the instance (k_fold adds those
+ * up).  All on one word per instance and sum, the atomics of a step queued
+ * for 30 us (287,000 entries of 64 instances: 48.7 us). */
+static __global__ void __launch_bounds__(T) k_coeffs(const __grid_constant__ Dev d, const __grid_constant__ Adj a, int t)
+{
+    const int n = d.nlist[t];
+    const long long base = tape_base(d, t, n);
+    if (base < 0)
+        return;
+    const int lane = threadIdx.x & 31;
+    double* sums = a.part + (size_t)(blockIdx.x % COPIES) * 2 * d.B;
+    const int stride = gridDim.x * T;
+    for (int k0 = ((threadIdx.x >> 5) * (int)gridDim.x + blockIdx.x) * 32; k0 < n; k0 += stride) {
+        const int k = k0 + lane;
+        const Entry e = k < n ? d.t_entry[base + k] : make_int2(-1, -1);
+        const unsigned elim = e.x >= 0 ? d.t_elim[base + k] : 31u;
+        const int kk = 5 - __popc(elim);
+        double er = 0.0, ee = 0.0;
+        if (kk > 0) {
+            const int c = e.x;
+            const Inst I = d.inst[e.y];
+            const int lc = (int)(c - I.off);
+            const int i = lc / I.cols, j = lc - i * I.cols;
+            const D4 diff = d.t_diff[base + k];
+            const double own = a.lam[c];
+            double S = 0.0, lf[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                lf[q] = 0.0;
+                if (!(elim & (2u << q))) {
+                    int na, nb;
+                    const bool in = nbr(I, i, j, q, &na, &nb);
+                    lf[q] = (in ? a.lam[I.off + (long long)na * I.cols + nb] : 0.0) - own;
+                    S += lf[q];
+                    er += lf[q] * diff.v[q];
+                }
+            }
+            const double g = cal_div_small(I.r, kk) * S; /* exact division by 1..5 on the integer pipe */
+            D4 w;
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                w.v[q] = (elim & (2u << q)) ? 0.0 : g - I.r * lf[q];
+            a.stamp[c] = t;
+            a.g[c] = g;
+            a.w[c] = w;
+            if (elim & 1u) {
+                ee = -cal_div_small(S * I.r, kk);
+                if (a.mu)
+                    a.mu[c] += g;
+            }
+        }
+        const int before = __shfl_up_sync(0xffffffffu, e.y, 1); /* every lane takes part */
+        const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || before != e.y);
+        const int head = 31 - __clz(heads & (0xffffffffu >> (31 - lane))); /* first lane of this lane's run */
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double r = __shfl_up_sync(0xffffffffu, er, o), p = __shfl_up_sync(0xffffffffu, ee, o);
+            if (lane - o >= head) {
+                er += r;
+                ee += p;
+            }
+        }
+        const bool tail = lane == 31 || ((heads >> (lane + 1)) & 1u);
+        if (tail && er != 0.0)
+            atomicAdd(sums + e.y, er);
+        if (tail && ee != 0.0)
+            atomicAdd(sums + d.B + e.y, ee);
+    }
+}
+
+/* the instances' dL/dr and dL/deps: their partial sums in a fixed order */
+static __global__ void k_fold(const double* __restrict__ part, double* __restrict__ grad, int n)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n)
+        return;
+    double v = 0.0;
+    for (int c = 0; c < COPIES; c++)
+        v += part[(size_t)c * n + q];
+    grad[q] = v;
+}
+
+/* lambda_t from lambda_{t+1}: every cell whose lambda changes lies in a tile
+ * that step t flagged (it kept a neighbour or is one that was kept) */
+static __global__ void __launch_bounds__(T) k_gather(const __grid_constant__ Dev d, const __grid_constant__ Adj a, int t)
+{
+    if (tape_base(d, t, d.nlist[t]) < 0)
+        return;
+    const int ntiles = d.counts[t];
+    const int* tiles = d.tiles + (size_t)t * d.ntiles;
+    for (int item = blockIdx.x; item < ntiles; item += gridDim.x) {
+        const int tile = tiles[item];
+        const Inst I = d.inst[d.tile_inst[tile]];
+        const int lt = tile - I.tile0;
+        const int ty = lt / I.tiles_x, tx = lt - ty * I.tiles_x;
+        for (int q = threadIdx.x; q < 1 << (d.lw + d.lh); q += T) {
+            const int i = (ty << d.lh) + (q >> d.lw), j = (tx << d.lw) + (q & ((1 << d.lw) - 1));
+            if (i >= I.rows || j >= I.cols)
+                continue;
+            const long long c = I.off + (long long)i * I.cols + j;
+            long long cn[4];
+            unsigned have = a.stamp[c] == t ? 16u : 0u;
+#pragma unroll
+            for (int s = 0; s < 4; s++) {
+                int na, nb;
+                const bool in = nbr(I, i, j, s, &na, &nb);
+                cn[s] = I.off + (long long)na * I.cols + nb;
+                if (in && a.stamp[cn[s]] == t)
+                    have |= 1u << s;
+            }
+            if (!have)
+                continue;
+            double from_nb = 0.0;
+#pragma unroll
+            for (int s = 0; s < 4; s++) /* x is neighbour 3 - s of its neighbour s */
+                if (have & (1u << s))
+                    from_nb += a.w[cn[s]].v[3 - s];
+            a.lam[c] = a.lam[c] + ((have & 16u) ? a.g[c] : 0.0) + from_nb;
+        }
+    }
+}
+
+/* lambda_T = 2 (h_T - target), mu_T the same, and the instances' losses */
+static __global__ void __launch_bounds__(T) k_loss(const __grid_constant__ Dev d, const __grid_constant__ Adj a,
+                                            const double* __restrict__ target, double* loss)
+{
+    extern __shared__ long long s_offs[];
+    double acc = 0.0;
+    int cur = -1; /* the instance acc belongs to, the same in every lane */
+    auto flush = [&]() {
+        double v = acc;
+        for (int o = 16; o > 0; o >>= 1)
+            v += __shfl_down_sync(0xffffffffu, v, o);
+        if ((threadIdx.x & 31) == 0 && cur >= 0 && v != 0.0)
+            atomicAdd(loss + cur, v);
+        acc = 0.0;
+    };
+    each_cell(d, s_offs, [&](long long c, int b, bool inside) {
+        const double diff = inside ? d.h[c] - target[c] : 0.0;
+        if (c < d.N) {
+            a.lam[c] = 2.0 * diff;
+            if (a.mu)
+                a.mu[c] = 2.0 * diff;
+        }
+        const int b0 = __shfl_sync(0xffffffffu, b, 0);
+        if (__all_sync(0xffffffffu, b == b0)) {
+            if (b0 != cur) {
+                flush();
+                cur = b0;
+            }
+            acc += diff * diff;
+        } else if (diff != 0.0) {
+            atomicAdd(loss + b, diff * diff);
+        }
+    });
+    flush();
+}
+
+/* dL/dh0 (see the top of the file) */
+static __global__ void k_final_grad(const double* __restrict__ h0, const double* __restrict__ lam,
+                             const double* __restrict__ mu, double* __restrict__ g_h0, long long n)
+{
+    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x)
+        g_h0[c] = h0[c] > 0.0 ? mu[c] : lam[c];
+}
+
+static int dense_blocks(long long n)
+{
+    const long long b = (n + T - 1) / T;
+    return (int)(b > 152 * 8 ? 152 * 8 : (b < 1 ? 1 : b));
+}
+
+/* steps [t0, t1) queued; epochs are unique per run since the stamps were
+ * cleared */
+static void queue_steps(const Dev& d, int t0, int t1, int epoch0, bool taped, cudaStream_t st)
+{
+    for (int t = t0; t < t1; t++) {
+        k_outflows<<<BLOCKS, T, 0, st>>>(d, t, epoch0 + t, taped ? 1 : 0);
+        k_update<<<BLOCKS, T, 0, st>>>(d, t, epoch0 + t);
+    }
+}
+
+/* the adjoint of steps [t0, t1), last first */
+static void queue_adjoint(const Dev& d, const Adj& a, int t0, int t1, cudaStream_t st)
+{
+    for (int t = t1 - 1; t >= t0; t--) {
+        k_coeffs<<<BLOCKS, T, 0, st>>>(d, a, t);
+        k_gather<<<BLOCKS, T, 0, st>>>(d, a, t);
+    }
+}
+
+} // namespace sdtw
