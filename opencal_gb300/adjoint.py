@@ -1,11 +1,11 @@
 """SCIDDICA-T rollout as a differentiable torch function (calibration only).
 
 ``rollout(z_dem, h0, p_r, p_eps, steps)`` runs ``steps`` plain-mode steps
-on the GPU (the bit-exact fused step kernel) and returns h_T; its backward
-calls the hand-written adjoint kernels of ``libopencal_models.so``
-(csrc/models/sciddicaT_adjoint.cu): elimination sets recomputed from the
-forward states and frozen, sqrt(T) checkpointing, gradients with respect to
-h0 (including the initialisation's z -= h0), p_r and p_eps.  Torch is used
+on the GPU (bit-exact, over the list of wet cells) and returns h_T; its
+backward calls the hand-written adjoint kernels of ``libopencal_models.so``
+(csrc/models/sciddicaT_adjoint.cu): the forward's elimination sets, taped and
+frozen (sqrt(T) checkpoints where the tape would not fit), gradients with
+respect to h0 (including the initialisation's z -= h0), p_r and p_eps.  Torch is used
 for device memory and streams only; the library itself stays C.
 """
 from __future__ import annotations
@@ -26,6 +26,7 @@ def _lib():
         m.cal_sdt_adj_create.restype = C.c_void_p
         m.cal_sdt_adj_create.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int]
         m.cal_sdt_adj_destroy.argtypes = [C.c_void_p]
+        m.cal_sdt_adj_set_tape.argtypes = [C.c_void_p, C.c_int]
         m.cal_sdt_adj_forward.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_double, C.c_double, C.c_void_p,
                                           C.c_void_p]
         m.cal_sdt_adj_backward.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(C.c_double),
@@ -54,6 +55,8 @@ class SciddicaTRollout(torch.autograd.Function):
         h0 = h0.contiguous()
         rows, cols = h0.shape
         ws = _Workspace(rows, cols, int(steps), toroidal)
+        if not any(ctx.needs_input_grad):
+            _lib().cal_sdt_adj_set_tape(ws.handle, 0)
         hT = torch.empty_like(h0)
         stream = torch.cuda.current_stream().cuda_stream
         rc = _lib().cal_sdt_adj_forward(ws.handle, z_dem.data_ptr(), h0.data_ptr(), float(p_r), float(p_eps),

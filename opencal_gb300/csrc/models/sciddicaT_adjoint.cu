@@ -1,6 +1,6 @@
 /*
  * sciddicaT_adjoint.cu -- reverse-mode adjoint of a SCIDDICA-T rollout
- * (plain mode), for calibration.
+ * (plain mode) of one grid, for calibration.
  *
  * Forward model (one step, every wet cell c, h_c > epsilon):
  *   m = h_c - eps, u_0 = z_c + eps, u_n = z_nb(n) + h_nb(n) (n = 1..4),
@@ -8,10 +8,9 @@
  *   avg_c = (m + sum_{n in A_c} u_n) / k_c,
  *   f_{c,n} = r (avg_c - u_n) for n in A_c, n >= 1, else 0;
  *   h'_x = h_x + sum_n (f_{nb(n), opp(n)} - f_{x,n}).
- * The elimination sets A_c and the wet set are discrete: they are taken
- * from the forward state (recomputed bit-identically from h_t) and frozen,
- * so the derivative is that of the piecewise-linear map the forward
- * actually evaluated.
+ * The elimination sets A_c and the wet set are discrete: they are the
+ * forward's, frozen, so the derivative is that of the piecewise-linear map
+ * the forward actually evaluated.
  *
  * Adjoint of one step, with lambda' = dL/dh_{t+1}:
  *   lf_{c,n} = lambda'_nb(n) - lambda'_c       (0 for absent neighbours'
@@ -25,324 +24,184 @@
  * and the initialisation z = z_dem - h0 where h0 > 0 adds
  *   dL/dh0 = lambda_0 - [h0 > 0] lambda_z.
  *
- * Memory: sqrt(T) checkpointing -- h is stored every K = ceil(sqrt(T))
- * steps during the forward; the backward recomputes one segment of K states
- * at a time from its checkpoint (bit-identical forward) and runs the
- * adjoint through it in reverse.
- *
- * Sparsity: the forward step (16 x 8 tiles) reports per tile whether a
- * cell of it is wet before and after the step; during the recompute those
- * flags are kept for every state of the segment.  The adjoint of a step
- * then visits only the tiles holding a wet cell (coefficients) and those
- * tiles and their edge neighbours (gather), updating lambda in place: in
- * every other cell g, gz and w are 0, so lambda and lambda_z are unchanged
- * there, bit for bit as the dense sweep leaves them.
- *
- * Reductions of the parameter gradients use per-block partials folded in a
- * fixed order (deterministic).
+ * The steps and their adjoint are the wet-cell list's (sciddicaT_wet.cuh)
+ * with one instance.  The forward tapes the rollout into a tape sized by a
+ * guess; the backward first learns what the tape needed.  When it was too
+ * small, the forward runs again with one that fits, or, when a whole-rollout
+ * tape would take more than half of the free device memory, with h stored
+ * every K = ceil(sqrt(T)) steps, and the sweep then recomputes and tapes one
+ * segment at a time.
  */
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
 
-#include "sciddicaT_kernels.cuh"
+#include <algorithm>
+
+#include "sciddicaT_wet.cuh"
 
 namespace sdtadj {
 
-constexpr int T = 256;      /* threads per block */
-constexpr int PBLOCKS = 1024; /* partials of the parameter gradients */
-constexpr int TW = 16, TH = 8; /* forward tiles, also the adjoint's unit of work */
+using sdtw::Adj;
+using sdtw::Dev;
+using sdtw::Inst;
+using sdtw::T;
+
+/* the unit of the update and the gather, as the ensembles' */
+constexpr int LW = 5, LH = 3;
 
 struct Work {
     int rows = 0, cols = 0, steps = 0, toroidal = 0, K = 0, nseg = 0;
-    long long n = 0;
     double r = 0, eps = 0;
-    double* z = nullptr;       /* z after the initialisation (z_dem - h0 where h0 > 0) */
-    double* h0 = nullptr;      /* initial thickness as given */
-    double* ckpt = nullptr;    /* (nseg) checkpoints: h at steps 0, K, 2K, ... */
-    double* seg = nullptr;     /* (K + 1) states of the segment being reversed */
-    double* lam[2] = {nullptr, nullptr};
-    double* lamz = nullptr;
-    double* g = nullptr;       /* g_c */
-    double* gz = nullptr;      /* [0 in A_c] g_c */
-    double* w = nullptr;       /* 4 * n: w_{c,m} */
-    unsigned char* flags = nullptr; /* (K + 1) x tiles: the forward's tile_wet of each step of the segment */
-    unsigned char* all_wet = nullptr; /* tiles: 3 (every tile visited) */
-    int tiles_x = 0, tiles_y = 0;
-    double* partial = nullptr; /* 2 * PBLOCKS */
-    double* result = nullptr;  /* 2 */
+    Dev d = {};
+    Adj a = {};
+    Inst* inst = nullptr;
+    long long* offs = nullptr;
+    double *z_dem = nullptr, *z = nullptr, *h0 = nullptr;
+    double* ckpt = nullptr; /* segments only */
+    char* slab = nullptr;   /* every array of fixed size, one allocation */
+    char* tape = nullptr;
+    bool want_tape = true;
+    bool flows_clear = false;
 };
 
-/* z after init and the canonical h0 (the first step turns -0 into +0) */
-__global__ void k_init(const double* __restrict__ z_dem, const double* __restrict__ h0, double* __restrict__ z,
-                       double* __restrict__ h, long long n)
+__global__ void k_instance(Inst I, long long n, Inst* inst, long long* offs)
 {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-        const double hv = h0[c];
-        z[c] = hv > 0.0 ? z_dem[c] - hv : z_dem[c];
-        h[c] = hv;
-    }
+    inst[0] = I;
+    offs[0] = 0;
+    offs[1] = n;
 }
 
-struct Geo {
-    int rows, cols, toroidal;
-    long long n;
+/* successive arrays of a slab, 256-byte aligned; with base NULL only sizes */
+struct Carve {
+    char* base;
+    size_t at = 0;
+    template <typename E>
+    void take(E** p, size_t count)
+    {
+        *p = (E*)(base + at);
+        at += (count * sizeof(E) + 255) & ~(size_t)255;
+    }
 };
 
-/* neighbour n = 1..4 (north, west, east, south) of (i, j); false outside a flat grid */
-static __device__ __forceinline__ bool nb(const Geo& g, int i, int j, int n, long long* c)
+static size_t carve(Work& W, char* base)
 {
-    int a = i + (n == 1 ? -1 : (n == 4 ? 1 : 0));
-    int b = j + (n == 2 ? -1 : (n == 3 ? 1 : 0));
-    if (g.toroidal) {
-        a = a < 0 ? a + g.rows : (a >= g.rows ? a - g.rows : a);
-        b = b < 0 ? b + g.cols : (b >= g.cols ? b - g.cols : b);
-    } else if ((unsigned)a >= (unsigned)g.rows || (unsigned)b >= (unsigned)g.cols) {
-        return false;
+    const size_t n = (size_t)W.rows * W.cols, steps = (size_t)W.steps + 1;
+    Dev& d = W.d;
+    Adj& a = W.a;
+    Carve c{base};
+    c.take(&W.inst, 1);
+    c.take(&W.offs, 2);
+    c.take((int**)&d.tile_inst, d.ntiles);
+    c.take(&W.z_dem, n);
+    c.take(&W.z, n);
+    c.take(&W.h0, n);
+    c.take(&d.h, n);
+    c.take(&d.zh, n);
+    c.take(&d.f, n);
+    c.take(&d.list[0], n);
+    c.take(&d.list[1], n);
+    c.take(&d.nlist, steps);
+    c.take(&d.counts, steps);
+    c.take(&d.tiles, (size_t)d.ntiles * steps);
+    c.take(&d.stamps, d.ntiles);
+    c.take(&d.toff, steps);
+    c.take(&d.need, 1);
+    c.take(&a.lam, n);
+    c.take(&a.mu, n);
+    c.take(&a.stamp, n);
+    c.take(&a.w, n);
+    c.take(&a.g, n);
+    c.take(&a.part, 2 * sdtw::COPIES);
+    c.take(&a.grad, 2);
+    d.inst = W.inst;
+    d.offs = W.offs;
+    d.z = W.z;
+    return c.at;
+}
+
+/* a tape of `entries` entries, instead of the one there was */
+static bool make_tape(Work& W, long long entries)
+{
+    Dev& d = W.d;
+    cudaFree(W.tape);
+    W.tape = nullptr;
+    d.cap = 0;
+    for (int pass = 0; pass < 2; pass++) {
+        Carve c{W.tape};
+        c.take(&d.t_diff, (size_t)entries);
+        c.take(&d.t_entry, (size_t)entries);
+        c.take(&d.t_elim, (size_t)entries);
+        if (pass == 0 && cudaMalloc(&W.tape, c.at) != cudaSuccess) {
+            (void)cudaGetLastError();
+            W.tape = nullptr;
+            return false;
+        }
     }
-    *c = (long long)a * g.cols + b;
+    d.cap = entries;
     return true;
 }
 
-/* the forward's elimination, returning the set, the count, the average and u */
-static __device__ __forceinline__ void eliminate(double hc, double zc, const double u14[4], double eps,
-                                                 unsigned* elim_out, int* k_out, double* avg_out, double u[5])
+/* the rollout from h0 and z_dem, queued: taped, or with checkpoints (keep) */
+static void queue_forward(Work& W, bool keep, cudaStream_t st)
 {
-    const double m = hc - eps;
-    u[0] = zc + eps;
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-        u[q + 1] = u14[q];
-    unsigned elim = 0;
-    double average;
-    int cells_count;
-    bool again;
-    do {
-        again = false;
-        average = m;
-        cells_count = 0;
-#pragma unroll
-        for (int q = 0; q < 5; q++)
-            if (!(elim & (1u << q))) {
-                average += u[q];
-                cells_count++;
-            }
-        if (cells_count != 0)
-            average = cal_div_small(average, cells_count);
-#pragma unroll
-        for (int q = 0; q < 5; q++)
-            if (!(elim & (1u << q)) && cal_le(average, u[q])) {
-                elim |= 1u << q;
-                again = true;
-            }
-    } while (again);
-    /* the set A (cells NOT eliminated) and its size when the last average was formed */
-    unsigned a_set = 0;
-    int k = 0;
-#pragma unroll
-    for (int q = 0; q < 5; q++)
-        if (!(elim & (1u << q))) {
-            a_set |= 1u << q;
-            k++;
-        }
-    (void)cells_count;
-    *elim_out = a_set;
-    *k_out = k;
-    *avg_out = average;
-}
-
-/* per cell of the visited tiles: coefficients g, gz, w and partials of
- * dL/dr, dL/deps; then lambda_t and lambda_z by a gather (no atomics) */
-static __device__ __forceinline__ int tile_of(int i, int j, int tiles_x)
-{
-    return (i / TH) * tiles_x + (j / TW);
-}
-
-/* k_coeffs_tiles: the tiles whose flag has `mask` set (a wet cell in h_t):
- * block b takes tiles b, b + gridDim.x, ...; every cell of a visited tile
- * is written (0 at dry cells) */
-__global__ void __launch_bounds__(T) k_coeffs_tiles(Geo geo, const double* __restrict__ z,
-                                                    const double* __restrict__ h, const double* __restrict__ lam,
-                                                    double r, double eps, long long eps_bits,
-                                                    double* __restrict__ g, double* __restrict__ gz,
-                                                    double* __restrict__ w, double* __restrict__ partial,
-                                                    const unsigned char* __restrict__ flags, int mask,
-                                                    int tiles_x, int ntiles)
-{
-    __shared__ double sr[T / 32], se[T / 32];
-    double pr = 0.0, pe = 0.0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        if (!(flags[t] & mask))
-            continue;
-        const int ty = t / tiles_x, tx = t - ty * tiles_x;
-        for (int k = threadIdx.x; k < TW * TH; k += T) {
-            const int i = ty * TH + k / TW, j = tx * TW + k % TW;
-            if (i >= geo.rows || j >= geo.cols)
-                continue;
-            const long long c = (long long)i * geo.cols + j;
-            const double hc = h[c];
-            double gc = 0.0, gzc = 0.0, wc[4] = {0.0, 0.0, 0.0, 0.0};
-            if (sdt::is_wet(hc, eps_bits)) {
-                double u14[4], lnb[4];
-                bool in[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    long long cn;
-                    in[q] = nb(geo, i, j, q + 1, &cn);
-                    u14[q] = in[q] ? z[cn] + h[cn] : 0.0 + 0.0;
-                    lnb[q] = in[q] ? lam[cn] : 0.0;
-                }
-                unsigned a_set;
-                int kk;
-                double avg, u[5];
-                eliminate(hc, z[c], u14, eps, &a_set, &kk, &avg, u);
-                if (kk > 0) {
-                    const double lc = lam[c];
-                    double S = 0.0, lf[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        lf[q] = 0.0;
-                        if (a_set & (1u << (q + 1))) {
-                            lf[q] = lnb[q] - lc;
-                            S += lf[q];
-                            pr += lf[q] * (avg - u[q + 1]);
-                        }
-                    }
-                    gc = cal_div_small(r, kk) * S; /* = (r / kk) * S: exact division by 1..5 on the integer pipe */
-                    gzc = (a_set & 1u) ? gc : 0.0;
-                    pe += cal_div_small(S * r * ((a_set & 1u) ? 0.0 : -1.0), kk);
-#pragma unroll
-                    for (int q = 0; q < 4; q++)
-                        if (a_set & (1u << (q + 1)))
-                            wc[q] = gc - r * lf[q];
-                }
-            }
-            g[c] = gc;
-            gz[c] = gzc;
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                w[q * geo.n + c] = wc[q];
-        }
+    Dev& d = W.d;
+    const size_t n = (size_t)d.N;
+    cudaMemsetAsync(d.stamps, 0, sizeof(int) * d.ntiles, st);
+    cudaMemsetAsync(d.counts, 0, sizeof(int) * (W.steps + 1), st);
+    cudaMemsetAsync(d.nlist, 0, sizeof(int) * (W.steps + 1), st);
+    cudaMemsetAsync(d.toff, 0, sizeof(long long), st);
+    cudaMemsetAsync(d.need, 0, sizeof(long long), st);
+    if (!W.flows_clear) {
+        cudaMemsetAsync(d.f, 0, n * sizeof(sdtw::D4), st);
+        W.flows_clear = true;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        pr += __shfl_down_sync(0xffffffffu, pr, o);
-        pe += __shfl_down_sync(0xffffffffu, pe, o);
+    sdtw::k_init<<<sdtw::dense_blocks(d.N), T, 2 * sizeof(long long), st>>>(d, W.z_dem, W.h0, W.z);
+    const int per = keep ? W.K : std::max(1, W.steps);
+    for (int t = 0; t < W.steps; t += per) {
+        if (keep)
+            cudaMemcpyAsync(W.ckpt + (size_t)(t / per) * n, d.h, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
+        sdtw::queue_steps(d, t, std::min(t + per, W.steps), 1, !keep, st);
     }
-    if ((threadIdx.x & 31) == 0) {
-        sr[threadIdx.x >> 5] = pr;
-        se[threadIdx.x >> 5] = pe;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0.0, b = 0.0;
-        for (int q = 0; q < T / 32; q++) {
-            a += sr[q];
-            b += se[q];
-        }
-        partial[blockIdx.x] += a;
-        partial[PBLOCKS + blockIdx.x] += b;
-    }
+    if (W.steps > 0)
+        sdtw::k_clear_flows<<<sdtw::BLOCKS, T, 0, st>>>(d, W.steps - 1);
 }
 
-/* is tile (ty, tx) flagged?  Outside a flat grid: no */
-static __device__ __forceinline__ bool tile_flag(const Geo& geo, const unsigned char* flags, int mask, int ty,
-                                                 int tx, int tiles_x, int tiles_y)
+/* the largest tape any step sequence asked for since the last forward */
+static cudaError_t tape_need(Work& W, long long* need, cudaStream_t st)
 {
-    if (geo.toroidal) {
-        ty = ty < 0 ? ty + tiles_y : (ty >= tiles_y ? ty - tiles_y : ty);
-        tx = tx < 0 ? tx + tiles_x : (tx >= tiles_x ? tx - tiles_x : tx);
-    } else if ((unsigned)ty >= (unsigned)tiles_y || (unsigned)tx >= (unsigned)tiles_x) {
-        return false;
+    cudaMemcpyAsync(need, W.d.need, sizeof(*need), cudaMemcpyDeviceToHost, st);
+    return cudaStreamSynchronize(st);
+}
+
+static void queue_seed(Work& W, const double* gT, cudaStream_t st)
+{
+    const size_t b = (size_t)W.d.N * sizeof(double);
+    cudaMemcpyAsync(W.a.lam, gT, b, cudaMemcpyDeviceToDevice, st);
+    cudaMemcpyAsync(W.a.mu, gT, b, cudaMemcpyDeviceToDevice, st);
+    cudaMemsetAsync(W.a.stamp, 0xff, sizeof(int) * (size_t)W.d.N, st);
+    cudaMemsetAsync(W.a.part, 0, sizeof(double) * 2 * sdtw::COPIES, st);
+}
+
+/* the reverse sweep recomputing segments from the checkpoints */
+static void queue_segments(Work& W, cudaStream_t st)
+{
+    Dev& d = W.d;
+    const size_t n = (size_t)d.N;
+    cudaMemsetAsync(d.need, 0, sizeof(long long), st);
+    for (int s = W.nseg - 1; s >= 0; s--) {
+        const int t0 = s * W.K, t1 = std::min(t0 + W.K, W.steps);
+        cudaMemcpyAsync(d.h, W.ckpt + (size_t)s * n, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
+        cudaMemsetAsync(d.nlist + t0, 0, sizeof(int) * (t1 - t0 + 1), st);
+        cudaMemsetAsync(d.counts + t0, 0, sizeof(int) * (t1 - t0), st);
+        cudaMemsetAsync(d.toff + t0, 0, sizeof(long long), st);
+        cudaMemsetAsync(d.stamps, 0, sizeof(int) * d.ntiles, st);
+        sdtw::k_relist<<<sdtw::dense_blocks(d.N), T, 2 * sizeof(long long), st>>>(d, t0);
+        sdtw::queue_steps(d, t0, t1, 1, true, st);
+        sdtw::k_clear_flows<<<sdtw::BLOCKS, T, 0, st>>>(d, t1 - 1);
+        sdtw::queue_adjoint(d, W.a, t0, t1, st);
     }
-    return (flags[ty * tiles_x + tx] & mask) != 0;
-}
-
-/* k_gather_tiles: in place, on the tiles that are flagged or have a flagged edge
- * neighbour; coefficients of unflagged tiles read as 0 (the dense sweep
- * wrote 0 there) */
-__global__ void __launch_bounds__(T) k_gather_tiles(Geo geo, double* __restrict__ lam,
-                                                    const double* __restrict__ g, const double* __restrict__ gz,
-                                                    const double* __restrict__ w, double* __restrict__ lamz,
-                                                    const unsigned char* __restrict__ flags, int mask, int tiles_x,
-                                                    int tiles_y)
-{
-    const int ntiles = tiles_x * tiles_y;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int ty = t / tiles_x, tx = t - ty * tiles_x;
-        const bool own = (flags[t] & mask) != 0;
-        if (!own && !tile_flag(geo, flags, mask, ty - 1, tx, tiles_x, tiles_y) &&
-            !tile_flag(geo, flags, mask, ty + 1, tx, tiles_x, tiles_y) &&
-            !tile_flag(geo, flags, mask, ty, tx - 1, tiles_x, tiles_y) &&
-            !tile_flag(geo, flags, mask, ty, tx + 1, tiles_x, tiles_y))
-            continue;
-        for (int k = threadIdx.x; k < TW * TH; k += T) {
-            const int i = ty * TH + k / TW, j = tx * TW + k % TW;
-            if (i >= geo.rows || j >= geo.cols)
-                continue;
-            const long long c = (long long)i * geo.cols + j;
-            double from_nb = 0.0;
-            long long cn;
-            /* x is neighbour opp(d) of its neighbour d: north<->south (1<->4), west<->east (2<->3) */
-            if (nb(geo, i, j, 1, &cn))
-                from_nb += (flags[tile_of((int)(cn / geo.cols), (int)(cn % geo.cols), tiles_x)] & mask)
-                               ? w[3 * geo.n + cn] : 0.0;
-            if (nb(geo, i, j, 2, &cn))
-                from_nb += (flags[tile_of((int)(cn / geo.cols), (int)(cn % geo.cols), tiles_x)] & mask)
-                               ? w[2 * geo.n + cn] : 0.0;
-            if (nb(geo, i, j, 3, &cn))
-                from_nb += (flags[tile_of((int)(cn / geo.cols), (int)(cn % geo.cols), tiles_x)] & mask)
-                               ? w[1 * geo.n + cn] : 0.0;
-            if (nb(geo, i, j, 4, &cn))
-                from_nb += (flags[tile_of((int)(cn / geo.cols), (int)(cn % geo.cols), tiles_x)] & mask)
-                               ? w[cn] : 0.0;
-            const double gc = own ? g[c] : 0.0, gzc = own ? gz[c] : 0.0;
-            lam[c] = lam[c] + gc + from_nb;
-            lamz[c] += gzc + from_nb;
-        }
-    }
-}
-
-__global__ void k_final_grad(const double* __restrict__ h0, const double* __restrict__ lam,
-                             const double* __restrict__ lamz, double* __restrict__ g_h0, long long n)
-{
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x)
-        g_h0[c] = lam[c] - (h0[c] > 0.0 ? lamz[c] : 0.0);
-}
-
-__global__ void k_fold_partials(const double* __restrict__ partial, double* __restrict__ out)
-{
-    if (threadIdx.x < 2) {
-        double a = 0.0;
-        for (int b = 0; b < PBLOCKS; b++)
-            a += partial[threadIdx.x * PBLOCKS + b];
-        out[threadIdx.x] = a;
-    }
-}
-
-static int grid_for(long long n)
-{
-    long long b = (n + T - 1) / T;
-    return (int)(b > 152 * 8 ? 152 * 8 : (b < 1 ? 1 : b));
-}
-
-/* one forward step from `h` into `h_next` (the fused kernel, bit-exact);
- * tile_wet: optional per-tile wet flags before / after the step */
-static void fwd_step(const Work& W, const double* h, double* h_next, cudaStream_t st,
-                     unsigned char* tile_wet = nullptr)
-{
-    sdt::Params p;
-    p.z = W.z;
-    p.h = h;
-    p.h_next = h_next;
-    p.rows = W.rows;
-    p.cols = W.cols;
-    p.toroidal = W.toroidal;
-    p.eps = W.eps;
-    p.r = W.r;
-    memcpy(&p.eps_bits, &W.eps, sizeof(double));
-    p.tile_wet = tile_wet;
-    sdt::launch<TW, TH>(p, st);
 }
 
 } // namespace sdtadj
@@ -355,31 +214,25 @@ extern "C" void* cal_sdt_adj_create(int rows, int cols, int steps, int toroidal)
     Work* W = new Work();
     W->rows = rows;
     W->cols = cols;
-    W->steps = steps;
+    W->steps = steps > 0 ? steps : 0;
     W->toroidal = toroidal;
-    W->n = (long long)rows * cols;
     W->K = (int)ceil(sqrt((double)(steps > 0 ? steps : 1)));
-    W->nseg = (steps + W->K - 1) / W->K;
-    if (W->nseg < 1)
-        W->nseg = 1;
-    const size_t b = W->n * sizeof(double);
-    bool ok = cudaMalloc(&W->z, b) == cudaSuccess && cudaMalloc(&W->h0, b) == cudaSuccess &&
-              cudaMalloc(&W->ckpt, b * (size_t)W->nseg) == cudaSuccess &&
-              cudaMalloc(&W->seg, b * (size_t)(W->K + 1)) == cudaSuccess &&
-              cudaMalloc(&W->lam[0], b) == cudaSuccess && cudaMalloc(&W->lam[1], b) == cudaSuccess &&
-              cudaMalloc(&W->lamz, b) == cudaSuccess && cudaMalloc(&W->g, b) == cudaSuccess &&
-              cudaMalloc(&W->gz, b) == cudaSuccess && cudaMalloc(&W->w, 4 * b) == cudaSuccess &&
-              cudaMalloc(&W->partial, 2 * sdtadj::PBLOCKS * sizeof(double)) == cudaSuccess &&
-              cudaMalloc(&W->result, 2 * sizeof(double)) == cudaSuccess;
-    W->tiles_x = (cols + sdtadj::TW - 1) / sdtadj::TW;
-    W->tiles_y = (rows + sdtadj::TH - 1) / sdtadj::TH;
-    const size_t nt = (size_t)W->tiles_x * W->tiles_y;
-    ok = ok && cudaMalloc(&W->flags, nt * (size_t)(W->K + 1)) == cudaSuccess &&
-         cudaMalloc(&W->all_wet, nt) == cudaSuccess && cudaMemset(W->all_wet, 3, nt) == cudaSuccess;
-    if (!ok) {
+    W->nseg = (W->steps + W->K - 1) / W->K;
+    sdtw::Dev& d = W->d;
+    d.B = 1;
+    d.N = (long long)rows * cols;
+    d.lw = sdtadj::LW;
+    d.lh = sdtadj::LH;
+    const int tx = (cols + (1 << d.lw) - 1) >> d.lw, ty = (rows + (1 << d.lh) - 1) >> d.lh;
+    d.ntiles = tx * ty;
+    const size_t bytes = sdtadj::carve(*W, nullptr);
+    if (rows <= 0 || cols <= 0 || d.N >= 0x7fffffffLL || cudaMalloc(&W->slab, bytes) != cudaSuccess) {
+        (void)cudaGetLastError();
         fprintf(stderr, "opencal-gb300: cal_sdt_adj_create: out of device memory\n");
+        delete W;
         return nullptr;
     }
+    sdtadj::carve(*W, W->slab);
     return W;
 }
 
@@ -388,48 +241,58 @@ extern "C" void cal_sdt_adj_destroy(void* handle)
     Work* W = (Work*)handle;
     if (!W)
         return;
-    cudaFree(W->z);
-    cudaFree(W->h0);
+    cudaFree(W->slab);
+    cudaFree(W->tape);
     cudaFree(W->ckpt);
-    cudaFree(W->seg);
-    cudaFree(W->lam[0]);
-    cudaFree(W->lam[1]);
-    cudaFree(W->lamz);
-    cudaFree(W->g);
-    cudaFree(W->gz);
-    cudaFree(W->w);
-    cudaFree(W->partial);
-    cudaFree(W->result);
-    cudaFree(W->flags);
-    cudaFree(W->all_wet);
     delete W;
 }
 
+/* 0: the next forwards leave no tape (no backward is expected; one that
+ * comes all the same runs the forward again); 1 (default): they do */
+extern "C" int cal_sdt_adj_set_tape(void* handle, int on)
+{
+    ((Work*)handle)->want_tape = on != 0;
+    return 0;
+}
+
 /* Forward rollout on device buffers: init (z = z_dem - h0 where h0 > 0),
- * `steps` steps, h_T into hT; checkpoints kept for the backward. */
+ * `steps` steps, h_T into hT; the tape kept for the backward. */
 extern "C" int cal_sdt_adj_forward(void* handle, const double* z_dem, const double* h0, double p_r, double p_eps,
                                    double* hT, void* stream)
 {
     Work* W = (Work*)handle;
     cudaStream_t st = (cudaStream_t)stream;
+    sdtw::Dev& d = W->d;
     W->r = p_r;
     W->eps = p_eps;
-    const size_t b = W->n * sizeof(double);
-    cudaMemcpyAsync(W->h0, h0, b, cudaMemcpyDeviceToDevice, st);
-    double* cur = W->seg;
-    double* nxt = W->seg + W->n;
-    sdtadj::k_init<<<sdtadj::grid_for(W->n), sdtadj::T, 0, st>>>(z_dem, h0, W->z, cur, W->n);
-    for (int t = 0; t < W->steps; t++) {
-        if (t % W->K == 0)
-            cudaMemcpyAsync(W->ckpt + (t / W->K) * W->n, cur, b, cudaMemcpyDeviceToDevice, st);
-        sdtadj::fwd_step(*W, cur, nxt, st);
-        double* tmp = cur;
-        cur = nxt;
-        nxt = tmp;
+    const size_t b = (size_t)d.N * sizeof(double);
+    if (W->want_tape && !d.cap && W->steps > 0) {
+        /* a first guess: a sixteenth of the cells wet on average, at most an
+         * eighth of the free memory */
+        size_t free_b = 0, total_b = 0;
+        cudaMemGetInfo(&free_b, &total_b);
+        const long long guess = (d.N / 16 + 1024) * W->steps;
+        const long long most = (long long)(free_b / 8 / sdtw::TAPE_BYTES);
+        if (most > 0)
+            sdtadj::make_tape(*W, std::min(guess, most));
     }
-    if (W->steps == 0)
-        cudaMemcpyAsync(W->ckpt, cur, b, cudaMemcpyDeviceToDevice, st);
-    cudaMemcpyAsync(hT, cur, b, cudaMemcpyDeviceToDevice, st);
+    sdtadj::Inst I;
+    memset(&I, 0, sizeof(I));
+    I.rows = W->rows;
+    I.cols = W->cols;
+    I.r = p_r;
+    I.eps = p_eps;
+    memcpy(&I.eps_bits, &p_eps, sizeof(double));
+    I.tiles_x = (W->cols + (1 << d.lw) - 1) >> d.lw;
+    I.tiles_y = (W->rows + (1 << d.lh) - 1) >> d.lh;
+    I.toroidal = W->toroidal;
+    sdtadj::k_instance<<<1, 1, 0, st>>>(I, d.N, W->inst, W->offs);
+    cudaMemsetAsync((void*)d.tile_inst, 0, sizeof(int) * d.ntiles, st);
+    cudaMemcpyAsync(W->h0, h0, b, cudaMemcpyDeviceToDevice, st);
+    cudaMemcpyAsync(W->z_dem, z_dem, b, cudaMemcpyDeviceToDevice, st);
+    sdtadj::queue_forward(*W, W->ckpt != nullptr, st);
+    /* no step: h0 as given, -0 and all */
+    cudaMemcpyAsync(hT, W->steps > 0 ? d.h : W->h0, b, cudaMemcpyDeviceToDevice, st);
     return (int)cudaGetLastError();
 }
 
@@ -440,70 +303,48 @@ extern "C" int cal_sdt_adj_backward(void* handle, const double* gT, double* g_h0
 {
     Work* W = (Work*)handle;
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t b = W->n * sizeof(double);
-    long long eps_bits;
-    memcpy(&eps_bits, &W->eps, sizeof(double));
-    sdtadj::Geo geo = {W->rows, W->cols, W->toroidal, W->n};
-    cudaMemcpyAsync(W->lam[0], gT, b, cudaMemcpyDeviceToDevice, st);
-    cudaMemsetAsync(W->lamz, 0, b, st);
-    cudaMemsetAsync(W->partial, 0, 2 * sdtadj::PBLOCKS * sizeof(double), st);
-    const int ntiles = W->tiles_x * W->tiles_y;
-    /* one resident wave of each kernel (blocks stride over the tiles): the
-     * dry tiles cost a flag test, not a block launch */
-    static int wave_c = 0, wave_g = 0;
-    if (!wave_c) {
-        int dev = 0, sms = 0, pc = 0, pg = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pc, sdtadj::k_coeffs_tiles, sdtadj::T, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pg, sdtadj::k_gather_tiles, sdtadj::T, 0);
-        wave_c = sms * (pc > 0 ? pc : 1);
-        wave_g = sms * (pg > 0 ? pg : 1);
-    }
-    int cgrid = ntiles < wave_c ? ntiles : wave_c;
-    if (cgrid > sdtadj::PBLOCKS)
-        cgrid = sdtadj::PBLOCKS;
-    const int ggrid = ntiles < wave_g ? ntiles : wave_g;
-    for (int s = W->nseg - 1; s >= 0; s--) {
-        const int t0 = s * W->K;
-        const int t1 = (t0 + W->K < W->steps) ? t0 + W->K : W->steps; /* states t0..t1-1 feed steps */
-        /* recompute the states of the segment from its checkpoint, keeping
-         * each step's tile flags (bit 0: wet before, bit 1: wet after) */
-        cudaMemcpyAsync(W->seg, W->ckpt + s * W->n, b, cudaMemcpyDeviceToDevice, st);
-        for (int t = t0; t < t1 - 1; t++)
-            sdtadj::fwd_step(*W, W->seg + (t - t0) * W->n, W->seg + (t - t0 + 1) * W->n, st,
-                             W->flags + (size_t)(t - t0) * ntiles);
-        /* reverse through the segment: state t's wet tiles are bit 0 of the
-         * step from t, or bit 1 of the step into it for the last state */
-        for (int t = t1 - 1; t >= t0; t--) {
-            const double* ht = W->seg + (t - t0) * W->n;
-            const unsigned char* fl;
-            int mask;
-            if (t < t1 - 1) {
-                fl = W->flags + (size_t)(t - t0) * ntiles;
-                mask = 1;
-            } else if (t > t0) {
-                fl = W->flags + (size_t)(t - 1 - t0) * ntiles;
-                mask = 2;
-            } else {
-                fl = W->all_wet; /* a one-state segment: no step reported on it */
-                mask = 1;
+    sdtw::Dev& d = W->d;
+    long long need = 0;
+    cudaError_t e = sdtadj::tape_need(*W, &need, st);
+    if (e != cudaSuccess)
+        return (int)e;
+    bool segments = W->ckpt != nullptr;
+    if (!segments && need > d.cap) {
+        size_t free_b = 0, total_b = 0;
+        cudaMemGetInfo(&free_b, &total_b);
+        segments = (size_t)need * sdtw::TAPE_BYTES > (free_b + (size_t)d.cap * sdtw::TAPE_BYTES) / 2 ||
+                   !sdtadj::make_tape(*W, need);
+        if (segments) {
+            if (cudaMalloc(&W->ckpt, (size_t)W->nseg * d.N * sizeof(double)) != cudaSuccess) {
+                (void)cudaGetLastError();
+                W->ckpt = nullptr;
+                return (int)cudaErrorMemoryAllocation;
             }
-            sdtadj::k_coeffs_tiles<<<cgrid, sdtadj::T, 0, st>>>(geo, W->z, ht, W->lam[0], W->r, W->eps, eps_bits, W->g,
-                                                               W->gz, W->w, W->partial, fl, mask, W->tiles_x, ntiles);
-            sdtadj::k_gather_tiles<<<ggrid, sdtadj::T, 0, st>>>(geo, W->lam[0], W->g, W->gz, W->w, W->lamz, fl, mask,
-                                                               W->tiles_x, W->tiles_y);
         }
+        sdtadj::queue_forward(*W, segments, st);
     }
-    const int cur = 0;
-    sdtadj::k_final_grad<<<sdtadj::grid_for(W->n), sdtadj::T, 0, st>>>(W->h0, W->lam[cur], W->lamz, g_h0, W->n);
-    sdtadj::k_fold_partials<<<1, 32, 0, st>>>(W->partial, W->result);
+    for (int attempt = 0;; attempt++) {
+        sdtadj::queue_seed(*W, gT, st);
+        if (!segments) {
+            sdtw::queue_adjoint(d, W->a, 0, W->steps, st);
+            break;
+        }
+        sdtadj::queue_segments(*W, st);
+        if ((e = sdtadj::tape_need(*W, &need, st)) != cudaSuccess)
+            return (int)e;
+        if (need <= d.cap)
+            break;
+        if (attempt || !sdtadj::make_tape(*W, need))
+            return (int)cudaErrorMemoryAllocation;
+    }
+    sdtw::k_final_grad<<<sdtw::dense_blocks(d.N), sdtadj::T, 0, st>>>(W->h0, W->a.lam, W->a.mu, g_h0, d.N);
+    sdtw::k_fold<<<1, 32, 0, st>>>(W->a.part, W->a.grad, 2);
     double res[2] = {0.0, 0.0};
-    cudaMemcpyAsync(res, W->result, sizeof(res), cudaMemcpyDeviceToHost, st);
-    cudaStreamSynchronize(st);
+    cudaMemcpyAsync(res, W->a.grad, sizeof(res), cudaMemcpyDeviceToHost, st);
+    e = cudaStreamSynchronize(st);
     if (g_r)
         *g_r = res[0];
     if (g_eps)
         *g_eps = res[1];
-    return (int)cudaGetLastError();
+    return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
