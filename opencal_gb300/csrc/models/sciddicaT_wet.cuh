@@ -36,18 +36,12 @@
  * dL/dh0 = lambda_0 - [h0 > 0] lambda_z is mu where h0 > 0, lambda elsewhere.
  *
  * Measured against the tile-by-tile step this replaced (fused tiles of 64 x
-<<<<<<< Updated upstream
  * 16 cells with their rings, the adjoint on whole tiles after restoring
  * them), 64 instances of 128..1024 cells a side, 500 steps, us per step:
  * forward 92 -> 16 (k_outflows) + 16 (k_update); reverse 10 + 65 + 29 -> 15
  * (k_coeffs) + 10 (k_gather).  k_outflows is bound by the FP64 pipe (60 % of
  * it over the launch, the rest is its chain of loads), the others by the
  * latency of theirs.
-=======
- * 16 with their rings, the adjoint on whole tiles after restoring them), 64
- * instances of 128..1024 cells a side, 500 steps, us per step: see the
- * kernels.
->>>>>>> Stashed changes
  */
 #pragma once
 
