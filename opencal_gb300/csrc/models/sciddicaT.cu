@@ -239,8 +239,7 @@ struct State {
     double* zeps = nullptr;      /* z + epsilon per cell (u[0] of the cell), from the priming */
     int* list[2] = {nullptr, nullptr}; /* a step's cells: c for a wet cell, ~c for one that dried */
     int* counts = nullptr;       /* [4] list parity, [6] step epoch; [C_TICKET] K2 block
-                                    ticket; [C_ARRIVED], [C_ERROR] the persistent kernel's
-                                    placement barrier counter and error flag */
+                                    ticket; [C_ERROR] the persistent kernel's error flag */
     unsigned long long* ctl = nullptr; /* 64-bit counters, one per 128-byte line (W_*) */
     int* tflag = nullptr;        /* per K2 tile: epoch of the step that flagged it */
     int* tlist = nullptr;        /* flagged tiles of the current step */
@@ -315,11 +314,8 @@ constexpr int K1_THREADS = 256;
 /* control words, each group on its own 128-byte line: the K2 ticket and the
  * persistent kernel's barrier counter are hit by every block and polled,
  * and must not share a line with the list and tile counters */
-constexpr int NCOUNTS = 512;
+constexpr int NCOUNTS = 128;
 constexpr int C_TICKET = 32, C_ARRIVED = 64, C_ERROR = 96;
-/* the persistent kernel's placement census: a flag (own line) and blocks
- * per SM, for SM ids below MAX_SM */
-constexpr int C_PLACE_BAD = 128, C_SMRANK = 256, MAX_SM = 256;
 /* 64-bit counters (State::ctl), each on a 128-byte line of its own; the low
  * 32 bits count appended items, the high 32 bits a barrier's arrivals:
  *   W_TILES + 16 * parity   tiles flagged in a step (per-step launches)
@@ -365,25 +361,23 @@ static __device__ __forceinline__ double ldh(const double* p)
 }
 
 /* flag tile t for this step's K2 and append it to the work-list once */
-template <bool CO>
 static __device__ __forceinline__ void flag_tile(int* tflag, int* tlist, unsigned long long* tcount, int t, int epoch)
 {
-    if (ldm<CO>(tflag + t) != epoch && atomicExch(tflag + t, epoch) != epoch)
+    if (atomicExch(tflag + t, epoch) != epoch)
         tlist[low32(atomicAdd(tcount, 1ull))] = t;
 }
 
 /* flag tile t for the lanes where `want` holds, once per distinct tile among
  * the lanes converged here: consecutive wet cells of the list mostly share
  * a tile, so the warp's leader for each tile does the (idempotent) flag
- * and the others skip its load and atomic */
-template <bool CO>
+ * and the others skip its atomic */
 static __device__ __forceinline__ void flag_tile_warp(bool want, int t, int* tflag, int* tlist,
                                                       unsigned long long* tcount, int epoch)
 {
     const unsigned act = __activemask();
     const unsigned peers = __match_any_sync(act, want ? t : -1);
     if (want && (threadIdx.x & 31) == __ffs(peers) - 1)
-        flag_tile<CO>(tflag, tlist, tcount, t, epoch);
+        flag_tile(tflag, tlist, tcount, t, epoch);
 }
 
 /* K1's work on the step's list (threads tid, tid + nthreads, ...): the
@@ -408,20 +402,24 @@ static __device__ __forceinline__ void k1_work(const K1Params& p, int par, int e
         /* neighbours in von Neumann order n = 1..4: north, west, east, south */
         int ni[4] = {i - 1, i, i, i + 1}, nj[4] = {j, j - 1, j + 1, j};
         double u[4];
-        bool in[4];
+        /* the receivers' tiles where they differ from the cell's own (which
+         * covers a receiver in it), and the tiles' stamps, loaded here so
+         * that they arrive while the minimisation runs */
+        const int own = tile_of(i, j, p.tiles_x);
+        int rt[4], stamp[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             int a = ni[q], b = nj[q];
-            in[q] = true;
+            bool in = true;
             if (p.toroidal) {
                 a = a < 0 ? a + p.rows : (a >= p.rows ? a - p.rows : a);
                 b = b < 0 ? b + p.cols : (b >= p.cols ? b - p.cols : b);
             } else if ((unsigned)a >= (unsigned)p.rows || (unsigned)b >= (unsigned)p.cols) {
-                in[q] = false;
+                in = false;
             }
-            ni[q] = a;
-            nj[q] = b;
-            if (in[q]) {
+            rt[q] = in ? tile_of(a, b, p.tiles_x) : own;
+            stamp[q] = rt[q] != own ? ldm<CO>(p.tflag + rt[q]) : epoch;
+            if (in) {
                 /* z + h of the neighbour, as K2 (or the priming) computed it
                  * from the same operands */
                 u[q] = ldh<CO>(p.zh + (long long)a * p.cols + b);
@@ -429,25 +427,20 @@ static __device__ __forceinline__ void k1_work(const K1Params& p, int par, int e
                 u[q] = 0.0 + 0.0; /* an absent neighbour reads z = 0, h = 0 */
             }
         }
+        const int own_stamp = ldm<CO>(p.tflag + own);
         double f[4];
         sdt::outflows_u0(ldh<CO>(p.h + c), __ldg(p.zeps + c), u[0], u[1], u[2], u[3], p.eps, p.r, f);
         bool any = false;
-        const int own = tile_of(i, j, p.tiles_x);
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             p.f[q * p.n + c] = f[q];
             if (__double_as_longlong(f[q]) != 0) {
                 any = true;
-                /* the receiver reads it; a receiver in this cell's own tile
-                 * is covered by the flag of the own tile below */
-                if (in[q]) {
-                    const int t = tile_of(ni[q], nj[q], p.tiles_x);
-                    if (t != own)
-                        flag_tile<CO>(p.tflag, p.tlist, tcount, t, epoch);
-                }
+                if (stamp[q] != epoch)
+                    flag_tile(p.tflag, p.tlist, tcount, rt[q], epoch);
             }
         }
-        flag_tile_warp<CO>(any, own, p.tflag, p.tlist, tcount, epoch);
+        flag_tile_warp(any && own_stamp != epoch, own, p.tflag, p.tlist, tcount, epoch);
     }
 }
 
@@ -491,15 +484,30 @@ static __device__ __forceinline__ void warp_append(bool pred, int value, int* li
         list[base + __popc(mask & ((1u << lane) - 1u))] = value;
 }
 
-/* Block-wide append of up to 4 items per thread to the next list, one
- * atomicAdd per block: item q as value[q] when want[q] (a wet cell) and as
+/* The update works in groups of THREADS threads: a block of the per-step
+ * kernel is one group, a block of the persistent kernel GROUPS of them that
+ * meet at barriers of their own. */
+template <int GROUPS>
+static __device__ __forceinline__ void group_sync()
+{
+    if (GROUPS == 1)
+        __syncthreads();
+    else
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)(threadIdx.x / THREADS)), "n"(THREADS) : "memory");
+}
+
+/* Group-wide append of up to 4 items per thread to the next list, one
+ * atomicAdd per group: item q as value[q] when want[q] (a wet cell) and as
  * ~value[q] when dried[q] (a cell whose outflows K1 must clear). */
+template <int GROUPS>
 static __device__ __forceinline__ void block_append4(const bool want[4], const bool dried[4], const int value[4],
                                                      int* list, unsigned long long* count)
 {
-    __shared__ int s_warp[2][THREADS / 32];
-    __shared__ int s_base[2];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ int s_warps[GROUPS][2][THREADS / 32];
+    __shared__ int s_bases[GROUPS][2];
+    int(*s_warp)[THREADS / 32] = s_warps[threadIdx.x / THREADS];
+    int* s_base = s_bases[threadIdx.x / THREADS];
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x % THREADS) >> 5;
     const unsigned below = (1u << lane) - 1u;
     unsigned mw[4], md[4];
     int nw = 0, nd = 0;
@@ -514,8 +522,8 @@ static __device__ __forceinline__ void block_append4(const bool want[4], const b
         s_warp[0][warp] = nw;
         s_warp[1][warp] = nd;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    group_sync<GROUPS>();
+    if (threadIdx.x % THREADS == 0) {
         int tw = 0, td = 0;
         for (int w = 0; w < THREADS / 32; w++) {
             tw += s_warp[0][w];
@@ -525,7 +533,7 @@ static __device__ __forceinline__ void block_append4(const bool want[4], const b
         s_base[0] = base;      /* wet entries first, */
         s_base[1] = base + tw; /* then the dried ones */
     }
-    __syncthreads();
+    group_sync<GROUPS>();
     int bw = s_base[0], bd = s_base[1];
     for (int w = 0; w < warp; w++) {
         bw += s_warp[0][w];
@@ -543,7 +551,7 @@ static __device__ __forceinline__ void block_append4(const bool want[4], const b
 }
 
 /* one flagged tile: h += inflows - outflows in place, then the wet test */
-template <bool CO>
+template <bool CO, int GROUPS>
 static __device__ __forceinline__ void k2_tile(const K2Params& p, int tile, int* list, unsigned long long* count)
 {
     const int ty = tile / p.tiles_x, tx = tile - ty * p.tiles_x;
@@ -552,8 +560,9 @@ static __device__ __forceinline__ void k2_tile(const K2Params& p, int tile, int*
      * half the serial FP64 chain per thread) */
     constexpr int CPT = (TW * TH >= 4 * THREADS) ? 4 : ((TW * TH >= 2 * THREADS) ? 2 : 1);
     static_assert((TW / CPT) * TH <= THREADS && TW % CPT == 0, "one group of CPT cells per thread at most");
-    const int r = threadIdx.x / (TW / CPT);         /* the tile's row; r >= TH: no cells */
-    const int j4 = (threadIdx.x % (TW / CPT)) * CPT; /* 0, CPT, ..., TW - CPT */
+    const int tid = threadIdx.x % THREADS;
+    const int r = tid / (TW / CPT);          /* the tile's row; r >= TH: no cells */
+    const int j4 = (tid % (TW / CPT)) * CPT; /* 0, CPT, ..., TW - CPT */
     const bool has = r < TH;
     const int i = ty * TH + r;
     const int jb = tx * TW + j4;
@@ -629,13 +638,13 @@ static __device__ __forceinline__ void k2_tile(const K2Params& p, int tile, int*
         dried[q] = wb && !want[q];
         value[q] = (int)c;
     }
-    block_append4(want, dried, value, list, count);
+    block_append4<GROUPS>(want, dried, value, list, count);
 }
 
-/* K2's work for blocks block, block + nblocks, ...: the flagged tiles, then
+/* K2's work for groups block, block + nblocks, ...: the flagged tiles, then
  * the current wet list in chunks of THREADS entries (carrying over the wet
  * cells of unflagged tiles, whose h did not change) */
-template <bool CO>
+template <bool CO, int GROUPS>
 static __device__ __forceinline__ void k2_work(const K2Params& p, int par, int epoch, int ntiles, int nlist,
                                                unsigned long long* count, int block, int nblocks)
 {
@@ -644,10 +653,10 @@ static __device__ __forceinline__ void k2_work(const K2Params& p, int par, int e
     const int items = ntiles + (nlist + THREADS - 1) / THREADS;
     for (int item = block; item < items; item += nblocks) {
         if (item < ntiles) {
-            k2_tile<CO>(p, ldm<CO>(p.tlist + item), list, count);
-            __syncthreads(); /* block_append4's shared words are reused */
+            k2_tile<CO, GROUPS>(p, ldm<CO>(p.tlist + item), list, count);
+            group_sync<GROUPS>(); /* block_append4's shared words are reused */
         } else {
-            const int k = (item - ntiles) * THREADS + threadIdx.x;
+            const int k = (item - ntiles) * THREADS + threadIdx.x % THREADS;
             bool carry = false;
             int c = 0;
             if (k < nlist) {
@@ -657,13 +666,13 @@ static __device__ __forceinline__ void k2_work(const K2Params& p, int par, int e
                     carry = ldm<CO>(p.tflag + tile_of(i, j, p.tiles_x)) != epoch;
                 }
             }
-            /* one atomic on the step's counter per block, not per warp:
-             * every block of the phase appends to that one word */
+            /* one atomic on the step's counter per group, not per warp:
+             * every group of the phase appends to that one word */
             const bool want[4] = {carry, false, false, false};
             const bool none[4] = {false, false, false, false};
             const int value[4] = {c, 0, 0, 0};
-            block_append4(want, none, value, list, count);
-            __syncthreads(); /* block_append4's shared words are reused */
+            block_append4<GROUPS>(want, none, value, list, count);
+            group_sync<GROUPS>(); /* block_append4's shared words are reused */
         }
     }
 }
@@ -673,7 +682,7 @@ __global__ void __launch_bounds__(THREADS) k2_update(const __grid_constant__ K2P
     const bool host = p.hpar >= 0;
     const int par = host ? p.hpar : p.counts[4];
     const int epoch = host ? p.hepoch : p.counts[6];
-    k2_work<false>(p, par, epoch, low32(p.ctl[W_TILES + 16 * par]), low32(p.ctl[W_LIST + 16 * par]),
+    k2_work<false, 1>(p, par, epoch, low32(p.ctl[W_TILES + 16 * par]), low32(p.ctl[W_LIST + 16 * par]),
                    p.ctl + W_LIST + 16 * (1 - par), blockIdx.x, gridDim.x);
     if (host) {
         /* nobody reads the device words during this launch */
@@ -698,16 +707,14 @@ __global__ void __launch_bounds__(THREADS) k2_update(const __grid_constant__ K2P
  * The two phases of each step (K1's and K2's work) are separated by a grid
  * barrier on the 64-bit word that counts what the phase appended (packed
  * barrier below), so that the poll that ends the wait also returns the count
- * the next phase needs.  counts[C_ARRIVED] is the arrival counter of the
- * one-off barrier of the placement census (zeroed before the launch),
- * counts[C_ERROR] the error flag.  Only one thread per block touches the
+ * the next phase needs.  counts[C_ERROR] is the error flag.  Only one thread per block touches the
  * shared words: it arrives, waits, and hands the count to its block through
  * shared memory, so that no L2 line is read by every thread of the grid. */
 constexpr unsigned BARRIER_SPIN_LIMIT = 1u << 22;
-/* pause between two polls of a barrier word: fewer polls leave the word's
- * L2 slice to the arrivals.  2048^2 x 4000 steps per run (same box, two
- * runs each): 32 ns 60.37 ms, 96 ns 59.70, 192 ns 59.46, 320 ns 60.19 */
-constexpr unsigned BARRIER_POLL_NS = 192;
+/* pause between two polls of a barrier word, us per step of SCIDDICA-T runs
+ * (96 x 80 / 2048 x 2048): 192 ns 10.59 / 13.18, 64 ns 10.56 / 13.14, 20 ns
+ * 10.53 / 13.12 */
+constexpr unsigned BARRIER_POLL_NS = 20;
 
 static __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p)
 {
@@ -770,37 +777,6 @@ static __device__ __forceinline__ bool grid_barrier(int* counts, unsigned nblock
     return s_ok != 0;
 }
 
-/* The order in which a persistent kernel deals work to its blocks:
- * v = (rank of the block on its SM) * SMs + SM, so that consecutive work
- * items go to different SMs first (a cooperative launch places its first
- * blocks several to an SM).  v is a permutation of the blocks when every
- * block finds its SM id below nsm and its rank below nb / nsm (nb distinct
- * pairs in nb places); if one does not, every block keeps its launch index.
- * Needs counts[C_PLACE_BAD] and counts[C_SMRANK ...] zeroed before the
- * launch; one grid barrier.  Returns -1 when that barrier gave up. */
-static __device__ int placement_order(int* counts, unsigned nb, int nsm, unsigned& round, int* s_tmp)
-{
-    __shared__ int s_v;
-    if (threadIdx.x == 0) {
-        unsigned smid;
-        asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-        int v = -1;
-        if (nsm > 0 && smid < (unsigned)nsm && smid < (unsigned)MAX_SM && nb % (unsigned)nsm == 0) {
-            const int rank = atomicAdd(counts + C_SMRANK + smid, 1);
-            if (rank < (int)(nb / (unsigned)nsm))
-                v = rank * nsm + (int)smid;
-        }
-        if (v < 0)
-            atomicExch(counts + C_PLACE_BAD, 1);
-        s_v = v;
-    }
-    if (!grid_barrier(counts, nb, round, counts + C_PLACE_BAD, counts + C_PLACE_BAD, s_tmp))
-        return -1;
-    const int vb = s_tmp[0] ? (int)blockIdx.x : s_v;
-    __syncthreads(); /* s_tmp is free again */
-    return vb;
-}
-
 static __device__ __forceinline__ unsigned long long ld_acquire_gpu_u64(const unsigned long long* p)
 {
     unsigned long long v;
@@ -841,19 +817,25 @@ static __device__ __forceinline__ bool packed_barrier(unsigned long long* word, 
     return s_ok != 0;
 }
 
-#ifndef SDT2_PERSIST_MINB
-#define SDT2_PERSIST_MINB 4 /* resident blocks per SM (5 measured slower: 78.4 against 72.8 ms per run) */
-#endif
-__global__ void __launch_bounds__(THREADS, SDT2_PERSIST_MINB) k_persist(const __grid_constant__ K1Params a,
-                                                     const __grid_constant__ K2Params b, int nsteps, int nsm)
+/* One block of 1024 threads on every SM.  A grid barrier costs by the
+ * blocks that arrive (empty barriers on this kernel's words, us: 608 blocks
+ * 3.2, 304 1.8, 152 1.45, 16 1.2) and a step has two, so the 155,648 threads
+ * that keep the FP64 pipes fed come in as few blocks as possible; within a
+ * block the update's groups of 256 threads stay independent.  More than 32
+ * registers a thread leave no room for a second block on an SM, so
+ * consecutive work items (block by block, then group by group) fall on
+ * different SMs. */
+constexpr int PGROUPS = 4, PTHREADS = PGROUPS * THREADS;
+__global__ void __launch_bounds__(PTHREADS, 1) k_persist(const __grid_constant__ K1Params a,
+                                                         const __grid_constant__ K2Params b, int nsteps,
+                                                         const int* done)
 {
+    nsteps -= *done;
+    if (nsteps <= 0)
+        return;
     __shared__ int s_cnt[2];
     __shared__ int s_state[3];
     const unsigned nb = gridDim.x;
-    unsigned round = 0;
-    const int vb = placement_order(a.counts, nb, nsm, round, s_cnt);
-    if (vb < 0)
-        return;
     if (threadIdx.x == 0) {
         s_state[0] = __ldcg(a.counts + 4);
         s_state[1] = __ldcg(a.counts + 6);
@@ -864,9 +846,10 @@ __global__ void __launch_bounds__(THREADS, SDT2_PERSIST_MINB) k_persist(const __
     int epoch = s_state[1];
     int nlist = s_state[2]; /* entries of the current step's list */
     /* K1's list entries in chunks of 32 (one per warp), consecutive chunks
-     * on consecutive blocks in the order v, so that the wet cells' FP64 work
-     * spreads over every SM whatever their number */
-    const int tid = ((threadIdx.x >> 5) * (int)nb + vb) * 32 + (threadIdx.x & 31);
+     * on consecutive blocks, so that the wet cells' FP64 work spreads over
+     * every SM whatever their number */
+    const int tid = ((threadIdx.x >> 5) * (int)nb + blockIdx.x) * 32 + (threadIdx.x & 31);
+    const int group = (threadIdx.x / THREADS) * (int)nb + blockIdx.x;
     for (int s = 0; s < nsteps; s++) {
         const int w = 16 * (s % 3);
         unsigned long long* tword = a.ctl + W_PT + w;
@@ -876,11 +859,11 @@ __global__ void __launch_bounds__(THREADS, SDT2_PERSIST_MINB) k_persist(const __
             const int wn = 16 * ((s + 1) % 3);
             a.ctl[(threadIdx.x ? W_PL : W_PT) + wn] = 0;
         }
-        k1_work<true>(a, par, epoch, nlist, tword, tid, nb * THREADS);
+        k1_work<true>(a, par, epoch, nlist, tword, tid, nb * PTHREADS);
         /* then: the flagged tiles of this step */
         if (!packed_barrier(tword, nb, a.counts, s_cnt))
             return;
-        k2_work<true>(b, par, epoch, s_cnt[0], nlist, lword, vb, nb);
+        k2_work<true, PGROUPS>(b, par, epoch, s_cnt[0], nlist, lword, group, nb * PGROUPS);
         par = 1 - par;
         epoch++;
         /* then: the entries of the next step's list */
@@ -900,11 +883,14 @@ __global__ void __launch_bounds__(THREADS, SDT2_PERSIST_MINB) k_persist(const __
 }
 
 /* -0 -> +0 in h, z + h and z + eps of every cell, and the first wet list
- * (its counter must be 0) */
+ * (its counter must be 0); nothing when *done has reached nsteps (done may
+ * be NULL) */
 __global__ void __launch_bounds__(THREADS) k_prime(double* h, const double* __restrict__ z, double* zh, double* zeps,
                                                   double eps, long long n, long long eps_bits, int* list,
-                                                  unsigned long long* count, int* counts)
+                                                  unsigned long long* count, int* counts, const int* done, int nsteps)
 {
+    if (done && *done >= nsteps)
+        return;
     if (blockIdx.x == 0 && threadIdx.x == 0)
         counts[6] = 1; /* first epoch (tile stamps start at 0) */
     for (long long c0 = (long long)blockIdx.x * blockDim.x; c0 < n; c0 += (long long)gridDim.x * blockDim.x) {
@@ -942,8 +928,10 @@ static void release()
     s = State();
 }
 
-/* (re)allocate for `ca` and prime from the current h and z */
-static bool prime(struct CALModel2D* ca, double* h, const double* z, double eps, long long eps_bits, cudaStream_t st)
+/* (re)allocate for `ca` and prime from the current h and z (done, nsteps:
+ * as for k_prime) */
+static bool prime(struct CALModel2D* ca, double* h, const double* z, double eps, long long eps_bits, cudaStream_t st,
+                  const int* done = nullptr, int nsteps = 0)
 {
     State& s = g_state;
     const long long n = (long long)ca->rows * ca->columns;
@@ -974,7 +962,8 @@ static bool prime(struct CALModel2D* ca, double* h, const double* z, double eps,
     int blocks = (int)((n + THREADS - 1) / THREADS);
     if (blocks > 152 * 16)
         blocks = 152 * 16;
-    k_prime<<<blocks, THREADS, 0, st>>>(h, z, s.zh, s.zeps, eps, n, eps_bits, s.list[0], s.ctl + W_LIST, s.counts);
+    k_prime<<<blocks, THREADS, 0, st>>>(h, z, s.zh, s.zeps, eps, n, eps_bits, s.list[0], s.ctl + W_LIST, s.counts,
+                                        done, nsteps);
     s.primed = true;
     s.hpar = 0; /* what k_prime leaves: parity 0, epoch 1 */
     s.hepoch = 1;
@@ -1060,27 +1049,20 @@ static bool step(struct CALModel2D* ca, const double* z, double* h, double eps, 
     return cudaGetLastError() == cudaSuccess;
 }
 
-/* `nsteps` steps in one cooperative launch of k_persist (one resident grid:
- * SMs x resident blocks per SM); false when the launch is refused or a
- * CUDA error is pending.  A barrier that gave up sets counts[C_ERROR], which
+/* The steps from *done to nsteps in one cooperative launch of k_persist (a
+ * block per SM); false when the launch is refused or a CUDA error is pending.  A barrier that gave up sets counts[C_ERROR], which
  * persist_failed() reports. */
 static bool persist(struct CALModel2D* ca, const double* z, double* h, double eps, double r, long long eps_bits,
-                    int nsteps, cudaStream_t st)
+                    int nsteps, const int* done, cudaStream_t st)
 {
     State& s = g_state;
     s.hknown = false; /* the kernel advances parity and epoch on the device */
-    static int grid = 0, sms_of_device = 0;
+    static int grid = 0;
     if (!grid) {
-        int per_sm = 0, dev = 0, sms = 0;
+        int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist, THREADS, 0);
-#ifdef SDT2_PERSIST_PER_SM /* compile-time cap (2 or 3 per SM measured slower than 4) */
-        if (per_sm > SDT2_PERSIST_PER_SM)
-            per_sm = SDT2_PERSIST_PER_SM;
-#endif
-        grid = sms * per_sm;
-        sms_of_device = sms;
+        grid = sms;
         if (grid <= 0)
             return false;
     }
@@ -1113,13 +1095,10 @@ static bool persist(struct CALModel2D* ca, const double* z, double* h, double ep
     b.eps_bits = eps_bits;
     a.hpar = b.hpar = -1;
     a.hepoch = b.hepoch = 0;
-    cudaMemsetAsync(s.counts + C_ARRIVED, 0, sizeof(int), st); /* placement barrier counter */
-    cudaMemsetAsync(s.counts + C_ERROR, 0, sizeof(int), st);   /* error flag */
-    cudaMemsetAsync(s.counts + C_PLACE_BAD, 0, (NCOUNTS - C_PLACE_BAD) * sizeof(int), st); /* placement census */
+    cudaMemsetAsync(s.counts + C_ERROR, 0, sizeof(int), st); /* error flag */
     cudaMemsetAsync(s.ctl + W_PT, 0, (NCTL - W_PT) * sizeof(unsigned long long), st); /* the steps' counters */
-    int nsm = sms_of_device;
-    void* args[] = {&a, &b, &nsteps, &nsm};
-    return cudaLaunchCooperativeKernel((const void*)k_persist, dim3(grid), dim3(THREADS), args, 0, st) ==
+    void* args[] = {&a, &b, &nsteps, &done};
+    return cudaLaunchCooperativeKernel((const void*)k_persist, dim3(grid), dim3(PTHREADS), args, 0, st) ==
            cudaSuccess;
 }
 
@@ -1209,6 +1188,401 @@ static int persist_failed(cudaStream_t st)
 
 } // namespace sdt2
 
+/* ================= the plain run in one cooperative launch ============== */
+/* Every step of a plain run in one launch with ONE grid barrier per step.  A
+ * step is a chain of dependent latencies whatever the flow's size, and the
+ * split step's two phases pay it twice (list entry, cell data, the
+ * minimisation, the atomics that flag a tile, a barrier; then tile, cell
+ * data, the atomic that appends, a barrier: 10.4 us a step on a grid with a
+ * few hundred wet cells).  Here the unit is a TW x TH tile, taken by a group
+ * of 256 threads: z and h with a ring of two cells into shared memory, the
+ * outflows of the tile and a ring of one -- the ring is computed by the
+ * neighbours too, which trades FP64 work for the second phase -- and the
+ * update of the tile from one h buffer into the other.
+ *
+ * L_t, the tiles of step t, is every tile whose h may change in step t or
+ * changed in step t - 1 (so that both buffers agree on every tile left
+ * out): a tile holding a wet cell and its four edge neighbours, for the wet
+ * cells of both h_{t-1} and h_t.  A tile of L_t that held a wet cell before
+ * the step marks itself and its neighbours for L_{t+1} as soon as its h is
+ * there, by one warp while the others compute, so that the two atomics of a
+ * mark (epoch stamp, append) are off the chain; one that is wet only after
+ * the step marks at its end.
+ *
+ * A block of four groups on every SM (sdt2::k_persist says why); consecutive
+ * tiles of the list go to different SMs. */
+namespace sdtp {
+
+/* us per step, 96 x 80 / 610 x 496 / 2048 x 2048 (whole runs in this form):
+ * 16 x 8 6.5 / 7.1 / 15.1, 8 x 8 6.4 / 6.9 / 17.5, 16 x 12 7.0 / 8.0 / 14.8,
+ * 16 x 16 7.2 / 10.9 / 17.0, 32 x 8 7.2 / 11.6 / 20.1; groups of 128 threads
+ * (eight a block) 6.8 / 10.0 / 15.7 */
+constexpr int TW = 16, TH = 8;
+/* More tiles than groups end this form's part of the run: the groups would
+ * take several tiles one after another and the rings' FP64 work weigh more
+ * than the split step's second barrier, so the split step (sdt2::k_persist)
+ * does the remaining steps.  2048 x 2048 x 4000, us per step when it ends at
+ * 456 / 608 (the groups) / 912 / 1216 tiles / never: 12.9 / 12.6 / 13.1 / 13.7
+ * / 15.0; the split step alone 13.1. */
+constexpr int GT = 256, GROUPS = 4, THREADS = GT * GROUPS; /* threads per group, groups per block */
+constexpr int R1W = TW + 2, R1H = TH + 2, R1 = R1W * R1H; /* outflow region */
+constexpr int R2W = TW + 4, R2H = TH + 4, R2 = R2W * R2H; /* load region */
+
+struct Shared {
+    double z[R2], h[R2], zh[R2];
+    double f[4][R1];
+    unsigned short list[R1];
+    /* of the group's current tile; the other set is cleared for the next
+     * tile, which may begin while a thread still reads this one */
+    struct Flags {
+        int count, any, own, late;
+    } flags[2];
+};
+
+struct State {
+    struct CALModel2D* ca = nullptr;
+    long long n = 0;
+    double* h2 = nullptr;
+    int* stamps = nullptr;
+    int* list[2] = {nullptr, nullptr};
+    unsigned long long* words = nullptr; /* three, 128 bytes apart */
+    int* counts = nullptr;               /* [C_ERROR] */
+    int tiles_x = 0, tiles_y = 0;
+};
+static State g_state;
+
+struct Params {
+    const double* __restrict__ z;
+    double* h0;
+    double* h1;
+    int* stamps;
+    int* list0;
+    int* list1;
+    unsigned long long* words;
+    int* counts;
+    int rows, cols, toroidal, tiles_x, tiles_y;
+    long long n;
+    double eps, r;
+    long long eps_bits;
+};
+
+constexpr int C_ERROR = sdt2::C_ERROR, C_DONE = 0, NCOUNTS = sdt2::NCOUNTS; /* [C_DONE]: steps done */
+
+static __device__ __forceinline__ void group_sync(int group)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(GT) : "memory");
+}
+
+/* A load of data that other blocks write while the kernel runs: a plain load
+ * through a pointer passed through a register move, so that the compiler
+ * cannot turn it into a non-coherent one and still batches it with others;
+ * the grid barrier between the steps (an acquire by one thread, then
+ * bar.sync) orders it after every write of the step before. */
+template <typename T>
+static __device__ __forceinline__ T ld(const T* p)
+{
+    const T* q;
+    asm("mov.b64 %0, %1;" : "=l"(q) : "l"(p));
+    return *q;
+}
+
+static __device__ __forceinline__ int modi(int x, int n)
+{
+    const int m = x % n;
+    return m < 0 ? m + n : m;
+}
+
+/* tile (ty, tx) moved by direction k (0: itself, 1..4: north, west, east,
+ * south) into the next list, once per step */
+static __device__ __forceinline__ void mark(const Params& p, int ty, int tx, int k, int epoch, int* list,
+                                            unsigned long long* word)
+{
+    int y = ty + (k == 1 ? -1 : (k == 4 ? 1 : 0)), x = tx + (k == 2 ? -1 : (k == 3 ? 1 : 0));
+    if (p.toroidal) {
+        y = y < 0 ? p.tiles_y - 1 : (y >= p.tiles_y ? 0 : y);
+        x = x < 0 ? p.tiles_x - 1 : (x >= p.tiles_x ? 0 : x);
+    } else if ((unsigned)y >= (unsigned)p.tiles_y || (unsigned)x >= (unsigned)p.tiles_x) {
+        return;
+    }
+    const int t = y * p.tiles_x + x;
+    if (atomicExch(p.stamps + t, epoch) != epoch)
+        list[sdt2::low32(atomicAdd(word, 1ull))] = t;
+}
+
+/* one tile of one step, by the 256 threads of a group */
+static __device__ __forceinline__ void tile_step(const Params& p, const double* hin, double* hout, int tile,
+                                                 int group, int tid, Shared& S, int turn, int epoch, int* next,
+                                                 unsigned long long* word)
+{
+    Shared::Flags& F = S.flags[turn];
+    const int ty = tile / p.tiles_x, tx = tile - ty * p.tiles_x;
+    const int i0 = ty * TH, j0 = tx * TW;
+    const bool edge = i0 < 2 || j0 < 2 || i0 + TH + 2 > p.rows || j0 + TW + 2 > p.cols;
+    double zv[(R2 + GT - 1) / GT], hv[(R2 + GT - 1) / GT];
+#pragma unroll
+    for (int k = 0; k < (R2 + GT - 1) / GT; k++) {
+        const int t = tid + k * GT;
+        int gi = i0 - 2 + t / R2W, gj = j0 - 2 + t % R2W;
+        bool in = t < R2;
+        if (edge) {
+            if (p.toroidal) {
+                gi = modi(gi, p.rows);
+                gj = modi(gj, p.cols);
+            } else {
+                in = in && (unsigned)gi < (unsigned)p.rows && (unsigned)gj < (unsigned)p.cols;
+            }
+        }
+        zv[k] = hv[k] = 0.0; /* absent neighbours read 0 */
+        if (in) {
+            const long long c = (long long)gi * p.cols + gj;
+            zv[k] = __ldg(p.z + c);
+            hv[k] = ld(hin + c);
+        }
+    }
+    group_sync(group); /* every thread is done with the tile before */
+    if (tid == 0)
+        S.flags[turn ^ 1] = Shared::Flags{0, 0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < (R2 + GT - 1) / GT; k++) {
+        const int t = tid + k * GT;
+        if (t < R2) {
+            const int a = t / R2W, b = t % R2W;
+            S.z[t] = zv[k];
+            S.h[t] = hv[k];
+            S.zh[t] = __double_as_longlong(hv[k]) != 0 ? zv[k] + hv[k] : sdt::plus_zero(zv[k]); /* z + 0.0 */
+            if (sdt::is_wet(hv[k], p.eps_bits)) {
+                F.any = 1;
+                if (a >= 2 && a < TH + 2 && b >= 2 && b < TW + 2 && i0 - 2 + a < p.rows && j0 - 2 + b < p.cols)
+                    F.own = 1;
+            }
+        }
+    }
+    group_sync(group);
+    const bool any = F.any != 0, own = F.own != 0;
+    if (own && tid >= GT - 32 && tid < GT - 27) /* the warp with the least left to do */
+        mark(p, ty, tx, tid - (GT - 32), epoch, next, word);
+    if (!any) {
+        /* changed last step, still now */
+        for (int q = tid; q < TW * TH; q += GT) {
+            const int i = i0 + q / TW, j = j0 + q % TW;
+            if (i < p.rows && j < p.cols)
+                hout[(long long)i * p.cols + j] = S.h[(q / TW + 2) * R2W + q % TW + 2];
+        }
+        return;
+    }
+    /* the outflows start at +0; the wet cells of the tile + 1 ring packed
+     * onto consecutive threads */
+    for (int t0 = 0; t0 < R1; t0 += GT) {
+        const int t = t0 + tid;
+        bool wet = false;
+        if (t < R1) {
+            const int a = t / R1W, b = t % R1W;
+            const bool in = p.toroidal || ((unsigned)(i0 - 1 + a) < (unsigned)p.rows &&
+                                           (unsigned)(j0 - 1 + b) < (unsigned)p.cols);
+            wet = in && sdt::is_wet(S.h[(a + 1) * R2W + b + 1], p.eps_bits);
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                S.f[q][t] = 0.0;
+        }
+        sdt::warp_append_shared(wet, t, S.list, &F.count);
+    }
+    group_sync(group);
+    for (int k = tid; k < F.count; k += GT) {
+        const int t = S.list[k];
+        const int a = t / R1W, b = t % R1W;
+        const int c = (a + 1) * R2W + b + 1;
+        double f[4];
+        sdt::outflows(S.h[c], S.z[c], S.zh[c - R2W], S.zh[c - 1], S.zh[c + 1], S.zh[c + R2W], p.eps, p.r, f);
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            S.f[q][t] = f[q];
+    }
+    group_sync(group);
+    bool late = false;
+    for (int q = tid; q < TW * TH; q += GT) {
+        const int a = q / TW, b = q % TW;
+        const int i = i0 + a, j = j0 + b;
+        if (i >= p.rows || j >= p.cols)
+            continue;
+        const int c = (a + 1) * R1W + b + 1;
+        /* inflow from neighbour n is its outflow f[4 - n] */
+        const double in[4] = {S.f[3][c - R1W], S.f[2][c - 1], S.f[1][c + 1], S.f[0][c + R1W]};
+        double x = S.h[(a + 2) * R2W + b + 2];
+        long long bits = 0;
+#pragma unroll
+        for (int n = 0; n < 4; n++)
+            bits |= __double_as_longlong(in[n]) | __double_as_longlong(S.f[n][c]);
+        if (bits != 0) {
+#pragma unroll
+            for (int n = 0; n < 4; n++)
+                x += in[n] - S.f[n][c];
+        }
+        hout[(long long)i * p.cols + j] = x;
+        late = late || sdt::is_wet(x, p.eps_bits);
+    }
+    if (!own) { /* the same for the whole group */
+        if (late)
+            F.late = 1;
+        group_sync(group);
+        if (F.late && tid < 5)
+            mark(p, ty, tx, tid, epoch, next, word);
+    }
+}
+
+__global__ void __launch_bounds__(THREADS, 1) k_persist(const __grid_constant__ Params p, int nsteps)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_cnt;
+    const int group = threadIdx.x / GT, tid = threadIdx.x % GT;
+    Shared& S = reinterpret_cast<Shared*>(smem)[group];
+    /* consecutive tiles on consecutive blocks, that is, SMs: more than 32
+     * registers a thread leave no room for two blocks on one */
+    const int first = group * (int)gridDim.x + blockIdx.x, stride = GROUPS * (int)gridDim.x;
+    if (threadIdx.x == 0)
+        s_cnt = sdt2::low32(__ldcg(p.words));
+    if (tid < 2)
+        S.flags[tid] = Shared::Flags{0, 0, 0, 0};
+    __syncthreads();
+    int n = s_cnt; /* tiles of the current step */
+    int turn = 0, s = 0;
+    for (; s < nsteps && n <= stride; s++) { /* n is the same in every block */
+        const int* list = (s & 1) ? p.list1 : p.list0;
+        int* next = (s & 1) ? p.list0 : p.list1;
+        unsigned long long* word = p.words + 16 * ((s + 1) % 3);
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            p.words[16 * ((s + 2) % 3)] = 0; /* the step after's, last polled at the end of step s - 2 */
+        for (int item = first; item < n; item += stride, turn ^= 1)
+            tile_step(p, (s & 1) ? p.h1 : p.h0, (s & 1) ? p.h0 : p.h1, ld(list + item), group, tid, S, turn, s + 2,
+                      next, word);
+        if (!sdt2::packed_barrier(word, gridDim.x, p.counts, &s_cnt))
+            return;
+        n = s_cnt;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        p.counts[C_DONE] = s;
+    if (s & 1) {
+        /* the state lies in h1: where the buffers can differ, the last
+         * step's changes, are tiles of the list it built */
+        const int* list = p.list1;
+        for (int item = first; item < n; item += stride) {
+            const int tile = ld(list + item);
+            const int ty = tile / p.tiles_x, tx = tile - ty * p.tiles_x;
+            for (int q = tid; q < TW * TH; q += GT) {
+                const int i = ty * TH + q / TW, j = tx * TW + q % TW;
+                if (i < p.rows && j < p.cols)
+                    p.h0[(long long)i * p.cols + j] = ld(p.h1 + (long long)i * p.cols + j);
+            }
+        }
+    }
+}
+
+/* -0 -> +0 in h (the first reference step adds 0.0 to every cell), the other
+ * buffer the same, and L_0 */
+__global__ void __launch_bounds__(256) k_prime(const __grid_constant__ Params p)
+{
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < p.n; c += stride) {
+        const double hv = sdt::plus_zero(p.h0[c]);
+        p.h0[c] = hv;
+        p.h1[c] = hv;
+        if (sdt::is_wet(hv, p.eps_bits)) {
+            const int ty = (int)(c / p.cols) / TH, tx = (int)(c % p.cols) / TW;
+            for (int k = 0; k < 5; k++)
+                mark(p, ty, tx, k, 1, p.list0, p.words);
+        }
+    }
+}
+
+static void release()
+{
+    State& s = g_state;
+    cudaFree(s.h2);
+    cudaFree(s.stamps);
+    cudaFree(s.list[0]);
+    cudaFree(s.list[1]);
+    cudaFree(s.words);
+    cudaFree(s.counts);
+    s = State();
+}
+
+/* Up to `nsteps` steps from h in one cooperative launch (a block per SM), as
+ * long as no group has two tiles; *done: where the device finds how many, or
+ * NULL when the grid has no more tiles than groups.  False when out
+ * of memory, when the launch is refused or a CUDA error is pending.  A
+ * barrier that gave up sets counts[C_ERROR], which persist_failed()
+ * reports. */
+static bool persist(struct CALModel2D* ca, const double* z, double* h, double eps, double r, long long eps_bits,
+                    int nsteps, const int** done, cudaStream_t st)
+{
+    State& s = g_state;
+    const long long n = (long long)ca->rows * ca->columns;
+    if (s.ca != ca || s.n != n) {
+        release();
+        s.ca = ca;
+        s.n = n;
+        s.tiles_x = (ca->columns + TW - 1) / TW;
+        s.tiles_y = (ca->rows + TH - 1) / TH;
+        const size_t nt = sizeof(int) * (size_t)s.tiles_x * s.tiles_y;
+        if (cudaMalloc(&s.h2, n * sizeof(double)) != cudaSuccess || cudaMalloc(&s.stamps, nt) != cudaSuccess ||
+            cudaMalloc(&s.list[0], nt) != cudaSuccess || cudaMalloc(&s.list[1], nt) != cudaSuccess ||
+            cudaMalloc(&s.words, 48 * sizeof(unsigned long long)) != cudaSuccess ||
+            cudaMalloc(&s.counts, NCOUNTS * sizeof(int)) != cudaSuccess) {
+            release();
+            return false;
+        }
+    }
+    static int grid = 0;
+    if (!grid) {
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (sms <= 0 || cudaFuncSetAttribute(k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(GROUPS * sizeof(Shared))) != cudaSuccess)
+            return false;
+        grid = sms;
+    }
+    Params p;
+    p.z = z;
+    p.h0 = h;
+    p.h1 = s.h2;
+    p.stamps = s.stamps;
+    p.list0 = s.list[0];
+    p.list1 = s.list[1];
+    p.words = s.words;
+    p.counts = s.counts;
+    p.rows = ca->rows;
+    p.cols = ca->columns;
+    p.toroidal = ca->T == CAL_SPACE_TOROIDAL;
+    p.tiles_x = s.tiles_x;
+    p.tiles_y = s.tiles_y;
+    p.n = n;
+    p.eps = eps;
+    p.r = r;
+    p.eps_bits = eps_bits;
+    cudaMemsetAsync(s.stamps, 0, sizeof(int) * (size_t)s.tiles_x * s.tiles_y, st);
+    cudaMemsetAsync(s.words, 0, 48 * sizeof(unsigned long long), st);
+    cudaMemsetAsync(s.counts, 0, NCOUNTS * sizeof(int), st);
+    const long long blocks = (n + 255) / 256;
+    k_prime<<<(int)(blocks > 152 * 16 ? 152 * 16 : blocks), 256, 0, st>>>(p);
+    *done = s.tiles_x * s.tiles_y > GROUPS * grid ? s.counts + C_DONE : nullptr;
+    void* args[] = {&p, &nsteps};
+    return cudaLaunchCooperativeKernel((const void*)k_persist, dim3(grid), dim3(THREADS), args,
+                                       GROUPS * sizeof(Shared), st) == cudaSuccess;
+}
+
+/* did the last persistent run give up at a barrier?  (synchronises) */
+static int persist_failed(cudaStream_t st)
+{
+    int flag = 0;
+    if (!g_state.counts)
+        return 0;
+    cudaStreamSynchronize(st);
+    cudaMemcpy(&flag, g_state.counts + C_ERROR, sizeof(int), cudaMemcpyDeviceToHost);
+    return flag;
+}
+
+} // namespace sdtp
+
 /* ======================= 2c. the split step with active cells ===========
  * OpenCAL's active-cells program (flows, width update and removal of dry
  * cells, an update after each, then the steering:
@@ -1242,7 +1616,7 @@ namespace sdtac {
 constexpr int THREADS = 256, BLOCKS = 152 * 4;
 /* counts[0..1] list lengths by parity, [4] parity, [6] epoch, [8 + parity]
  * cells activated by the step's flows, [32] K2 block ticket (own line); the
- * persistent kernel's barrier and placement words at sdt2's offsets */
+ * persistent kernel's barrier words at sdt2's offsets */
 constexpr int NCOUNTS = sdt2::NCOUNTS, C_PAR = 4, C_EPOCH = 6, C_EXT = 8, C_TICKET = sdt2::C_TICKET;
 
 struct State {
@@ -1404,16 +1778,13 @@ __global__ void __launch_bounds__(THREADS) k2_update(const __grid_constant__ Par
 }
 
 /* every step of a run in one cooperative launch: the flows phase, a grid
- * barrier, the update phase, a grid barrier; work dealt in the placement
- * order (sdt2::placement_order) */
-__global__ void __launch_bounds__(THREADS, 4) k_persist(const __grid_constant__ Params p, int nsteps, int nsm)
+ * barrier, the update phase, a grid barrier; a block of 1024 threads per SM
+ * (sdt2::k_persist says why) */
+__global__ void __launch_bounds__(sdt2::PTHREADS, 1) k_persist(const __grid_constant__ Params p, int nsteps)
 {
     __shared__ int s_cnt[2];
     const unsigned nb = gridDim.x;
     unsigned round = 0;
-    const int vb = sdt2::placement_order(p.counts, nb, nsm, round, s_cnt);
-    if (vb < 0)
-        return;
     if (threadIdx.x == 0) {
         s_cnt[0] = __ldcg(p.counts + C_PAR);
         s_cnt[1] = __ldcg(p.counts + C_EPOCH);
@@ -1425,7 +1796,7 @@ __global__ void __launch_bounds__(THREADS, 4) k_persist(const __grid_constant__ 
         s_cnt[0] = __ldcg(p.counts + par);
     __syncthreads();
     int na = s_cnt[0];
-    const int g0 = first_chunk(vb, (int)nb), gs = (int)nb * (THREADS / 32);
+    const int g0 = first_chunk(blockIdx.x, (int)nb), gs = (int)nb * (sdt2::PTHREADS / 32);
     for (int s = 0; s < nsteps; s++) {
         if (blockIdx.x == 0 && threadIdx.x == 0)
             p.counts[1 - par] = 0; /* the list the update phase appends to */
@@ -1541,31 +1912,28 @@ static bool step(struct CALModel2D* ca, const double* z, double* h, double eps, 
     return cudaGetLastError() == cudaSuccess;
 }
 
-/* `nsteps` steps in one cooperative launch of k_persist (SMs x resident
- * blocks per SM); false when the launch is refused or a CUDA error is
+/* `nsteps` steps in one cooperative launch of k_persist (a block per SM);
+ * false when the launch is refused or a CUDA error is
  * pending.  A barrier that gave up sets the error word persist_failed()
  * reports. */
 static bool persist(struct CALModel2D* ca, const double* z, double* h, double eps, double r, long long eps_bits,
                     int nsteps, cudaStream_t st)
 {
     State& s = g_state;
-    static int grid = 0, nsm = 0;
+    static int grid = 0;
     if (!grid) {
-        int per_sm = 0, dev = 0, sms = 0;
+        int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist, THREADS, 0);
-        grid = sms * per_sm;
-        nsm = sms;
+        grid = sms;
         if (grid <= 0)
             return false;
     }
     Params p = params(ca, z, h, eps, r, eps_bits);
     cudaMemsetAsync(s.counts + sdt2::C_ARRIVED, 0, sizeof(int), st);
     cudaMemsetAsync(s.counts + sdt2::C_ERROR, 0, sizeof(int), st);
-    cudaMemsetAsync(s.counts + sdt2::C_PLACE_BAD, 0, (NCOUNTS - sdt2::C_PLACE_BAD) * sizeof(int), st);
-    void* args[] = {&p, &nsteps, &nsm};
-    return cudaLaunchCooperativeKernel((const void*)k_persist, dim3(grid), dim3(THREADS), args, 0, st) ==
+    void* args[] = {&p, &nsteps};
+    return cudaLaunchCooperativeKernel((const void*)k_persist, dim3(grid), dim3(sdt2::PTHREADS), args, 0, st) ==
            cudaSuccess;
 }
 
@@ -2155,8 +2523,14 @@ static int g_fallbacks = 0;
 static void cal_note_fallback() { g_fallbacks++; }
 extern "C" int cal_sciddicaT_device_loop_fallbacks(void) { return g_fallbacks; }
 
-/* every one of `steps` steps in one cooperative launch: the persistent
- * split step (plain) or the persistent active-cells split step; the state
+/* did a grid barrier of the last plain persistent run give up?  (synchronises) */
+static int sciddicaT_persist_gave_up(cudaStream_t st)
+{
+    return sdtp::persist_failed(st) || sdt2::persist_failed(st);
+}
+
+/* every one of `steps` steps in cooperative launches: tile by tile, then the
+ * persistent split step (plain), or the persistent active-cells split step; the state
  * must be initialised.  Returns a CALError code (CAL_ERROR_CUDA also when a
  * grid barrier gave up, which synchronises). */
 static int sciddicaT_persist_steps(struct CALModel2D* ca, int steps, bool fused_ac)
@@ -2168,17 +2542,25 @@ static int sciddicaT_persist_steps(struct CALModel2D* ca, int steps, bool fused_
         sciddicaT_ac_prepare_now(ca);
         if (!sdtac::g_state.primed)
             return CAL_ERROR_OUT_OF_MEMORY;
-    } else {
-        sciddicaT_split_prepare_now(ca);
-        if (!sdt2::g_state.primed)
-            return CAL_ERROR_OUT_OF_MEMORY;
+    } else if (sdt3::g_state.primed && sdt3::g_state.ca == ca) {
+        sciddicaT_sparse_resolve(ca); /* h back from the sparse step's buffers */
+        sciddicaT_sparse_invalidate();
     }
     const double* z = (const double*)calGetDeviceBuffer2Dr(ca, Q.z, 0);
     double* h = (double*)calGetDeviceBuffer2Dr(ca, Q.h, 0);
-    const bool ok = fused_ac ? sdtac::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, st)
-                             : sdt2::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, st);
+    bool ok;
+    if (fused_ac) {
+        ok = sdtac::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, st);
+    } else {
+        const int* done = nullptr;
+        ok = sdtp::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, &done, st);
+        if (ok && done)
+            ok = sdt2::prime(ca, h, z, P.epsilon, eps_bits, st, done, steps) &&
+                 sdt2::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, done, st);
+        sdt2::g_state.primed = false; /* the split step's lists were not kept in the first part */
+    }
     if (!ok)
-        return CAL_ERROR_CUDA;
+        return !fused_ac && (!sdtp::g_state.h2 || !sdt2::g_state.f) ? CAL_ERROR_OUT_OF_MEMORY : CAL_ERROR_CUDA;
     calMarkCurrentWritten2Dr(ca, Q.h);
     return calGetLastError();
 }
@@ -2263,7 +2645,7 @@ extern "C" int cal_sciddicaT_run(int rows, int cols, int toroidal, int ac, int s
     } else if (graph == 4 && mode == SDT_MODE_FUSED) {
         /* every step in one cooperative launch (the persistent split step) */
         if (steps > 0 && sciddicaT_persist_steps(ca, steps, fused_ac) == CAL_SUCCESS &&
-            (fused_ac ? sdtac::persist_failed(s) : sdt2::persist_failed(s)) != 0)
+            (fused_ac ? sdtac::persist_failed(s) : sciddicaT_persist_gave_up(s)) != 0)
             cal::set_error(CAL_ERROR_CUDA, "SCIDDICA-T persistent step: a grid barrier gave up");
     } else {
         for (run->step = run->initial_step; run->step <= run->final_step; run->step++)
@@ -2299,6 +2681,7 @@ extern "C" int cal_sciddicaT_run(int rows, int cols, int toroidal, int ac, int s
     }
     int err = calGetLastError();
     sdt2::release();
+    sdtp::release();
     sdtac::release();
     g_fused_ac = false;
     calRunFinalize2D(run);
@@ -2495,7 +2878,7 @@ extern "C" int cal_sciddicaT_persist_failed(void* handle)
 {
     SdtSession* s = (SdtSession*)handle;
     cudaStream_t st = (cudaStream_t)calGetStream2D(s->ca);
-    return s->fused_ac ? sdtac::persist_failed(st) : sdt2::persist_failed(st);
+    return s->fused_ac ? sdtac::persist_failed(st) : sciddicaT_persist_gave_up(st);
 }
 
 /* host-buffer round trip through the API: z and h from the caller's arrays
@@ -2559,6 +2942,8 @@ extern "C" int cal_sciddicaT_wet_count(void* handle)
     SdtSession* s = (SdtSession*)handle;
     if (!sdt2::g_state.counts)
         return -1;
+    if (s->mode == SDT_MODE_FUSED && !s->fused_ac)
+        sciddicaT_split_prepare_now(s->ca); /* after a persistent run the lists are not there */
     /* the model's stream does not synchronise with the legacy stream */
     cudaStreamSynchronize((cudaStream_t)calGetStream2D(s->ca));
     int c[6] = {0, 0, 0, 0, 0, 0};
@@ -2649,6 +3034,7 @@ extern "C" void cal_sciddicaT_close(void* handle)
             cudaFree(s->snap[k][l]);
     cudaFree(s->snap_flags);
     sdt2::release();
+    sdtp::release();
     sdtac::release();
     g_fused_ac = false;
     calRunFinalize2D(s->run);
