@@ -1413,15 +1413,17 @@ namespace sci2 {
  * that.  Every byte written here is overwritten by the copy. */
 static void touch_pages(void* dst, size_t bytes)
 {
-    constexpr size_t STEP = 4096, MIN_SHARE = 4u << 20;
-    const int nthreads = (int)std::min<size_t>(4, bytes / MIN_SHARE);
+    /* the C library keeps freed blocks below 32 MB mapped for reuse, larger
+     * ones come fresh from the system every time */
+    constexpr size_t STEP = 4096, MIN_BYTES = 32u << 20;
+    const int nthreads = 4;
+    if (bytes < MIN_BYTES)
+        return;
     volatile char* p = (volatile char*)dst;
     auto share = [=](int k, int n) {
         for (size_t q = bytes / n * k; q < (k + 1 == n ? bytes : bytes / n * (k + 1)); q += STEP)
             p[q] = 0;
     };
-    if (nthreads < 1)
-        return; /* small results: the faults cost less than the threads */
     std::vector<std::thread> others;
     int started = 1;
     try {
