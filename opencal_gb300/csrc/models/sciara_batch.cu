@@ -64,6 +64,7 @@ constexpr int MAX_INST = 1024;
 struct Phys {
     double Pclock, Pc, Pac, PTsol, PTvent, a, b, c, d, Pcool, Prho, Pepsilon, Psigma, Pcv, rad2;
     double rrad2, w2; /* RN(1 / rad2), Pc * Pc */
+    double cool3;     /* 3 Pepsilon Psigma Pclock Pcool / (Prho Pcv Pac) */
     int rad2_recip;   /* x / rad2 by cal_div_recip (its precondition holds) */
 };
 
@@ -615,9 +616,11 @@ __global__ void __launch_bounds__(K1T) k_update(const __grid_constant__ Dev d, c
  *      own adjoints; keeps, per entry, dL/dh' (A_h), dL/dt' / D (A_t) and
  *      t' for the outflow adjoints;
  *   B1 (lava entries): the adjoint of each outflow gathered from the two
- *      cells it connects, then the minimisation backward, scattered (FP64
- *      atomics) to the thickness, altitude and temperature adjoints of the
- *      nine cells it read; then, by its last block, the emission backward --
+ *      cells it connects, then the minimisation backward to the nine cells
+ *      it read: the cell's own adjoints directly, its neighbours' through
+ *      one FP64 atomic each onto two sums per cell, of the neighbours across
+ *      an edge (H = z + h: dL/dh and dL/dz alike) and across a corner
+ *      (dL/dz by 1 / sqrt 2); B2 folds a cell's sums into its adjoints; then, by its last block, the emission backward --
  *      dL/drate += dL/dSlt(vent) * Pclock / Pac for the vent whose emission
  *      took effect, the temperature adjoint of the vent cell reset (the
  *      emission overwrote it).
@@ -634,6 +637,8 @@ struct Adj {
     double* lh;   /* dense: dL/dSlt */
     double* lt;   /* dense: dL/dSt */
     double* lz;   /* dense: dL/dSz */
+    double* side; /* dense: dL/dH from the cells across an edge, */
+    double* diag; /* and across a corner, not yet in lh and lz */
     Mix* mix;     /* per entry of the step */
     double* grad; /* nvents x nphases, internal vent order */
 };
@@ -648,32 +653,35 @@ __global__ void __launch_bounds__(BT) k_bcells(const __grid_constant__ Dev d, co
     const int x = tp.cell[e];
     const unsigned flag = tp.flag[e];
     const double t = tp.val[e], tn = tp.val[tp.cap + e];
-    const double lh = a.lh[x], lt = a.lt[x];
+    const double side = a.side[x], diag = a.diag[x];
+    const double lh = a.lh[x] + (side + diag), lt = a.lt[x];
+    const double lz = a.lz[x] + (side + diag * d.ph.rrad2);
     double Lh = lh, Lt = lt; /* adjoints of h', t' */
     if (flag & E_BORDER) {
         Lh = 0.0;
         Lt = 0.0;
     } else if (flag & E_SOLID) {
-        Lh = a.lz[x]; /* Sz += h' */
+        Lh = lz; /* Sz += h' */
         Lt = 0.0;
     } else if (flag & E_LAVA) {
-        /* st = t' / aus^(1/3), aus = 1 + 3 K t'^3 / (C h') */
-        const double K = d.ph.Pepsilon * d.ph.Psigma * d.ph.Pclock * d.ph.Pcool;
-        const double Cc = d.ph.Prho * d.ph.Pcv * d.ph.Pac;
+        /* st = t' / aus^(1/3), aus = 1 + q, q = cool3 t'^3 / h' */
         const double hn = tp.val[2 * tp.cap + e], aus = tp.val[5 * tp.cap + e], st = tp.val[6 * tp.cap + e];
+        const double rh = 1.0 / hn, rt = 1.0 / tn;
+        const double q = d.ph.cool3 * (tn * tn * tn) * rh;
         const double dst_daus = -st / (3.0 * aus);
-        const double daus_dT = 9.0 * K * tn * tn / (Cc * hn);
-        const double daus_dh = -3.0 * K * tn * tn * tn / (Cc * hn * hn);
-        Lh = lh + lt * (dst_daus * daus_dh);
-        Lt = lt * (st / tn + dst_daus * daus_dT);
+        Lh = lh - lt * (dst_daus * q * rh);
+        Lt = lt * ((st + 3.0 * dst_daus * q) * rt);
     }
     Mix m = {Lh, 0.0, tn, 0.0};
     if (flag & E_FLOW) {
         const double residual = tp.val[3 * tp.cap + e], D = tp.val[4 * tp.cap + e];
         m.At = Lt / D;
-        Lh = Lh + Lt * (t - tn) / D;
-        Lt = Lt * residual / D;
+        Lh = Lh + m.At * (t - tn);
+        Lt = m.At * residual;
     }
+    a.side[x] = 0.0;
+    a.diag[x] = 0.0;
+    a.lz[x] = lz;
     a.lh[x] = Lh;
     a.lt[x] = Lt;
     a.mix[k] = m;
@@ -724,7 +732,7 @@ __global__ void __launch_bounds__(BT) k_bflows(const __grid_constant__ Dev d, co
             lt_add += v * dlog * fk;
         }
         const double g = cal_div_small(G, __popc(S));
-        const double inv = 1.0 / d.ph.rad2;
+        const double inv = d.ph.rrad2;
         double lz_own = 0.0;
 #pragma unroll
         for (int k = 0; k < 9; k++) {
@@ -738,16 +746,13 @@ __global__ void __launch_bounds__(BT) k_bflows(const __grid_constant__ Dev d, co
                 lz_own += lH[k];
             if (k >= 5)
                 lz_own += lH[k] * (1.0 - inv);
-            if (k >= 1 && ((inside >> k) & 1u)) {
-                const int cn = x + kMi[k] * cols + kMj[k];
-                atomicAdd(a.lh + cn, lH[k]);
-                atomicAdd(a.lz + cn, k < 5 ? lH[k] : lH[k] * inv);
-            }
+            if (k >= 1 && ((inside >> k) & 1u))
+                atomicAdd((k < 5 ? a.side : a.diag) + x + kMi[k] * cols + kMj[k], lH[k]);
         }
-        atomicAdd(a.lh + x, g); /* avg's h[0] */
-        atomicAdd(a.lt + x, lt_add);
-        if (lz_own != 0.0)
-            atomicAdd(a.lz + x, lz_own);
+        /* no other thread of the launch touches these */
+        a.lh[x] += g; /* avg's h[0] */
+        a.lt[x] += lt_add;
+        a.lz[x] += lz_own;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -762,7 +767,8 @@ __global__ void __launch_bounds__(BT) k_bflows(const __grid_constant__ Dev d, co
         const int eff = phase < (unsigned)d.nphases ? d.g_eff[(size_t)q * d.nphases + phase] : -1;
         if (eff >= 0) {
             const int c = d.g_cell[q];
-            a.grad[(size_t)eff * d.nphases + phase] += __ldcg(a.lh + c) * d.ph.Pclock / d.ph.Pac;
+            const double lh = __ldcg(a.lh + c) + (__ldcg(a.side + c) + __ldcg(a.diag + c));
+            a.grad[(size_t)eff * d.nphases + phase] += lh * d.ph.Pclock / d.ph.Pac;
             a.lt[c] = 0.0;
         }
     }
@@ -805,6 +811,8 @@ __global__ void __launch_bounds__(T) k_bloss(const __grid_constant__ Dev d, cons
             a.lh[c] = 2.0 * diff;
             a.lt[c] = 0.0;
             a.lz[c] = 0.0;
+            a.side[c] = 0.0;
+            a.diag[c] = 0.0;
         }
         const int b0 = __shfl_sync(0xffffffffu, b, 0);
         if (__all_sync(0xffffffffu, b == b0 || b < 0)) {
@@ -970,6 +978,8 @@ static void free_work(Batch& bt)
     wfree(&bt.adj.lh);
     wfree(&bt.adj.lt);
     wfree(&bt.adj.lz);
+    wfree(&bt.adj.side);
+    wfree(&bt.adj.diag);
     wfree(&bt.adj.mix);
     wfree(&bt.adj.grad);
     wfree(&bt.tgt);
@@ -1125,6 +1135,7 @@ extern "C" void* cal_sciara_batch_create(int B, const int* dims, const double* z
     d.ph.rrad2 = 1.0 / d.ph.rad2;
     d.ph.rad2_recip = cal_recip_exact_ok(d.ph.rad2, d.ph.rrad2) ? 1 : 0;
     d.ph.w2 = d.ph.Pc * d.ph.Pc;
+    d.ph.cool3 = 3.0 * d.ph.Pepsilon * d.ph.Psigma * d.ph.Pclock * d.ph.Pcool / (d.ph.Prho * d.ph.Pcv * d.ph.Pac);
     /* evaluatePowerLawParams (Sciara.cpp:199-204), C library log10 */
     d.ph.b = (log10(Pr_Tvent) - log10(Pr_Tsol)) / (d.ph.PTvent - d.ph.PTsol);
     d.ph.a = log10(Pr_Tsol) - d.ph.b * (d.ph.PTsol);
@@ -1324,7 +1335,8 @@ static int loss_grad(Batch* bt, const double* target, int max_steps, double* los
     if (!walloc(&tp.used, 1) || !walloc(&tp.step_base, (size_t)bt->tape_steps) ||
         !walloc(&tp.step_lava, (size_t)bt->tape_steps) || !walloc(&tp.step_n, (size_t)bt->tape_steps) ||
         !walloc(&bt->tgt, (size_t)bt->N) || !walloc(&bt->loss, (size_t)bt->B) || !walloc(&a.lh, (size_t)bt->N) ||
-        !walloc(&a.lt, (size_t)bt->N) || !walloc(&a.lz, (size_t)bt->N) || !walloc(&a.grad, ngrad))
+        !walloc(&a.lt, (size_t)bt->N) || !walloc(&a.lz, (size_t)bt->N) ||
+        !walloc(&a.side, (size_t)bt->N) || !walloc(&a.diag, (size_t)bt->N) || !walloc(&a.grad, ngrad))
         return OOM;
     if (!tp.cap && !grow_tape(*bt, first_tape(*bt, steps)) && !grow_tape(*bt, 4096))
         return OOM;
@@ -1426,7 +1438,7 @@ extern "C" int cal_sciara_batch_loss_grad(void* handle, const double* target, in
      * sixteenth of the device's memory */
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
-    const size_t held = (size_t)bt->tp.cap * sci2::ENTRY_BYTES + sizeof(double) * 4 * (size_t)bt->N +
+    const size_t held = (size_t)bt->tp.cap * sci2::ENTRY_BYTES + sizeof(double) * 6 * (size_t)bt->N +
                         sizeof(sci2::Mix) * (size_t)bt->mix_cap;
     if (rc || held > total_b / 16) {
         cudaStreamSynchronize(bt->st);
