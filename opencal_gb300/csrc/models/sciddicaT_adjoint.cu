@@ -25,7 +25,7 @@
  *   dL/dh0 = lambda_0 - [h0 > 0] lambda_z.
  *
  * The steps and their adjoint are the wet-cell list's (sciddicaT_wet.cuh)
- * with one instance.  The forward tapes the rollout into a tape sized by a
+ * with one instance, in one cooperative launch each way.  The forward tapes the rollout into a tape sized by a
  * guess; the backward first learns what the tape needed.  When it was too
  * small, the forward runs again with one that fits, or, when a whole-rollout
  * tape would take more than half of the free device memory, with h stored
@@ -62,6 +62,7 @@ struct Work {
     double* ckpt = nullptr; /* segments only */
     char* slab = nullptr;   /* every array of fixed size, one allocation */
     char* tape = nullptr;
+    unsigned long long* words = nullptr; /* of the cooperative launches */
     bool want_tape = true;
     bool flows_clear = false;
 };
@@ -108,6 +109,7 @@ static size_t carve(Work& W, char* base)
     c.take(&d.stamps, d.ntiles);
     c.take(&d.toff, steps);
     c.take(&d.need, 1);
+    c.take(&W.words, 16 * sdtw::NWORDS);
     c.take(&a.lam, n);
     c.take(&a.mu, n);
     c.take(&a.stamp, n);
@@ -153,6 +155,7 @@ static void queue_forward(Work& W, bool keep, cudaStream_t st)
     cudaMemsetAsync(d.nlist, 0, sizeof(int) * (W.steps + 1), st);
     cudaMemsetAsync(d.toff, 0, sizeof(long long), st);
     cudaMemsetAsync(d.need, 0, sizeof(long long), st);
+    cudaMemsetAsync(W.words, 0, sizeof(unsigned long long) * 16 * sdtw::NWORDS, st);
     if (!W.flows_clear) {
         cudaMemsetAsync(d.f, 0, n * sizeof(sdtw::D4), st);
         W.flows_clear = true;
@@ -162,7 +165,7 @@ static void queue_forward(Work& W, bool keep, cudaStream_t st)
     for (int t = 0; t < W.steps; t += per) {
         if (keep)
             cudaMemcpyAsync(W.ckpt + (size_t)(t / per) * n, d.h, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
-        sdtw::queue_steps(d, t, std::min(t + per, W.steps), 1, !keep, st);
+        sdtw::launch_steps(d, t, std::min(t + per, W.steps), 1, !keep, W.words, st);
     }
     if (W.steps > 0)
         sdtw::k_clear_flows<<<sdtw::BLOCKS, T, 0, st>>>(d, W.steps - 1);
@@ -198,9 +201,9 @@ static void queue_segments(Work& W, cudaStream_t st)
         cudaMemsetAsync(d.toff + t0, 0, sizeof(long long), st);
         cudaMemsetAsync(d.stamps, 0, sizeof(int) * d.ntiles, st);
         sdtw::k_relist<<<sdtw::dense_blocks(d.N), T, 2 * sizeof(long long), st>>>(d, t0);
-        sdtw::queue_steps(d, t0, t1, 1, true, st);
+        sdtw::launch_steps(d, t0, t1, 1, true, W.words, st);
         sdtw::k_clear_flows<<<sdtw::BLOCKS, T, 0, st>>>(d, t1 - 1);
-        sdtw::queue_adjoint(d, W.a, t0, t1, st);
+        sdtw::launch_sweep(d, W.a, t0, t1, W.words, st);
     }
 }
 
@@ -292,7 +295,7 @@ extern "C" int cal_sdt_adj_forward(void* handle, const double* z_dem, const doub
     cudaMemcpyAsync(W->z_dem, z_dem, b, cudaMemcpyDeviceToDevice, st);
     sdtadj::queue_forward(*W, W->ckpt != nullptr, st);
     /* no step: h0 as given, -0 and all */
-    cudaMemcpyAsync(hT, W->steps > 0 ? d.h : W->h0, b, cudaMemcpyDeviceToDevice, st);
+    sdtw::k_out<<<sdtw::dense_blocks(d.N), sdtadj::T, 0, st>>>(W->steps > 0 ? d.h : W->h0, hT, d.N, W->words);
     return (int)cudaGetLastError();
 }
 
@@ -326,7 +329,7 @@ extern "C" int cal_sdt_adj_backward(void* handle, const double* gT, double* g_h0
     for (int attempt = 0;; attempt++) {
         sdtadj::queue_seed(*W, gT, st);
         if (!segments) {
-            sdtw::queue_adjoint(d, W->a, 0, W->steps, st);
+            sdtw::launch_sweep(d, W->a, 0, W->steps, W->words, st);
             break;
         }
         sdtadj::queue_segments(*W, st);
@@ -340,8 +343,12 @@ extern "C" int cal_sdt_adj_backward(void* handle, const double* gT, double* g_h0
     sdtw::k_final_grad<<<sdtw::dense_blocks(d.N), sdtadj::T, 0, st>>>(W->h0, W->a.lam, W->a.mu, g_h0, d.N);
     sdtw::k_fold<<<1, 32, 0, st>>>(W->a.part, W->a.grad, 2);
     double res[2] = {0.0, 0.0};
+    unsigned long long gave_up = 0; /* a grid barrier did */
     cudaMemcpyAsync(res, W->a.grad, sizeof(res), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(&gave_up, W->words + 16 * 7, sizeof(gave_up), cudaMemcpyDeviceToHost, st);
     e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess && gave_up)
+        e = cudaErrorUnknown;
     if (g_r)
         *g_r = res[0];
     if (g_eps)

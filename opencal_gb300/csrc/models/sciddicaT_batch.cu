@@ -13,7 +13,8 @@
  * the tiles of all instances are numbered in one range.
  *
  * Forward and adjoint: one list of the wet cells of all instances per step
- * (sciddicaT_wet.cuh), two launches per step each way.  Dry regions cost
+ * (sciddicaT_wet.cuh), two launches per step each way in the recorded
+ * evaluation, all steps in one cooperative launch otherwise.  Dry regions cost
  * nothing, and every instance stays bit-identical to a run of its own.
  *
  * Tape.  The forward TAPES each wet cell's elimination set and differences,
@@ -66,14 +67,15 @@ struct Batch {
     double *z_dem = nullptr, *z = nullptr, *h0 = nullptr;
     double* ckpt = nullptr; /* nseg x N, segments only */
     double* loss = nullptr; /* B */
+    unsigned long long* words = nullptr; /* of the cooperative launches */
     cudaStream_t st = nullptr;
     bool flows_clear = false; /* f is zero everywhere */
     /* the loss + gradient evaluation recorded once as a CUDA graph and
      * replayed every call: tape offsets chained on the device, results
      * copied into pinned host memory (h_out: B losses, 2B gradients, then
-     * the tape entries needed); valid for the target, dL/dh0 buffer, tile
+     * the tape entries needed and the cooperative launches' error word); valid for the target, dL/dh0 buffer, tile
      * shape and tape it was recorded with */
-    double* h_out = nullptr; /* pinned: 3B doubles + one long long */
+    double* h_out = nullptr; /* pinned: 3B doubles + two long longs */
     cudaGraphExec_t gexec = nullptr;
     const double* g_target = nullptr;
     const double* g_gh0 = nullptr;
@@ -162,10 +164,28 @@ static bool tiles_for(Batch& bt)
     return true;
 }
 
+/* steps [t0, t1) queued: in one cooperative launch, or, to be recorded,
+ * launch by launch */
+static void queue_steps(Batch& bt, int t0, int t1, int epoch0, bool taped, bool recorded)
+{
+    if (recorded)
+        sdtw::queue_steps(bt.d, t0, t1, epoch0, taped, bt.st);
+    else
+        sdtw::launch_steps(bt.d, t0, t1, epoch0, taped, bt.words, bt.st);
+}
+
+static void queue_adjoint(Batch& bt, Adj& a, int t0, int t1, bool recorded)
+{
+    if (recorded)
+        sdtw::queue_adjoint(bt.d, a, t0, t1, bt.st);
+    else
+        sdtw::launch_sweep(bt.d, a, t0, t1, bt.words, bt.st);
+}
+
 /* The initial state and `steps` steps from it, queued.  keep: h every K
  * steps into the checkpoints; taped: every step onto the tape (toff[0] = 0,
  * need reset). */
-static void forward(Batch& bt, int steps, bool keep, bool taped)
+static void forward(Batch& bt, int steps, bool keep, bool taped, bool recorded)
 {
     Dev& d = bt.d;
     cudaStream_t st = bt.st;
@@ -173,6 +193,7 @@ static void forward(Batch& bt, int steps, bool keep, bool taped)
     cudaMemsetAsync(d.stamps, 0, sizeof(int) * d.ntiles, st);
     cudaMemsetAsync(d.counts, 0, sizeof(int) * (bt.steps + 1), st);
     cudaMemsetAsync(d.nlist, 0, sizeof(int) * (bt.steps + 1), st);
+    cudaMemsetAsync(bt.words, 0, sizeof(unsigned long long) * 16 * sdtw::NWORDS, st);
     if (taped || keep) {
         cudaMemsetAsync(d.toff, 0, sizeof(long long), st);
         cudaMemsetAsync(d.need, 0, sizeof(long long), st);
@@ -187,7 +208,7 @@ static void forward(Batch& bt, int steps, bool keep, bool taped)
         if (keep)
             cudaMemcpyAsync(bt.ckpt + (size_t)(t / bt.K) * d.N, d.h, (size_t)d.N * sizeof(double),
                             cudaMemcpyDeviceToDevice, st);
-        sdtw::queue_steps(d, t, t1, 1, taped, st);
+        queue_steps(bt, t, t1, 1, taped, recorded);
     }
     if (steps > 0)
         sdtw::k_clear_flows<<<sdtw::BLOCKS, T, 0, st>>>(d, steps - 1);
@@ -205,7 +226,7 @@ static void destroy(Batch* bt)
     void* ptrs[] = {(void*)d.inst, (void*)d.offs, (void*)d.tile_inst, d.h,     d.zh,    d.f,       d.list[0], d.list[1],
                     d.nlist,       d.tiles,       d.counts,           d.stamps, d.t_entry, d.t_elim, d.t_diff,  d.toff,
                     d.need,        a.lam,         a.mu,               a.stamp, a.w,     a.g,       a.grad,    a.part,
-                    bt->z_dem,     bt->z,         bt->h0,             bt->ckpt, bt->loss};
+                    bt->z_dem,     bt->z,         bt->h0,             bt->ckpt, bt->loss, bt->words};
     for (void* p : ptrs)
         cudaFree(p);
     if (bt->st)
@@ -261,7 +282,9 @@ extern "C" void* cal_sdt_batch_create(int B, const int* dims, const double* para
               cudaMalloc(&d.counts, sizeof(int) * (steps + 1)) == cudaSuccess &&
               cudaMalloc(&d.nlist, sizeof(int) * (steps + 1)) == cudaSuccess &&
               cudaMalloc(&d.toff, sizeof(long long) * (steps + 1)) == cudaSuccess &&
-              cudaMalloc(&d.need, sizeof(long long)) == cudaSuccess && cudaMalloc(&bt->z_dem, nb) == cudaSuccess &&
+              cudaMalloc(&d.need, sizeof(long long)) == cudaSuccess &&
+              cudaMalloc(&bt->words, sizeof(unsigned long long) * 16 * sdtw::NWORDS) == cudaSuccess &&
+              cudaMalloc(&bt->z_dem, nb) == cudaSuccess &&
               cudaMalloc(&bt->z, nb) == cudaSuccess && cudaMalloc(&bt->h0, nb) == cudaSuccess &&
               cudaMalloc(&d.h, nb) == cudaSuccess && cudaMalloc(&d.zh, nb) == cudaSuccess &&
               cudaMalloc(&d.f, (size_t)d.N * sizeof(sdtw::D4)) == cudaSuccess &&
@@ -328,9 +351,9 @@ extern "C" int cal_sdt_batch_set_params(void* handle, const double* params)
 extern "C" int cal_sdt_batch_forward(void* handle, double* hT)
 {
     Batch* bt = (Batch*)handle;
-    sdtb::forward(*bt, bt->steps, false, false);
+    sdtb::forward(*bt, bt->steps, false, false, false);
     if (hT)
-        cudaMemcpyAsync(hT, bt->d.h, (size_t)bt->d.N * sizeof(double), cudaMemcpyDeviceToDevice, bt->st);
+        sdtw::k_out<<<sdtw::dense_blocks(bt->d.N), sdtw::T, 0, bt->st>>>(bt->d.h, hT, bt->d.N, bt->words);
     return (int)cudaGetLastError();
 }
 
@@ -350,7 +373,7 @@ namespace sdtb {
  * by segment where the rollout is not on the tape), dL/dh0, and the losses,
  * gradients and the tape entries needed copied into the pinned h_out.
  * Nothing in it waits for the host, so it can be recorded. */
-static void queue_loss_grad(Batch& bt, const double* target, double* g_h0)
+static void queue_loss_grad(Batch& bt, const double* target, double* g_h0, bool recorded)
 {
     Dev& d = bt.d;
     Adj a = bt.a;
@@ -358,13 +381,13 @@ static void queue_loss_grad(Batch& bt, const double* target, double* g_h0)
         a.mu = nullptr; /* nothing reads it */
     const size_t nb = (size_t)d.N * sizeof(double), offs = sizeof(long long) * (bt.B + 1);
     cudaStream_t st = bt.st;
-    forward(bt, bt.steps, !bt.run_full, bt.run_full);
+    forward(bt, bt.steps, !bt.run_full, bt.run_full, recorded);
     cudaMemsetAsync(bt.loss, 0, bt.B * sizeof(double), st);
     cudaMemsetAsync(a.part, 0, 2 * bt.B * sizeof(double) * sdtw::COPIES, st);
     cudaMemsetAsync(a.stamp, 0xff, sizeof(int) * (size_t)d.N, st);
     sdtw::k_loss<<<sdtw::dense_blocks(d.N), T, offs, st>>>(d, a, target, bt.loss);
     if (bt.run_full) {
-        sdtw::queue_adjoint(d, a, 0, bt.steps, st);
+        queue_adjoint(bt, a, 0, bt.steps, recorded);
     } else {
         for (int s = bt.nseg - 1; s >= 0; s--) {
             const int t0 = s * bt.K, t1 = std::min(t0 + bt.K, bt.steps);
@@ -375,9 +398,9 @@ static void queue_loss_grad(Batch& bt, const double* target, double* g_h0)
             cudaMemsetAsync(d.counts + t0, 0, sizeof(int) * (t1 - t0), st);
             cudaMemsetAsync(d.toff + t0, 0, sizeof(long long), st);
             sdtw::k_relist<<<sdtw::dense_blocks(d.N), T, offs, st>>>(d, t0);
-            sdtw::queue_steps(d, t0, t1, bt.steps + 1, true, st);
+            queue_steps(bt, t0, t1, bt.steps + 1, true, recorded);
             sdtw::k_clear_flows<<<sdtw::BLOCKS, T, 0, st>>>(d, t1 - 1);
-            sdtw::queue_adjoint(d, a, t0, t1, st);
+            queue_adjoint(bt, a, t0, t1, recorded);
         }
     }
     if (g_h0)
@@ -386,6 +409,7 @@ static void queue_loss_grad(Batch& bt, const double* target, double* g_h0)
     cudaMemcpyAsync(bt.h_out, bt.loss, bt.B * sizeof(double), cudaMemcpyDeviceToHost, st);
     cudaMemcpyAsync(bt.h_out + bt.B, a.grad, 2 * bt.B * sizeof(double), cudaMemcpyDeviceToHost, st);
     cudaMemcpyAsync(bt.h_out + 3 * bt.B, d.need, sizeof(long long), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(bt.h_out + 3 * bt.B + 1, bt.words + 16 * 7, sizeof(long long), cudaMemcpyDeviceToHost, st);
 }
 
 /* arrays that only the gradient needs, allocated by the first call that
@@ -416,14 +440,14 @@ static bool adjoint_arrays(Batch& bt, bool want_mu)
  * quarter) and the evaluation run again; a first call, without a tape, runs
  * the forward alone to learn that size.  In the memory-chosen mode a
  * whole-rollout tape that would not fit switches the ensemble to segments.
- * Segments of more than 32 steps (rollouts over 1024 steps) always run
- * launch by launch: the recording would hold over six launches a step, and
- * instantiating it costs as much as launching them. */
+ * Segments of more than 32 steps (rollouts over 1024 steps) are not
+ * recorded: six launches a step would make a graph that costs more to
+ * instantiate than the cooperative launches to run. */
 static int loss_grad(Batch& bt, const double* target, double* loss_out, double* grad_out, double* g_h0)
 {
     Dev& d = bt.d;
     cudaStream_t st = bt.st;
-    if (!bt.h_out && cudaMallocHost(&bt.h_out, sizeof(double) * (3 * bt.B + 1)) != cudaSuccess)
+    if (!bt.h_out && cudaMallocHost(&bt.h_out, sizeof(double) * (3 * bt.B + 2)) != cudaSuccess)
         return (int)cudaErrorMemoryAllocation;
     for (int attempt = 0; attempt < 5; attempt++) {
         if (!adjoint_arrays(bt, g_h0 != nullptr)) {
@@ -432,8 +456,9 @@ static int loss_grad(Batch& bt, const double* target, double* loss_out, double* 
         }
         const bool measure = bt.run_full && d.cap == 0 && bt.steps > 0;
         if (measure) {
-            forward(bt, bt.steps, false, true);
+            forward(bt, bt.steps, false, true, false);
             cudaMemcpyAsync(bt.h_out + 3 * bt.B, d.need, sizeof(long long), cudaMemcpyDeviceToHost, st);
+            cudaMemcpyAsync(bt.h_out + 3 * bt.B + 1, bt.words + 16 * 7, sizeof(long long), cudaMemcpyDeviceToHost, st);
         } else if (bt.use_graph && bt.steps > 0 && (bt.run_full || bt.K <= 32)) {
             if (!bt.gexec || bt.g_target != target || bt.g_gh0 != g_h0 || bt.g_shape != bt.shape ||
                 bt.g_tape != d.t_diff || bt.g_full != bt.run_full) {
@@ -445,7 +470,7 @@ static int loss_grad(Batch& bt, const double* target, double* loss_out, double* 
                 }
                 if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
                     return (int)cudaGetLastError();
-                queue_loss_grad(bt, target, g_h0);
+                queue_loss_grad(bt, target, g_h0, true);
                 cudaError_t e = cudaStreamEndCapture(st, &graph);
                 if (e != cudaSuccess || !graph) {
                     (void)cudaGetLastError();
@@ -468,14 +493,19 @@ static int loss_grad(Batch& bt, const double* target, double* loss_out, double* 
                 return (int)cudaGetLastError();
             bt.graph_launches++;
         } else {
-            queue_loss_grad(bt, target, g_h0);
+            queue_loss_grad(bt, target, g_h0, false);
         }
         if (cudaStreamSynchronize(st) != cudaSuccess) {
             bt.flows_clear = false;
             return (int)cudaGetLastError();
         }
-        long long need = 0;
+        long long need = 0, gave_up = 0;
         memcpy(&need, bt.h_out + 3 * bt.B, sizeof(need));
+        memcpy(&gave_up, bt.h_out + 3 * bt.B + 1, sizeof(gave_up));
+        if (gave_up) { /* a grid barrier did */
+            bt.flows_clear = false;
+            return (int)cudaErrorUnknown;
+        }
         bt.last_need = need;
         if (!measure && need <= d.cap) {
             if (loss_out)
@@ -547,9 +577,9 @@ extern "C" int cal_sdt_batch_autotune(void* handle, int probe_steps, float* ms)
             best = -1;
             break;
         }
-        sdtb::forward(*bt, probe_steps, false, false);
+        sdtb::forward(*bt, probe_steps, false, false, false);
         cudaEventRecord(e0, bt->st);
-        sdtb::forward(*bt, probe_steps, false, false);
+        sdtb::forward(*bt, probe_steps, false, false, false);
         cudaEventRecord(e1, bt->st);
         cudaEventSynchronize(e1);
         float t = 0.f;

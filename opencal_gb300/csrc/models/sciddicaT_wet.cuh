@@ -128,24 +128,21 @@ static __device__ __forceinline__ long long tape_base(const Dev& d, int t, int n
     return off + n <= d.cap ? off : -1;
 }
 
-static __global__ void __launch_bounds__(T) k_outflows(const __grid_constant__ Dev d, int t, int epoch, int taped)
+static __device__ __forceinline__ int add(int* count, int v) { return atomicAdd(count, v); }
+static __device__ __forceinline__ int add(unsigned long long* count, int v)
 {
-    const int n = d.nlist[t];
+    return (int)(unsigned)atomicAdd(count, (unsigned long long)v);
+}
+
+/* the outflows of the n entries of list t, by warp `warp` of `nwarps`; base:
+ * where they go on the tape, or -1; ntiles: counter of the flagged tiles */
+template <typename C>
+static __device__ __forceinline__ void outflows(const Dev& d, int t, int epoch, int n, long long base, C* ntiles,
+                                                int warp, int nwarps)
+{
     const Entry* list = d.list[t & 1];
-    long long base = -1;
-    if (taped) {
-        base = tape_base(d, t, n);
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            const long long end = d.toff[t] + n;
-            d.toff[t + 1] = end;
-            if (*d.need < end) /* one step at a time runs */
-                *d.need = end;
-        }
-    }
     int* tiles = d.tiles + (size_t)t * d.ntiles;
-    /* chunks of 32 entries on consecutive blocks */
-    const int stride = gridDim.x * T;
-    for (int k = ((threadIdx.x >> 5) * (int)gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31); k < n; k += stride) {
+    for (int k = warp * 32 + (threadIdx.x & 31); k < n; k += nwarps * 32) {
         const Entry e = list[k];
         if (base >= 0)
             d.t_entry[base + k] = e;
@@ -187,7 +184,7 @@ static __global__ void __launch_bounds__(T) k_outflows(const __grid_constant__ D
         const bool any = (elim & 0x1eu) != 0x1eu;
         auto flag = [&](int tile) {
             if (atomicExch(d.stamps + tile, epoch) != epoch)
-                tiles[atomicAdd(d.counts + t, 1)] = tile;
+                tiles[add(ntiles, 1)] = tile;
         };
 #pragma unroll
         for (int q = 0; q < 4; q++)
@@ -201,14 +198,46 @@ static __global__ void __launch_bounds__(T) k_outflows(const __grid_constant__ D
     }
 }
 
-/* one entry per thread at most onto the next list, one atomic per block */
-static __device__ __forceinline__ void block_append(bool want, Entry e, Entry* list, int* count, int* s_warp)
+static __global__ void __launch_bounds__(T) k_outflows(const __grid_constant__ Dev d, int t, int epoch, int taped)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n = d.nlist[t];
+    long long base = -1;
+    if (taped) {
+        base = tape_base(d, t, n);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            const long long end = d.toff[t] + n;
+            d.toff[t + 1] = end;
+            if (*d.need < end) /* one step at a time runs */
+                *d.need = end;
+        }
+    }
+    /* chunks of 32 entries on consecutive blocks */
+    outflows(d, t, epoch, n, base, d.counts + t, (threadIdx.x >> 5) * gridDim.x + blockIdx.x, gridDim.x * (T / 32));
+}
+
+/* the update works in groups of T threads: a block of the per-step kernel is
+ * one group, a block of the persistent kernels GROUPS that meet at barriers
+ * of their own */
+template <int NG>
+static __device__ __forceinline__ void group_sync()
+{
+    if (NG == 1)
+        __syncthreads();
+    else
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)(threadIdx.x / T)), "n"(T) : "memory");
+}
+
+/* one entry per thread at most onto the next list, one atomic per group */
+template <int NG, typename C>
+static __device__ __forceinline__ void group_append(bool want, Entry e, Entry* list, C* count)
+{
+    __shared__ int s_warps[NG][T / 32];
+    int* s_warp = s_warps[threadIdx.x / T];
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x % T) >> 5;
     const unsigned m = __ballot_sync(0xffffffffu, want);
     if (lane == 0)
         s_warp[warp] = __popc(m);
-    __syncthreads();
+    group_sync<NG>();
     if (warp == 0) {
         const int v = lane < T / 32 ? s_warp[lane] : 0;
         int incl = v;
@@ -220,29 +249,32 @@ static __device__ __forceinline__ void block_append(bool want, Entry e, Entry* l
         }
         int at = 0;
         if (lane == T / 32 - 1 && incl > 0)
-            at = atomicAdd(count, incl);
+            at = add(count, incl);
         at = __shfl_sync(0xffffffffu, at, T / 32 - 1);
         if (lane < T / 32)
             s_warp[lane] = at + incl - v;
     }
-    __syncthreads();
+    group_sync<NG>();
     if (want)
         list[s_warp[warp] + __popc(m & ((1u << lane) - 1u))] = e;
-    __syncthreads(); /* s_warp is reused */
+    group_sync<NG>(); /* s_warp is reused */
 }
 
-static __global__ void __launch_bounds__(T) k_update(const __grid_constant__ Dev d, int t, int epoch)
+/* the update of step t's ntiles flagged tiles and the next list, whose
+ * counter is `count`, by group `group` of `ngroups` */
+template <int NG, typename C>
+static __device__ __forceinline__ void update(const Dev& d, int t, int epoch, int ntiles, int nlist, C* count,
+                                              int group, int ngroups)
 {
-    __shared__ int s_warp[T / 32];
-    const int ntiles = d.counts[t], nlist = d.nlist[t];
+    const int tid = threadIdx.x % T;
     const int* tiles = d.tiles + (size_t)t * d.ntiles;
     const Entry* cur = d.list[t & 1];
     Entry* next = d.list[(t + 1) & 1];
     const int items = ntiles + (nlist + T - 1) / T;
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+    for (int item = group; item < items; item += ngroups) {
         if (item >= ntiles) {
             /* wet cells of tiles that no flow touched: they stay wet */
-            const int k = (item - ntiles) * T + threadIdx.x;
+            const int k = (item - ntiles) * T + tid;
             bool carry = false;
             Entry e = make_int2(-1, 0);
             if (k < nlist) {
@@ -254,7 +286,7 @@ static __global__ void __launch_bounds__(T) k_update(const __grid_constant__ Dev
                     carry = d.stamps[I.tile0 + (i >> d.lh) * I.tiles_x + (j >> d.lw)] != epoch;
                 }
             }
-            block_append(carry, e, next, d.nlist + t + 1, s_warp);
+            group_append<NG>(carry, e, next, count);
             continue;
         }
         const int tile = tiles[item];
@@ -263,7 +295,7 @@ static __global__ void __launch_bounds__(T) k_update(const __grid_constant__ Dev
         const int lt = tile - I.tile0;
         const int ty = lt / I.tiles_x, tx = lt - ty * I.tiles_x;
         for (int q0 = 0; q0 < 1 << (d.lw + d.lh); q0 += T) {
-            const int q = q0 + threadIdx.x;
+            const int q = q0 + tid;
             const int i = (ty << d.lh) + (q >> d.lw), j = (tx << d.lw) + (q & ((1 << d.lw) - 1));
             bool want = false;
             Entry e = make_int2(-1, bi);
@@ -293,9 +325,14 @@ static __global__ void __launch_bounds__(T) k_update(const __grid_constant__ Dev
                 want = wet || sdt::is_wet(hc, I.eps_bits);
                 e.x = wet ? c : ~c;
             }
-            block_append(want, e, next, d.nlist + t + 1, s_warp);
+            group_append<NG>(want, e, next, count);
         }
     }
+}
+
+static __global__ void __launch_bounds__(T) k_update(const __grid_constant__ Dev d, int t, int epoch)
+{
+    update<1>(d, t, epoch, d.counts[t], d.nlist[t], d.nlist + t + 1, blockIdx.x, gridDim.x);
 }
 
 /* f back to zero after the last step run: the cells wet in step t */
@@ -399,16 +436,12 @@ static __global__ void __launch_bounds__(T) k_relist(const __grid_constant__ Dev
  * adds it to one of COPIES partial sums of the instance (k_fold adds those
  * up).  All on one word per instance and sum, the atomics of a step queued
  * for 30 us (287,000 entries of 64 instances: 48.7 us). */
-static __global__ void __launch_bounds__(T) k_coeffs(const __grid_constant__ Dev d, const __grid_constant__ Adj a, int t)
+static __device__ __forceinline__ void coeffs(const Dev& d, const Adj& a, int t, int n, long long base, int warp,
+                                              int nwarps)
 {
-    const int n = d.nlist[t];
-    const long long base = tape_base(d, t, n);
-    if (base < 0)
-        return;
     const int lane = threadIdx.x & 31;
-    double* sums = a.part + (size_t)(blockIdx.x % COPIES) * 2 * d.B;
-    const int stride = gridDim.x * T;
-    for (int k0 = ((threadIdx.x >> 5) * (int)gridDim.x + blockIdx.x) * 32; k0 < n; k0 += stride) {
+    double* sums = a.part + (size_t)(warp % COPIES) * 2 * d.B;
+    for (int k0 = warp * 32; k0 < n; k0 += nwarps * 32) {
         const int k = k0 + lane;
         const Entry e = k < n ? d.t_entry[base + k] : make_int2(-1, -1);
         const unsigned elim = e.x >= 0 ? d.t_elim[base + k] : 31u;
@@ -466,6 +499,14 @@ static __global__ void __launch_bounds__(T) k_coeffs(const __grid_constant__ Dev
     }
 }
 
+static __global__ void __launch_bounds__(T) k_coeffs(const __grid_constant__ Dev d, const __grid_constant__ Adj a, int t)
+{
+    const int n = d.nlist[t];
+    const long long base = tape_base(d, t, n);
+    if (base >= 0)
+        coeffs(d, a, t, n, base, (threadIdx.x >> 5) * gridDim.x + blockIdx.x, gridDim.x * (T / 32));
+}
+
 /* the instances' dL/dr and dL/deps: their partial sums in a fixed order */
 static __global__ void k_fold(const double* __restrict__ part, double* __restrict__ grad, int n)
 {
@@ -480,18 +521,15 @@ static __global__ void k_fold(const double* __restrict__ part, double* __restric
 
 /* lambda_t from lambda_{t+1}: every cell whose lambda changes lies in a tile
  * that step t flagged (it kept a neighbour or is one that was kept) */
-static __global__ void __launch_bounds__(T) k_gather(const __grid_constant__ Dev d, const __grid_constant__ Adj a, int t)
+static __device__ __forceinline__ void gather(const Dev& d, const Adj& a, int t, int ntiles, int group, int ngroups)
 {
-    if (tape_base(d, t, d.nlist[t]) < 0)
-        return;
-    const int ntiles = d.counts[t];
     const int* tiles = d.tiles + (size_t)t * d.ntiles;
-    for (int item = blockIdx.x; item < ntiles; item += gridDim.x) {
+    for (int item = group; item < ntiles; item += ngroups) {
         const int tile = tiles[item];
         const Inst I = d.inst[d.tile_inst[tile]];
         const int lt = tile - I.tile0;
         const int ty = lt / I.tiles_x, tx = lt - ty * I.tiles_x;
-        for (int q = threadIdx.x; q < 1 << (d.lw + d.lh); q += T) {
+        for (int q = threadIdx.x % T; q < 1 << (d.lw + d.lh); q += T) {
             const int i = (ty << d.lh) + (q >> d.lw), j = (tx << d.lw) + (q & ((1 << d.lw) - 1));
             if (i >= I.rows || j >= I.cols)
                 continue;
@@ -516,6 +554,135 @@ static __global__ void __launch_bounds__(T) k_gather(const __grid_constant__ Dev
             a.lam[c] = a.lam[c] + ((have & 16u) ? a.g[c] : 0.0) + from_nb;
         }
     }
+}
+
+static __global__ void __launch_bounds__(T) k_gather(const __grid_constant__ Dev d, const __grid_constant__ Adj a, int t)
+{
+    if (tape_base(d, t, d.nlist[t]) >= 0)
+        gather(d, a, t, d.counts[t], blockIdx.x, gridDim.x);
+}
+
+/* ---- all steps in one cooperative launch --------------------------------
+ * Launched one after another on a stream, dependent kernels that read their
+ * counts from memory start 4.1 us apart at least (1.2 us as nodes of a
+ * graph); the phases of a step separated by grid barriers of one block of
+ * 1024 threads per SM take 1.45 us each (sciddicaT.cu, sdt2::k_persist), so
+ * runs that are not recorded go this way (one grid of 512 x 480, us per step:
+ * forward 16 -> 10.8, reverse 15 -> 8.0; 40 instances forward 21 -> 17). */
+constexpr int GROUPS = 4, PT = GROUPS * T;
+constexpr unsigned SPIN_LIMIT = 1u << 22;
+
+/* words[16 k]: k = 0, 1, 2 the flagged tiles of steps by t % 3; 3, 4, 5 the
+ * next list's entries; 6 arrivals of the plain barrier; counts in the low 32
+ * bits, a phase's arrivals in the high 32 (words zero at launch); word 7:
+ * not 0 when a wait gave up */
+constexpr int NWORDS = 8;
+
+/* End of a phase: the block's arrival on *word, then the wait for all of
+ * `rounds` x gridDim.x arrivals (a word counted afresh each use: rounds = 1);
+ * bounded, and false for the whole block when it gave up.  *low: the word's
+ * low half when complete. */
+static __device__ __forceinline__ bool phase_end(unsigned long long* word, unsigned rounds, unsigned long long* err,
+                                                 int* low)
+{
+    __shared__ int s_ok, s_low;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(1ull << 32) : "memory");
+        unsigned long long v = 0;
+        int ok = 0;
+        for (unsigned polls = 0; polls < SPIN_LIMIT; polls++) {
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word) : "memory");
+            if ((unsigned)(v >> 32) >= rounds * gridDim.x) {
+                ok = 1;
+                break;
+            }
+            __nanosleep(20);
+        }
+        if (!ok)
+            atomicExch(err, 1ull);
+        s_ok = ok;
+        s_low = (int)(unsigned)v;
+    }
+    __syncthreads();
+    *low = s_low;
+    return s_ok != 0;
+}
+
+/* steps [t0, t1) from list t0 */
+static __global__ void __launch_bounds__(PT, 1) k_steps(const __grid_constant__ Dev d, int t0, int t1, int epoch0,
+                                                       int taped, unsigned long long* words)
+{
+    const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps = gridDim.x * (PT / 32);
+    const int group = (threadIdx.x / T) * gridDim.x + blockIdx.x, ngroups = gridDim.x * GROUPS;
+    int n = d.nlist[t0];
+    long long off = taped ? d.toff[t0] : 0, most = 0;
+    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+    for (int t = t0; t < t1; t++) {
+        unsigned long long* tword = words + 16 * (t % 3);
+        unsigned long long* lword = words + 16 * (3 + t % 3);
+        if (first) {
+            /* the next step's words, last polled two steps ago */
+            words[16 * ((t + 1) % 3)] = 0;
+            words[16 * (3 + (t + 1) % 3)] = 0;
+        }
+        outflows(d, t, epoch0 + t, n, taped && off + n <= d.cap ? off : -1, tword, warp, nwarps);
+        if (taped) {
+            off += n;
+            most = off > most ? off : most;
+            if (first)
+                d.toff[t + 1] = off;
+        }
+        int ntiles;
+        if (!phase_end(tword, 1, words + 16 * 7, &ntiles))
+            return;
+        update<GROUPS>(d, t, epoch0 + t, ntiles, n, lword, group, ngroups);
+        if (first)
+            d.counts[t] = ntiles;
+        if (!phase_end(lword, 1, words + 16 * 7, &n))
+            return;
+        if (first)
+            d.nlist[t + 1] = n;
+    }
+    if (taped && first && *d.need < most)
+        *d.need = most;
+}
+
+/* the adjoint of steps [t0, t1), last first (steps that did not fit the tape
+ * are left out, as by k_coeffs) */
+static __global__ void __launch_bounds__(PT, 1) k_sweep(const __grid_constant__ Dev d, const __grid_constant__ Adj a,
+                                                       int t0, int t1, unsigned long long* words)
+{
+    const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps = gridDim.x * (PT / 32);
+    const int group = (threadIdx.x / T) * gridDim.x + blockIdx.x, ngroups = gridDim.x * GROUPS;
+    unsigned round = 0;
+    int unused;
+    int n = d.nlist[t1 - 1], ntiles = d.counts[t1 - 1];
+    long long base = tape_base(d, t1 - 1, n);
+    for (int t = t1 - 1; t >= t0; t--) {
+        if (base >= 0)
+            coeffs(d, a, t, n, base, warp, nwarps);
+        if (!phase_end(words + 16 * 6, ++round, words + 16 * 7, &unused))
+            return;
+        if (base >= 0)
+            gather(d, a, t, ntiles, group, ngroups);
+        if (t > t0) { /* known since the forward: loaded before the wait */
+            n = d.nlist[t - 1];
+            ntiles = d.counts[t - 1];
+            base = tape_base(d, t - 1, n);
+        }
+        if (!phase_end(words + 16 * 6, ++round, words + 16 * 7, &unused))
+            return;
+    }
+}
+
+/* h into the caller's array; NaN everywhere when a wait gave up */
+static __global__ void k_out(const double* __restrict__ h, double* __restrict__ out, long long n,
+                             const unsigned long long* words)
+{
+    const bool bad = words[16 * 7] != 0;
+    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x)
+        out[c] = bad ? __longlong_as_double(0x7ff8000000000000LL) : h[c];
 }
 
 /* lambda_T = 2 (h_T - target), mu_T the same, and the instances' losses */
@@ -585,6 +752,38 @@ static void queue_adjoint(const Dev& d, const Adj& a, int t0, int t1, cudaStream
         k_coeffs<<<BLOCKS, T, 0, st>>>(d, a, t);
         k_gather<<<BLOCKS, T, 0, st>>>(d, a, t);
     }
+}
+
+static int sm_count()
+{
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    }
+    return sms;
+}
+
+/* as queue_steps, queue_adjoint, in one launch each; words: NWORDS x 16 */
+static bool launch_steps(Dev& d, int t0, int t1, int epoch0, bool taped, unsigned long long* words, cudaStream_t st)
+{
+    if (t1 <= t0)
+        return true;
+    /* word 7, an error of an earlier part of the run, stays */
+    cudaMemsetAsync(words, 0, sizeof(unsigned long long) * 16 * 7, st);
+    int on = taped ? 1 : 0;
+    void* args[] = {&d, &t0, &t1, &epoch0, &on, &words};
+    return cudaLaunchCooperativeKernel((const void*)k_steps, dim3(sm_count()), dim3(PT), args, 0, st) == cudaSuccess;
+}
+
+static bool launch_sweep(Dev& d, Adj& a, int t0, int t1, unsigned long long* words, cudaStream_t st)
+{
+    if (t1 <= t0)
+        return true;
+    cudaMemsetAsync(words, 0, sizeof(unsigned long long) * 16 * 7, st);
+    void* args[] = {&d, &a, &t0, &t1, &words};
+    return cudaLaunchCooperativeKernel((const void*)k_sweep, dim3(sm_count()), dim3(PT), args, 0, st) == cudaSuccess;
 }
 
 } // namespace sdtw
