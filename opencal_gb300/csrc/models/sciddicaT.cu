@@ -1201,13 +1201,21 @@ static int persist_failed(cudaStream_t st)
  * update of the tile from one h buffer into the other.
  *
  * L_t, the tiles of step t, is every tile whose h may change in step t or
- * changed in step t - 1 (so that both buffers agree on every tile left
- * out): a tile holding a wet cell and its four edge neighbours, for the wet
- * cells of both h_{t-1} and h_t.  A tile of L_t that held a wet cell before
- * the step marks itself and its neighbours for L_{t+1} as soon as its h is
- * there, by one warp while the others compute, so that the two atomics of a
- * mark (epoch stamp, append) are off the chain; one that is wet only after
- * the step marks at its end.
+ * changed in step t - 1 (so that both buffers agree on every tile left out).
+ * A cell's outflows depend on its own thickness and its neighbours', so a
+ * flow that was 0 stays 0 unless one of those cells changed: L_{t+1} is
+ * every tile that a flow touched in step t and every tile within two cells of
+ * a cell it touched (by rows plus columns); L_0 the tiles of the wet cells
+ * and their edge neighbours.  Wet tiles at rest drop out: at the end of a
+ * 2048 x 2048 run half of the wet cells are.  A tile that moved in the step
+ * before marks itself and the tiles within three cells for L_{t+1} at once,
+ * by one warp while the others compute, so that the two atomics of a mark
+ * (epoch stamp, append) are off the chain; what it reaches beyond that, it
+ * marks at its end.  Two cells for the early marks measured 12.6 us a step
+ * of the whole 2048 x 2048 run, three 12.7, four 12.8 when the form ended at
+ * 912 tiles, all alike on the smaller grids; against lists of all wet tiles:
+ * 96 x 80 6.5 -> 6.1 us a step, 610 x 496 7.2 -> 7.2, 2048 x 2048 12.7 ->
+ * 12.3, and 46.3 -> 41.6 ms for a flow of which more comes to rest.
  *
  * A block of four groups on every SM (sdt2::k_persist says why); consecutive
  * tiles of the list go to different SMs. */
@@ -1222,8 +1230,8 @@ constexpr int TW = 16, TH = 8;
  * take several tiles one after another and the rings' FP64 work weigh more
  * than the split step's second barrier, so the split step (sdt2::k_persist)
  * does the remaining steps.  2048 x 2048 x 4000, us per step when it ends at
- * 456 / 608 (the groups) / 912 / 1216 tiles / never: 12.9 / 12.6 / 13.1 / 13.7
- * / 15.0; the split step alone 13.1. */
+ * 608 (the groups) / 912 / 1216 tiles: 12.3 / 12.7 / 12.8; the split step
+ * alone 13.1. */
 constexpr int GT = 256, GROUPS = 4, THREADS = GT * GROUPS; /* threads per group, groups per block */
 constexpr int R1W = TW + 2, R1H = TH + 2, R1 = R1W * R1H; /* outflow region */
 constexpr int R2W = TW + 4, R2H = TH + 4, R2 = R2W * R2H; /* load region */
@@ -1235,7 +1243,8 @@ struct Shared {
     /* of the group's current tile; the other set is cleared for the next
      * tile, which may begin while a thread still reads this one */
     struct Flags {
-        int count, any, own, late;
+        int count, any;
+        unsigned reach; /* reach() of the cells that flows touched */
     } flags[2];
 };
 
@@ -1244,6 +1253,7 @@ struct State {
     long long n = 0;
     double* h2 = nullptr;
     int* stamps = nullptr;
+    unsigned long long* moved = nullptr;
     int* list[2] = {nullptr, nullptr};
     unsigned long long* words = nullptr; /* three, 128 bytes apart */
     int* counts = nullptr;               /* [C_ERROR] */
@@ -1256,6 +1266,7 @@ struct Params {
     double* h0;
     double* h1;
     int* stamps;
+    unsigned long long* moved; /* per tile: the epoch of the last step that moved it (high half), its reach then */
     int* list0;
     int* list1;
     unsigned long long* words;
@@ -1292,21 +1303,50 @@ static __device__ __forceinline__ int modi(int x, int n)
     return m < 0 ? m + n : m;
 }
 
-/* tile (ty, tx) moved by direction k (0: itself, 1..4: north, west, east,
- * south) into the next list, once per step */
-static __device__ __forceinline__ void mark(const Params& p, int ty, int tx, int k, int epoch, int* list,
-                                            unsigned long long* word)
+/* tile (y, x) into the next list, once per step */
+static __device__ __forceinline__ void mark_tile(const Params& p, int y, int x, int epoch, int* list,
+                                                 unsigned long long* word)
 {
-    int y = ty + (k == 1 ? -1 : (k == 4 ? 1 : 0)), x = tx + (k == 2 ? -1 : (k == 3 ? 1 : 0));
-    if (p.toroidal) {
-        y = y < 0 ? p.tiles_y - 1 : (y >= p.tiles_y ? 0 : y);
-        x = x < 0 ? p.tiles_x - 1 : (x >= p.tiles_x ? 0 : x);
-    } else if ((unsigned)y >= (unsigned)p.tiles_y || (unsigned)x >= (unsigned)p.tiles_x) {
-        return;
-    }
     const int t = y * p.tiles_x + x;
     if (atomicExch(p.stamps + t, epoch) != epoch)
         list[sdt2::low32(atomicAdd(word, 1ull))] = t;
+}
+
+/* the tile beside (ty, tx) in direction k (0: itself, 1..4: north, west,
+ * east, south, 5..8: north-west, north-east, south-west, south-east) into
+ * the next list; on a toroidal grid a last tile of one row or column has the
+ * tile behind it within the reach of two cells as well */
+static __device__ __forceinline__ void mark(const Params& p, int ty, int tx, int k, int epoch, int* list,
+                                            unsigned long long* word)
+{
+    const int dy = (k == 1 || k == 5 || k == 6) ? -1 : ((k == 4 || k == 7 || k == 8) ? 1 : 0);
+    const int dx = (k == 2 || k == 5 || k == 7) ? -1 : ((k == 3 || k == 6 || k == 8) ? 1 : 0);
+    int y = ty + dy, x = tx + dx;
+    if (!p.toroidal) {
+        if ((unsigned)y < (unsigned)p.tiles_y && (unsigned)x < (unsigned)p.tiles_x)
+            mark_tile(p, y, x, epoch, list, word);
+        return;
+    }
+    y = y < 0 ? p.tiles_y - 1 : (y >= p.tiles_y ? 0 : y);
+    x = x < 0 ? p.tiles_x - 1 : (x >= p.tiles_x ? 0 : x);
+    mark_tile(p, y, x, epoch, list, word);
+    if (k >= 1 && k <= 4 && ((dy && p.rows - y * TH == 1) || (dx && p.cols - x * TW == 1))) {
+        y += dy;
+        x += dx;
+        y = y < 0 ? p.tiles_y - 1 : (y >= p.tiles_y ? 0 : y);
+        x = x < 0 ? p.tiles_x - 1 : (x >= p.tiles_x ? 0 : x);
+        mark_tile(p, y, x, epoch, list, word);
+    }
+}
+
+/* the directions (bit k as in mark) of the tiles within m cells, by rows
+ * plus columns, of cell (a, b) of a tile of hx x wx cells */
+static __device__ __forceinline__ unsigned reach(int a, int b, int hx, int wx, int m)
+{
+    const int n = a, w = b, e = wx - 1 - b, t = hx - 1 - a; /* cells between it and each edge */
+    return 1u | (n < m ? 2u : 0u) | (w < m ? 4u : 0u) | (e < m ? 8u : 0u) | (t < m ? 16u : 0u) |
+           (n + w + 2 <= m ? 32u : 0u) | (n + e + 2 <= m ? 64u : 0u) | (t + w + 2 <= m ? 128u : 0u) |
+           (t + e + 2 <= m ? 256u : 0u);
 }
 
 /* one tile of one step, by the 256 threads of a group */
@@ -1339,28 +1379,32 @@ static __device__ __forceinline__ void tile_step(const Params& p, const double* 
             hv[k] = ld(hin + c);
         }
     }
+    /* the warp with the least left to do marks: where the tile moved in the
+     * step before, it is taken to move again and reach one cell further */
+    unsigned early = 0;
+    if (tid >= GT - 32) {
+        const unsigned long long mv = ld(p.moved + tile);
+        if ((int)(mv >> 32) == epoch - 1)
+            early = (unsigned)mv & 0x1ffu;
+    }
     group_sync(group); /* every thread is done with the tile before */
     if (tid == 0)
-        S.flags[turn ^ 1] = Shared::Flags{0, 0, 0, 0};
+        S.flags[turn ^ 1] = Shared::Flags{0, 0, 0};
 #pragma unroll
     for (int k = 0; k < (R2 + GT - 1) / GT; k++) {
         const int t = tid + k * GT;
         if (t < R2) {
-            const int a = t / R2W, b = t % R2W;
             S.z[t] = zv[k];
             S.h[t] = hv[k];
             S.zh[t] = __double_as_longlong(hv[k]) != 0 ? zv[k] + hv[k] : sdt::plus_zero(zv[k]); /* z + 0.0 */
-            if (sdt::is_wet(hv[k], p.eps_bits)) {
+            if (sdt::is_wet(hv[k], p.eps_bits))
                 F.any = 1;
-                if (a >= 2 && a < TH + 2 && b >= 2 && b < TW + 2 && i0 - 2 + a < p.rows && j0 - 2 + b < p.cols)
-                    F.own = 1;
-            }
         }
     }
     group_sync(group);
-    const bool any = F.any != 0, own = F.own != 0;
-    if (own && tid >= GT - 32 && tid < GT - 27) /* the warp with the least left to do */
-        mark(p, ty, tx, tid - (GT - 32), epoch, next, word);
+    const bool any = F.any != 0;
+    if (early >> (tid & 31) & 1)
+        mark(p, ty, tx, tid & 31, epoch, next, word);
     if (!any) {
         /* changed last step, still now */
         for (int q = tid; q < TW * TH; q += GT) {
@@ -1398,7 +1442,8 @@ static __device__ __forceinline__ void tile_step(const Params& p, const double* 
             S.f[q][t] = f[q];
     }
     group_sync(group);
-    bool late = false;
+    const int hx = min(TH, p.rows - i0), wx = min(TW, p.cols - j0);
+    unsigned dirs = 0; /* low half: one cell further than the high half */
     for (int q = tid; q < TW * TH; q += GT) {
         const int a = q / TW, b = q % TW;
         const int i = i0 + a, j = j0 + b;
@@ -1416,16 +1461,19 @@ static __device__ __forceinline__ void tile_step(const Params& p, const double* 
 #pragma unroll
             for (int n = 0; n < 4; n++)
                 x += in[n] - S.f[n][c];
+            dirs |= reach(a, b, hx, wx, 3) | reach(a, b, hx, wx, 2) << 16;
         }
         hout[(long long)i * p.cols + j] = x;
-        late = late || sdt::is_wet(x, p.eps_bits);
     }
-    if (!own) { /* the same for the whole group */
-        if (late)
-            F.late = 1;
-        group_sync(group);
-        if (F.late && tid < 5)
-            mark(p, ty, tx, tid, epoch, next, word);
+    dirs = __reduce_or_sync(0xffffffffu, dirs);
+    if (dirs && (tid & 31) == 0)
+        atomicOr(&F.reach, dirs);
+    group_sync(group);
+    if (tid >= GT - 32 && F.reach) {
+        if ((F.reach >> 16 & ~early) >> (tid & 31) & 1)
+            mark(p, ty, tx, tid & 31, epoch, next, word);
+        if (tid == GT - 1)
+            p.moved[tile] = (unsigned long long)epoch << 32 | (F.reach & 0x1ffu);
     }
 }
 
@@ -1441,7 +1489,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_persist(const __grid_constant__ 
     if (threadIdx.x == 0)
         s_cnt = sdt2::low32(__ldcg(p.words));
     if (tid < 2)
-        S.flags[tid] = Shared::Flags{0, 0, 0, 0};
+        S.flags[tid] = Shared::Flags{0, 0, 0};
     __syncthreads();
     int n = s_cnt; /* tiles of the current step */
     int turn = 0, s = 0;
@@ -1498,6 +1546,7 @@ static void release()
     State& s = g_state;
     cudaFree(s.h2);
     cudaFree(s.stamps);
+    cudaFree(s.moved);
     cudaFree(s.list[0]);
     cudaFree(s.list[1]);
     cudaFree(s.words);
@@ -1524,7 +1573,7 @@ static bool persist(struct CALModel2D* ca, const double* z, double* h, double ep
         s.tiles_y = (ca->rows + TH - 1) / TH;
         const size_t nt = sizeof(int) * (size_t)s.tiles_x * s.tiles_y;
         if (cudaMalloc(&s.h2, n * sizeof(double)) != cudaSuccess || cudaMalloc(&s.stamps, nt) != cudaSuccess ||
-            cudaMalloc(&s.list[0], nt) != cudaSuccess || cudaMalloc(&s.list[1], nt) != cudaSuccess ||
+            cudaMalloc(&s.moved, 2 * nt) != cudaSuccess || cudaMalloc(&s.list[0], nt) != cudaSuccess || cudaMalloc(&s.list[1], nt) != cudaSuccess ||
             cudaMalloc(&s.words, 48 * sizeof(unsigned long long)) != cudaSuccess ||
             cudaMalloc(&s.counts, NCOUNTS * sizeof(int)) != cudaSuccess) {
             release();
@@ -1546,6 +1595,7 @@ static bool persist(struct CALModel2D* ca, const double* z, double* h, double ep
     p.h0 = h;
     p.h1 = s.h2;
     p.stamps = s.stamps;
+    p.moved = s.moved;
     p.list0 = s.list[0];
     p.list1 = s.list[1];
     p.words = s.words;
@@ -1560,6 +1610,7 @@ static bool persist(struct CALModel2D* ca, const double* z, double* h, double ep
     p.r = r;
     p.eps_bits = eps_bits;
     cudaMemsetAsync(s.stamps, 0, sizeof(int) * (size_t)s.tiles_x * s.tiles_y, st);
+    cudaMemsetAsync(s.moved, 0, sizeof(unsigned long long) * (size_t)s.tiles_x * s.tiles_y, st);
     cudaMemsetAsync(s.words, 0, 48 * sizeof(unsigned long long), st);
     cudaMemsetAsync(s.counts, 0, NCOUNTS * sizeof(int), st);
     const long long blocks = (n + 255) / 256;

@@ -51,6 +51,21 @@ def test_flat_grids_flow_across_the_edges(env, rows, cols, steps):
     assert got.tobytes() == per_step.tobytes()
 
 
+@pytest.mark.parametrize("rows,cols", [(17, 33), (41, 48), (49, 65), (64, 96)])
+@pytest.mark.parametrize("toroidal", [0, 1])
+def test_flows_that_come_to_rest(env, rows, cols, toroidal):
+    """long runs: tiles of wet cells at rest leave the list and come back when
+    a flow arrives, across last tiles of one row or column too"""
+    cal, oracle, _ = env
+    z, h = _inputs(rows, cols, rows + cols)
+    z = z * 0.5
+    h[rows // 4:] = 0.0
+    got = cal.sciddicaT(z, h, 400, toroidal=bool(toroidal), mode=cal.MODE_FUSED, graph=4)[1]
+    per_step = cal.sciddicaT(z, h, 400, toroidal=bool(toroidal), mode=cal.MODE_FUSED, graph=0)[1]
+    assert got.tobytes() == per_step.tobytes()
+    assert got.tobytes() == oracle.sciddicaT(z, h, 400, toroidal=bool(toroidal), ac=False)[1].tobytes()
+
+
 @pytest.mark.parametrize("steps", [60, 61])
 @pytest.mark.parametrize("toroidal", [0, 1])
 def test_flow_outgrows_a_tile_per_group(env, steps, toroidal):
