@@ -1215,7 +1215,7 @@ static int persist_failed(cudaStream_t st)
  * of the whole 2048 x 2048 run, three 12.7, four 12.8 when the form ended at
  * 912 tiles, all alike on the smaller grids; against lists of all wet tiles:
  * 96 x 80 6.5 -> 6.1 us a step, 610 x 496 7.2 -> 7.2, 2048 x 2048 12.7 ->
- * 12.3, and 46.3 -> 41.6 ms for a flow of which more comes to rest.
+ * 12.3.
  *
  * A block of four groups on every SM (sdt2::k_persist says why); consecutive
  * tiles of the list go to different SMs. */
