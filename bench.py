@@ -76,7 +76,8 @@ def launches_per_step(loop):
     return base + (1 if loop == "device" else 0)
 
 
-LAUNCHES_PER_RUN = {"eager": 1, "graph": 1, "device": 1, "persistent": 2}
+# persistent: the priming and the steps of the tile form, then of the split step
+LAUNCHES_PER_RUN = {"eager": 1, "graph": 1, "device": 1, "persistent": 4}
 
 
 def _peaks():
@@ -311,8 +312,9 @@ def gpu_arm(args):
     elif STEP_KERNEL == "single":
         kernel_desc = "SCIDDICA-T dense fused step sdt::fused_step (every tile every step)"
     if args.loop == "persistent":
-        kernel_desc = ("SCIDDICA-T split step, all 4000 steps in one cooperative launch of sdt2::k_persist "
-                       "(K1 and K2 phases separated by grid barriers)")
+        kernel_desc = ("SCIDDICA-T, all 4000 steps in two cooperative launches: sdtp::k_persist (a tile per group, "
+                       "one grid barrier a step) while the tiles in motion are no more than the groups, then "
+                       "sdt2::k_persist (K1 and K2 phases separated by grid barriers)")
     peak, peak_kind = _peaks()
     # the metric's formula: cell-updates/s of the timed runs x 24 B; per step,
     # the runs' event time / 4000 (launch gaps included)
@@ -707,9 +709,9 @@ def calibration_section(args):
             "fd_sample_recovered": fd_traj["recovered"],
             "batched_sample_recovered": batched_on_sample,
         },
-        # one launch of the recorded evaluation; its nodes: forward (init +
-        # one step kernel per step, each taping its tiles), loss; backward
-        # per step: tape restore, coefficients, gather; the result copies
+        # one launch of the recorded evaluation; its nodes: forward (init,
+        # per step the outflows with their tape entries and the update),
+        # loss; backward per step: coefficients, gather; the result copies
         "gpu_launches_per_batched_iter": 1,
         "graph_nodes_per_batched_iter": g_nodes,
         "batched_iter_s_launch_by_launch": batched_eager_s,

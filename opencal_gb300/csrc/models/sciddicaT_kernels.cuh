@@ -1,6 +1,6 @@
 /*
  * sciddicaT_kernels.cuh -- device code of the SCIDDICA-T step shared by the
- * forward paths (sciddicaT.cu) and the adjoint (sciddicaT_adjoint.cu): the
+ * single-grid paths (sciddicaT.cu) and the wet-cell list (sciddicaT_wet.cuh): the
  * wet test, the outflow computation (the reference's minimisation of
  * differences, operation by operation) and the single fused step kernel.
  * Reference: OpenCAL-OMP/examples/calomp_sciddicaT/source/sciddicaT.c:36-100.
@@ -29,9 +29,6 @@ struct Params {
     int toroidal;
     double eps, r;
     long long eps_bits;
-    /* dense step only, optional: per tile (row-major over the launch grid)
-     * bit 0 = a cell of the tile is wet before the step, bit 1 = after */
-    unsigned char* tile_wet = nullptr;
 };
 
 /* h > eps as the reference evaluates `!(h <= eps)`, on the bit pattern:
@@ -155,8 +152,7 @@ static __device__ __forceinline__ void warp_append_shared(bool pred, int value, 
  * the block-uniform result has bit 0 set when a cell of the tile was wet
  * before the step and bit 1 when one is wet after it (0 without TRACK). */
 template <int TW, int TH, bool TRACK = false>
-__device__ __forceinline__ int fused_tile(const Params& p, int i0, int j0, double* smem, bool staged = false,
-                                          unsigned char* elim_tile = nullptr)
+__device__ __forceinline__ int fused_tile(const Params& p, int i0, int j0, double* smem, bool staged = false)
 {
     using T = Tile<TW, TH>;
     double* sz = smem;                      /* [R2H][R2W] */
@@ -267,15 +263,10 @@ __device__ __forceinline__ int fused_tile(const Params& p, int i0, int j0, doubl
         const double u3 = sz[c + 1] + sh[c + 1];
         const double u4 = sz[c + T::R2W] + sh[c + T::R2W];
         double f[4];
-        unsigned elim;
-        outflows(sh[c], sz[c], u1, u2, u3, u4, p.eps, p.r, f, &elim);
+        outflows(sh[c], sz[c], u1, u2, u3, u4, p.eps, p.r, f);
 #pragma unroll
         for (int q = 0; q < 4; q++)
             sf[q * F + t] = f[q];
-        /* the tile's own cells' elimination sets, for an adjoint that
-         * reuses them (elim_tile: TW x TH bytes, row-major) */
-        if (elim_tile && a >= 1 && a <= TH && b >= 1 && b <= TW)
-            elim_tile[(a - 1) * TW + (b - 1)] = (unsigned char)elim;
     }
     __syncthreads();
 
@@ -322,13 +313,7 @@ template <int TW, int TH>
 __global__ void __launch_bounds__(THREADS) fused_step(const __grid_constant__ Params p)
 {
     extern __shared__ __align__(16) double smem[];
-    if (p.tile_wet) {
-        const int wet = fused_tile<TW, TH, true>(p, blockIdx.y * TH, blockIdx.x * TW, smem);
-        if (threadIdx.x == 0)
-            p.tile_wet[blockIdx.y * gridDim.x + blockIdx.x] = (unsigned char)wet;
-    } else {
-        fused_tile<TW, TH>(p, blockIdx.y * TH, blockIdx.x * TW, smem);
-    }
+    fused_tile<TW, TH>(p, blockIdx.y * TH, blockIdx.x * TW, smem);
 }
 
 /* The dense step with z and h staged by TMA: thread 0 arms an mbarrier with
@@ -367,13 +352,7 @@ __global__ void __launch_bounds__(THREADS) fused_step_tma(const __grid_constant_
         __syncthreads();
         return;
     }
-    if (p.tile_wet) {
-        const int wet = fused_tile<TW, TH, true>(p, i0, j0, smem, true);
-        if (threadIdx.x == 0)
-            p.tile_wet[blockIdx.y * gridDim.x + blockIdx.x] = (unsigned char)wet;
-    } else {
-        fused_tile<TW, TH>(p, i0, j0, smem, true);
-    }
+    fused_tile<TW, TH>(p, i0, j0, smem, true);
 }
 
 /* TMA launches queued and blocks whose copies timed out, per translation
