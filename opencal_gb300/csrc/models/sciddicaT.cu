@@ -360,10 +360,12 @@ static __device__ __forceinline__ double ldh(const double* p)
     return CO ? *launder(p) : __ldg(p);
 }
 
-/* flag tile t for this step's K2 and append it to the work-list once */
+/* flag tile t for this step's K2 and append it to the work-list once; with
+ * LOOK, not without a look at the stamp (the caller has not had one) */
+template <bool LOOK>
 static __device__ __forceinline__ void flag_tile(int* tflag, int* tlist, unsigned long long* tcount, int t, int epoch)
 {
-    if (atomicExch(tflag + t, epoch) != epoch)
+    if ((!LOOK || tflag[t] != epoch) && atomicExch(tflag + t, epoch) != epoch)
         tlist[low32(atomicAdd(tcount, 1ull))] = t;
 }
 
@@ -371,13 +373,14 @@ static __device__ __forceinline__ void flag_tile(int* tflag, int* tlist, unsigne
  * the lanes converged here: consecutive wet cells of the list mostly share
  * a tile, so the warp's leader for each tile does the (idempotent) flag
  * and the others skip its atomic */
+template <bool LOOK>
 static __device__ __forceinline__ void flag_tile_warp(bool want, int t, int* tflag, int* tlist,
                                                       unsigned long long* tcount, int epoch)
 {
     const unsigned act = __activemask();
     const unsigned peers = __match_any_sync(act, want ? t : -1);
     if (want && (threadIdx.x & 31) == __ffs(peers) - 1)
-        flag_tile(tflag, tlist, tcount, t, epoch);
+        flag_tile<LOOK>(tflag, tlist, tcount, t, epoch);
 }
 
 /* K1's work on the step's list (threads tid, tid + nthreads, ...): the
@@ -403,8 +406,12 @@ static __device__ __forceinline__ void k1_work(const K1Params& p, int par, int e
         int ni[4] = {i - 1, i, i, i + 1}, nj[4] = {j, j - 1, j + 1, j};
         double u[4];
         /* the receivers' tiles where they differ from the cell's own (which
-         * covers a receiver in it), and the tiles' stamps, loaded here so
-         * that they arrive while the minimisation runs */
+         * covers a receiver in it).  In the persistent kernel, where a step
+         * is one chain of latencies, the tiles' stamps are loaded here so
+         * that they arrive while the minimisation runs; in the per-step
+         * kernel the other blocks on the SM hide that, and a stamp looked at
+         * late saves an atomic more often (4000 launches with active
+         * cells at 2048 x 2048: 98.9 ms early, 94.4 late) */
         const int own = tile_of(i, j, p.tiles_x);
         int rt[4], stamp[4];
 #pragma unroll
@@ -418,7 +425,7 @@ static __device__ __forceinline__ void k1_work(const K1Params& p, int par, int e
                 in = false;
             }
             rt[q] = in ? tile_of(a, b, p.tiles_x) : own;
-            stamp[q] = rt[q] != own ? ldm<CO>(p.tflag + rt[q]) : epoch;
+            stamp[q] = rt[q] == own ? epoch : (CO ? ldm<CO>(p.tflag + rt[q]) : epoch - 1);
             if (in) {
                 /* z + h of the neighbour, as K2 (or the priming) computed it
                  * from the same operands */
@@ -427,7 +434,7 @@ static __device__ __forceinline__ void k1_work(const K1Params& p, int par, int e
                 u[q] = 0.0 + 0.0; /* an absent neighbour reads z = 0, h = 0 */
             }
         }
-        const int own_stamp = ldm<CO>(p.tflag + own);
+        const int own_stamp = CO ? ldm<CO>(p.tflag + own) : epoch - 1;
         double f[4];
         sdt::outflows_u0(ldh<CO>(p.h + c), __ldg(p.zeps + c), u[0], u[1], u[2], u[3], p.eps, p.r, f);
         bool any = false;
@@ -437,10 +444,10 @@ static __device__ __forceinline__ void k1_work(const K1Params& p, int par, int e
             if (__double_as_longlong(f[q]) != 0) {
                 any = true;
                 if (stamp[q] != epoch)
-                    flag_tile(p.tflag, p.tlist, tcount, rt[q], epoch);
+                    flag_tile<!CO>(p.tflag, p.tlist, tcount, rt[q], epoch);
             }
         }
-        flag_tile_warp(any && own_stamp != epoch, own, p.tflag, p.tlist, tcount, epoch);
+        flag_tile_warp<!CO>(any && own_stamp != epoch, own, p.tflag, p.tlist, tcount, epoch);
     }
 }
 
@@ -488,6 +495,16 @@ static __device__ __forceinline__ void warp_append(bool pred, int value, int* li
  * kernel is one group, a block of the persistent kernel GROUPS of them that
  * meet at barriers of their own. */
 template <int GROUPS>
+static __device__ __forceinline__ int group_index()
+{
+    return GROUPS == 1 ? 0 : (int)threadIdx.x / THREADS;
+}
+template <int GROUPS>
+static __device__ __forceinline__ int group_thread()
+{
+    return GROUPS == 1 ? (int)threadIdx.x : (int)threadIdx.x % THREADS;
+}
+template <int GROUPS>
 static __device__ __forceinline__ void group_sync()
 {
     if (GROUPS == 1)
@@ -505,9 +522,9 @@ static __device__ __forceinline__ void block_append4(const bool want[4], const b
 {
     __shared__ int s_warps[GROUPS][2][THREADS / 32];
     __shared__ int s_bases[GROUPS][2];
-    int(*s_warp)[THREADS / 32] = s_warps[threadIdx.x / THREADS];
-    int* s_base = s_bases[threadIdx.x / THREADS];
-    const int lane = threadIdx.x & 31, warp = (threadIdx.x % THREADS) >> 5;
+    int(*s_warp)[THREADS / 32] = s_warps[group_index<GROUPS>()];
+    int* s_base = s_bases[group_index<GROUPS>()];
+    const int lane = threadIdx.x & 31, warp = group_thread<GROUPS>() >> 5;
     const unsigned below = (1u << lane) - 1u;
     unsigned mw[4], md[4];
     int nw = 0, nd = 0;
@@ -523,7 +540,7 @@ static __device__ __forceinline__ void block_append4(const bool want[4], const b
         s_warp[1][warp] = nd;
     }
     group_sync<GROUPS>();
-    if (threadIdx.x % THREADS == 0) {
+    if (group_thread<GROUPS>() == 0) {
         int tw = 0, td = 0;
         for (int w = 0; w < THREADS / 32; w++) {
             tw += s_warp[0][w];
@@ -560,7 +577,7 @@ static __device__ __forceinline__ void k2_tile(const K2Params& p, int tile, int*
      * half the serial FP64 chain per thread) */
     constexpr int CPT = (TW * TH >= 4 * THREADS) ? 4 : ((TW * TH >= 2 * THREADS) ? 2 : 1);
     static_assert((TW / CPT) * TH <= THREADS && TW % CPT == 0, "one group of CPT cells per thread at most");
-    const int tid = threadIdx.x % THREADS;
+    const int tid = group_thread<GROUPS>();
     const int r = tid / (TW / CPT);          /* the tile's row; r >= TH: no cells */
     const int j4 = (tid % (TW / CPT)) * CPT; /* 0, CPT, ..., TW - CPT */
     const bool has = r < TH;
@@ -656,7 +673,7 @@ static __device__ __forceinline__ void k2_work(const K2Params& p, int par, int e
             k2_tile<CO, GROUPS>(p, ldm<CO>(p.tlist + item), list, count);
             group_sync<GROUPS>(); /* block_append4's shared words are reused */
         } else {
-            const int k = (item - ntiles) * THREADS + threadIdx.x % THREADS;
+            const int k = (item - ntiles) * THREADS + group_thread<GROUPS>();
             bool carry = false;
             int c = 0;
             if (k < nlist) {
@@ -1727,6 +1744,7 @@ static __device__ __forceinline__ void warp_append(bool pred, int value, int* li
 
 /* The flows process over the na entries of the active list, in chunks of
  * 32 entries (one per warp): chunks g0, g0 + gs, ... */
+template <bool EARLY>
 static __device__ __forceinline__ void flows_work(const Params& p, int par, int epoch, int na, int g0, int gs)
 {
     int* list = par ? p.list1 : p.list0;
@@ -1743,7 +1761,8 @@ static __device__ __forceinline__ void flows_work(const Params& p, int par, int 
         double u[4];
         /* the neighbours' marks are loaded here, together, so that they
          * arrive while the minimisation runs (one after another behind it:
-         * 11.2 us a step of 1021 x 983 cells against 10.7) */
+         * 11.2 us a step of 1021 x 983 cells against 10.7) in the persistent
+         * kernel; not in the per-step one, as in sdt2::k1_work */
         int nc[4], mark[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) {
@@ -1751,7 +1770,7 @@ static __device__ __forceinline__ void flows_work(const Params& p, int par, int 
             const bool in = nbr(p, i, j, q, a, b);
             nc[q] = a * p.cols + b;
             u[q] = in ? __ldg(p.z + nc[q]) + p.h[nc[q]] : 0.0 + 0.0;
-            mark[q] = in ? p.mark[nc[q]] : epoch;
+            mark[q] = in ? (EARLY ? p.mark[nc[q]] : epoch - 1) : epoch;
         }
         double f[4];
         unsigned elim;
@@ -1760,7 +1779,8 @@ static __device__ __forceinline__ void flows_work(const Params& p, int par, int 
         for (int q = 0; q < 4; q++) {
             p.f[q * p.n + c] = f[q];
             /* calAddActiveCellX2D for every neighbour whose flow is kept */
-            if (!(elim & (2u << q)) && mark[q] != epoch && atomicExch(p.mark + nc[q], epoch) != epoch)
+            if (!(elim & (2u << q)) && mark[q] != epoch && (EARLY || p.mark[nc[q]] != epoch) &&
+                atomicExch(p.mark + nc[q], epoch) != epoch)
                 list[na + atomicAdd(p.counts + C_EXT + par, 1)] = nc[q];
         }
     }
@@ -1810,7 +1830,7 @@ __global__ void __launch_bounds__(THREADS) k1_flows(const __grid_constant__ Para
     const int par = p.counts[C_PAR], epoch = p.counts[C_EPOCH];
     if (blockIdx.x == 0 && threadIdx.x == 0)
         p.counts[1 - par] = 0; /* the list K2 appends to */
-    flows_work(p, par, epoch, p.counts[par], first_chunk(blockIdx.x, gridDim.x), gridDim.x * (THREADS / 32));
+    flows_work<false>(p, par, epoch, p.counts[par], first_chunk(blockIdx.x, gridDim.x), gridDim.x * (THREADS / 32));
 }
 
 __global__ void __launch_bounds__(THREADS) k2_update(const __grid_constant__ Params p)
@@ -1853,7 +1873,7 @@ __global__ void __launch_bounds__(sdt2::PTHREADS, 1) k_persist(const __grid_cons
     for (int s = 0; s < nsteps; s++) {
         if (blockIdx.x == 0 && threadIdx.x == 0)
             p.counts[1 - par] = 0; /* the list the update phase appends to */
-        flows_work(p, par, epoch, na, g0, gs);
+        flows_work<true>(p, par, epoch, na, g0, gs);
         /* then: the extended list's length */
         if (!sdt2::grid_barrier(p.counts, nb, round, p.counts + par, p.counts + C_EXT + par, s_cnt))
             return;
