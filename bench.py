@@ -785,7 +785,7 @@ def sciara_arm(args):
                    "input_generation_s": gen_s, "l2": "no flush: the step touches only the lava cells' tiles"},
         "forward_ms": fw_ms, "forward_runs_ms": fw, "loss_grad_ms": lg_ms,
         "adjoint": {"what": "dL/d(emission rate) of every vent and phase, L = sum (Slt_T - target)^2, "
-                            "decisions frozen, undo tape; loss_grad_ms = forward with tape + adjoint",
+                            "decisions frozen, tape of the visited cells; loss_grad_ms = forward with tape + adjoint",
                     "loss_median": float(np.median(loss)),
                     "grad_abs_max": float(max(np.abs(g).max() for g in grads))},
         "lava_cells_final": lava,
@@ -860,7 +860,7 @@ def adjoint_arm(args):
     """SCIDDICA-T single-grid adjoint: 1024^2, T = 2000 steps, L = sum (h_T -
     h_target)^2 with the target from the run at p_r = 0.42, p_eps = 0.0015,
     gradient with respect to p_r, p_eps and h0 at p_r = 0.5, p_eps = 0.001 by
-    the hand-written adjoint (forward with sqrt(T) checkpoints + reverse
+    the hand-written adjoint (taped forward + reverse
     sweep, csrc/models/sciddicaT_adjoint.cu) through torch.autograd.  One
     bench step = one gradient evaluation; metric cell-updates/s of the
     forward (rows x cols x T per evaluation).  Compared with central finite
@@ -915,7 +915,7 @@ def adjoint_arm(args):
     e1.synchronize()
     fd_ms = e0.elapsed_time(e1)
     # the same loss and gradients by the ensemble engine with one instance:
-    # tile work-lists, so dry regions cost nothing (csrc/models/sciddicaT_batch.cu)
+    # its wet cells' list, so dry regions cost nothing (csrc/models/sciddicaT_batch.cu)
     from opencal_gb300.ensemble import Ensemble
     ens = Ensemble([(ADJ_SIZE, ADJ_SIZE)], [(0.5, 0.001)], [z], [h0], ADJ_STEPS, device=dev)
     tgt = ens.pack([target.cpu().numpy()])
@@ -949,13 +949,13 @@ def adjoint_arm(args):
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": adj_ms, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded DEM + source, seed 3)",
         "config": {"workload": f"SCIDDICA-T adjoint {ADJ_SIZE}^2 FP64, VN, flat, plain, T = {ADJ_STEPS}: one "
-                               "gradient evaluation (forward with sqrt(T) checkpoints + reverse sweep) w.r.t. "
+                               "gradient evaluation (taped forward + reverse sweep) w.r.t. "
                                "p_r, p_eps and h0",
                    "l2": "no flush: 8 MiB grids"},
         "gradient_ms": adj_ms, "gradient_runs_ms": times,
         "fd_gradient_ms": fd_ms, "adjoint_vs_fd_speedup": fd_ms / adj_ms,
         "sparse_engine": {"what": "the same loss and gradients (p_r, p_eps, h0) by the ensemble engine with one "
-                                  "instance (tile work-lists; host-timed, synchronised)",
+                                  "instance (host-timed, synchronised)",
                           "gradient_ms": sparse_ms, "runs_ms": sparse, "loss": float(s_loss[0]),
                           "grad_rel_diff_vs_dense": [abs(s_grad[0, 0] - gr) / max(abs(gr), 1e-300),
                                                      abs(s_grad[0, 1] - ge) / max(abs(ge), 1e-300)]},

@@ -3,7 +3,7 @@
 ``Ensemble`` wraps the ensemble entry points of ``libopencal_models.so``
 (csrc/models/sciddicaT_batch.cu): many independent plain-mode SCIDDICA-T
 instances (flat boundary; each with its own grid size, DEM, source, p_r and
-p_epsilon) advanced by one launch per step over a packed tile work-list, with
+p_epsilon) advanced together over one list of their wet cells, with
 a hand-written adjoint giving every instance's dL/dp_r and dL/dp_eps of
 L = sum (h_T - target)^2 in one backward pass.
 
