@@ -73,14 +73,13 @@ struct Batch {
     /* the loss + gradient evaluation recorded once as a CUDA graph and
      * replayed every call: tape offsets chained on the device, results
      * copied into pinned host memory (h_out: B losses, 2B gradients, then
-     * the tape entries needed and the cooperative launches' error word); valid for the target, dL/dh0 buffer, tile
-     * shape and tape it was recorded with */
+     * the tape entries needed and the cooperative launches' error word); valid
+     * for the target, the dL/dh0 buffer and what the tape holds (dropped with
+     * the tiles and the tape it was recorded with) */
     double* h_out = nullptr; /* pinned: 3B doubles + two long longs */
     cudaGraphExec_t gexec = nullptr;
     const double* g_target = nullptr;
     const double* g_gh0 = nullptr;
-    const void* g_tape = nullptr;
-    int g_shape = -1;
     long long graph_launches = 0;
     long long graph_nodes = 0; /* kernel and copy nodes of the recorded evaluation */
     bool use_graph = true;
@@ -102,10 +101,13 @@ static void drop_graph(Batch& bt)
     bt.gexec = nullptr;
 }
 
-/* a tape of `cap` entries; false when out of memory */
+/* a tape of `cap` entries; false when out of memory.  A recorded evaluation
+ * holds the old arrays and the old capacity in its nodes, and the new arrays
+ * may lie where some of the old ones did: it goes with them. */
 static bool grow_tape(Batch& bt, long long cap)
 {
     Dev& d = bt.d;
+    drop_graph(bt);
     cudaFree(d.t_entry);
     cudaFree(d.t_elim);
     cudaFree(d.t_diff);
@@ -434,11 +436,11 @@ static bool adjoint_arrays(Batch& bt, bool want_mu)
 }
 
 /* One evaluation: as one launch of the recorded graph (recorded again when
- * the target, the dL/dh0 buffer, the tile shape, the tape or what it holds
- * changed), or launch by launch.  When the tape was too small the evaluation
- * is discarded, the tape grown to the size the device reported (plus a
- * quarter) and the evaluation run again; a first call, without a tape, runs
- * the forward alone to learn that size.  In the memory-chosen mode a
+ * the target, the dL/dh0 buffer or what the tape holds changed, or when the
+ * tiles or the tape were allocated again), or launch by launch.  When the
+ * tape was too small the evaluation is discarded, the tape grown to the size
+ * the device reported (plus a quarter) and the evaluation run again; a first
+ * call, without a tape, runs the forward alone to learn that size.  In the memory-chosen mode a
  * whole-rollout tape that would not fit switches the ensemble to segments.
  * Segments of more than 32 steps (rollouts over 1024 steps) are not
  * recorded: six launches a step would make a graph that costs more to
@@ -460,8 +462,7 @@ static int loss_grad(Batch& bt, const double* target, double* loss_out, double* 
             cudaMemcpyAsync(bt.h_out + 3 * bt.B, d.need, sizeof(long long), cudaMemcpyDeviceToHost, st);
             cudaMemcpyAsync(bt.h_out + 3 * bt.B + 1, bt.words + 16 * 7, sizeof(long long), cudaMemcpyDeviceToHost, st);
         } else if (bt.use_graph && bt.steps > 0 && (bt.run_full || bt.K <= 32)) {
-            if (!bt.gexec || bt.g_target != target || bt.g_gh0 != g_h0 || bt.g_shape != bt.shape ||
-                bt.g_tape != d.t_diff || bt.g_full != bt.run_full) {
+            if (!bt.gexec || bt.g_target != target || bt.g_gh0 != g_h0 || bt.g_full != bt.run_full) {
                 drop_graph(bt);
                 cudaGraph_t graph = nullptr;
                 if (!bt.flows_clear) { /* the recording must not hold the one-off clear */
@@ -485,8 +486,6 @@ static int loss_grad(Batch& bt, const double* target, double* loss_out, double* 
                     return (int)e;
                 bt.g_target = target;
                 bt.g_gh0 = g_h0;
-                bt.g_shape = bt.shape;
-                bt.g_tape = d.t_diff;
                 bt.g_full = bt.run_full;
             }
             if (cudaGraphLaunch(bt.gexec, st) != cudaSuccess)
