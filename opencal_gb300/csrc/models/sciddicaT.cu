@@ -847,7 +847,8 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_persist(const __grid_constant__
                                                          const __grid_constant__ K2Params b, int nsteps,
                                                          const int* done)
 {
-    nsteps -= *done;
+    if (done)
+        nsteps -= *done;
     if (nsteps <= 0)
         return;
     __shared__ int s_cnt[2];
@@ -945,10 +946,8 @@ static void release()
     s = State();
 }
 
-/* (re)allocate for `ca` and prime from the current h and z (done, nsteps:
- * as for k_prime) */
-static bool prime(struct CALModel2D* ca, double* h, const double* z, double eps, long long eps_bits, cudaStream_t st,
-                  const int* done = nullptr, int nsteps = 0)
+/* the arrays for `ca`; false when out of memory */
+static bool reserve(struct CALModel2D* ca)
 {
     State& s = g_state;
     const long long n = (long long)ca->rows * ca->columns;
@@ -968,10 +967,23 @@ static bool prime(struct CALModel2D* ca, double* h, const double* z, double eps,
         for (int k = 0; k < 2 && ok; k++)
             ok = cudaMalloc(&s.list[k], n * sizeof(int)) == cudaSuccess;
         if (!ok) {
+            (void)cudaGetLastError();
             release();
             return false;
         }
     }
+    return true;
+}
+
+/* (re)allocate for `ca` and prime from the current h and z (done, nsteps:
+ * as for k_prime) */
+static bool prime(struct CALModel2D* ca, double* h, const double* z, double eps, long long eps_bits, cudaStream_t st,
+                  const int* done = nullptr, int nsteps = 0)
+{
+    if (!reserve(ca))
+        return false;
+    State& s = g_state;
+    const long long n = s.n;
     cudaMemsetAsync(s.f, 0, 4 * n * sizeof(double), st);
     cudaMemsetAsync(s.counts, 0, NCOUNTS * sizeof(int), st); /* parity 0, tickets 0 */
     cudaMemsetAsync(s.ctl, 0, NCTL * sizeof(unsigned long long), st); /* empty lists, no flagged tile */
@@ -1066,9 +1078,9 @@ static bool step(struct CALModel2D* ca, const double* z, double* h, double eps, 
     return cudaGetLastError() == cudaSuccess;
 }
 
-/* The steps from *done to nsteps in one cooperative launch of k_persist (a
- * block per SM); false when the launch is refused or a CUDA error is pending.  A barrier that gave up sets counts[C_ERROR], which
- * persist_failed() reports. */
+/* The steps from *done (NULL: 0) to nsteps in one cooperative launch of
+ * k_persist (a block per SM); false when the launch is refused or a CUDA
+ * error is pending.  A barrier that gave up sets counts[C_ERROR]. */
 static bool persist(struct CALModel2D* ca, const double* z, double* h, double eps, double r, long long eps_bits,
                     int nsteps, const int* done, cudaStream_t st)
 {
@@ -1571,14 +1583,10 @@ static void release()
     s = State();
 }
 
-/* Up to `nsteps` steps from h in one cooperative launch (a block per SM), as
- * long as no group has two tiles; *done: where the device finds how many, or
- * NULL when the grid has no more tiles than groups.  False when out
- * of memory, when the launch is refused or a CUDA error is pending.  A
- * barrier that gave up sets counts[C_ERROR], which persist_failed()
- * reports. */
-static bool persist(struct CALModel2D* ca, const double* z, double* h, double eps, double r, long long eps_bits,
-                    int nsteps, const int** done, cudaStream_t st)
+/* the arrays for `ca`, and whether its grid has more tiles than there are
+ * groups (the split step may then have to take over); false when out of
+ * memory */
+static bool reserve(struct CALModel2D* ca, int* grid, bool* more_tiles)
 {
     State& s = g_state;
     const long long n = (long long)ca->rows * ca->columns;
@@ -1590,23 +1598,39 @@ static bool persist(struct CALModel2D* ca, const double* z, double* h, double ep
         s.tiles_y = (ca->rows + TH - 1) / TH;
         const size_t nt = sizeof(int) * (size_t)s.tiles_x * s.tiles_y;
         if (cudaMalloc(&s.h2, n * sizeof(double)) != cudaSuccess || cudaMalloc(&s.stamps, nt) != cudaSuccess ||
-            cudaMalloc(&s.moved, 2 * nt) != cudaSuccess || cudaMalloc(&s.list[0], nt) != cudaSuccess || cudaMalloc(&s.list[1], nt) != cudaSuccess ||
+            cudaMalloc(&s.moved, 2 * nt) != cudaSuccess || cudaMalloc(&s.list[0], nt) != cudaSuccess ||
+            cudaMalloc(&s.list[1], nt) != cudaSuccess ||
             cudaMalloc(&s.words, 48 * sizeof(unsigned long long)) != cudaSuccess ||
             cudaMalloc(&s.counts, NCOUNTS * sizeof(int)) != cudaSuccess) {
+            (void)cudaGetLastError();
             release();
             return false;
         }
     }
-    static int grid = 0;
-    if (!grid) {
-        int dev = 0, sms = 0;
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0, count = 0;
         cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0 || cudaFuncSetAttribute(k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)(GROUPS * sizeof(Shared))) != cudaSuccess)
+        cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+        if (count <= 0 || cudaFuncSetAttribute(k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)(GROUPS * sizeof(Shared))) != cudaSuccess)
             return false;
-        grid = sms;
+        sms = count;
     }
+    *grid = sms;
+    *more_tiles = s.tiles_x * s.tiles_y > GROUPS * sms;
+    return true;
+}
+
+/* Up to `nsteps` steps from h in one cooperative launch (reserve's grid: a
+ * block per SM), as long as no group has two tiles; counts[C_DONE]: how many.
+ * False when the launch is refused or a CUDA error is pending.  A barrier
+ * that gave up sets counts[C_ERROR]. */
+static bool persist(struct CALModel2D* ca, const double* z, double* h, double eps, double r, long long eps_bits,
+                    int nsteps, int grid, cudaStream_t st)
+{
+    State& s = g_state;
+    const long long n = s.n;
     Params p;
     p.z = z;
     p.h0 = h;
@@ -1632,7 +1656,6 @@ static bool persist(struct CALModel2D* ca, const double* z, double* h, double ep
     cudaMemsetAsync(s.counts, 0, NCOUNTS * sizeof(int), st);
     const long long blocks = (n + 255) / 256;
     k_prime<<<(int)(blocks > 152 * 16 ? 152 * 16 : blocks), 256, 0, st>>>(p);
-    *done = s.tiles_x * s.tiles_y > GROUPS * grid ? s.counts + C_DONE : nullptr;
     void* args[] = {&p, &nsteps};
     return cudaLaunchCooperativeKernel((const void*)k_persist, dim3(grid), dim3(THREADS), args,
                                        GROUPS * sizeof(Shared), st) == cudaSuccess;
@@ -2602,10 +2625,19 @@ static int sciddicaT_persist_gave_up(cudaStream_t st)
     return sdtp::persist_failed(st) || sdt2::persist_failed(st);
 }
 
-/* every one of `steps` steps in cooperative launches: tile by tile, then the
- * persistent split step (plain), or the persistent active-cells split step; the state
- * must be initialised.  Returns a CALError code (CAL_ERROR_CUDA also when a
- * grid barrier gave up, which synchronises). */
+static int sciddicaT_persist_error(CALError code)
+{
+    const cudaError_t e = cudaGetLastError();
+    cal::set_error(code, std::string("SCIDDICA-T persistent step: ") +
+                             (code == CAL_ERROR_OUT_OF_MEMORY ? "out of device memory" : cudaGetErrorString(e)));
+    return code;
+}
+
+/* Every one of `steps` steps in cooperative launches: tile by tile, then the
+ * persistent split step (plain; the split step alone where the tile form's
+ * arrays do not fit), or the persistent active-cells split step; the state
+ * must be initialised.  Asynchronous.  A CALError code, which the library's
+ * error is set to; whether a grid barrier gave up is asked for afterwards. */
 static int sciddicaT_persist_steps(struct CALModel2D* ca, int steps, bool fused_ac)
 {
     long long eps_bits;
@@ -2614,7 +2646,7 @@ static int sciddicaT_persist_steps(struct CALModel2D* ca, int steps, bool fused_
     if (fused_ac) {
         sciddicaT_ac_prepare_now(ca);
         if (!sdtac::g_state.primed)
-            return CAL_ERROR_OUT_OF_MEMORY;
+            return sciddicaT_persist_error(CAL_ERROR_OUT_OF_MEMORY);
     } else if (sdt3::g_state.primed && sdt3::g_state.ca == ca) {
         sciddicaT_sparse_resolve(ca); /* h back from the sparse step's buffers */
         sciddicaT_sparse_invalidate();
@@ -2625,16 +2657,23 @@ static int sciddicaT_persist_steps(struct CALModel2D* ca, int steps, bool fused_
     if (fused_ac) {
         ok = sdtac::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, st);
     } else {
-        const int* done = nullptr;
-        ok = sdtp::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, &done, st);
-        if (ok && done)
+        int grid = 0;
+        bool more = true;
+        const bool tiles = sdtp::reserve(ca, &grid, &more);
+        /* everything the run may need before its first step */
+        if ((more || !tiles) && !sdt2::reserve(ca))
+            return sciddicaT_persist_error(CAL_ERROR_OUT_OF_MEMORY);
+        ok = !tiles || sdtp::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, grid, st);
+        if (ok && (more || !tiles)) {
+            const int* done = tiles ? sdtp::g_state.counts + sdtp::C_DONE : nullptr;
             ok = sdt2::prime(ca, h, z, P.epsilon, eps_bits, st, done, steps) &&
                  sdt2::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, done, st);
+        }
         sdt2::g_state.primed = false; /* the split step's lists were not kept in the first part */
     }
-    if (!ok)
-        return !fused_ac && (!sdtp::g_state.h2 || !sdt2::g_state.f) ? CAL_ERROR_OUT_OF_MEMORY : CAL_ERROR_CUDA;
     calMarkCurrentWritten2Dr(ca, Q.h);
+    if (!ok)
+        return sciddicaT_persist_error(CAL_ERROR_CUDA);
     return calGetLastError();
 }
 
@@ -2776,6 +2815,7 @@ struct SdtSession {
     size_t bytes;
     double* snap[6][2]; /* device copies of z, h, f0..f3 (both layers) after init */
     CALbyte* snap_flags;
+    volatile int* gave_up; /* [2], pinned: error words of the persistent kernels */
 };
 
 static struct CALSubstate2Dr* sdt_sub(int k) { return k == 0 ? Q.z : (k == 1 ? Q.h : Q.f[k - 2]); }
@@ -2793,6 +2833,12 @@ extern "C" void* cal_sciddicaT_open(int rows, int cols, int toroidal, int ac, do
     s->bytes = sizeof(double) * (size_t)rows * cols;
     s->ca = calCADef2D(rows, cols, CAL_VON_NEUMANN_NEIGHBORHOOD_2D, toroidal ? CAL_SPACE_TOROIDAL : CAL_SPACE_FLAT,
                        (ac && !s->fused_ac) ? CAL_OPT_ACTIVE_CELLS : CAL_NO_OPT);
+    if (s->ca && cudaMallocHost((void**)&s->gave_up, 2 * sizeof(int)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        calFinalize2D(s->ca);
+        s->ca = nullptr;
+        cal::set_error(CAL_ERROR_OUT_OF_MEMORY, "cal_sciddicaT_open: pinned memory");
+    }
     if (!s->ca) {
         g_fused_ac = false;
         free(s);
@@ -2970,9 +3016,23 @@ extern "C" int cal_sciddicaT_host_run(void* handle, const double* z_host, const 
     calCopySubstateFromHost2Dr(s->ca, Q.h, h_host);
     sciddicaT_step_invalidate();
     calRunInitSimulation2D(s->run); /* the program's init: z -= h at the source, f = 0 */
-    cal_sciddicaT_steps(handle, steps, graph);
+    const int rc = cal_sciddicaT_steps(handle, steps, graph);
+    if (rc != CAL_SUCCESS)
+        return rc;
     sciddicaT_sparse_resolve(s->ca);
+    /* the persistent kernels' error words, read by the wait for the result */
+    s->gave_up[0] = s->gave_up[1] = 0;
+    if (graph == 4) {
+        const int* words[2] = {s->fused_ac ? sdtac::g_state.counts : sdt2::g_state.counts,
+                               s->fused_ac ? nullptr : sdtp::g_state.counts};
+        for (int k = 0; k < 2; k++)
+            if (words[k])
+                cudaMemcpyAsync((void*)&s->gave_up[k], words[k] + sdt2::C_ERROR, sizeof(int), cudaMemcpyDeviceToHost,
+                                (cudaStream_t)calGetStream2D(s->ca));
+    }
     calCopySubstateToHost2Dr(s->ca, Q.h, h_out);
+    if (s->gave_up[0] || s->gave_up[1])
+        cal::set_error(CAL_ERROR_CUDA, "SCIDDICA-T persistent step: a grid barrier gave up");
     return calGetLastError();
 }
 
@@ -3106,6 +3166,7 @@ extern "C" void cal_sciddicaT_close(void* handle)
         for (int l = 0; l < 2; l++)
             cudaFree(s->snap[k][l]);
     cudaFree(s->snap_flags);
+    cudaFreeHost((void*)s->gave_up);
     sdt2::release();
     sdtp::release();
     sdtac::release();
