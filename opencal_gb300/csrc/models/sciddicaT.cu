@@ -2633,10 +2633,23 @@ static int sciddicaT_persist_error(CALError code)
     return code;
 }
 
+/* The steps from which a run on a grid with more tiles than groups starts in
+ * the tile form.  That form, and the split step's lists when it hands over,
+ * are built from the whole grid on every call (25 us and 1 us per 65,000
+ * cells), while the split step goes on with the lists of the call before; so
+ * that this costs a wide flow, which soon outgrows the tile form, a twentieth
+ * of its 13 us a step at most.  us a call of 1 / 16 / 64 steps, 610 x 496:
+ * always the tile form 53 / 160 / 518, by this rule 17 / 176 / 509; 2048 x
+ * 2048: 117 / 342 / 1062 and 21 / 241 / 960. */
+static int sciddicaT_tile_steps(struct CALModel2D* ca)
+{
+    return 40 + (int)((long long)ca->rows * ca->columns / 40000);
+}
+
 /* Every one of `steps` steps in cooperative launches: tile by tile, then the
- * persistent split step (plain; the split step alone where the tile form's
- * arrays do not fit), or the persistent active-cells split step; the state
- * must be initialised.  Asynchronous.  A CALError code, which the library's
+ * persistent split step (plain; the split step alone for a few steps or where
+ * the tile form's arrays do not fit), or the persistent active-cells split
+ * step; the state must be initialised.  Asynchronous.  A CALError code, which the library's
  * error is set to; whether a grid barrier gave up is asked for afterwards. */
 static int sciddicaT_persist_steps(struct CALModel2D* ca, int steps, bool fused_ac)
 {
@@ -2659,17 +2672,20 @@ static int sciddicaT_persist_steps(struct CALModel2D* ca, int steps, bool fused_
     } else {
         int grid = 0;
         bool more = true;
-        const bool tiles = sdtp::reserve(ca, &grid, &more);
+        const bool tiles = sdtp::reserve(ca, &grid, &more) && (!more || steps >= sciddicaT_tile_steps(ca));
         /* everything the run may need before its first step */
         if ((more || !tiles) && !sdt2::reserve(ca))
             return sciddicaT_persist_error(CAL_ERROR_OUT_OF_MEMORY);
-        ok = !tiles || sdtp::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, grid, st);
-        if (ok && (more || !tiles)) {
-            const int* done = tiles ? sdtp::g_state.counts + sdtp::C_DONE : nullptr;
-            ok = sdt2::prime(ca, h, z, P.epsilon, eps_bits, st, done, steps) &&
-                 sdt2::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, done, st);
+        if (tiles) {
+            const int* done = sdtp::g_state.counts + sdtp::C_DONE;
+            ok = sdtp::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, grid, st) &&
+                 (!more || (sdt2::prime(ca, h, z, P.epsilon, eps_bits, st, done, steps) &&
+                            sdt2::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, done, st)));
+            sdt2::g_state.primed = false; /* the split step's lists were not kept in the first part */
+        } else {
+            sciddicaT_split_prepare_now(ca);
+            ok = sdt2::persist(ca, z, h, P.epsilon, P.r, eps_bits, steps, nullptr, st);
         }
-        sdt2::g_state.primed = false; /* the split step's lists were not kept in the first part */
     }
     calMarkCurrentWritten2Dr(ca, Q.h);
     if (!ok)
@@ -2952,6 +2968,8 @@ extern "C" int cal_sciddicaT_set_params(void* handle, double p_r, double p_eps)
 {
     SdtSession* s = (SdtSession*)handle;
     P.r = p_r;
+    if (memcmp(&P.epsilon, &p_eps, sizeof(double)) != 0)
+        sdt2::g_state.primed = false; /* its list of wet cells was made for the other epsilon */
     P.epsilon = p_eps;
     if (s->mode == SDT_MODE_PROCESSES)
         sciddicaT_declare_pure(s->ca); /* the guard holds epsilon's value */
