@@ -155,12 +155,14 @@ static void queue_forward(Work& W, bool keep, cudaStream_t st)
     cudaMemsetAsync(d.nlist, 0, sizeof(int) * (W.steps + 1), st);
     cudaMemsetAsync(d.toff, 0, sizeof(long long), st);
     cudaMemsetAsync(d.need, 0, sizeof(long long), st);
-    cudaMemsetAsync(W.words, 0, sizeof(unsigned long long) * 16 * sdtw::NWORDS, st);
-    if (!W.flows_clear) {
+    const size_t words = sizeof(unsigned long long) * 16 * sdtw::NWORDS;
+    if (!W.flows_clear) { /* before the first run: no outflows, and no run that gave up */
         cudaMemsetAsync(d.f, 0, n * sizeof(sdtw::D4), st);
+        cudaMemsetAsync(W.words, 0, words, st);
         W.flows_clear = true;
     }
-    sdtw::k_init<<<sdtw::dense_blocks(d.N), T, 2 * sizeof(long long), st>>>(d, W.z_dem, W.h0, W.z);
+    sdtw::k_init<<<sdtw::dense_blocks(d.N), T, 2 * sizeof(long long), st>>>(d, W.z_dem, W.h0, W.z, W.words);
+    cudaMemsetAsync(W.words, 0, words, st);
     const int per = keep ? W.K : std::max(1, W.steps);
     for (int t = 0; t < W.steps; t += per) {
         if (keep)

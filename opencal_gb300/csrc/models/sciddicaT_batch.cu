@@ -69,7 +69,9 @@ struct Batch {
     double* loss = nullptr; /* B */
     unsigned long long* words = nullptr; /* of the cooperative launches */
     cudaStream_t st = nullptr;
-    bool flows_clear = false; /* f is zero everywhere */
+    /* f is zero everywhere before a run, but after one that gave up (words
+     * say so, and k_init clears it) */
+    bool flows_clear = false;
     /* the loss + gradient evaluation recorded once as a CUDA graph and
      * replayed every call: tape offsets chained on the device, results
      * copied into pinned host memory (h_out: B losses, 2B gradients, then
@@ -184,6 +186,16 @@ static void queue_adjoint(Batch& bt, Adj& a, int t0, int t1, bool recorded)
         sdtw::launch_sweep(bt.d, a, t0, t1, bt.words, bt.st);
 }
 
+/* before the first run: no outflows, and no run that gave up */
+static void first_state(Batch& bt)
+{
+    if (bt.flows_clear)
+        return;
+    cudaMemsetAsync(bt.d.f, 0, (size_t)bt.d.N * sizeof(sdtw::D4), bt.st);
+    cudaMemsetAsync(bt.words, 0, sizeof(unsigned long long) * 16 * sdtw::NWORDS, bt.st);
+    bt.flows_clear = true;
+}
+
 /* The initial state and `steps` steps from it, queued.  keep: h every K
  * steps into the checkpoints; taped: every step onto the tape (toff[0] = 0,
  * need reset). */
@@ -195,16 +207,13 @@ static void forward(Batch& bt, int steps, bool keep, bool taped, bool recorded)
     cudaMemsetAsync(d.stamps, 0, sizeof(int) * d.ntiles, st);
     cudaMemsetAsync(d.counts, 0, sizeof(int) * (bt.steps + 1), st);
     cudaMemsetAsync(d.nlist, 0, sizeof(int) * (bt.steps + 1), st);
-    cudaMemsetAsync(bt.words, 0, sizeof(unsigned long long) * 16 * sdtw::NWORDS, st);
     if (taped || keep) {
         cudaMemsetAsync(d.toff, 0, sizeof(long long), st);
         cudaMemsetAsync(d.need, 0, sizeof(long long), st);
     }
-    if (!bt.flows_clear) {
-        cudaMemsetAsync(d.f, 0, (size_t)d.N * sizeof(sdtw::D4), st);
-        bt.flows_clear = true;
-    }
-    sdtw::k_init<<<sdtw::dense_blocks(d.N), T, offs, st>>>(d, bt.z_dem, bt.h0, bt.z);
+    first_state(bt);
+    sdtw::k_init<<<sdtw::dense_blocks(d.N), T, offs, st>>>(d, bt.z_dem, bt.h0, bt.z, bt.words);
+    cudaMemsetAsync(bt.words, 0, sizeof(unsigned long long) * 16 * sdtw::NWORDS, st);
     for (int t = 0; t < steps; t += keep ? bt.K : steps) {
         const int t1 = std::min(t + (keep ? bt.K : steps), steps);
         if (keep)
@@ -349,7 +358,7 @@ extern "C" int cal_sdt_batch_set_params(void* handle, const double* params)
 
 /* Forward rollout of every instance (`steps` steps); h_T copied into hT (a
  * device array in the padded layout, or NULL).  Asynchronous on the
- * ensemble's stream. */
+ * ensemble's stream; hT is NaN when a grid barrier gave up. */
 extern "C" int cal_sdt_batch_forward(void* handle, double* hT)
 {
     Batch* bt = (Batch*)handle;
@@ -360,11 +369,17 @@ extern "C" int cal_sdt_batch_forward(void* handle, double* hT)
 }
 
 /* Tiles updated by each step of the last rollout: steps + 1 counts, the last
- * 0 (no step).  Synchronises. */
+ * 0 (no step).  Synchronises; an error when the rollout gave up at a grid
+ * barrier. */
 extern "C" int cal_sdt_batch_active_tiles(void* handle, int* out)
 {
     Batch* bt = (Batch*)handle;
     cudaStreamSynchronize(bt->st);
+    unsigned long long gave_up = 0;
+    if (bt->flows_clear)
+        cudaMemcpy(&gave_up, bt->words + 16 * 7, sizeof(gave_up), cudaMemcpyDeviceToHost);
+    if (gave_up)
+        return (int)cudaErrorUnknown;
     return (int)cudaMemcpy(out, bt->d.counts, sizeof(int) * (bt->steps + 1), cudaMemcpyDeviceToHost);
 }
 
@@ -465,10 +480,7 @@ static int loss_grad(Batch& bt, const double* target, double* loss_out, double* 
             if (!bt.gexec || bt.g_target != target || bt.g_gh0 != g_h0 || bt.g_full != bt.run_full) {
                 drop_graph(bt);
                 cudaGraph_t graph = nullptr;
-                if (!bt.flows_clear) { /* the recording must not hold the one-off clear */
-                    cudaMemsetAsync(d.f, 0, (size_t)d.N * sizeof(sdtw::D4), st);
-                    bt.flows_clear = true;
-                }
+                first_state(bt); /* the recording must not hold the one-off clear */
                 if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
                     return (int)cudaGetLastError();
                 queue_loss_grad(bt, target, g_h0, true);
@@ -501,10 +513,8 @@ static int loss_grad(Batch& bt, const double* target, double* loss_out, double* 
         long long need = 0, gave_up = 0;
         memcpy(&need, bt.h_out + 3 * bt.B, sizeof(need));
         memcpy(&gave_up, bt.h_out + 3 * bt.B + 1, sizeof(gave_up));
-        if (gave_up) { /* a grid barrier did */
-            bt.flows_clear = false;
+        if (gave_up) /* a grid barrier did (the next run clears what it left) */
             return (int)cudaErrorUnknown;
-        }
         bt.last_need = need;
         if (!measure && need <= d.cap) {
             if (loss_out)

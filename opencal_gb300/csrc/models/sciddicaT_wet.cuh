@@ -375,13 +375,20 @@ static __device__ __forceinline__ void each_cell(const Dev& d, long long* s_offs
 }
 
 /* z after the initialisation (z_dem - h0 where h0 > 0), h = h0 with -0 made
- * +0 (the first reference step adds 0.0 to every cell), z + h, and list 0 */
+ * +0 (the first reference step adds 0.0 to every cell), z + h, and list 0.
+ * words: of the run before; one that gave up left outflows in f */
 static __global__ void __launch_bounds__(T) k_init(const __grid_constant__ Dev d, const double* __restrict__ z_dem,
-                                            const double* __restrict__ h0, double* z)
+                                            const double* __restrict__ h0, double* z,
+                                            const unsigned long long* words)
 {
     extern __shared__ long long s_offs[];
+    const bool gave_up = words[16 * 7] != 0;
     each_cell(d, s_offs, [&](long long c, int b, bool inside) {
         bool wet = false;
+        if (gave_up && c < d.N) {
+            const D4 zero = {{0.0, 0.0, 0.0, 0.0}};
+            d.f[c] = zero;
+        }
         if (inside) {
             const double hv = h0[c];
             const double zv = hv > 0.0 ? z_dem[c] - hv : z_dem[c];

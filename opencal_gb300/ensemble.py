@@ -192,7 +192,9 @@ class Ensemble:
 
     def active_tiles(self) -> np.ndarray:
         out = np.zeros(self.steps + 1, dtype=np.int32)
-        self._lib.cal_sdt_batch_active_tiles(self.handle, _ptr(out, C.c_int))
+        rc = self._lib.cal_sdt_batch_active_tiles(self.handle, _ptr(out, C.c_int))
+        if rc:
+            raise CALError(f"cal_sdt_batch_active_tiles failed ({rc})")
         return out
 
     def autotune(self, probe_steps: int = 50):

@@ -14,6 +14,9 @@ int fake_malloc_at = -1;  /* the n-th cudaMalloc from now is refused (once) */
 int fake_launch_at = -1;  /* the n-th cooperative launch from now is refused (once); -2: all */
 int fake_read4 = 0;       /* 4-byte asynchronous reads return 1 */
 int fake_launches = 0;    /* cooperative launches asked for */
+int fake_cut_at = -1;     /* the n-th cooperative launch from now, one of sdtw::k_steps (Dev, t0, t1, epoch0, taped,
+                           * words), runs the first half of its steps and leaves word 7 as after a barrier that gave
+                           * up (once) */
 
 cudaError_t cudaMalloc(void** p, size_t bytes)
 {
@@ -35,6 +38,14 @@ cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3 grid, dim3 block, vo
     fake_launches++;
     if (fake_launch_at == -2 || (fake_launch_at >= 0 && fake_launch_at-- == 0))
         grid.x *= 1024;
+    if (fake_cut_at >= 0 && fake_cut_at-- == 0) {
+        const int t0 = *(int*)args[1], t1 = *(int*)args[2];
+        int half = (t0 + t1) / 2;
+        void* cut[6] = {args[0], args[1], &half, args[3], args[4], args[5]};
+        cudaError_t e = real(f, grid, block, cut, smem, st);
+        cudaMemsetAsync(*(char**)args[5] + 8 * 16 * 7, 1, 8, st);
+        return e;
+    }
     return real(f, grid, block, args, smem, st);
 }
 
