@@ -772,25 +772,34 @@ static int sm_count()
     return sms;
 }
 
-/* as queue_steps, queue_adjoint, in one launch each; words: NWORDS x 16 */
-static bool launch_steps(Dev& d, int t0, int t1, int epoch0, bool taped, unsigned long long* words, cudaStream_t st)
+/* As queue_steps, queue_adjoint, in one cooperative launch each (words:
+ * NWORDS x 16), or like them where that is refused: a process that is given
+ * a part of the SMs cannot have a block on each.  (A launch that fails for
+ * another reason leaves an error that the plain launches meet again.) */
+static void launch_steps(Dev& d, int t0, int t1, int epoch0, bool taped, unsigned long long* words, cudaStream_t st)
 {
     if (t1 <= t0)
-        return true;
+        return;
     /* word 7, an error of an earlier part of the run, stays */
     cudaMemsetAsync(words, 0, sizeof(unsigned long long) * 16 * 7, st);
     int on = taped ? 1 : 0;
     void* args[] = {&d, &t0, &t1, &epoch0, &on, &words};
-    return cudaLaunchCooperativeKernel((const void*)k_steps, dim3(sm_count()), dim3(PT), args, 0, st) == cudaSuccess;
+    if (cudaLaunchCooperativeKernel((const void*)k_steps, dim3(sm_count()), dim3(PT), args, 0, st) != cudaSuccess) {
+        (void)cudaGetLastError();
+        queue_steps(d, t0, t1, epoch0, taped, st);
+    }
 }
 
-static bool launch_sweep(Dev& d, Adj& a, int t0, int t1, unsigned long long* words, cudaStream_t st)
+static void launch_sweep(Dev& d, Adj& a, int t0, int t1, unsigned long long* words, cudaStream_t st)
 {
     if (t1 <= t0)
-        return true;
+        return;
     cudaMemsetAsync(words, 0, sizeof(unsigned long long) * 16 * 7, st);
     void* args[] = {&d, &a, &t0, &t1, &words};
-    return cudaLaunchCooperativeKernel((const void*)k_sweep, dim3(sm_count()), dim3(PT), args, 0, st) == cudaSuccess;
+    if (cudaLaunchCooperativeKernel((const void*)k_sweep, dim3(sm_count()), dim3(PT), args, 0, st) != cudaSuccess) {
+        (void)cudaGetLastError();
+        queue_adjoint(d, a, t0, t1, st);
+    }
 }
 
 } // namespace sdtw
