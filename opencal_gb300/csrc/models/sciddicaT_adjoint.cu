@@ -115,7 +115,8 @@ static size_t carve(Work& W, char* base)
     c.take(&a.stamp, n);
     c.take(&a.w, n);
     c.take(&a.g, n);
-    c.take(&a.part, 2 * sdtw::COPIES);
+    c.take(&a.sums, n);
+    c.take(&a.part, 2 * sdtw::PARTS);
     c.take(&a.grad, 2);
     d.inst = W.inst;
     d.offs = W.offs;
@@ -186,7 +187,7 @@ static void queue_seed(Work& W, const double* gT, cudaStream_t st)
     cudaMemcpyAsync(W.a.lam, gT, b, cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(W.a.mu, gT, b, cudaMemcpyDeviceToDevice, st);
     cudaMemsetAsync(W.a.stamp, 0xff, sizeof(int) * (size_t)W.d.N, st);
-    cudaMemsetAsync(W.a.part, 0, sizeof(double) * 2 * sdtw::COPIES, st);
+    cudaMemsetAsync(W.a.sums, 0, sizeof(double2) * (size_t)W.d.N, st);
 }
 
 /* the reverse sweep recomputing segments from the checkpoints */
@@ -343,7 +344,7 @@ extern "C" int cal_sdt_adj_backward(void* handle, const double* gT, double* g_h0
             return (int)cudaErrorMemoryAllocation;
     }
     sdtw::k_final_grad<<<sdtw::dense_blocks(d.N), sdtadj::T, 0, st>>>(W->h0, W->a.lam, W->a.mu, g_h0, d.N);
-    sdtw::k_fold<<<1, 32, 0, st>>>(W->a.part, W->a.grad, 2);
+    sdtw::queue_grad(d, W->a, st);
     double res[2] = {0.0, 0.0};
     unsigned long long gave_up = 0; /* a grid barrier did */
     cudaMemcpyAsync(res, W->a.grad, sizeof(res), cudaMemcpyDeviceToHost, st);

@@ -24,9 +24,9 @@
  * when it would not fit in device memory the ensemble falls back to sqrt(T)
  * checkpointing: h is stored every K = ceil(sqrt(T)) steps and the backward
  * recomputes one segment at a time from its checkpoint, taping that segment
- * only.  lambda is updated in place in a fixed order; per-instance dL/dp_r
- * and dL/dp_eps are reduced per warp and added with atomics to a few partial
- * sums (so their summation order is not fixed).
+ * only.  lambda is updated in place, and dL/dp_r and dL/dp_eps are added up,
+ * in a fixed order: the gradients repeat bit for bit (the losses, added up
+ * with atomics, need not).
  *
  * The tile shape -- the unit of the update and of the gather -- is chosen by
  * a small autotuner (cal_sdt_batch_autotune): each candidate shape times a
@@ -236,7 +236,7 @@ static void destroy(Batch* bt)
     Adj& a = bt->a;
     void* ptrs[] = {(void*)d.inst, (void*)d.offs, (void*)d.tile_inst, d.h,     d.zh,    d.f,       d.list[0], d.list[1],
                     d.nlist,       d.tiles,       d.counts,           d.stamps, d.t_entry, d.t_elim, d.t_diff,  d.toff,
-                    d.need,        a.lam,         a.mu,               a.stamp, a.w,     a.g,       a.grad,    a.part,
+                    d.need,        a.lam,         a.mu,               a.stamp, a.w,     a.g,       a.grad,    a.part,   a.sums,
                     bt->z_dem,     bt->z,         bt->h0,             bt->ckpt, bt->loss, bt->words};
     for (void* p : ptrs)
         cudaFree(p);
@@ -400,7 +400,6 @@ static void queue_loss_grad(Batch& bt, const double* target, double* g_h0, bool 
     cudaStream_t st = bt.st;
     forward(bt, bt.steps, !bt.run_full, bt.run_full, recorded);
     cudaMemsetAsync(bt.loss, 0, bt.B * sizeof(double), st);
-    cudaMemsetAsync(a.part, 0, 2 * bt.B * sizeof(double) * sdtw::COPIES, st);
     cudaMemsetAsync(a.stamp, 0xff, sizeof(int) * (size_t)d.N, st);
     sdtw::k_loss<<<sdtw::dense_blocks(d.N), T, offs, st>>>(d, a, target, bt.loss);
     if (bt.run_full) {
@@ -422,7 +421,7 @@ static void queue_loss_grad(Batch& bt, const double* target, double* g_h0, bool 
     }
     if (g_h0)
         sdtw::k_final_grad<<<sdtw::dense_blocks(d.N), T, 0, st>>>(bt.h0, a.lam, a.mu, g_h0, d.N);
-    sdtw::k_fold<<<(2 * bt.B + T - 1) / T, T, 0, st>>>(a.part, a.grad, 2 * bt.B);
+    sdtw::queue_grad(d, a, st);
     cudaMemcpyAsync(bt.h_out, bt.loss, bt.B * sizeof(double), cudaMemcpyDeviceToHost, st);
     cudaMemcpyAsync(bt.h_out + bt.B, a.grad, 2 * bt.B * sizeof(double), cudaMemcpyDeviceToHost, st);
     cudaMemcpyAsync(bt.h_out + 3 * bt.B, d.need, sizeof(long long), cudaMemcpyDeviceToHost, st);
@@ -445,8 +444,8 @@ static bool adjoint_arrays(Batch& bt, bool want_mu)
         return false;
     };
     return need(&a.lam, n) && need(&a.stamp, n) && need(&a.w, n) && need(&a.g, n) && need(&a.grad, 2 * (size_t)bt.B) &&
-           need(&a.part, 2 * (size_t)bt.B * sdtw::COPIES) &&
-           need(&bt.loss, (size_t)bt.B) && (!want_mu || need(&a.mu, n)) &&
+           need(&a.part, 2 * (size_t)bt.B * sdtw::PARTS) && need(&a.sums, n) && need(&bt.loss, (size_t)bt.B) &&
+           (!want_mu || need(&a.mu, n)) &&
            (bt.run_full || bt.steps == 0 || need(&bt.ckpt, n * bt.nseg));
 }
 

@@ -26,7 +26,7 @@
  *
  *   k_coeffs    one thread per taped wet cell: g and the four w (the
  *               formulas of sciddicaT_adjoint.cu) beside the step's stamp,
- *               and the sums dL/dr, dL/deps of its instance;
+ *               and its parts of dL/dr and dL/deps;
  *   k_gather    the step's flagged tiles: lambda = lambda + g + the
  *               neighbours' w, in place, in a fixed order (results do not
  *               depend on the order of the list).
@@ -101,10 +101,11 @@ struct Adj {
     int* stamp; /* per cell: step whose coefficients it holds */
     D4* w;
     double* g;
-    double* part; /* COPIES x 2B partial sums of grad */
-    double* grad; /* 2B: dL/dr[0..B), dL/deps[B..2B) */
+    double2* sums; /* per cell: its parts of dL/dr and dL/deps, all steps */
+    double* part;  /* PARTS x 2B: sums of runs of cells */
+    double* grad;  /* 2B: dL/dr[0..B), dL/deps[B..2B) */
 };
-constexpr int COPIES = 32;
+constexpr int PARTS = 64;
 
 /* neighbour q = 0..3 (north, west, east, south) of (i, j); false where a
  * flat grid ends */
@@ -438,71 +439,54 @@ static __global__ void __launch_bounds__(T) k_relist(const __grid_constant__ Dev
 }
 
 /* The coefficients of step t's wet cells and their parts of dL/dr, dL/deps.
- * Neighbouring entries come from a few tiles, so a warp holds a few runs of
- * entries of one instance: a segmented scan sums each run, and its last lane
- * adds it to one of COPIES partial sums of the instance (k_fold adds those
- * up).  All on one word per instance and sum, the atomics of a step queued
- * for 30 us (287,000 entries of 64 instances: 48.7 us). */
+ * A cell adds its parts to sums of its own, which are added up after the last
+ * step in a fixed order (k_parts, k_fold), so that the gradients repeat bit
+ * for bit whatever order the lists were appended in, and no atomics queue on
+ * an instance's two words (287,000 entries of 64 instances, all on one word
+ * per instance and sum: 48.7 us a step). */
 static __device__ __forceinline__ void coeffs(const Dev& d, const Adj& a, int t, int n, long long base, int warp,
                                               int nwarps)
 {
-    const int lane = threadIdx.x & 31;
-    double* sums = a.part + (size_t)(warp % COPIES) * 2 * d.B;
-    for (int k0 = warp * 32; k0 < n; k0 += nwarps * 32) {
-        const int k = k0 + lane;
-        const Entry e = k < n ? d.t_entry[base + k] : make_int2(-1, -1);
+    for (int k = warp * 32 + (int)(threadIdx.x & 31); k < n; k += nwarps * 32) {
+        const Entry e = d.t_entry[base + k];
         const unsigned elim = e.x >= 0 ? d.t_elim[base + k] : 31u;
         const int kk = 5 - __popc(elim);
-        double er = 0.0, ee = 0.0;
-        if (kk > 0) {
-            const int c = e.x;
-            const Inst I = d.inst[e.y];
-            const int lc = (int)(c - I.off);
-            const int i = lc / I.cols, j = lc - i * I.cols;
-            const D4 diff = d.t_diff[base + k];
-            const double own = a.lam[c];
-            double S = 0.0, lf[4];
+        if (kk == 0)
+            continue;
+        const int c = e.x;
+        const Inst I = d.inst[e.y];
+        const int lc = (int)(c - I.off);
+        const int i = lc / I.cols, j = lc - i * I.cols;
+        const D4 diff = d.t_diff[base + k];
+        const double own = a.lam[c];
+        double2 sum = a.sums[c];
+        double S = 0.0, lf[4], er = 0.0;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                lf[q] = 0.0;
-                if (!(elim & (2u << q))) {
-                    int na, nb;
-                    const bool in = nbr(I, i, j, q, &na, &nb);
-                    lf[q] = (in ? a.lam[I.off + (long long)na * I.cols + nb] : 0.0) - own;
-                    S += lf[q];
-                    er += lf[q] * diff.v[q];
-                }
-            }
-            const double g = cal_div_small(I.r, kk) * S; /* exact division by 1..5 on the integer pipe */
-            D4 w;
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                w.v[q] = (elim & (2u << q)) ? 0.0 : g - I.r * lf[q];
-            a.stamp[c] = t;
-            a.g[c] = g;
-            a.w[c] = w;
-            if (elim & 1u) {
-                ee = -cal_div_small(S * I.r, kk);
-                if (a.mu)
-                    a.mu[c] += g;
+        for (int q = 0; q < 4; q++) {
+            lf[q] = 0.0;
+            if (!(elim & (2u << q))) {
+                int na, nb;
+                const bool in = nbr(I, i, j, q, &na, &nb);
+                lf[q] = (in ? a.lam[I.off + (long long)na * I.cols + nb] : 0.0) - own;
+                S += lf[q];
+                er += lf[q] * diff.v[q];
             }
         }
-        const int before = __shfl_up_sync(0xffffffffu, e.y, 1); /* every lane takes part */
-        const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || before != e.y);
-        const int head = 31 - __clz(heads & (0xffffffffu >> (31 - lane))); /* first lane of this lane's run */
+        const double g = cal_div_small(I.r, kk) * S; /* exact division by 1..5 on the integer pipe */
+        D4 w;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double r = __shfl_up_sync(0xffffffffu, er, o), p = __shfl_up_sync(0xffffffffu, ee, o);
-            if (lane - o >= head) {
-                er += r;
-                ee += p;
-            }
+        for (int q = 0; q < 4; q++)
+            w.v[q] = (elim & (2u << q)) ? 0.0 : g - I.r * lf[q];
+        a.stamp[c] = t;
+        a.g[c] = g;
+        a.w[c] = w;
+        sum.x += er;
+        if (elim & 1u) {
+            sum.y -= cal_div_small(S * I.r, kk);
+            if (a.mu)
+                a.mu[c] += g;
         }
-        const bool tail = lane == 31 || ((heads >> (lane + 1)) & 1u);
-        if (tail && er != 0.0)
-            atomicAdd(sums + e.y, er);
-        if (tail && ee != 0.0)
-            atomicAdd(sums + d.B + e.y, ee);
+        a.sums[c] = sum;
     }
 }
 
@@ -514,6 +498,36 @@ static __global__ void __launch_bounds__(T) k_coeffs(const __grid_constant__ Dev
         coeffs(d, a, t, n, base, (threadIdx.x >> 5) * gridDim.x + blockIdx.x, gridDim.x * (T / 32));
 }
 
+/* block (p, b): the sums of the p-th run of instance b's cells */
+static __global__ void __launch_bounds__(T) k_parts(const __grid_constant__ Dev d, const __grid_constant__ Adj a)
+{
+    __shared__ double s_sum[2][T / 32];
+    const Inst I = d.inst[blockIdx.y];
+    const long long n = (long long)I.rows * I.cols, per = (n + PARTS - 1) / PARTS;
+    const long long c1 = min(n, per * (blockIdx.x + 1));
+    double r = 0.0, e = 0.0;
+    for (long long c = per * blockIdx.x + threadIdx.x; c < c1; c += T) {
+        const double2 v = a.sums[I.off + c];
+        r += v.x;
+        e += v.y;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        r += __shfl_down_sync(0xffffffffu, r, o);
+        e += __shfl_down_sync(0xffffffffu, e, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        s_sum[0][threadIdx.x >> 5] = r;
+        s_sum[1][threadIdx.x >> 5] = e;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double v = 0.0;
+        for (int w = 0; w < T / 32; w++)
+            v += s_sum[threadIdx.x][w];
+        a.part[(size_t)blockIdx.x * 2 * d.B + threadIdx.x * d.B + blockIdx.y] = v;
+    }
+}
+
 /* the instances' dL/dr and dL/deps: their partial sums in a fixed order */
 static __global__ void k_fold(const double* __restrict__ part, double* __restrict__ grad, int n)
 {
@@ -521,8 +535,8 @@ static __global__ void k_fold(const double* __restrict__ part, double* __restric
     if (q >= n)
         return;
     double v = 0.0;
-    for (int c = 0; c < COPIES; c++)
-        v += part[(size_t)c * n + q];
+    for (int p = 0; p < PARTS; p++)
+        v += part[(size_t)p * n + q];
     grad[q] = v;
 }
 
@@ -692,7 +706,8 @@ static __global__ void k_out(const double* __restrict__ h, double* __restrict__ 
         out[c] = bad ? __longlong_as_double(0x7ff8000000000000LL) : h[c];
 }
 
-/* lambda_T = 2 (h_T - target), mu_T the same, and the instances' losses */
+/* lambda_T = 2 (h_T - target), mu_T the same, the cells' sums 0, and the
+ * instances' losses */
 static __global__ void __launch_bounds__(T) k_loss(const __grid_constant__ Dev d, const __grid_constant__ Adj a,
                                             const double* __restrict__ target, double* loss)
 {
@@ -713,6 +728,7 @@ static __global__ void __launch_bounds__(T) k_loss(const __grid_constant__ Dev d
             a.lam[c] = 2.0 * diff;
             if (a.mu)
                 a.mu[c] = 2.0 * diff;
+            a.sums[c] = make_double2(0.0, 0.0);
         }
         const int b0 = __shfl_sync(0xffffffffu, b, 0);
         if (__all_sync(0xffffffffu, b == b0)) {
@@ -759,6 +775,13 @@ static void queue_adjoint(const Dev& d, const Adj& a, int t0, int t1, cudaStream
         k_coeffs<<<BLOCKS, T, 0, st>>>(d, a, t);
         k_gather<<<BLOCKS, T, 0, st>>>(d, a, t);
     }
+}
+
+/* dL/dr and dL/deps from the cells' sums */
+static void queue_grad(const Dev& d, const Adj& a, cudaStream_t st)
+{
+    k_parts<<<dim3(PARTS, d.B), T, 0, st>>>(d, a);
+    k_fold<<<(2 * d.B + T - 1) / T, T, 0, st>>>(a.part, a.grad, 2 * d.B);
 }
 
 static int sm_count()
