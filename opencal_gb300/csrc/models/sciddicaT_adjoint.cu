@@ -68,7 +68,18 @@ struct Work {
     unsigned long long* words = nullptr; /* of the cooperative launches */
     bool want_tape = true;
     bool flows_clear = false;
+    /* counts the changes of tape and checkpoints; need[1] holds the one that
+     * the last forward to run left its record in (a captured forward may run
+     * after they were changed) */
+    long long record = 0;
 };
+
+__global__ void k_start(long long* toff, long long* need, long long record)
+{
+    toff[0] = 0;
+    need[0] = 0;
+    need[1] = record;
+}
 
 __global__ void k_instance(Inst I, long long n, Inst* inst, long long* offs)
 {
@@ -111,7 +122,7 @@ static size_t carve(Work& W, char* base)
     c.take(&d.tiles, (size_t)d.ntiles * steps);
     c.take(&d.stamps, d.ntiles);
     c.take(&d.toff, steps);
-    c.take(&d.need, 1);
+    c.take(&d.need, 2);
     c.take(&W.words, 16 * sdtw::NWORDS);
     c.take(&a.lam, n);
     c.take(&a.mu, n);
@@ -132,6 +143,8 @@ static void drop_tape(Work& W)
     cudaFree(W.tape);
     W.tape = nullptr;
     W.d.cap = 0;
+    if (!W.ckpt) /* with checkpoints it holds one segment at a time */
+        W.record++;
 }
 
 /* a tape of `entries` entries, instead of the one there was */
@@ -164,21 +177,25 @@ static long long kept_tape(const Work& W)
     return std::max<long long>(1, std::min(states / (long long)sdtw::TAPE_BYTES, (n / 16 + 1024) * W.steps));
 }
 
-/* the rollout from h0 and z_dem, queued: taped, or with checkpoints (keep) */
+/* The rollout from h0 and z_dem, queued: taped, or with checkpoints (keep).
+ * A captured one is not taped: its nodes would keep the address of a tape
+ * that a backward may allocate again. */
 static void queue_forward(Work& W, bool keep, cudaStream_t st)
 {
-    Dev& d = W.d;
+    Dev d = W.d;
     const size_t n = (size_t)d.N;
+    const bool captured = sdtw::capturing(st);
+    if (captured)
+        d.cap = 0;
+    k_start<<<1, 1, 0, st>>>(d.toff, d.need, captured && !keep ? -1 : W.record);
     cudaMemsetAsync(d.stamps, 0, sizeof(int) * d.ntiles, st);
     cudaMemsetAsync(d.counts, 0, sizeof(int) * (W.steps + 1), st);
     cudaMemsetAsync(d.nlist, 0, sizeof(int) * (W.steps + 1), st);
-    cudaMemsetAsync(d.toff, 0, sizeof(long long), st);
-    cudaMemsetAsync(d.need, 0, sizeof(long long), st);
     const size_t words = sizeof(unsigned long long) * 16 * sdtw::NWORDS;
     if (!W.flows_clear) { /* before the first run: no outflows, and no run that gave up */
         cudaMemsetAsync(d.f, 0, n * sizeof(sdtw::D4), st);
         cudaMemsetAsync(W.words, 0, words, st);
-        W.flows_clear = true;
+        W.flows_clear = !captured; /* what is captured has not run yet */
     }
     sdtw::k_init<<<sdtw::dense_blocks(d.N), T, 2 * sizeof(long long), st>>>(d, W.z_dem, W.h0, W.z, W.words);
     cudaMemsetAsync(W.words, 0, words, st);
@@ -192,10 +209,11 @@ static void queue_forward(Work& W, bool keep, cudaStream_t st)
         sdtw::k_clear_flows<<<sdtw::BLOCKS, T, 0, st>>>(d, W.steps - 1);
 }
 
-/* the largest tape any step sequence asked for since the last forward */
-static cudaError_t tape_need(Work& W, long long* need, cudaStream_t st)
+/* need[0]: the largest tape any step sequence asked for since the last
+ * forward; need[1]: that forward's record */
+static cudaError_t tape_need(Work& W, long long need[2], cudaStream_t st)
 {
-    cudaMemcpyAsync(need, W.d.need, sizeof(*need), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(need, W.d.need, 2 * sizeof(*need), cudaMemcpyDeviceToHost, st);
     return cudaStreamSynchronize(st);
 }
 
@@ -280,7 +298,9 @@ extern "C" int cal_sdt_adj_set_tape(void* handle, int on)
 }
 
 /* Forward rollout on device buffers: init (z = z_dem - h0 where h0 > 0),
- * `steps` steps, h_T into hT; the tape kept for the backward. */
+ * `steps` steps, h_T into hT; the tape kept for the backward.  May be
+ * captured into a graph (nothing is allocated then: without a tape from an
+ * earlier forward the backward runs the forward again). */
 extern "C" int cal_sdt_adj_forward(void* handle, const double* z_dem, const double* h0, double p_r, double p_eps,
                                    double* hT, void* stream)
 {
@@ -290,7 +310,7 @@ extern "C" int cal_sdt_adj_forward(void* handle, const double* z_dem, const doub
     W->r = p_r;
     W->eps = p_eps;
     const size_t b = (size_t)d.N * sizeof(double);
-    if (W->want_tape && !d.cap && W->steps > 0) {
+    if (W->want_tape && !d.cap && W->steps > 0 && !sdtw::capturing(st)) {
         /* at most an eighth of the free memory */
         size_t free_b = 0, total_b = 0;
         cudaMemGetInfo(&free_b, &total_b);
@@ -326,25 +346,27 @@ extern "C" int cal_sdt_adj_backward(void* handle, const double* gT, double* g_h0
     Work* W = (Work*)handle;
     cudaStream_t st = (cudaStream_t)stream;
     sdtw::Dev& d = W->d;
-    long long need = 0;
-    cudaError_t e = sdtadj::tape_need(*W, &need, st);
+    long long need[2] = {0, 0};
+    cudaError_t e = sdtadj::tape_need(*W, need, st);
     if (e != cudaSuccess)
         return (int)e;
     bool segments = W->ckpt != nullptr;
-    if (!segments && need > d.cap) {
+    if (!segments && need[0] > d.cap) {
         size_t free_b = 0, total_b = 0;
         cudaMemGetInfo(&free_b, &total_b);
-        segments = (size_t)need * sdtw::TAPE_BYTES > (free_b + (size_t)d.cap * sdtw::TAPE_BYTES) / 2 ||
-                   !sdtadj::make_tape(*W, need);
+        segments = (size_t)need[0] * sdtw::TAPE_BYTES > (free_b + (size_t)d.cap * sdtw::TAPE_BYTES) / 2 ||
+                   !sdtadj::make_tape(*W, need[0]);
         if (segments) {
             if (cudaMalloc(&W->ckpt, (size_t)W->nseg * d.N * sizeof(double)) != cudaSuccess) {
                 (void)cudaGetLastError();
                 W->ckpt = nullptr;
                 return (int)cudaErrorMemoryAllocation;
             }
+            W->record++;
         }
-        sdtadj::queue_forward(*W, segments, st);
     }
+    if (need[1] != W->record)
+        sdtadj::queue_forward(*W, segments, st);
     for (int attempt = 0;; attempt++) {
         sdtadj::queue_seed(*W, gT, st);
         if (!segments) {
@@ -352,11 +374,11 @@ extern "C" int cal_sdt_adj_backward(void* handle, const double* gT, double* g_h0
             break;
         }
         sdtadj::queue_segments(*W, st);
-        if ((e = sdtadj::tape_need(*W, &need, st)) != cudaSuccess)
+        if ((e = sdtadj::tape_need(*W, need, st)) != cudaSuccess)
             return (int)e;
-        if (need <= d.cap)
+        if (need[0] <= d.cap)
             break;
-        if (attempt || !sdtadj::make_tape(*W, need))
+        if (attempt || !sdtadj::make_tape(*W, need[0]))
             return (int)cudaErrorMemoryAllocation;
     }
     sdtw::k_final_grad<<<sdtw::dense_blocks(d.N), sdtadj::T, 0, st>>>(W->h0, W->a.lam, W->a.mu, g_h0, d.N);

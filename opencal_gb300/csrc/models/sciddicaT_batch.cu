@@ -193,7 +193,7 @@ static void first_state(Batch& bt)
         return;
     cudaMemsetAsync(bt.d.f, 0, (size_t)bt.d.N * sizeof(sdtw::D4), bt.st);
     cudaMemsetAsync(bt.words, 0, sizeof(unsigned long long) * 16 * sdtw::NWORDS, bt.st);
-    bt.flows_clear = true;
+    bt.flows_clear = !sdtw::capturing(bt.st); /* what a caller captures has not run yet */
 }
 
 /* The initial state and `steps` steps from it, queued.  keep: h every K

@@ -795,14 +795,25 @@ static int sm_count()
     return sms;
 }
 
+static bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &c) == cudaSuccess && c != cudaStreamCaptureStatusNone;
+}
+
 /* As queue_steps, queue_adjoint, in one cooperative launch each (words:
- * NWORDS x 16), or like them where that is refused: a process that is given
+ * NWORDS x 16), or like them while a caller captures the stream and where
+ * the launch is refused: a process that is given
  * a part of the SMs cannot have a block on each.  (A launch that fails for
  * another reason leaves an error that the plain launches meet again.) */
 static void launch_steps(Dev& d, int t0, int t1, int epoch0, bool taped, unsigned long long* words, cudaStream_t st)
 {
     if (t1 <= t0)
         return;
+    if (capturing(st)) {
+        queue_steps(d, t0, t1, epoch0, taped, st);
+        return;
+    }
     /* word 7, an error of an earlier part of the run, stays */
     cudaMemsetAsync(words, 0, sizeof(unsigned long long) * 16 * 7, st);
     int on = taped ? 1 : 0;
