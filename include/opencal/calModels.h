@@ -93,8 +93,9 @@ void cal_sciddicaT_close(void* session);
 void* cal_sdt_adj_create(int rows, int cols, int steps, int toroidal);
 void cal_sdt_adj_destroy(void* work);
 /* 0: the next forwards leave no tape for a backward (which then runs the
- * forward again); 1 (default): they do */
-int cal_sdt_adj_set_tape(void* work, int on);
+ * forward again); 1 (default): they do; 2: checkpoints, every segment taped
+ * in its turn by the backward */
+int cal_sdt_adj_set_tape(void* work, int mode);
 int cal_sdt_adj_forward(void* work, const double* z_dem, const double* h0, double p_r, double p_eps, double* hT,
                         void* stream);
 int cal_sdt_adj_backward(void* work, const double* dL_dhT, double* dL_dh0, double* dL_dpr, double* dL_dpeps,

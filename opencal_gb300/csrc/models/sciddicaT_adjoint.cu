@@ -66,7 +66,7 @@ struct Work {
     char* slab = nullptr;   /* every array of fixed size, one allocation */
     char* tape = nullptr;
     unsigned long long* words = nullptr; /* of the cooperative launches */
-    bool want_tape = true;
+    bool want_tape = true, want_segments = false;
     bool flows_clear = false;
     /* counts the changes of tape and checkpoints; need[1] holds the one that
      * the last forward to run left its record in (a captured forward may run
@@ -175,6 +175,17 @@ static long long kept_tape(const Work& W)
     const long long n = W.d.N;
     const long long states = (long long)(W.nseg + W.K + 1) * n * (long long)sizeof(double);
     return std::max<long long>(1, std::min(states / (long long)sdtw::TAPE_BYTES, (n / 16 + 1024) * W.steps));
+}
+
+static bool make_checkpoints(Work& W)
+{
+    if (cudaMalloc(&W.ckpt, (size_t)W.nseg * W.d.N * sizeof(double)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        W.ckpt = nullptr;
+        return false;
+    }
+    W.record++;
+    return true;
 }
 
 /* The rollout from h0 and z_dem, queued: taped, or with checkpoints (keep).
@@ -290,10 +301,16 @@ extern "C" void cal_sdt_adj_destroy(void* handle)
 }
 
 /* 0: the next forwards leave no tape (no backward is expected; one that
- * comes all the same runs the forward again); 1 (default): they do */
-extern "C" int cal_sdt_adj_set_tape(void* handle, int on)
+ * comes all the same runs the forward again); 1 (default): they do; 2: they
+ * leave checkpoints, and backwards recompute and tape a segment at a time (a
+ * workspace that has checkpoints stays with them).  1 on a bad mode. */
+extern "C" int cal_sdt_adj_set_tape(void* handle, int mode)
 {
-    ((Work*)handle)->want_tape = on != 0;
+    Work* W = (Work*)handle;
+    if (mode < 0 || mode > 2)
+        return 1;
+    W->want_tape = mode == 1;
+    W->want_segments = mode == 2;
     return 0;
 }
 
@@ -310,7 +327,9 @@ extern "C" int cal_sdt_adj_forward(void* handle, const double* z_dem, const doub
     W->r = p_r;
     W->eps = p_eps;
     const size_t b = (size_t)d.N * sizeof(double);
-    if (W->want_tape && !d.cap && W->steps > 0 && !sdtw::capturing(st)) {
+    if (W->want_segments && !W->ckpt && W->steps > 0 && !sdtw::capturing(st) && !sdtadj::make_checkpoints(*W))
+        return (int)cudaErrorMemoryAllocation;
+    if (W->want_tape && !W->ckpt && !d.cap && W->steps > 0 && !sdtw::capturing(st)) {
         /* at most an eighth of the free memory */
         size_t free_b = 0, total_b = 0;
         cudaMemGetInfo(&free_b, &total_b);
@@ -356,14 +375,8 @@ extern "C" int cal_sdt_adj_backward(void* handle, const double* gT, double* g_h0
         cudaMemGetInfo(&free_b, &total_b);
         segments = (size_t)need[0] * sdtw::TAPE_BYTES > (free_b + (size_t)d.cap * sdtw::TAPE_BYTES) / 2 ||
                    !sdtadj::make_tape(*W, need[0]);
-        if (segments) {
-            if (cudaMalloc(&W->ckpt, (size_t)W->nseg * d.N * sizeof(double)) != cudaSuccess) {
-                (void)cudaGetLastError();
-                W->ckpt = nullptr;
-                return (int)cudaErrorMemoryAllocation;
-            }
-            W->record++;
-        }
+        if (segments && !sdtadj::make_checkpoints(*W))
+            return (int)cudaErrorMemoryAllocation;
     }
     if (need[1] != W->record)
         sdtadj::queue_forward(*W, segments, st);
