@@ -87,8 +87,8 @@ struct Dev {
     double* St;
     double* Msl;
     const unsigned char* Mb;
-    double* fc;   /* 16 doubles per list slot: f[8], f * St[8]; only the positive flows' are written */
-    unsigned char* fmask; /* per lava cell: bit k - 1 = a positive outflow to neighbour k */
+    double* fc;   /* 16 doubles per list slot: f[8], f * St[8]; only those in fmask are written */
+    unsigned char* fmask; /* per lava cell: bit k - 1 = neighbour k must add the outflow to it (k_flows) */
     int2* map;    /* per cell: (epoch, slot) */
     int* recv;    /* per cell: epoch in which it was listed as a receiver */
     int* rlist;   /* cells without lava that receive a flow this step */
@@ -359,6 +359,7 @@ struct Tape {
     int* step_n;    /* all entries */
 };
 constexpr int NVAL = 7;
+constexpr long long EXPONENT = 0x7ff0000000000000LL; /* all ones: infinite or NaN */
 constexpr size_t ENTRY_BYTES = sizeof(int) * 2 + 1 + sizeof(double) * (1 + 16 + NVAL);
 constexpr unsigned char E_FLOW = 1, E_BORDER = 2, E_LAVA = 4, E_SOLID = 8;
 
@@ -398,14 +399,18 @@ __global__ void __launch_bounds__(K1T) k_flows(const __grid_constant__ Dev d, co
             tp.pr[base + k] = F.Pr;
         }
         double* slot = slots + (size_t)k * 16;
-        d.fmask[c] = (unsigned char)(F.F >> 1);
+        /* a flow that is 0 changes nothing where it arrives (update_cell
+         * leaves it out), unless the temperature is not finite: 0 x t is
+         * then NaN, in the model's sum of the receiver too */
+        const unsigned sent = (__double_as_longlong(F.t) & EXPONENT) == EXPONENT ? 0x1feu : F.F;
+        d.fmask[c] = (unsigned char)(sent >> 1);
 #pragma unroll
         for (int q = 1; q < 9; q++) {
-            if (!((F.F >> q) & 1u))
+            if (!((sent >> q) & 1u))
                 continue;
             slot[q - 1] = F.f[q];
             slot[8 + q - 1] = F.f[q] * F.t;
-            if ((F.inside >> q) & 1u) {
+            if ((F.F >> q) & (F.inside >> q) & 1u) {
                 const int cn = (int)F.cn[q];
                 if (!cal_pos(F.h[q]) && d.recv[cn] != epoch && atomicExch(d.recv + cn, epoch) != epoch) {
                     append(d.rlist, d.counts + 11, d.capacity, d.counts + 8, cn);
@@ -440,7 +445,8 @@ static __device__ __forceinline__ void compute_cell(const Dev& d, const double* 
     const unsigned out = me.x == epoch ? d.fmask[x] : 0u;
     /* which neighbours' flows arrive here, and their slots: most of a cell's
      * eight neighbours send nothing, and a zero added changes nothing, so
-     * only the flows there are get loaded and added (16 scenarios of 700 x
+     * only the flows there are (and those of a neighbour whose temperature is
+     * not finite) get loaded and added (16 scenarios of 700 x
      * 768, us a step: 23.3 with all sixteen loads and 24 additions of a cell
      * amid lava, 21.7 so; k_flows, which then stores no zeros, 34.3 and
      * 31.4) */
