@@ -181,6 +181,9 @@ int cal_sciara_batch_read(void* batch, double* z, double* slt, double* st, doubl
  * a limit on the tiles flagged, summed over the steps (0: none) */
 int cal_sciara_batch_loss_grad(void* batch, const double* target, int max_steps, double* loss, double* grad,
                                int* steps_done, long long tape_slots, float* ms);
+/* the most entries the tape of cal_sciara_batch_loss_grad may hold (0: as the
+ * memory allows); a run that needs more is taped and swept in stretches */
+int cal_sciara_batch_set_tape_limit(void* batch, long long entries);
 int cal_sciara_batch_lava_cells(void* batch);
 
 /* ---- mbusu, 3D subsurface flow (OpenCAL/examples/cal_mbusu-glut/source/mbusu.c) ----

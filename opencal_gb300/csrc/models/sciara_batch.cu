@@ -924,6 +924,7 @@ struct Batch {
     double* tgt = nullptr;  /* target, padded layout */
     double* loss = nullptr; /* B */
     int tape_steps = 0, mix_cap = 0;
+    long long tape_limit = 0; /* entries; 0: none */
 };
 
 template <typename T>
@@ -966,12 +967,16 @@ static void free_tape(Batch& bt)
     tp.cap = 0;
 }
 
-/* a tape for `entries` entries (kept when it is large enough already) */
+/* a tape for `entries` entries (kept when it is large enough already); false
+ * when that is more than the caller allows or the memory holds (what there
+ * was is then given up in the second case) */
 static bool grow_tape(Batch& bt, long long entries)
 {
     Tape& tp = bt.tp;
     if (tp.cap >= entries)
         return true;
+    if (bt.tape_limit > 0 && entries > bt.tape_limit)
+        return false;
     free_tape(bt);
     const size_t n = (size_t)entries;
     if (walloc(&tp.cell, n) && walloc(&tp.mask, n) && walloc(&tp.flag, n) && walloc(&tp.pr, n) &&
@@ -1227,10 +1232,10 @@ extern "C" void cal_sciara_batch_destroy(void* handle)
 namespace sci2 {
 
 /* the run from the initial state: calRun2D's loop with the stop condition
- * of Sciara.cpp:177-183 (elapsed time >= emission's end).  With a tape
- * every step's entries are kept. */
-static int forward(Batch* bt, int max_steps, const Tape* tape, std::vector<double>* elapsed_of, int* steps_done,
-                   float* ms)
+ * of Sciara.cpp:177-183 (elapsed time >= emission's end).  With a tape the
+ * entries of the steps from taped_from on are kept. */
+static int forward(Batch* bt, int max_steps, const Tape* tape, int taped_from, std::vector<double>* elapsed_of,
+                   int* steps_done, float* ms)
 {
     Dev& d = bt->d;
     cudaStream_t st = bt->st;
@@ -1248,12 +1253,9 @@ static int forward(Batch* bt, int max_steps, const Tape* tape, std::vector<doubl
     cudaMemcpyAsync(d.counts + 6, &one, sizeof(int), cudaMemcpyHostToDevice, st);
     int blocks = (int)std::min<long long>((bt->N + T - 1) / T, 152 * 16);
     k_prime<<<blocks, T, 0, st>>>(d);
-    Tape tp;
-    memset(&tp, 0, sizeof(tp));
-    if (tape) {
-        tp = *tape;
-        cudaMemsetAsync(tp.used, 0, sizeof(long long), st);
-    }
+    const Tape none = {};
+    if (tape)
+        cudaMemsetAsync(tape->used, 0, sizeof(long long), st);
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -1265,6 +1267,7 @@ static int forward(Batch* bt, int max_steps, const Tape* tape, std::vector<doubl
             elapsed_of->push_back(elapsed);
         /* the phase as the vent process forms it: (unsigned)(elapsed / emission_time) */
         const unsigned phase = (unsigned)(elapsed / (double)bt->emission_time);
+        const Tape& tp = tape && done >= taped_from ? *tape : none;
         k_collect<<<K2_BLOCKS, T, 0, st>>>(d, phase, done > 0);
         k_flows<<<152 * 32, K1T, 0, st>>>(d, tp);
         k_update<<<152 * 32, K1T, 0, st>>>(d, tp, done);
@@ -1312,7 +1315,7 @@ static int run_length(const Batch* bt, int max_steps)
  * loop.  0, or a CALError code (CAL_ERROR_OUT_OF_MEMORY = list overflow). */
 extern "C" int cal_sciara_batch_run(void* handle, int max_steps, int* steps_done, float* ms)
 {
-    return sci2::forward((Batch*)handle, max_steps, nullptr, nullptr, steps_done, ms);
+    return sci2::forward((Batch*)handle, max_steps, nullptr, 0, nullptr, steps_done, ms);
 }
 
 namespace sci2 {
@@ -1328,7 +1331,8 @@ static long long first_tape(const Batch& bt, int steps)
         sum += std::min<long long>(bt.N, 64 + 24LL * std::max(1, bt.nvents) * t);
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
-    return std::max<long long>(4096, std::min<long long>(sum, (long long)(free_b / 4 / ENTRY_BYTES)));
+    sum = std::max<long long>(4096, std::min<long long>(sum, (long long)(free_b / 4 / ENTRY_BYTES)));
+    return bt.tape_limit > 0 ? std::min(sum, bt.tape_limit) : sum;
 }
 
 static int loss_grad(Batch* bt, const double* target, int max_steps, double* loss_out, double* grad_out,
@@ -1353,7 +1357,7 @@ static int loss_grad(Batch* bt, const double* target, int max_steps, double* los
         !walloc(&a.lt, (size_t)bt->N) || !walloc(&a.lz, (size_t)bt->N) ||
         !walloc(&a.side, (size_t)bt->N) || !walloc(&a.diag, (size_t)bt->N) || !walloc(&a.grad, ngrad))
         return OOM;
-    if (!tp.cap && !grow_tape(*bt, first_tape(*bt, steps)) && !grow_tape(*bt, 4096))
+    if (!tp.cap && !grow_tape(*bt, first_tape(*bt, steps)) && !grow_tape(*bt, 1))
         return OOM;
     /* target in the padded layout: an input, copied before the timed region */
     cudaMemsetAsync(bt->tgt, 0, (size_t)bt->N * sizeof(double), st);
@@ -1364,37 +1368,26 @@ static int loss_grad(Batch* bt, const double* target, int max_steps, double* los
         src += n;
     }
     std::vector<double> elapsed_of;
+    std::vector<int> n;
     int done = 0;
+    long long need = 0;
     for (int attempt = 0;; attempt++) {
         elapsed_of.clear();
         cudaEventRecord(e0, st);
-        const int rc = forward(bt, max_steps, &tp, &elapsed_of, &done, nullptr);
+        const int rc = forward(bt, max_steps, &tp, 0, &elapsed_of, &done, nullptr);
         if (rc)
             return rc;
-        long long need = 0;
         int tiles = 0;
+        n.resize(done);
         cudaMemcpy(&need, tp.used, sizeof(need), cudaMemcpyDeviceToHost);
         cudaMemcpy(&tiles, d.counts + 9, sizeof(tiles), cudaMemcpyDeviceToHost);
+        cudaMemcpy(n.data(), tp.step_n, sizeof(int) * done, cudaMemcpyDeviceToHost);
         if (tape_slots > 0 && tiles > tape_slots)
             return OOM; /* the caller's limit */
-        if (need <= tp.cap)
+        if (need <= tp.cap || attempt || !grow_tape(*bt, need))
             break;
-        if (attempt || !grow_tape(*bt, need))
-            return OOM;
     }
-    cudaMemsetAsync(bt->loss, 0, sizeof(double) * bt->B, st);
-    cudaMemsetAsync(a.grad, 0, sizeof(double) * ngrad, st);
-    const size_t offs_bytes = sizeof(long long) * (bt->B + 1);
-    k_bloss<<<(int)std::min<long long>((bt->N + T - 1) / T, 152 * 8), T, offs_bytes, st>>>(d, a, bt->tgt, bt->loss);
-    std::vector<long long> base(done);
-    std::vector<int> nlava(done), n(done);
-    cudaMemcpyAsync(base.data(), tp.step_base, sizeof(long long) * done, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(nlava.data(), tp.step_lava, sizeof(int) * done, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(n.data(), tp.step_n, sizeof(int) * done, cudaMemcpyDeviceToHost, st);
-    cudaStreamSynchronize(st);
-    int most = 1;
-    for (int t = 0; t < done; t++)
-        most = std::max(most, n[t]);
+    const int most = std::max(1, *std::max_element(n.begin(), n.end()));
     if (most > bt->mix_cap) {
         wfree(&a.mix);
         bt->mix_cap = 0;
@@ -1402,16 +1395,55 @@ static int loss_grad(Batch* bt, const double* target, int max_steps, double* los
             return OOM;
         bt->mix_cap = most;
     }
-    for (int t = done - 1; t >= 0; t--) {
-        const int epoch_b = -(t + 1);
-        const unsigned phase = (unsigned)(elapsed_of[t] / bt->emission_time);
-        if (n[t] > 0)
-            k_bcells<<<(n[t] + BT - 1) / BT, BT, 0, st>>>(d, tp, a, base[t], n[t], epoch_b);
-        /* an emitting vent cell is a lava cell of the step */
-        if (nlava[t] > 0)
-            k_bflows<<<(nlava[t] + BT - 1) / BT, BT, offs_bytes, st>>>(d, tp, a, base[t], nlava[t], epoch_b, phase);
+    /* A run whose tape does not fit is taped and swept a stretch of steps at
+     * a time, the last first, each after a forward to its end (no state is
+     * kept: a tape of half the size costs two and a half forwards more) */
+    const bool stretches = need > tp.cap;
+    if (stretches) {
+        long long entries = need;
+        while (entries > most && !grow_tape(*bt, entries))
+            entries /= 2;
+        if (!grow_tape(*bt, std::max<long long>(most, entries)))
+            return OOM;
+    }
+    cudaMemsetAsync(bt->loss, 0, sizeof(double) * bt->B, st);
+    cudaMemsetAsync(a.grad, 0, sizeof(double) * ngrad, st);
+    const size_t offs_bytes = sizeof(long long) * (bt->B + 1);
+    std::vector<long long> base(done);
+    std::vector<int> nlava(done);
+    for (int t1 = done, t0; t1 > 0; t1 = t0) {
+        t0 = 0;
+        if (stretches) {
+            long long room = tp.cap;
+            for (t0 = t1; t0 > 0 && n[t0 - 1] <= room; t0--)
+                room -= n[t0 - 1];
+            const int rc = forward(bt, t1, &tp, t0, nullptr, nullptr, nullptr);
+            if (rc)
+                return rc;
+        }
+        if (t1 == done)
+            k_bloss<<<(int)std::min<long long>((bt->N + T - 1) / T, 152 * 8), T, offs_bytes, st>>>(d, a, bt->tgt,
+                                                                                                   bt->loss);
+        cudaMemcpyAsync(&base[t0], tp.step_base + t0, sizeof(long long) * (t1 - t0), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(&nlava[t0], tp.step_lava + t0, sizeof(int) * (t1 - t0), cudaMemcpyDeviceToHost, st);
+        cudaStreamSynchronize(st);
+        for (int t = t1 - 1; t >= t0; t--) {
+            const int epoch_b = -(t + 1);
+            const unsigned phase = (unsigned)(elapsed_of[t] / bt->emission_time);
+            if (n[t] > 0)
+                k_bcells<<<(n[t] + BT - 1) / BT, BT, 0, st>>>(d, tp, a, base[t], n[t], epoch_b);
+            /* an emitting vent cell is a lava cell of the step */
+            if (nlava[t] > 0)
+                k_bflows<<<(nlava[t] + BT - 1) / BT, BT, offs_bytes, st>>>(d, tp, a, base[t], nlava[t], epoch_b,
+                                                                           phase);
+        }
     }
     cudaEventRecord(e1, st);
+    if (stretches) { /* the run's final state */
+        const int rc = forward(bt, max_steps, nullptr, 0, nullptr, nullptr, nullptr);
+        if (rc)
+            return rc;
+    }
     std::vector<double> grad(ngrad);
     cudaMemcpyAsync(grad.data(), a.grad, sizeof(double) * ngrad, cudaMemcpyDeviceToHost, st);
     if (loss_out)
@@ -1430,6 +1462,21 @@ static int loss_grad(Batch* bt, const double* target, int max_steps, double* los
 
 } // namespace sci2
 
+/* The most entries that loss_grad's tape may hold (0, the default: as many as
+ * the device memory holds); runs that need more are taped in stretches. */
+extern "C" int cal_sciara_batch_set_tape_limit(void* handle, long long entries)
+{
+    Batch* bt = (Batch*)handle;
+    if (entries < 0)
+        return 1; /* CAL_ERROR_INVALID_ARGUMENT */
+    bt->tape_limit = entries;
+    if (entries > 0 && bt->tp.cap > entries) {
+        cudaStreamSynchronize(bt->st);
+        sci2::free_tape(*bt);
+    }
+    return 0;
+}
+
 /* Loss L_b = sum over scenario b of (Slt_T - target)^2 and its gradient
  * with respect to every emission rate, by the adjoint with the forward's
  * decisions frozen.  target: host array, the scenarios' grids back to back
@@ -1437,7 +1484,8 @@ static int loss_grad(Batch* bt, const double* target, int max_steps, double* los
  * order.  tape_slots: a limit on the tiles flagged, summed over the steps
  * (0: none); a run that flags more is an error.  The tape grows to the run:
  * when it proves too small the forward runs once more with a tape of the
- * size it asked for.  The state after the call is the run's final one.  0
+ * size it asked for, and where that does not fit the steps are taped and
+ * swept in stretches.  The state after the call is the run's final one.  0
  * or a CALError code; ms: device time of forward + adjoint. */
 extern "C" int cal_sciara_batch_loss_grad(void* handle, const double* target, int max_steps, double* loss_out,
                                           double* grad_out, int* steps_done, long long tape_slots, float* ms)
