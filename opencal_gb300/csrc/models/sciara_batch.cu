@@ -46,6 +46,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <thread>
 #include <vector>
 
@@ -917,14 +918,15 @@ struct Batch {
     void* allocs[32] = {};
     int nalloc = 0;
     bool primed = false;
-    /* loss_grad's workspace: kept for the next call while it is a small
-     * part of the device's memory (free_work) */
+    /* loss_grad's workspace: kept for the next call while what all handles
+     * keep is a small part of the device's memory (keep_work) */
     Tape tp = {};
     Adj adj = {};
     double* tgt = nullptr;  /* target, padded layout */
     double* loss = nullptr; /* B */
     int tape_steps = 0, mix_cap = 0;
     long long tape_limit = 0; /* entries; 0: none */
+    long long kept = 0;       /* bytes of the workspace in g_kept */
 };
 
 template <typename T>
@@ -988,6 +990,8 @@ static bool grow_tape(Batch& bt, long long entries)
     return false;
 }
 
+static std::atomic<long long> g_kept{0}; /* bytes that handles keep between calls */
+
 static void free_work(Batch& bt)
 {
     free_tape(bt);
@@ -1005,6 +1009,25 @@ static void free_work(Batch& bt)
     wfree(&bt.tgt);
     wfree(&bt.loss);
     bt.tape_steps = bt.mix_cap = 0;
+    g_kept -= bt.kept;
+    bt.kept = 0;
+}
+
+/* the workspace stays for the next call while those of all handles together
+ * take at most a sixteenth of the device's memory; else it is given back */
+static void keep_work(Batch& bt)
+{
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    const long long bytes = bt.tp.cap * (long long)ENTRY_BYTES + (long long)sizeof(double) * 6 * bt.N +
+                            (long long)sizeof(Mix) * bt.mix_cap;
+    const long long before = g_kept.fetch_add(bytes - bt.kept);
+    const long long all = before + bytes - bt.kept;
+    bt.kept = bytes;
+    if (all > (long long)(total_b / 16)) {
+        cudaStreamSynchronize(bt.st);
+        free_work(bt);
+    }
 }
 
 static void destroy(Batch* bt)
@@ -1497,15 +1520,11 @@ extern "C" int cal_sciara_batch_loss_grad(void* handle, const double* target, in
     const int rc = sci2::loss_grad(bt, target, max_steps, loss_out, grad_out, steps_done, tape_slots, ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    /* the workspace stays for the next call while it takes at most a
-     * sixteenth of the device's memory */
-    size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
-    const size_t held = (size_t)bt->tp.cap * sci2::ENTRY_BYTES + sizeof(double) * 6 * (size_t)bt->N +
-                        sizeof(sci2::Mix) * (size_t)bt->mix_cap;
-    if (rc || held > total_b / 16) {
+    if (rc) {
         cudaStreamSynchronize(bt->st);
         sci2::free_work(*bt);
+    } else {
+        sci2::keep_work(*bt);
     }
     return rc;
 }
