@@ -28,9 +28,10 @@
  * in a fixed order: the gradients repeat bit for bit (the losses, added up
  * with atomics, need not).
  *
- * The tile shape -- the unit of the update and of the gather -- is chosen by
- * a small autotuner (cal_sdt_batch_autotune): each candidate shape times a
- * forward probe with CUDA events and the fastest is kept for the ensemble.
+ * The tile shape -- the unit of the update and of the gather -- is 32x8 or
+ * chosen by a small autotuner (cal_sdt_batch_autotune): each candidate shape
+ * times a forward probe with CUDA events and the fastest is kept for the
+ * ensemble.
  */
 #include <math.h>
 #include <stdio.h>
@@ -561,11 +562,13 @@ extern "C" int cal_sdt_batch_loss_grad(void* handle, const double* target, doubl
 }
 
 /* Pick the fastest tile shape for this ensemble: a forward of `probe_steps`
- * steps per candidate (0: 32x16, 1: 64x16, 2: 64x32), timed with CUDA
- * events after one untimed probe.  Writes the milliseconds to ms[0..2]
- * (ms[3..4] = 0) and returns the chosen shape, or -1 on a CUDA error.  The
- * smaller shapes 3 (16x8) and 4 (32x8, an ensemble's shape until another is
- * chosen) are selected by cal_sdt_batch_set_shape. */
+ * steps per candidate (0: 32x16, 1: 64x16, 2: 64x32, 4: 32x8, the shape until
+ * another is chosen), timed with CUDA events after one untimed probe.  (The
+ * recorded evaluation launches other kernels; they rank the shapes alike:
+ * 100 steps of 64 instances, ms, cooperative 2.17 / 2.65 / 3.33 / 2.11,
+ * recorded 2.09 / 2.56 / 3.32 / 2.01.)  Writes the milliseconds to ms[0..2]
+ * and ms[4] (ms[3] = 0) and returns the chosen shape, or -1 on a CUDA error.
+ * Shape 3 (16x8) is selected by cal_sdt_batch_set_shape. */
 extern "C" int cal_sdt_batch_autotune(void* handle, int probe_steps, float* ms)
 {
     Batch* bt = (Batch*)handle;
@@ -579,7 +582,7 @@ extern "C" int cal_sdt_batch_autotune(void* handle, int probe_steps, float* ms)
     for (int s = 0; s < sdtb::NSHAPES; s++)
         if (ms)
             ms[s] = 0.f;
-    for (int s = 0; s < 3; s++) {
+    for (int s : {0, 1, 2, 4}) {
         bt->shape = s;
         if (!sdtb::tiles_for(*bt)) {
             best = -1;

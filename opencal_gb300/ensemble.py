@@ -204,7 +204,7 @@ class Ensemble:
         best = self._lib.cal_sdt_batch_autotune(self.handle, int(probe_steps), ms)
         if best < 0:
             raise CALError("cal_sdt_batch_autotune failed")
-        return SHAPES[best], {SHAPES[k]: float(ms[k]) for k in range(3)}
+        return SHAPES[best], {SHAPES[k]: float(ms[k]) for k in (0, 1, 2, 4)}
 
     def set_shape(self, name: str):
         if self._lib.cal_sdt_batch_set_shape(self.handle, SHAPES.index(name)):
