@@ -132,7 +132,8 @@ static bool grow_tape(Batch& bt, long long cap)
     return true;
 }
 
-/* re-tile every instance for the current shape */
+/* re-tile every instance for the current shape; false when out of memory
+ * (d.tiles is then NULL, and nothing runs until another shape fits) */
 static bool tiles_for(Batch& bt)
 {
     Dev& d = bt.d;
@@ -162,8 +163,12 @@ static bool tiles_for(Batch& bt)
     bool ok = cudaMalloc((void**)&d.tile_inst, sizeof(int) * tinst.size()) == cudaSuccess &&
               cudaMalloc(&d.stamps, sizeof(int) * tinst.size()) == cudaSuccess &&
               cudaMalloc(&d.tiles, sizeof(int) * std::max<size_t>(1, (size_t)d.ntiles * bt.steps)) == cudaSuccess;
-    if (!ok)
+    if (!ok) {
+        (void)cudaGetLastError();
+        cudaFree(d.tiles);
+        d.tiles = nullptr;
         return false;
+    }
     cudaMemcpy((void*)d.tile_inst, tinst.data(), sizeof(int) * tinst.size(), cudaMemcpyHostToDevice);
     cudaMemcpy((void*)d.inst, bt.inst.data(), sizeof(Inst) * bt.B, cudaMemcpyHostToDevice);
     return true;
@@ -363,6 +368,8 @@ extern "C" int cal_sdt_batch_set_params(void* handle, const double* params)
 extern "C" int cal_sdt_batch_forward(void* handle, double* hT)
 {
     Batch* bt = (Batch*)handle;
+    if (!bt->d.tiles)
+        return (int)cudaErrorMemoryAllocation;
     sdtb::forward(*bt, bt->steps, false, false, false);
     if (hT)
         sdtw::k_out<<<sdtw::dense_blocks(bt->d.N), sdtw::T, 0, bt->st>>>(bt->d.h, hT, bt->d.N, bt->words);
@@ -464,7 +471,7 @@ static int loss_grad(Batch& bt, const double* target, double* loss_out, double* 
 {
     Dev& d = bt.d;
     cudaStream_t st = bt.st;
-    if (!bt.h_out && cudaMallocHost(&bt.h_out, sizeof(double) * (3 * bt.B + 2)) != cudaSuccess)
+    if (!d.tiles || (!bt.h_out && cudaMallocHost(&bt.h_out, sizeof(double) * (3 * bt.B + 2)) != cudaSuccess))
         return (int)cudaErrorMemoryAllocation;
     for (int attempt = 0; attempt < 5; attempt++) {
         if (!adjoint_arrays(bt, g_h0 != nullptr)) {
