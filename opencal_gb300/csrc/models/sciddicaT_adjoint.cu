@@ -26,10 +26,10 @@
  *
  * The steps and their adjoint are the wet-cell list's (sciddicaT_wet.cuh)
  * with one instance, in one cooperative launch each way.  The forward tapes
- * the rollout into a tape that takes no more memory than checkpoints every
- * K = ceil(sqrt(T)) steps and the states of a segment between two would (a
- * program may hold many rollouts between their forwards and backwards; 2 % of
- * the cells wet fit in it at 400 steps, 0.6 % at 4000).  The backward first
+ * the rollout into a tape that, where memory matters, takes no more of it than
+ * checkpoints every K = ceil(sqrt(T)) steps and the states of a segment
+ * between two would (kept_tape: a program may hold many rollouts between
+ * their forwards and backwards).  The backward first
  * learns what the tape needed.  When it was too small, the forward runs again
  * with one that fits, given back after the sweep, or, when that would take
  * more than half of the free device memory, with h stored every K steps, and
@@ -68,6 +68,7 @@ struct Work {
     unsigned long long* words = nullptr; /* of the cooperative launches */
     bool want_tape = true, want_segments = false;
     bool flows_clear = false;
+    long long kept = 0; /* entries of the tape kept after a backward */
     /* counts the changes of tape and checkpoints; need[1] holds the one that
      * the last forward to run left its record in (a captured forward may run
      * after they were changed) */
@@ -167,14 +168,21 @@ static bool make_tape(Work& W, long long entries)
     return true;
 }
 
-/* entries of the tape a rollout keeps between its forward and its backward:
- * no more bytes than sqrt(T) checkpointing keeps (nseg checkpoints, K + 1
- * states), and no more than a sixteenth of the cells wet on average need */
+/* Entries of the tape a rollout may keep between its forward and its
+ * backward: no more bytes than sqrt(T) checkpointing keeps (nseg checkpoints,
+ * K + 1 states), or than a 1024th of the device's memory while 256 of them
+ * would still fit, and no more than a sixteenth of the cells wet on average
+ * need.  (512 x 480 x 400: 81 MB, 290 MB, 268 MB; of 40 flows two fifths of
+ * the first is the median need and 1.6 times it the largest.) */
 static long long kept_tape(const Work& W)
 {
     const long long n = W.d.N;
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
     const long long states = (long long)(W.nseg + W.K + 1) * n * (long long)sizeof(double);
-    return std::max<long long>(1, std::min(states / (long long)sdtw::TAPE_BYTES, (n / 16 + 1024) * W.steps));
+    const long long bytes = std::max(states, (long long)std::min(total_b / 1024, free_b / 256));
+    return std::max<long long>(1, std::min(std::min(bytes, (long long)free_b / 8) / (long long)sdtw::TAPE_BYTES,
+                                           (n / 16 + 1024) * W.steps));
 }
 
 static bool make_checkpoints(Work& W)
@@ -330,12 +338,8 @@ extern "C" int cal_sdt_adj_forward(void* handle, const double* z_dem, const doub
     if (W->want_segments && !W->ckpt && W->steps > 0 && !sdtw::capturing(st) && !sdtadj::make_checkpoints(*W))
         return (int)cudaErrorMemoryAllocation;
     if (W->want_tape && !W->ckpt && !d.cap && W->steps > 0 && !sdtw::capturing(st)) {
-        /* at most an eighth of the free memory */
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        const long long most = (long long)(free_b / 8 / sdtw::TAPE_BYTES);
-        if (most > 0)
-            sdtadj::make_tape(*W, std::min(sdtadj::kept_tape(*W), most));
+        W->kept = sdtadj::kept_tape(*W);
+        sdtadj::make_tape(*W, W->kept);
     }
     sdtadj::Inst I;
     memset(&I, 0, sizeof(I));
@@ -403,7 +407,7 @@ extern "C" int cal_sdt_adj_backward(void* handle, const double* gT, double* g_h0
     e = cudaStreamSynchronize(st);
     if (e == cudaSuccess && gave_up)
         e = cudaErrorUnknown;
-    if (d.cap > sdtadj::kept_tape(*W))
+    if (d.cap > W->kept)
         sdtadj::drop_tape(*W); /* another backward runs the forward again */
     if (g_r)
         *g_r = res[0];
