@@ -67,6 +67,10 @@ struct Work {
     char* tape = nullptr;
     unsigned long long* words = nullptr; /* of the cooperative launches */
     bool want_tape = true, want_segments = false;
+    /* the flagged tiles of all steps, which a whole tape needs, would take
+     * more than the checkpoints (over a million steps, or 270,000 on a grid
+     * of few cells): room for one segment's */
+    bool only_segments = false;
     bool flows_clear = false;
     long long kept = 0; /* entries of the tape kept after a backward */
     /* counts the changes of tape and checkpoints; need[1] holds the one that
@@ -120,7 +124,7 @@ static size_t carve(Work& W, char* base)
     c.take(&d.list[1], n);
     c.take(&d.nlist, steps);
     c.take(&d.counts, steps);
-    c.take(&d.tiles, (size_t)d.ntiles * steps);
+    c.take(&d.tiles, (size_t)d.ntiles * (W.only_segments ? W.K : steps));
     c.take(&d.stamps, d.ntiles);
     c.take(&d.toff, steps);
     c.take(&d.need, 2);
@@ -137,6 +141,14 @@ static size_t carve(Work& W, char* base)
     d.offs = W.offs;
     d.z = W.z;
     return c.at;
+}
+
+/* d with the flagged tiles of the steps from t0 on at the start of d.tiles */
+static Dev from_step(const Dev& d, int t0)
+{
+    Dev s = d;
+    s.tiles = (int*)((char*)d.tiles - sizeof(int) * (size_t)t0 * d.ntiles);
+    return s;
 }
 
 static void drop_tape(Work& W)
@@ -206,7 +218,7 @@ static void queue_forward(Work& W, bool keep, cudaStream_t st)
     const bool captured = sdtw::capturing(st);
     if (captured)
         d.cap = 0;
-    k_start<<<1, 1, 0, st>>>(d.toff, d.need, captured && !keep ? -1 : W.record);
+    k_start<<<1, 1, 0, st>>>(d.toff, d.need, (captured || W.only_segments) && !keep ? -1 : W.record);
     cudaMemsetAsync(d.stamps, 0, sizeof(int) * d.ntiles, st);
     cudaMemsetAsync(d.counts, 0, sizeof(int) * (W.steps + 1), st);
     cudaMemsetAsync(d.nlist, 0, sizeof(int) * (W.steps + 1), st);
@@ -218,11 +230,13 @@ static void queue_forward(Work& W, bool keep, cudaStream_t st)
     }
     sdtw::k_init<<<sdtw::dense_blocks(d.N), T, 2 * sizeof(long long), st>>>(d, W.z_dem, W.h0, W.z, W.words);
     cudaMemsetAsync(W.words, 0, words, st);
-    const int per = keep ? W.K : std::max(1, W.steps);
+    const bool parts = keep || W.only_segments;
+    const int per = parts ? W.K : std::max(1, W.steps);
     for (int t = 0; t < W.steps; t += per) {
         if (keep)
             cudaMemcpyAsync(W.ckpt + (size_t)(t / per) * n, d.h, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
-        sdtw::launch_steps(d, t, std::min(t + per, W.steps), 1, !keep, W.words, st);
+        Dev part = parts ? from_step(d, t) : d;
+        sdtw::launch_steps(part, t, std::min(t + per, W.steps), 1, !parts, W.words, st);
     }
     if (W.steps > 0)
         sdtw::k_clear_flows<<<sdtw::BLOCKS, T, 0, st>>>(d, W.steps - 1);
@@ -248,11 +262,11 @@ static void queue_seed(Work& W, const double* gT, cudaStream_t st)
 /* the reverse sweep recomputing segments from the checkpoints */
 static void queue_segments(Work& W, cudaStream_t st)
 {
-    Dev& d = W.d;
-    const size_t n = (size_t)d.N;
-    cudaMemsetAsync(d.need, 0, sizeof(long long), st);
+    const size_t n = (size_t)W.d.N;
+    cudaMemsetAsync(W.d.need, 0, sizeof(long long), st);
     for (int s = W.nseg - 1; s >= 0; s--) {
         const int t0 = s * W.K, t1 = std::min(t0 + W.K, W.steps);
+        Dev d = from_step(W.d, t0);
         cudaMemcpyAsync(d.h, W.ckpt + (size_t)s * n, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
         cudaMemsetAsync(d.nlist + t0, 0, sizeof(int) * (t1 - t0 + 1), st);
         cudaMemsetAsync(d.counts + t0, 0, sizeof(int) * (t1 - t0), st);
@@ -286,6 +300,8 @@ extern "C" void* cal_sdt_adj_create(int rows, int cols, int steps, int toroidal)
     d.lh = sdtadj::LH;
     const int tx = (cols + (1 << d.lw) - 1) >> d.lw, ty = (rows + (1 << d.lh) - 1) >> d.lh;
     d.ntiles = tx * ty;
+    const double lists = (double)d.ntiles * sizeof(int) * W->steps;
+    W->only_segments = lists > 1 << 20 && lists > (double)(W->nseg + W->K + 1) * d.N * sizeof(double);
     const size_t bytes = sdtadj::carve(*W, nullptr);
     if (rows <= 0 || cols <= 0 || d.N >= 0x7fffffffLL || cudaMalloc(&W->slab, bytes) != cudaSuccess) {
         (void)cudaGetLastError();
@@ -335,7 +351,7 @@ extern "C" int cal_sdt_adj_forward(void* handle, const double* z_dem, const doub
     W->r = p_r;
     W->eps = p_eps;
     const size_t b = (size_t)d.N * sizeof(double);
-    if (W->want_segments && !W->ckpt && W->steps > 0 && !sdtw::capturing(st) && !sdtadj::make_checkpoints(*W))
+    if ((W->want_segments || W->only_segments) && !W->ckpt && W->steps > 0 && !sdtw::capturing(st) && !sdtadj::make_checkpoints(*W))
         return (int)cudaErrorMemoryAllocation;
     if (W->want_tape && !W->ckpt && !d.cap && W->steps > 0 && !sdtw::capturing(st)) {
         W->kept = sdtadj::kept_tape(*W);
@@ -374,10 +390,11 @@ extern "C" int cal_sdt_adj_backward(void* handle, const double* gT, double* g_h0
     if (e != cudaSuccess)
         return (int)e;
     bool segments = W->ckpt != nullptr;
-    if (!segments && need[0] > d.cap) {
+    if (!segments && (W->only_segments || need[0] > d.cap)) {
         size_t free_b = 0, total_b = 0;
         cudaMemGetInfo(&free_b, &total_b);
-        segments = (size_t)need[0] * sdtw::TAPE_BYTES > (free_b + (size_t)d.cap * sdtw::TAPE_BYTES) / 2 ||
+        segments = W->only_segments ||
+                   (size_t)need[0] * sdtw::TAPE_BYTES > (free_b + (size_t)d.cap * sdtw::TAPE_BYTES) / 2 ||
                    !sdtadj::make_tape(*W, need[0]);
         if (segments && !sdtadj::make_checkpoints(*W))
             return (int)cudaErrorMemoryAllocation;
