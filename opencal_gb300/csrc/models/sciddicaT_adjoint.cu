@@ -135,7 +135,7 @@ static size_t carve(Work& W, char* base)
     c.take(&a.w, n);
     c.take(&a.g, n);
     c.take(&a.sums, n);
-    c.take(&a.part, 2 * sdtw::PARTS);
+    c.take(&a.part, 4 * sdtw::PARTS);
     c.take(&a.grad, 2);
     d.inst = W.inst;
     d.offs = W.offs;
@@ -256,7 +256,6 @@ static void queue_seed(Work& W, const double* gT, cudaStream_t st)
     cudaMemcpyAsync(W.a.lam, gT, b, cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(W.a.mu, gT, b, cudaMemcpyDeviceToDevice, st);
     cudaMemsetAsync(W.a.stamp, 0xff, sizeof(int) * (size_t)W.d.N, st);
-    cudaMemsetAsync(W.a.sums, 0, sizeof(double2) * (size_t)W.d.N, st);
 }
 
 /* the reverse sweep recomputing segments from the checkpoints */

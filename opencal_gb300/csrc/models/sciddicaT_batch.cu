@@ -242,7 +242,7 @@ static void destroy(Batch* bt)
     Adj& a = bt->a;
     void* ptrs[] = {(void*)d.inst, (void*)d.offs, (void*)d.tile_inst, d.h,     d.zh,    d.f,       d.list[0], d.list[1],
                     d.nlist,       d.tiles,       d.counts,           d.stamps, d.t_entry, d.t_elim, d.t_diff,  d.toff,
-                    d.need,        a.lam,         a.mu,               a.stamp, a.w,     a.g,       a.grad,    a.part,   a.sums,
+                    d.need,        a.lam,         a.mu,               a.stamp, a.w,     a.g,       a.grad,    a.part,
                     bt->z_dem,     bt->z,         bt->h0,             bt->ckpt, bt->loss, bt->words};
     for (void* p : ptrs)
         cudaFree(p);
@@ -451,8 +451,11 @@ static bool adjoint_arrays(Batch& bt, bool want_mu)
         *p = nullptr;
         return false;
     };
-    return need(&a.lam, n) && need(&a.stamp, n) && need(&a.w, n) && need(&a.g, n) && need(&a.grad, 2 * (size_t)bt.B) &&
-           need(&a.part, 2 * (size_t)bt.B * sdtw::PARTS) && need(&a.sums, n) && need(&bt.loss, (size_t)bt.B) &&
+    if (!need(&a.w, 2 * n)) /* and the cells' sums */
+        return false;
+    a.sums = a.w + n;
+    return need(&a.lam, n) && need(&a.stamp, n) && need(&a.g, n) && need(&a.grad, 2 * (size_t)bt.B) &&
+           need(&a.part, 4 * (size_t)bt.B * sdtw::PARTS) && need(&bt.loss, (size_t)bt.B) &&
            (!want_mu || need(&a.mu, n)) &&
            (bt.run_full || bt.steps == 0 || need(&bt.ckpt, n * bt.nseg));
 }

@@ -98,14 +98,42 @@ constexpr size_t TAPE_BYTES = sizeof(Entry) + 1 + sizeof(D4); /* per entry */
 struct Adj {
     double* lam;
     double* mu; /* or NULL */
-    int* stamp; /* per cell: step whose coefficients it holds */
+    int* stamp; /* per cell: step whose coefficients it holds; -1 before its first */
     D4* w;
     double* g;
-    double2* sums; /* per cell: its parts of dL/dr and dL/deps, all steps */
-    double* part;  /* PARTS x 2B: sums of runs of cells */
+    D4* sums;      /* per cell: its parts of dL/dr, dL/deps of all steps (Sum, Sum) */
+    double* part;  /* PARTS x 4B: sums of runs of cells */
     double* grad;  /* 2B: dL/dr[0..B), dL/deps[B..2B) */
 };
 constexpr int PARTS = 64;
+
+/* Kahan's sum: the value is v - c.  The parts of the cells cancel within a
+ * step more than those of a cell over the steps, so that plain sums cell by
+ * cell lost what sums step by step keep (errors of up to 1.2e-14 where those
+ * had 9e-16). */
+struct Sum {
+    double v, c;
+};
+
+static __device__ __forceinline__ bool sum_finite(double v)
+{
+    return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; /* on the integer pipe */
+}
+
+static __device__ __forceinline__ void sum_add(Sum& s, double x)
+{
+    const double y = x - s.c, t = s.v + y, c = (t - s.v) - y;
+    s.c = sum_finite(t) ? c : 0.0; /* an infinite sum stays one */
+    s.v = t;
+}
+
+/* a + b with the rounding of a.v + b.v kept whatever their order */
+static __device__ __forceinline__ void sum_add(Sum& a, const Sum& b)
+{
+    const double t = a.v + b.v, z = t - a.v, c = a.c + b.c - ((a.v - (t - z)) + (b.v - z));
+    a.c = sum_finite(t) ? c : 0.0;
+    a.v = t;
+}
 
 /* neighbour q = 0..3 (north, west, east, south) of (i, j); false where a
  * flat grid ends */
@@ -459,7 +487,10 @@ static __device__ __forceinline__ void coeffs(const Dev& d, const Adj& a, int t,
         const int i = lc / I.cols, j = lc - i * I.cols;
         const D4 diff = d.t_diff[base + k];
         const double own = a.lam[c];
-        double2 sum = a.sums[c];
+        const D4 sums = a.sums[c]; /* counts from the cell's second step on */
+        const bool later = a.stamp[c] >= 0;
+        Sum sr = {later ? sums.v[0] : 0.0, later ? sums.v[1] : 0.0};
+        Sum se = {later ? sums.v[2] : 0.0, later ? sums.v[3] : 0.0};
         double S = 0.0, lf[4], er = 0.0;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
@@ -480,13 +511,14 @@ static __device__ __forceinline__ void coeffs(const Dev& d, const Adj& a, int t,
         a.stamp[c] = t;
         a.g[c] = g;
         a.w[c] = w;
-        sum.x += er;
+        sum_add(sr, er);
         if (elim & 1u) {
-            sum.y -= cal_div_small(S * I.r, kk);
+            sum_add(se, -cal_div_small(S * I.r, kk));
             if (a.mu)
                 a.mu[c] += g;
         }
-        a.sums[c] = sum;
+        const D4 sums1 = {{sr.v, sr.c, se.v, se.c}};
+        a.sums[c] = sums1;
     }
 }
 
@@ -498,46 +530,79 @@ static __global__ void __launch_bounds__(T) k_coeffs(const __grid_constant__ Dev
         coeffs(d, a, t, n, base, (threadIdx.x >> 5) * gridDim.x + blockIdx.x, gridDim.x * (T / 32));
 }
 
-/* block (p, b): the sums of the p-th run of instance b's cells */
+/* Block (p, b): the sums of the p-th run of instance b's cells.  Few cells
+ * were ever wet; the rest of the work is the additions that join the
+ * threads' sums, on an FP64 pipe that takes some 19 clocks a warp: one warp
+ * joins them (64 instances, 84 MB of stamps: in every warp, with 64 runs an
+ * instance, 1081 us) */
 static __global__ void __launch_bounds__(T) k_parts(const __grid_constant__ Dev d, const __grid_constant__ Adj a)
 {
-    __shared__ double s_sum[2][T / 32];
+    __shared__ Sum s_sum[2][T];
     const Inst I = d.inst[blockIdx.y];
     const long long n = (long long)I.rows * I.cols, per = (n + PARTS - 1) / PARTS;
     const long long c1 = min(n, per * (blockIdx.x + 1));
-    double r = 0.0, e = 0.0;
-    for (long long c = per * blockIdx.x + threadIdx.x; c < c1; c += T) {
-        const double2 v = a.sums[I.off + c];
-        r += v.x;
-        e += v.y;
+    Sum q[2] = {{0.0, 0.0}, {0.0, 0.0}};
+    for (long long c0 = per * blockIdx.x; c0 < c1; c0 += 8 * T) {
+        int stamp[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const long long c = c0 + u * T + threadIdx.x;
+            stamp[u] = c < c1 ? a.stamp[I.off + c] : -1;
+        }
+#pragma unroll
+        for (int h = 0; h < 8; h += 4) {
+            D4 v[4];
+            bool any = false;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                v[u] = {{0.0, 0.0, 0.0, 0.0}};
+                if (stamp[h + u] >= 0) {
+                    v[u] = a.sums[I.off + c0 + (h + u) * T + threadIdx.x];
+                    any = true;
+                }
+            }
+            if (any) /* in the flow, mostly the whole warp */
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        sum_add(q[k], v[u].v[2 * k]);
+                        q[k].c += v[u].v[2 * k + 1];
+                    }
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        r += __shfl_down_sync(0xffffffffu, r, o);
-        e += __shfl_down_sync(0xffffffffu, e, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        s_sum[0][threadIdx.x >> 5] = r;
-        s_sum[1][threadIdx.x >> 5] = e;
-    }
+    s_sum[0][threadIdx.x] = q[0];
+    s_sum[1][threadIdx.x] = q[1];
     __syncthreads();
-    if (threadIdx.x < 2) {
-        double v = 0.0;
-        for (int w = 0; w < T / 32; w++)
-            v += s_sum[threadIdx.x][w];
-        a.part[(size_t)blockIdx.x * 2 * d.B + threadIdx.x * d.B + blockIdx.y] = v;
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (k >= 2)
+        return;
+    Sum v = s_sum[k][lane];
+    for (int w = 1; w < T / 32; w++)
+        sum_add(v, s_sum[k][w * 32 + lane]);
+    for (int o = 16; o > 0; o >>= 1)
+        sum_add(v, Sum{__shfl_down_sync(0xffffffffu, v.v, o), __shfl_down_sync(0xffffffffu, v.c, o)});
+    if (lane == 0) {
+        double* out = a.part + (size_t)blockIdx.x * 4 * d.B + k * d.B + blockIdx.y;
+        out[0] = v.v;
+        out[2 * d.B] = v.c;
     }
 }
 
-/* the instances' dL/dr and dL/deps: their partial sums in a fixed order */
-static __global__ void k_fold(const double* __restrict__ part, double* __restrict__ grad, int n)
+/* the instances' dL/dr and dL/deps (n = 2B): their partial sums in a fixed
+ * order, a warp each */
+static __global__ void __launch_bounds__(T) k_fold(const double* __restrict__ part, double* __restrict__ grad, int n)
 {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int q = blockIdx.x * (T / 32) + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (q >= n)
         return;
-    double v = 0.0;
-    for (int p = 0; p < PARTS; p++)
-        v += part[(size_t)p * n + q];
-    grad[q] = v;
+    Sum v = {0.0, 0.0};
+    for (int p = lane; p < PARTS; p += 32)
+        sum_add(v, Sum{part[(size_t)p * 2 * n + q], part[(size_t)p * 2 * n + n + q]});
+    for (int o = 16; o > 0; o >>= 1)
+        sum_add(v, Sum{__shfl_down_sync(0xffffffffu, v.v, o), __shfl_down_sync(0xffffffffu, v.c, o)});
+    if (lane == 0)
+        grad[q] = v.v - v.c;
 }
 
 /* lambda_t from lambda_{t+1}: every cell whose lambda changes lies in a tile
@@ -706,8 +771,7 @@ static __global__ void k_out(const double* __restrict__ h, double* __restrict__ 
         out[c] = bad ? __longlong_as_double(0x7ff8000000000000LL) : h[c];
 }
 
-/* lambda_T = 2 (h_T - target), mu_T the same, the cells' sums 0, and the
- * instances' losses */
+/* lambda_T = 2 (h_T - target), mu_T the same, and the instances' losses */
 static __global__ void __launch_bounds__(T) k_loss(const __grid_constant__ Dev d, const __grid_constant__ Adj a,
                                             const double* __restrict__ target, double* loss)
 {
@@ -728,7 +792,6 @@ static __global__ void __launch_bounds__(T) k_loss(const __grid_constant__ Dev d
             a.lam[c] = 2.0 * diff;
             if (a.mu)
                 a.mu[c] = 2.0 * diff;
-            a.sums[c] = make_double2(0.0, 0.0);
         }
         const int b0 = __shfl_sync(0xffffffffu, b, 0);
         if (__all_sync(0xffffffffu, b == b0)) {
@@ -781,7 +844,7 @@ static void queue_adjoint(const Dev& d, const Adj& a, int t0, int t1, cudaStream
 static void queue_grad(const Dev& d, const Adj& a, cudaStream_t st)
 {
     k_parts<<<dim3(PARTS, d.B), T, 0, st>>>(d, a);
-    k_fold<<<(2 * d.B + T - 1) / T, T, 0, st>>>(a.part, a.grad, 2 * d.B);
+    k_fold<<<(2 * d.B + T / 32 - 1) / (T / 32), T, 0, st>>>(a.part, a.grad, 2 * d.B);
 }
 
 static int sm_count()
