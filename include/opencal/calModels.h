@@ -96,6 +96,9 @@ void cal_sdt_adj_destroy(void* work);
  * forward again); 1 (default): they do; 2: checkpoints, every segment taped
  * in its turn by the backward */
 int cal_sdt_adj_set_tape(void* work, int mode);
+/* the most entries of tape kept between a forward and its backward (0: as the
+ * memory allows) */
+int cal_sdt_adj_set_tape_limit(void* work, long long entries);
 int cal_sdt_adj_forward(void* work, const double* z_dem, const double* h0, double p_r, double p_eps, double* hT,
                         void* stream);
 int cal_sdt_adj_backward(void* work, const double* dL_dhT, double* dL_dh0, double* dL_dpr, double* dL_dpeps,

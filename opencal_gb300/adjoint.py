@@ -5,8 +5,10 @@ on the GPU (bit-exact, over the list of wet cells) and returns h_T; its
 backward calls the hand-written adjoint kernels of ``libopencal_models.so``
 (csrc/models/sciddicaT_adjoint.cu): the forward's elimination sets, taped and
 frozen (sqrt(T) checkpoints where the tape would not fit), gradients with
-respect to h0 (including the initialisation's z -= h0), p_r and p_eps.  Torch is used
-for device memory and streams only; the library itself stays C.
+respect to h0 (including the initialisation's z -= h0), p_r and p_eps, which
+repeat bit for bit.  What a rollout holds between its forward and its backward
+is bounded by what sqrt(T) checkpointing holds, or a 128th of the free memory.  Torch is used for device memory and streams only; the library itself
+stays C.
 """
 from __future__ import annotations
 
@@ -27,6 +29,7 @@ def _lib():
         m.cal_sdt_adj_create.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int]
         m.cal_sdt_adj_destroy.argtypes = [C.c_void_p]
         m.cal_sdt_adj_set_tape.argtypes = [C.c_void_p, C.c_int]
+        m.cal_sdt_adj_set_tape_limit.argtypes = [C.c_void_p, C.c_longlong]
         m.cal_sdt_adj_forward.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_double, C.c_double, C.c_void_p,
                                           C.c_void_p]
         m.cal_sdt_adj_backward.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(C.c_double),

@@ -29,11 +29,14 @@
  * the rollout into a tape that, where memory matters, takes no more of it than
  * checkpoints every K = ceil(sqrt(T)) steps and the states of a segment
  * between two would (kept_tape: a program may hold many rollouts between
- * their forwards and backwards).  The backward first
- * learns what the tape needed.  When it was too small, the forward runs again
- * with one that fits, given back after the sweep, or, when that would take
- * more than half of the free device memory, with h stored every K steps, and
- * the sweep then recomputes and tapes one segment at a time.
+ * their forwards and backwards).  The backward first learns what the tape
+ * needed.  One that was too small holds the last steps; when running the
+ * steps before them again, as often as it takes, costs no more than one
+ * forward, the sweep goes on so (1024 x 1024 x 2000 with 0.6 of the tape it
+ * needs: 45 -> 54 ms, with a forward into a larger one 65).  Else the forward
+ * runs again with a tape that fits, given back after the sweep, or, when that
+ * would take more than half of the free device memory, with h stored every K
+ * steps, and the sweep then recomputes and tapes one segment at a time.
  */
 #include <math.h>
 #include <stdio.h>
@@ -41,6 +44,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <vector>
 
 #include "sciddicaT_wet.cuh"
 
@@ -72,16 +76,22 @@ struct Work {
      * of few cells): room for one segment's */
     bool only_segments = false;
     bool flows_clear = false;
-    long long kept = 0; /* entries of the tape kept after a backward */
+    long long kept = 0;  /* entries of the tape kept after a backward */
+    long long limit = 0; /* on those (0: none) */
     /* counts the changes of tape and checkpoints; need[1] holds the one that
      * the last forward to run left its record in (a captured forward may run
      * after they were changed) */
     long long record = 0;
 };
 
-__global__ void k_start(long long* toff, long long* need, long long record)
+/* need[1] of a forward that cannot be reversed as it is: captured, or run in
+ * part (need[0] is then the part's) */
+constexpr long long NOT_TAPED = -1, IN_PART = -2;
+
+__global__ void k_start(long long* toff, long long* tpos, long long* need, long long record)
 {
     toff[0] = 0;
+    tpos[0] = 0;
     need[0] = 0;
     need[1] = record;
 }
@@ -127,6 +137,7 @@ static size_t carve(Work& W, char* base)
     c.take(&d.tiles, (size_t)d.ntiles * (W.only_segments ? W.K : steps));
     c.take(&d.stamps, d.ntiles);
     c.take(&d.toff, steps);
+    c.take(&d.tpos, steps);
     c.take(&d.need, 2);
     c.take(&W.words, 16 * sdtw::NWORDS);
     c.take(&a.lam, n);
@@ -182,19 +193,20 @@ static bool make_tape(Work& W, long long entries)
 
 /* Entries of the tape a rollout may keep between its forward and its
  * backward: no more bytes than sqrt(T) checkpointing keeps (nseg checkpoints,
- * K + 1 states), or than a 1024th of the device's memory while 256 of them
- * would still fit, and no more than a sixteenth of the cells wet on average
- * need.  (512 x 480 x 400: 81 MB, 290 MB, 268 MB; of 40 flows two fifths of
- * the first is the median need and 1.6 times it the largest.) */
+ * K + 1 states) or than a 128th of the free memory, and no more than a
+ * sixteenth of the cells wet on average need.  (512 x 480 x 400: 81 MB, 2 GB,
+ * 268 MB; of 40 flows two fifths of the first is the median need and 1.6 times
+ * it the largest.) */
 static long long kept_tape(const Work& W)
 {
     const long long n = W.d.N;
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     const long long states = (long long)(W.nseg + W.K + 1) * n * (long long)sizeof(double);
-    const long long bytes = std::max(states, (long long)std::min(total_b / 1024, free_b / 256));
-    return std::max<long long>(1, std::min(std::min(bytes, (long long)free_b / 8) / (long long)sdtw::TAPE_BYTES,
-                                           (n / 16 + 1024) * W.steps));
+    const long long bytes = std::max(states, (long long)(free_b / 128));
+    const long long entries = std::min(std::min(bytes, (long long)free_b / 8) / (long long)sdtw::TAPE_BYTES,
+                                       (n / 16 + 1024) * W.steps);
+    return std::max<long long>(1, W.limit > 0 ? std::min(entries, W.limit) : entries);
 }
 
 static bool make_checkpoints(Work& W)
@@ -208,17 +220,19 @@ static bool make_checkpoints(Work& W)
     return true;
 }
 
-/* The rollout from h0 and z_dem, queued: taped, or with checkpoints (keep).
- * A captured one is not taped: its nodes would keep the address of a tape
+/* The first `steps` steps of the rollout from h0 and z_dem, queued: taped, or
+ * with checkpoints (keep).  A captured one is not taped: its nodes would keep the address of a tape
  * that a backward may allocate again. */
-static void queue_forward(Work& W, bool keep, cudaStream_t st)
+static void queue_forward(Work& W, int steps, bool keep, cudaStream_t st)
 {
     Dev d = W.d;
     const size_t n = (size_t)d.N;
     const bool captured = sdtw::capturing(st);
     if (captured)
         d.cap = 0;
-    k_start<<<1, 1, 0, st>>>(d.toff, d.need, (captured || W.only_segments) && !keep ? -1 : W.record);
+    k_start<<<1, 1, 0, st>>>(d.toff, d.tpos, d.need,
+                             steps < W.steps ? IN_PART
+                                             : ((captured || W.only_segments) && !keep ? NOT_TAPED : W.record));
     cudaMemsetAsync(d.stamps, 0, sizeof(int) * d.ntiles, st);
     cudaMemsetAsync(d.counts, 0, sizeof(int) * (W.steps + 1), st);
     cudaMemsetAsync(d.nlist, 0, sizeof(int) * (W.steps + 1), st);
@@ -229,17 +243,18 @@ static void queue_forward(Work& W, bool keep, cudaStream_t st)
         W.flows_clear = !captured; /* what is captured has not run yet */
     }
     sdtw::k_init<<<sdtw::dense_blocks(d.N), T, 2 * sizeof(long long), st>>>(d, W.z_dem, W.h0, W.z, W.words);
-    cudaMemsetAsync(W.words, 0, words, st);
+    if (steps == W.steps) /* else a part of a sweep that may have given up already */
+        cudaMemsetAsync(W.words, 0, words, st);
     const bool parts = keep || W.only_segments;
-    const int per = parts ? W.K : std::max(1, W.steps);
-    for (int t = 0; t < W.steps; t += per) {
+    const int per = parts ? W.K : std::max(1, steps);
+    for (int t = 0; t < steps; t += per) {
         if (keep)
             cudaMemcpyAsync(W.ckpt + (size_t)(t / per) * n, d.h, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
         Dev part = parts ? from_step(d, t) : d;
-        sdtw::launch_steps(part, t, std::min(t + per, W.steps), 1, !parts, W.words, st);
+        sdtw::launch_steps(part, t, std::min(t + per, steps), 1, !parts, W.words, st);
     }
-    if (W.steps > 0)
-        sdtw::k_clear_flows<<<sdtw::BLOCKS, T, 0, st>>>(d, W.steps - 1);
+    if (steps > 0)
+        sdtw::k_clear_flows<<<sdtw::BLOCKS, T, 0, st>>>(d, steps - 1);
 }
 
 /* need[0]: the largest tape any step sequence asked for since the last
@@ -248,6 +263,43 @@ static cudaError_t tape_need(Work& W, long long need[2], cudaStream_t st)
 {
     cudaMemcpyAsync(need, W.d.need, 2 * sizeof(*need), cudaMemcpyDeviceToHost, st);
     return cudaStreamSynchronize(st);
+}
+
+/* The stretches [c, t1) of steps, last first, that a tape too small for all
+ * holds one at a time after a forward to t1; none when a step does not fit at
+ * all or the forwards would take more than `steps` steps together. */
+static std::vector<std::pair<int, int>> stretches(const Work& W, const std::vector<long long>& toff)
+{
+    std::vector<std::pair<int, int>> out;
+    std::vector<long long> base(W.steps);
+    long long pos = 0, again = 0;
+    for (int t = 0; t < W.steps; t++) {
+        const int n = (int)(toff[t + 1] - toff[t]);
+        base[t] = sdtw::tape_slot(W.d.cap, true, pos, n);
+        if (base[t] < 0)
+            return out;
+        pos = sdtw::tape_next(true, pos, base[t], n);
+    }
+    for (int t1 = W.steps, c; t1 > 0; t1 = c) {
+        long long end = 0; /* of what lies at the start of the tape since it began again */
+        int lap = 0;
+        for (c = t1; c > 0; c--) {
+            const long long from = base[c - 1], to = from + (toff[c] - toff[c - 1]);
+            if (c < t1 && to > base[c]) /* step c began at 0 again */
+                lap++;
+            if (lap == 2 || (lap == 1 && from < end))
+                break;
+            if (lap == 0)
+                end = std::max(end, to);
+        }
+        out.push_back(std::make_pair(c, t1));
+        again += c;
+        if (again > W.steps) {
+            out.clear();
+            return out;
+        }
+    }
+    return out;
 }
 
 static void queue_seed(Work& W, const double* gT, cudaStream_t st)
@@ -266,6 +318,7 @@ static void queue_segments(Work& W, cudaStream_t st)
     for (int s = W.nseg - 1; s >= 0; s--) {
         const int t0 = s * W.K, t1 = std::min(t0 + W.K, W.steps);
         Dev d = from_step(W.d, t0);
+        d.tpos = nullptr;
         cudaMemcpyAsync(d.h, W.ckpt + (size_t)s * n, n * sizeof(double), cudaMemcpyDeviceToDevice, st);
         cudaMemsetAsync(d.nlist + t0, 0, sizeof(int) * (t1 - t0 + 1), st);
         cudaMemsetAsync(d.counts + t0, 0, sizeof(int) * (t1 - t0), st);
@@ -337,6 +390,17 @@ extern "C" int cal_sdt_adj_set_tape(void* handle, int mode)
     return 0;
 }
 
+/* The most entries of tape (41 bytes each) that the workspace keeps between a
+ * forward and its backward; 0 (default): as the memory allows.  For the
+ * tapes allocated from now on. */
+extern "C" int cal_sdt_adj_set_tape_limit(void* handle, long long entries)
+{
+    if (entries < 0)
+        return 1;
+    ((Work*)handle)->limit = entries;
+    return 0;
+}
+
 /* Forward rollout on device buffers: init (z = z_dem - h0 where h0 > 0),
  * `steps` steps, h_T into hT; the tape kept for the backward.  May be
  * captured into a graph (nothing is allocated then: without a tape from an
@@ -350,7 +414,8 @@ extern "C" int cal_sdt_adj_forward(void* handle, const double* z_dem, const doub
     W->r = p_r;
     W->eps = p_eps;
     const size_t b = (size_t)d.N * sizeof(double);
-    if ((W->want_segments || W->only_segments) && !W->ckpt && W->steps > 0 && !sdtw::capturing(st) && !sdtadj::make_checkpoints(*W))
+    if ((W->want_segments || W->only_segments) && !W->ckpt && W->steps > 0 && !sdtw::capturing(st) &&
+        !sdtadj::make_checkpoints(*W))
         return (int)cudaErrorMemoryAllocation;
     if (W->want_tape && !W->ckpt && !d.cap && W->steps > 0 && !sdtw::capturing(st)) {
         W->kept = sdtadj::kept_tape(*W);
@@ -370,7 +435,7 @@ extern "C" int cal_sdt_adj_forward(void* handle, const double* z_dem, const doub
     cudaMemsetAsync((void*)d.tile_inst, 0, sizeof(int) * d.ntiles, st);
     cudaMemcpyAsync(W->h0, h0, b, cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(W->z_dem, z_dem, b, cudaMemcpyDeviceToDevice, st);
-    sdtadj::queue_forward(*W, W->ckpt != nullptr, st);
+    sdtadj::queue_forward(*W, W->steps, W->ckpt != nullptr, st);
     /* no step: h0 as given, -0 and all */
     sdtw::k_out<<<sdtw::dense_blocks(d.N), sdtadj::T, 0, st>>>(W->steps > 0 ? d.h : W->h0, hT, d.N, W->words);
     return (int)cudaGetLastError();
@@ -386,24 +451,43 @@ extern "C" int cal_sdt_adj_backward(void* handle, const double* gT, double* g_h0
     sdtw::Dev& d = W->d;
     long long need[2] = {0, 0};
     cudaError_t e = sdtadj::tape_need(*W, need, st);
+    if (e == cudaSuccess && need[1] == sdtadj::IN_PART) {
+        sdtadj::queue_forward(*W, W->steps, W->ckpt != nullptr, st);
+        e = sdtadj::tape_need(*W, need, st);
+    }
     if (e != cudaSuccess)
         return (int)e;
     bool segments = W->ckpt != nullptr;
-    if (!segments && (W->only_segments || need[0] > d.cap)) {
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        segments = W->only_segments ||
-                   (size_t)need[0] * sdtw::TAPE_BYTES > (free_b + (size_t)d.cap * sdtw::TAPE_BYTES) / 2 ||
-                   !sdtadj::make_tape(*W, need[0]);
-        if (segments && !sdtadj::make_checkpoints(*W))
-            return (int)cudaErrorMemoryAllocation;
+    std::vector<std::pair<int, int>> parts;
+    if (!segments && !W->only_segments && need[0] > d.cap && d.cap > 0 && need[1] == W->record) {
+        std::vector<long long> toff(W->steps + 1);
+        cudaMemcpyAsync(toff.data(), d.toff, sizeof(long long) * toff.size(), cudaMemcpyDeviceToHost, st);
+        if ((e = cudaStreamSynchronize(st)) != cudaSuccess)
+            return (int)e;
+        parts = sdtadj::stretches(*W, toff);
     }
-    if (need[1] != W->record)
-        sdtadj::queue_forward(*W, segments, st);
+    if (parts.empty()) {
+        if (!segments && (W->only_segments || need[0] > d.cap)) {
+            size_t free_b = 0, total_b = 0;
+            cudaMemGetInfo(&free_b, &total_b);
+            segments = W->only_segments ||
+                       (size_t)need[0] * sdtw::TAPE_BYTES > (free_b + (size_t)d.cap * sdtw::TAPE_BYTES) / 2 ||
+                       !sdtadj::make_tape(*W, need[0]);
+            if (segments && !sdtadj::make_checkpoints(*W))
+                return (int)cudaErrorMemoryAllocation;
+        }
+        if (need[1] != W->record)
+            sdtadj::queue_forward(*W, W->steps, segments, st);
+        parts.push_back(std::make_pair(0, W->steps));
+    }
     for (int attempt = 0;; attempt++) {
         sdtadj::queue_seed(*W, gT, st);
         if (!segments) {
-            sdtw::launch_sweep(d, W->a, 0, W->steps, W->words, st);
+            for (const auto& part : parts) {
+                if (part.second < W->steps)
+                    sdtadj::queue_forward(*W, part.second, false, st);
+                sdtw::launch_sweep(d, W->a, part.first, part.second, W->words, st);
+            }
             break;
         }
         sdtadj::queue_segments(*W, st);

@@ -38,7 +38,7 @@
  * Measured against the tile-by-tile step this replaced (fused tiles of 64 x
  * 16 cells with their rings, the adjoint on whole tiles after restoring
  * them), 64 instances of 128..1024 cells a side, 500 steps, us per step:
- * forward 92 -> 16 (k_outflows) + 16 (k_update); reverse 10 + 65 + 29 -> 15
+ * forward 92 -> 16 (k_outflows) + 16 (k_update); reverse 10 + 65 + 29 -> 13
  * (k_coeffs) + 10 (k_gather).  k_outflows is bound by the FP64 pipe (60 % of
  * it over the launch, the rest is its chain of loads), the others by the
  * latency of theirs.
@@ -89,7 +89,9 @@ struct Dev {
     unsigned char* t_elim;
     D4* t_diff;
     long long cap;   /* its entries */
-    long long* toff; /* per step: first entry; toff[t + 1] chained by step t */
+    long long* toff; /* per step: entries before it; toff[t + 1] chained by step t */
+    long long* tpos; /* a tape that starts again from its first entry when a step does not fit behind the one
+                      * before (NULL: later steps are left out): per step, where the step before ended */
     long long* need; /* the most entries any rollout or segment asked for */
 };
 
@@ -149,12 +151,21 @@ static __device__ __forceinline__ bool nbr(const Inst& I, int i, int j, int q, i
     return (unsigned)*a < (unsigned)I.rows && (unsigned)*b < (unsigned)I.cols;
 }
 
-/* the tape entries of step t start here; -1: they do not fit (the
- * evaluation is discarded and repeated with a larger tape) */
+/* the n tape entries of a step start here; -1: they do not fit (the
+ * evaluation is repeated).  at: where the step before ended, or, when later
+ * steps are left out, the entries before */
+static __host__ __device__ __forceinline__ long long tape_slot(long long cap, bool again, long long at, int n)
+{
+    return at + n <= cap ? at : (again && n <= cap ? 0 : -1);
+}
+/* and the step's end */
+static __host__ __device__ __forceinline__ long long tape_next(bool again, long long at, long long base, int n)
+{
+    return again ? (base >= 0 ? base + n : at) : at + n;
+}
 static __device__ __forceinline__ long long tape_base(const Dev& d, int t, int n)
 {
-    const long long off = d.toff[t];
-    return off + n <= d.cap ? off : -1;
+    return tape_slot(d.cap, d.tpos != nullptr, d.tpos ? d.tpos[t] : d.toff[t], n);
 }
 
 static __device__ __forceinline__ int add(int* count, int v) { return atomicAdd(count, v); }
@@ -236,6 +247,8 @@ static __global__ void __launch_bounds__(T) k_outflows(const __grid_constant__ D
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             const long long end = d.toff[t] + n;
             d.toff[t + 1] = end;
+            if (d.tpos)
+                d.tpos[t + 1] = tape_next(true, d.tpos[t], base, n);
             if (*d.need < end) /* one step at a time runs */
                 *d.need = end;
         }
@@ -470,8 +483,9 @@ static __global__ void __launch_bounds__(T) k_relist(const __grid_constant__ Dev
  * A cell adds its parts to sums of its own, which are added up after the last
  * step in a fixed order (k_parts, k_fold), so that the gradients repeat bit
  * for bit whatever order the lists were appended in, and no atomics queue on
- * an instance's two words (287,000 entries of 64 instances, all on one word
- * per instance and sum: 48.7 us a step). */
+ * an instance's two words.  287,000 entries of 64 instances, us a step: all
+ * added to one word per instance and sum 48.7, a segmented scan over each warp
+ * and 32 copies of the words 15, so 13.3 (11.0 were the sums not compensated). */
 static __device__ __forceinline__ void coeffs(const Dev& d, const Adj& a, int t, int n, long long base, int warp,
                                               int nwarps)
 {
@@ -654,7 +668,9 @@ static __global__ void __launch_bounds__(T) k_gather(const __grid_constant__ Dev
  * graph); the phases of a step separated by grid barriers of one block of
  * 1024 threads per SM take 1.45 us each (sciddicaT.cu, sdt2::k_persist), so
  * runs that are not recorded go this way (one grid of 512 x 480, us per step:
- * forward 16 -> 10.8, reverse 15 -> 8.0; 40 instances forward 21 -> 17). */
+ * forward 16 -> 10.8, reverse 15 -> 7.7; 40 instances forward 21 -> 17).  The
+ * blocks take every SM's registers, so that kernels of other streams wait for
+ * the end of the launch; the recorded form leaves them room between its own. */
 constexpr int GROUPS = 4, PT = GROUPS * T;
 constexpr unsigned SPIN_LIMIT = 1u << 22;
 
@@ -702,8 +718,15 @@ static __global__ void __launch_bounds__(PT, 1) k_steps(const __grid_constant__ 
     const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps = gridDim.x * (PT / 32);
     const int group = (threadIdx.x / T) * gridDim.x + blockIdx.x, ngroups = gridDim.x * GROUPS;
     int n = d.nlist[t0];
-    long long off = taped ? d.toff[t0] : 0, most = 0;
-    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+    /* the tape's state lies in shared memory: the two phases leave no
+     * register for it */
+    __shared__ long long s_at, s_off; /* as for tape_slot; entries so far */
+    const bool again = d.tpos != nullptr, first = blockIdx.x == 0 && threadIdx.x == 0;
+    if (threadIdx.x == 0 && taped) {
+        s_off = d.toff[t0];
+        s_at = again ? d.tpos[t0] : s_off;
+    }
+    __syncthreads();
     for (int t = t0; t < t1; t++) {
         unsigned long long* tword = words + 16 * (t % 3);
         unsigned long long* lword = words + 16 * (3 + t % 3);
@@ -712,16 +735,19 @@ static __global__ void __launch_bounds__(PT, 1) k_steps(const __grid_constant__ 
             words[16 * ((t + 1) % 3)] = 0;
             words[16 * (3 + (t + 1) % 3)] = 0;
         }
-        outflows(d, t, epoch0 + t, n, taped && off + n <= d.cap ? off : -1, tword, warp, nwarps);
-        if (taped) {
-            off += n;
-            most = off > most ? off : most;
-            if (first)
-                d.toff[t + 1] = off;
-        }
+        outflows(d, t, epoch0 + t, n, taped ? tape_slot(d.cap, again, s_at, n) : -1, tword, warp, nwarps);
         int ntiles;
         if (!phase_end(tword, 1, words + 16 * 7, &ntiles))
             return;
+        if (threadIdx.x == 0 && taped) { /* read again after the next barrier */
+            s_at = tape_next(again, s_at, tape_slot(d.cap, again, s_at, n), n);
+            s_off += n;
+            if (first) {
+                d.toff[t + 1] = s_off;
+                if (again)
+                    d.tpos[t + 1] = s_at;
+            }
+        }
         update<GROUPS>(d, t, epoch0 + t, ntiles, n, lword, group, ngroups);
         if (first)
             d.counts[t] = ntiles;
@@ -730,8 +756,8 @@ static __global__ void __launch_bounds__(PT, 1) k_steps(const __grid_constant__ 
         if (first)
             d.nlist[t + 1] = n;
     }
-    if (taped && first && *d.need < most)
-        *d.need = most;
+    if (taped && first && *d.need < s_off)
+        *d.need = s_off;
 }
 
 /* the adjoint of steps [t0, t1), last first (steps that did not fit the tape

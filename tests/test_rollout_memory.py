@@ -1,6 +1,6 @@
 """Device memory of live rollouts: what one holds between its forward and its
-backward, and after it, is bounded by what sqrt(T) checkpointing holds (and a
-1024th of the device's memory, where that is more), and the gradients do not
+backward, and after it, is bounded by what sqrt(T) checkpointing holds (or a
+128th of the free memory, where that is more), and the gradients do not
 depend on whether the tape fitted."""
 import math
 
@@ -29,7 +29,7 @@ def test_bounded_by_checkpointing(rows, cols, steps, wet):
     K = math.ceil(math.sqrt(steps))
     n = rows * cols
     # the tape, 24 fields of the workspace, the tiles of every step, allocation granules
-    tape = max(8 * n * (K + math.ceil(steps / K) + 1), torch.cuda.mem_get_info()[1] // 1024)
+    tape = max(8 * n * (K + math.ceil(steps / K) + 1), torch.cuda.mem_get_info()[0] // 128)
     bound = tape + 8 * n * 24 + 4 * (n // 256 + rows + cols) * (steps + 1) + (64 << 20)
 
     def rollout():
